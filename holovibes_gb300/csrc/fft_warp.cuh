@@ -42,7 +42,7 @@ __device__ __forceinline__ float2 w32mul(int m, float2 a)
     if (r == 0)
         b = a;
     else if (r == 4)
-        b = fft::w8mul<1>(a);
+        b = fft::w8mul<1, true>(a);
     else
     {
         const float c = c32(r), s = s32(r);
@@ -58,9 +58,12 @@ __device__ __forceinline__ float2 w32mul(int m, float2 a)
 }
 
 // Forward 32-point DFT in place (natural order): n = 4 n1 + n2, k = k1 + 8 k2; DFT8 over n1,
-// twiddle w32^(n2 k1), DFT4 over n2.
+// twiddle w32^(n2 k1), DFT4 over n2. The twiddles that are eighth roots (n2 k1 = 4, 12) are taken
+// into the DFT4's first sums as fused multiply-adds.
 __device__ __forceinline__ void dft32(float2 (&x)[32])
 {
+    constexpr float c = 0.707106781186547524400844362104849039f;
+    const float2 cc = make_float2(c, c), nc = make_float2(-c, -c);
     float2 a[4][8];
 #pragma unroll
     for (int n2 = 0; n2 < 4; ++n2)
@@ -68,21 +71,42 @@ __device__ __forceinline__ void dft32(float2 (&x)[32])
 #pragma unroll
         for (int n1 = 0; n1 < 8; ++n1)
             a[n2][n1] = x[4 * n1 + n2];
-        fft::dft8(a[n2]);
+        fft::dft8<true>(a[n2]);
     }
-#pragma unroll
-    for (int n2 = 1; n2 < 4; ++n2)
-#pragma unroll
-        for (int k1 = 1; k1 < 8; ++k1)
-            a[n2][k1] = w32mul(n2 * k1, a[n2][k1]);
 #pragma unroll
     for (int k1 = 0; k1 < 8; ++k1)
     {
-        fft::dft4(a[0][k1], a[1][k1], a[2][k1], a[3][k1]);
-        x[k1] = a[0][k1];
-        x[k1 + 8] = a[1][k1];
-        x[k1 + 16] = a[2][k1];
-        x[k1 + 24] = a[3][k1];
+        float2 s02, d02, s13, d13;
+        if (k1 == 2 || k1 == 6)  // n2 = 2: c (1 - i), times -i for k1 = 6
+        {
+            const float2 u = make_float2(a[2][k1].x + a[2][k1].y, a[2][k1].y - a[2][k1].x);
+            const float2 v = k1 == 2 ? u : cmul_negi(u);
+            s02 = fft::pfma(v, cc, a[0][k1]);
+            d02 = fft::pfma(v, nc, a[0][k1]);
+        }
+        else
+        {
+            const float2 v = w32mul(2 * k1, a[2][k1]);
+            s02 = fft::padd(a[0][k1], v);
+            d02 = fft::psub(a[0][k1], v);
+        }
+        if (k1 == 4)  // n2 = 1: c (1 - i), n2 = 3: -i c (1 - i)
+        {
+            const float2 u = make_float2(a[1][4].x + a[1][4].y, a[1][4].y - a[1][4].x);
+            const float2 v = fft::pmul(make_float2(a[3][4].y - a[3][4].x, -a[3][4].x - a[3][4].y), cc);
+            s13 = fft::pfma(u, cc, v);
+            d13 = fft::pfma(u, cc, make_float2(-v.x, -v.y));
+        }
+        else
+        {
+            const float2 v1 = w32mul(k1, a[1][k1]), v3 = w32mul(3 * k1, a[3][k1]);
+            s13 = fft::padd(v1, v3);
+            d13 = fft::psub(v1, v3);
+        }
+        x[k1] = fft::padd(s02, s13);
+        x[k1 + 16] = fft::psub(s02, s13);
+        x[k1 + 8] = make_float2(d02.x + d13.y, d02.y - d13.x);
+        x[k1 + 24] = make_float2(d02.x - d13.y, d02.y + d13.x);
     }
 }
 
@@ -107,7 +131,7 @@ struct Warp
             const float2* t = tw + g;
 #pragma unroll
             for (int k1 = 1; k1 < 32; ++k1)
-                x[k1] = cmul(x[k1], t[(k1 - 1) * 32]);
+                x[k1] = cmul_tw(x[k1], t[(k1 - 1) * 32]);
         }
         else
         {
@@ -118,8 +142,8 @@ struct Warp
                 a[j] = x[2 * j];      // group g:      samples g + 32 j
                 b[j] = x[2 * j + 1];  // group g + 16: samples g + 16 + 32 j
             }
-            fft::dft16(a);
-            fft::dft16(b);
+            fft::dft16<true>(a);
+            fft::dft16<true>(b);
             const float2* ta = tw + g;
             const float2* tb = tw + g + 16;
             x[0] = a[0];
@@ -127,8 +151,8 @@ struct Warp
 #pragma unroll
             for (int k1 = 1; k1 < 16; ++k1)
             {
-                x[k1] = cmul(a[k1], ta[(k1 - 1) * 32]);
-                x[16 + k1] = cmul(b[k1], tb[(k1 - 1) * 32]);
+                x[k1] = cmul_tw(a[k1], ta[(k1 - 1) * 32]);
+                x[16 + k1] = cmul_tw(b[k1], tb[(k1 - 1) * 32]);
             }
         }
     }
@@ -175,7 +199,7 @@ __device__ __forceinline__ float2 w24mul(int m, float2 a)
     if (r == 0)
         b = a;
     else if (r == 3)
-        b = fft::w8mul<1>(a);
+        b = fft::w8mul<1, true>(a);
     else
     {
         const float c = c24(r), s = s24(r);
@@ -201,7 +225,7 @@ __device__ __forceinline__ void dft24(float2* x)
 #pragma unroll
         for (int n1 = 0; n1 < 8; ++n1)
             a[n2][n1] = x[3 * n1 + n2];
-        fft::dft8(a[n2]);
+        fft::dft8<true>(a[n2]);
     }
 #pragma unroll
     for (int n2 = 1; n2 < 3; ++n2)
@@ -211,7 +235,7 @@ __device__ __forceinline__ void dft24(float2* x)
 #pragma unroll
     for (int k1 = 0; k1 < 8; ++k1)
     {
-        fft::dft3(a[0][k1], a[1][k1], a[2][k1]);
+        fft::dft3<true>(a[0][k1], a[1][k1], a[2][k1]);
         x[k1] = a[0][k1];
         x[k1 + 8] = a[1][k1];
         x[k1 + 16] = a[2][k1];
@@ -232,7 +256,7 @@ struct W768
         const float2* t = tw + g;
 #pragma unroll
         for (int k1 = 1; k1 < 24; ++k1)
-            x[k1] = cmul(x[k1], t[(k1 - 1) * 32]);
+            x[k1] = cmul_tw(x[k1], t[(k1 - 1) * 32]);
     }
     // V32 stage A: x[i] = sample g + 24 i (i < 32, g < 24) -> z[g][k1] * w^(g k1) in x[k1]
     __device__ __forceinline__ static void stage_a32(float2 (&x)[32], const float2* tw, int g)
@@ -241,7 +265,7 @@ struct W768
         const float2* t = tw + TW24 + g;
 #pragma unroll
         for (int k1 = 1; k1 < 32; ++k1)
-            x[k1] = cmul(x[k1], t[(k1 - 1) * 24]);
+            x[k1] = cmul_tw(x[k1], t[(k1 - 1) * 24]);
     }
 
     static void twiddle_fill(float2* out)

@@ -14,6 +14,17 @@ __host__ __device__ __forceinline__ float2 cmul(float2 a, float2 b)
 {
     return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
+// The product with its fused multiply-adds written out (the compiler may fuse either product of
+// cmul's sums): a transform's bits do not depend on the kernel that it is inlined in. The two forms
+// differ in the imaginary part's fused product: twiddles (_tw) and full-frame multipliers.
+__device__ __forceinline__ float2 cmul_tw(float2 a, float2 b)
+{
+    return make_float2(fmaf(a.x, b.x, -__fmul_rn(a.y, b.y)), fmaf(a.y, b.x, __fmul_rn(a.x, b.y)));
+}
+__device__ __forceinline__ float2 cmul_fma(float2 a, float2 b)
+{
+    return make_float2(fmaf(a.x, b.x, -__fmul_rn(a.y, b.y)), fmaf(a.x, b.y, __fmul_rn(a.y, b.x)));
+}
 __host__ __device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
 __host__ __device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
 __host__ __device__ __forceinline__ float2 cconj(float2 a) { return make_float2(a.x, -a.y); }

@@ -44,7 +44,7 @@ hv_status make_fresnel_lens(float2* lens, int W, int H, float lam, float z, floa
 hv_status make_spectral_lens(float2* lens, int W, int H, float lam, float z, float ps, int mode, cudaStream_t st);
 // real_planes (no spatial transform, frames of a multiple of 8 pixels): the real split-BF16 planes
 // of the ring slots written are produced in the same pass (cov_tc.cu layout, real rows).
-// reserve_sms: the persistent (TMA-fed) FFT passes leave that many SMs to kernels of other streams
+// reserve_sms: the persistent FFT passes leave that many SMs to kernels of other streams
 // (a Pipe's render lanes).
 hv_status spatial_transform(const void* raw, int kind, int W, int H, int batch, int space, const float2* lens,
                             float2* work, float2* ring, int slot0, int nslots, cudaStream_t st,

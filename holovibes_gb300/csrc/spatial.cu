@@ -17,8 +17,8 @@
 //   row pass   : inverse row FFT * 1/(H*W) (AS only)
 // and the last pass writes straight into the time-ring slots, so the reference's separate
 // mask, divide and ring-copy passes disappear. Passes of 512, 768 and 1024 points use the warp
-// engine (fft_warp.cuh: 32 samples per thread, one transpose; the 1024-point passes persistent and
-// fed by TMA where they apply), every other length the shared-memory Stockham tile engine
+// engine (fft_warp.cuh: 32 samples per thread, one transpose; the passes are persistent and
+// fed by bulk copies), every other length the shared-memory Stockham tile engine
 // (fft_smem.cuh).
 #include <math.h>
 
@@ -355,725 +355,446 @@ __global__ void __launch_bounds__(fft::Tile<N, F, true>::NT) k_fft_cols(ColPass 
     }
 }
 
-// ------------------------------------------------------------------ warp engine (N = 512, 1024)
-// Rows: 32 / NG rows per warp (1 or 2), 8 warps per CTA; lane (r, g) = (lane / NG, lane % NG);
-// the transpose in the warp's own [row][n2][k1] block, k1 rows padded to NG + 1 entries
-// (conflict-free both ways). Columns: 256 / NG adjacent columns per CTA (8 or 16), thread
-// (c, g) = (t % C, t / C) holds samples g + NG i of column c (a warp load covers 32 / C rows of
-// C * 8 bytes); the transpose goes through a [k1][n2][c] block (conflict-free: k1 rows padded
-// to 264 entries when C = 8).
+// ------------------------------------------------------------------ warp engine (N = 512, 768, 1024)
+// Persistent passes of two 256-thread CTAs per SM, fed by bulk copies into the buffer that the
+// transpose has just left: a row warp (or a column CTA) asks for its next tile as soon as the
+// transposed samples are in registers, so the copy runs beside the second half of the transform
+// and the stores. The waits are bounded; one that gives up sets g_fft_wait_error, lets the copy
+// already issued land and ends the warp (or the CTA).
+//
+// Rows: 32 / NG rows per warp (2 for N = 512), lane (r, g) = (lane / NG, lane % NG); the transpose
+// in the warp's own [row][n2][k1] block, k1 rows padded by one entry (conflict-free both ways), no
+// CTA barrier inside the loop. N = 768 runs DFT24 first: 32 lanes load 24 samples each, lanes
+// 0..23 run the DFT32 and store.
+// Columns: 256 / NG adjacent columns per CTA (8, or 16 for N = 512), thread (c, g) = (t % C, t / C)
+// holds samples g + NG i of column c; the transpose goes through a [k1][n2][c] block
+// (conflict-free: k1 rows padded to 264 entries when C = 8).
+//
+// What bounds them: issue slots and latency at 16 warps per SM (64 data registers per thread), and
+// DRAM for large batches of complex input. Measured (us; one CTA per row block or column tile,
+// its own loads and scalar arithmetic -> here): rows of 16-bit frames, 64 x 768 x 768 102.7 -> 74.4,
+// 32 x 1024 x 1024 78.1 -> 63.1, times a lens 89.2 -> 71.1; columns forward, 768 141.7 -> 103.8, 1024
+// 93.1 -> 89.0 (0.89 of the measured copy bandwidth); columns * G inverse, 768 207.6 -> 168.2, 1024
+// 169.3 -> 138.1. The kernels are specialised on the input encoding and the multiplier, or on the
+// column mode: run-time branches on them spilled and cost a quarter of the instructions (rows of
+// 64 x 768 x 768: 69.8 M against 52.4 M with the packed arithmetic).
+__device__ int g_fft_wait_error = 0;
+
 constexpr int W32_WARPS = 8;
 constexpr int W32_THREADS = 256;
 
 template <int N>
 struct W32Geom
 {
-    static constexpr int NG = fftw::Warp<N>::NG;
+    static constexpr int NG = N == 768 ? 32 : N / 32;   // threads per transform
+    static constexpr int NS = N / NG;                   // samples a thread loads (32; 24 for 768)
+    static constexpr int K1 = N == 768 ? 24 : NG;       // stage-A outputs per n2
     static constexpr int RPW = 32 / NG;                 // rows per warp
-    static constexpr int ROWS = W32_WARPS * RPW;        // rows per CTA
-    static constexpr int ROW_PAD = NG + 1;
-    static constexpr int ROW_BUF = RPW * 32 * ROW_PAD;  // per warp
+    static constexpr int ROW_PAD = K1 + 1;
+    static constexpr int ROW_BUF = RPW * 32 * ROW_PAD;  // float2 per warp; holds RPW rows of input too
     static constexpr int COLS = W32_THREADS / NG;       // columns per CTA
     static constexpr int COL_PAD = 32 * COLS + (COLS == 8 ? 8 : 0);
-    static constexpr int TW = fftw::Warp<N>::TW_COUNT;
-    static constexpr size_t ROW_SMEM = (TW + static_cast<size_t>(W32_WARPS) * ROW_BUF) * sizeof(float2);
-    static constexpr size_t COL_SMEM = (TW + static_cast<size_t>(NG) * COL_PAD) * sizeof(float2);
+    static constexpr int COL_BUF = (N == 768 ? 32 : NG) * COL_PAD;  // float2 per CTA; holds a tile too
+    static constexpr int tw_count()
+    {
+        if constexpr (N == 768)
+            return fftw::W768::TW_COUNT;
+        else
+            return fftw::Warp<N>::TW_COUNT;
+    }
+    static constexpr int TW = tw_count();
+    static_assert(ROW_BUF >= RPW * N && COL_BUF >= COLS * N, "the transpose buffers hold the input tiles");
+    static_assert(TW % 2 == 0 && ROW_BUF % 2 == 0 && COL_BUF % 2 == 0, "16-byte aligned buffers");
+    // the column tile sits on a 128-byte boundary (tensor copies)
+    static constexpr size_t ROW_SMEM =
+        (TW + static_cast<size_t>(W32_WARPS) * ROW_BUF) * sizeof(float2) + W32_WARPS * sizeof(uint64_t);
+    static constexpr size_t COL_SMEM =
+        128 + (TW + static_cast<size_t>(COL_BUF)) * sizeof(float2) + 2 * sizeof(uint64_t);
 };
 
-// First-stage samples of one row: x[j] = converted sample at e0 + STRIDE j (j < NS) of the input,
-// times premul[l0 + STRIDE j] when the pass has one, conjugated for an inverse pass. Every load of
-// the thread is issued before any is used (the input kind is a uniform branch).
-template <int NS, int STRIDE>
-__device__ __forceinline__ void load_row_samples(const RowPass& p, const void* p_in, size_t e0, size_t l0,
-                                                 float2 (&x)[32])
+// Converted sample j of a row in shared memory at `row` + STRIDE j.
+template <int KIND>
+__device__ __forceinline__ float2 staged_sample(const void* row, int at, bool swap)
 {
-    const bool inv = p.inverse != 0;
-    if (p.in_kind == IN_C64)
+    if constexpr (KIND == IN_U8)
+        return make_float2(static_cast<float>(static_cast<const uint8_t*>(row)[at]) * 257.0f, 0.f);
+    else if constexpr (KIND == IN_U16)
     {
-        const float2* in = static_cast<const float2*>(p_in) + e0;
-#pragma unroll
-        for (int j = 0; j < NS; ++j)
-            x[j] = __ldg(in + STRIDE * j);
-        if (p.premul)
-        {
-            const float2* L = p.premul + l0;
-#pragma unroll
-            for (int j = 0; j < NS; ++j)
-                x[j] = cmul(x[j], __ldg(L + STRIDE * j));
-        }
+        uint16_t u = static_cast<const uint16_t*>(row)[at];
+        if (swap)
+            u = static_cast<uint16_t>((u << 8) | (u >> 8));
+        return make_float2(static_cast<float>(u), 0.f);
     }
+    else if constexpr (KIND == IN_F32)
+        return make_float2(static_cast<const float*>(row)[at], 0.f);
     else
-    {
-        float v[NS];
-        bool pre_done = false;  // x already holds the converted, premultiplied samples
-        switch (p.in_kind)
-        {
-        case IN_U8:
-        {
-            const uint8_t* in = static_cast<const uint8_t*>(p_in) + e0;
-            uint8_t u[NS];
-#pragma unroll
-            for (int j = 0; j < NS; ++j)
-                u[j] = __ldcs(in + STRIDE * j);
-            if (p.premul)
-            {
-                // the lens loads go out before the pixels are used: one memory round trip, not two
-                const float2* L = p.premul + l0;
-#pragma unroll
-                for (int j = 0; j < NS; ++j)
-                    x[j] = __ldg(L + STRIDE * j);
-#pragma unroll
-                for (int j = 0; j < NS; ++j)
-                {
-                    const float f = static_cast<float>(u[j]) * 257.0f;
-                    x[j] = make_float2(f * x[j].x, f * x[j].y);
-                }
-                pre_done = true;
-                break;
-            }
-#pragma unroll
-            for (int j = 0; j < NS; ++j)
-                v[j] = static_cast<float>(u[j]) * 257.0f;
-            break;
-        }
-        case IN_U16:
-        case IN_U16_BE:
-        {
-            const uint16_t* in = static_cast<const uint16_t*>(p_in) + e0;
-            uint16_t u[NS];
-#pragma unroll
-            for (int j = 0; j < NS; ++j)
-                u[j] = __ldcs(in + STRIDE * j);
-            const bool swap = p.in_kind == IN_U16_BE;
-#pragma unroll
-            for (int j = 0; j < NS; ++j)
-                v[j] = static_cast<float>(swap ? static_cast<uint16_t>((u[j] << 8) | (u[j] >> 8)) : u[j]);
-            break;
-        }
-        default:
-        {
-            const float* in = static_cast<const float*>(p_in) + e0;
-#pragma unroll
-            for (int j = 0; j < NS; ++j)
-                v[j] = __ldcs(in + STRIDE * j);
-            break;
-        }
-        }
-        if (pre_done)
-        {
-        }
-        else if (p.premul)
-        {
-            const float2* L = p.premul + l0;
-#pragma unroll
-            for (int j = 0; j < NS; ++j)
-            {
-                const float2 l = __ldg(L + STRIDE * j);
-                x[j] = make_float2(v[j] * l.x, v[j] * l.y);
-            }
-        }
-        else
-        {
-#pragma unroll
-            for (int j = 0; j < NS; ++j)
-                x[j] = make_float2(v[j], 0.f);
-        }
-    }
-    if (inv)
-    {
-#pragma unroll
-        for (int j = 0; j < NS; ++j)
-            x[j] = cconj(x[j]);
-    }
+        return static_cast<const float2*>(row)[at];
 }
 
-template <int N>
-__global__ void __launch_bounds__(W32_THREADS, 2) k_fft_rows_w32(RowPass p)
+// Row pass: units of RPW rows, `per_frame` per frame; with a premultiplier the frames of one row
+// block are adjacent (the multiplier rows stay in L1), else the rows of one frame. KIND: the input
+// encoding (IN_U16 for both byte orders). The input rows of the next unit land in the warp's
+// transpose block by one bulk copy; without `bulk` (input off 16-byte alignment, engine mode 2)
+// the lanes copy them there.
+template <int N, int KIND, bool PREMUL>
+__global__ void __launch_bounds__(W32_THREADS, 2) k_fft_rows_warp(RowPass p, int per_frame, int nframes, int bulk)
 {
     using Gm = W32Geom<N>;
-    using Wp = fftw::Warp<N>;
-    constexpr int NG = Gm::NG;
-    extern __shared__ float2 smem[];
+    constexpr int NG = Gm::NG, NS = Gm::NS;
+    constexpr int ESIZE = KIND == IN_U8 ? 1 : KIND == IN_U16 ? 2 : KIND == IN_F32 ? 4 : 8;
+    extern __shared__ __align__(16) float2 smem[];
     if (!ctl_active(p.ctl))
         return;
-    const float2* tw = stage_twiddles(smem, p.tw, Gm::TW, W32_THREADS);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    float2* buf = smem + Gm::TW + warp * Gm::ROW_BUF;
+    uint64_t* bar = reinterpret_cast<uint64_t*>(smem + Gm::TW + W32_WARPS * Gm::ROW_BUF) + warp;
+    const uint8_t* p_in = static_cast<const uint8_t*>(p.in) + (p.raw_from_ctl ? p.ctl->raw_offset : 0);
+    const int units = per_frame * nframes;
+    const bool inv = p.inverse != 0, swap = p.in_kind == IN_U16_BE;
+    // unit u: rows y0 .. of frame f
+    auto locate = [&](int u, int& f, int& y0) {
+        if (PREMUL)
+        {
+            const int rb = u / nframes;
+            f = u - rb * nframes;
+            y0 = rb * Gm::RPW;
+        }
+        else
+        {
+            f = u / per_frame;
+            y0 = (u - f * per_frame) * Gm::RPW;
+        }
+    };
+    auto source = [&](int f, int y0) {
+        return p_in + (static_cast<size_t>(f) * p.in_frame + static_cast<size_t>(y0) * N) * ESIZE;
+    };
+    auto issue = [&](int u) {
+        int f, y0;
+        locate(u, f, y0);
+        const uint32_t bytes = static_cast<uint32_t>(min(Gm::RPW, p.rows - y0)) * N * ESIZE;
+        tc::mbar_arrive_expect_tx(bar, bytes);
+        tc::bulk_g2s(buf, source(f, y0), bytes, bar);
+    };
+    const int u0 = blockIdx.x * W32_WARPS + warp, du = gridDim.x * W32_WARPS;
+    if (lane == 0)
+    {
+        tc::mbar_init(bar, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        tc::fence_async_smem();
+        if (bulk && u0 < units)
+            issue(u0);
+    }
+    const float2* tw = stage_twiddles(smem, p.tw, Gm::TW, W32_THREADS);  // ends with a CTA barrier
+
     const int r = lane / NG, g = lane % NG;
-    const int y = blockIdx.x * Gm::ROWS + warp * Gm::RPW + r;
-    // lanes of a row past the frame's last row compute on zeros and store nothing (they take part
-    // in the warp's transpose)
-    const bool row_ok = y < p.rows;
-    const int yc = row_ok ? y : 0;
-    float2* buf = smem + Gm::TW + warp * Gm::ROW_BUF + r * 32 * Gm::ROW_PAD;
-    const int b = blockIdx.y;
-    const void* p_in = p.raw_from_ctl ? static_cast<const void*>(static_cast<const uint8_t*>(p.in) + p.ctl->raw_offset)
-                                      : p.in;
-    const size_t e0 = static_cast<size_t>(b) * p.in_frame + static_cast<size_t>(yc) * N + g;
-    const bool inv = p.inverse != 0;
-
-    float2 x[32];
-    load_row_samples<32, NG>(p, p_in, e0, static_cast<size_t>(yc) * N + g, x);
-    Wp::stage_a(x, tw, g);
-    // transpose: z[n2][k1] at buf[n2 * ROW_PAD + k1]; thread g then reads z[n2][g] for every n2
-#pragma unroll
-    for (int e = 0; e < 32; ++e)
-        buf[Wp::n2_of(e, g) * Gm::ROW_PAD + Wp::k1_of(e)] = x[e];
-    __syncwarp();
-#pragma unroll
-    for (int n2 = 0; n2 < 32; ++n2)
-        x[n2] = buf[n2 * Gm::ROW_PAD + g];
-    fftw::dft32(x);
-
-    if (!row_ok)
-        return;
-    float2* o = p.out + p.out_map.offset(b) + static_cast<size_t>(y) * N + g;
-    const float sc = p.scale;
-#pragma unroll
-    for (int k2 = 0; k2 < 32; ++k2)
+    const float2 scale = make_float2(p.scale, inv ? -p.scale : p.scale);
+    uint32_t phase = 0;
+    for (int u = u0; u < units; u += du)
     {
-        float2 v = x[k2];
-        if (inv)
-            v = cconj(v);
-        v = cscale(v, sc);
-        if (p.stream_out)
-            __stcs(o + NG * k2, v);
-        else
-            o[NG * k2] = v;
-    }
-}
-
-// Column transpose through shared memory: thread (c, g) writes its z[n2][k1], then reads z[n2][g]
-// for every n2 (g now the k1 it owns). Ends with a barrier so the block can be reused.
-template <int N>
-__device__ __forceinline__ void w32_col_exchange(float2 (&x)[32], float2* S, int c, int g)
-{
-    using Gm = W32Geom<N>;
-    using Wp = fftw::Warp<N>;
-#pragma unroll
-    for (int e = 0; e < 32; ++e)
-        S[Wp::k1_of(e) * Gm::COL_PAD + Wp::n2_of(e, g) * Gm::COLS + c] = x[e];
-    __syncthreads();
-    const float2* rd = S + g * Gm::COL_PAD + c;
-#pragma unroll
-    for (int n2 = 0; n2 < 32; ++n2)
-        x[n2] = rd[n2 * Gm::COLS];
-    __syncthreads();
-}
-
-template <int N>
-__global__ void __launch_bounds__(W32_THREADS, 2) k_fft_cols_w32(ColPass p)
-{
-    using Gm = W32Geom<N>;
-    using Wp = fftw::Warp<N>;
-    constexpr int NG = Gm::NG;
-    extern __shared__ float2 smem[];
-    if (!ctl_active(p.ctl))
-        return;
-    const float2* tw = stage_twiddles(smem, p.tw, Gm::TW, W32_THREADS);
-    float2* S = smem + Gm::TW;
-    const int c = threadIdx.x % Gm::COLS, g = threadIdx.x / Gm::COLS;
-    const int W = p.width;
-    const int col = blockIdx.x * Gm::COLS + c;
-    const bool in_range = col < W;
-    const int b = blockIdx.y;
-    // sample g + NG j of column `col` sits at g W + col + j (NG W)
-    const size_t e0 = static_cast<size_t>(g) * W + col;
-    const size_t step = static_cast<size_t>(NG) * W;
-    const float2* in = p.in + static_cast<size_t>(b) * p.in_frame + e0;
-    const bool inv_in = p.mode == 1;
-
-    float2 x[32];
-#pragma unroll
-    for (int j = 0; j < 32; ++j)
-        x[j] = in_range ? in[j * step] : make_float2(0.f, 0.f);
-    if (inv_in)
-    {
-#pragma unroll
-        for (int j = 0; j < 32; ++j)
-            x[j] = cconj(x[j]);
-    }
-    Wp::stage_a(x, tw, g);
-    w32_col_exchange<N>(x, S, c, g);
-    fftw::dft32(x);
-
-    float2* o = p.out + p.out_map.offset(b) + e0;
-    const float sc = p.scale;
-    if (p.mode == 2)
-    {
-        // * G, conjugate, inverse transform (stage B left X[g + NG k2], stage A's input shape)
-        const float2* Gp = p.postmul + e0;
-#pragma unroll
-        for (int k2 = 0; k2 < 32; ++k2)
-        {
-            const float2 gv = in_range ? __ldg(Gp + k2 * step) : make_float2(0.f, 0.f);
-            x[k2] = cconj(cmul(x[k2], gv));
-        }
-        Wp::stage_a(x, tw, g);
-        w32_col_exchange<N>(x, S, c, g);
-        fftw::dft32(x);
-        if (in_range)
-        {
-#pragma unroll
-            for (int k2 = 0; k2 < 32; ++k2)
-                o[k2 * step] = cscale(cconj(x[k2]), sc);
-        }
-        return;
-    }
-    if (!in_range)
-        return;
-#pragma unroll
-    for (int k2 = 0; k2 < 32; ++k2)
-    {
-        float2 v = x[k2];
-        if (inv_in)
-            v = cconj(v);
-        v = cscale(v, sc);
-        if (p.stream_out)
-            __stcs(o + k2 * step, v);
-        else
-            o[k2 * step] = v;
-    }
-}
-
-// ------------------------------------------------------------------ warp engine, TMA-fed columns
-// Persistent column pass (N = 1024): one CTA per SM walks the tiles blockIdx.x, + gridDim.x, ...
-// (a tile = 8 columns x 1024 rows of one frame, 64 KB). The tile two steps ahead is loaded by TMA
-// (four 256-row boxes) into one of two staging buffers while the current tile is transformed
-// from registers, so the column reads stream without the per-tile load latency of the
-// register-loading kernel. The waits are bounded; a wait that gives up sets g_fft_wait_error,
-// lets the copies already issued land and ends the CTA.
-__device__ int g_fft_wait_error = 0;
-
-constexpr int WT_N = 1024;
-constexpr int WT_COLS = W32Geom<WT_N>::COLS;
-constexpr int WT_TILE = WT_N * WT_COLS;  // float2 per tile
-constexpr size_t WT_SMEM = 1024 + (2 * static_cast<size_t>(WT_TILE) + fftw::Warp<WT_N>::NG * W32Geom<WT_N>::COL_PAD +
-                                   fftw::Warp<WT_N>::TW_COUNT) * sizeof(float2) + 64;
-
-__global__ void __launch_bounds__(W32_THREADS, 1) k_fft_cols_w32_tma(const __grid_constant__ CUtensorMap tmap,
-                                                                       ColPass p, int tiles_x, int ntiles)
-{
-    using Gm = W32Geom<WT_N>;
-    using Wp = fftw::Warp<WT_N>;
-    constexpr int NG = Gm::NG;
-    constexpr int COLS = Gm::COLS;
-    extern __shared__ unsigned char smem_raw[];
-    if (!ctl_active(p.ctl))
-        return;
-    float2* stage = reinterpret_cast<float2*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    float2* S = stage + 2 * WT_TILE;
-    float2* tws = S + NG * Gm::COL_PAD;
-    uint64_t* bar = reinterpret_cast<uint64_t*>(tws + Gm::TW);
-    __shared__ int s_abort;
-    volatile int* abort = &s_abort;
-    const int tid = threadIdx.x;
-    if (tid == 0)
-    {
-        tc::mbar_init(&bar[0], 1);
-        tc::mbar_init(&bar[1], 1);
-        s_abort = 0;
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    for (int e = tid; e < Gm::TW; e += W32_THREADS)
-        tws[e] = __ldg(p.tw + e);
-    tc::fence_async_smem();
-    __syncthreads();
-
-    auto issue = [&](int t, int sb) {
-        const int fb = t / tiles_x, tx = t - fb * tiles_x;
-        tc::mbar_arrive_expect_tx(&bar[sb], WT_TILE * sizeof(float2));
-#pragma unroll
-        for (int q = 0; q < WT_N / 256; ++q)
-            tc::tma_load_2d(stage + sb * WT_TILE + q * 256 * COLS, &tmap, tx * COLS * 2, fb * WT_N + q * 256, &bar[sb]);
-    };
-    if (tid == 0)
-    {
-        if (static_cast<int>(blockIdx.x) < ntiles)
-            issue(blockIdx.x, 0);
-        if (static_cast<int>(blockIdx.x + gridDim.x) < ntiles)
-            issue(blockIdx.x + gridDim.x, 1);
-    }
-    const int c = tid % COLS, g = tid / COLS;
-    const int W = p.width;
-    const size_t step = static_cast<size_t>(NG) * W;
-    const bool inv_in = p.mode == 1;
-    const float sc = p.scale;
-    int k = 0;
-    for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++k)
-    {
-        const int sb = k & 1;
-        // every thread waits; the CTA agrees on the outcome so that all of it leaves together
-        const bool landed = tc::mbar_wait(&bar[sb], static_cast<uint32_t>((k >> 1) & 1), abort);
-        if (!__syncthreads_and(landed))
-        {
-            if (tid == 0)
-                s_abort = 1;
-            break;
-        }
+        int f, y0;
+        locate(u, f, y0);
+        const int y = y0 + r;
+        // lanes of a row past the frame's last row compute on other rows' samples and store nothing
+        const bool row_ok = y < p.rows;
         float2 x[32];
+        if constexpr (PREMUL)
         {
-            const float2* src = stage + sb * WT_TILE + g * COLS + c;  // row g + NG j at (g + NG j) * COLS
+            const float2* L = p.premul + static_cast<size_t>(row_ok ? y : y0) * N + g;
 #pragma unroll
-            for (int j = 0; j < 32; ++j)
-                x[j] = src[j * NG * COLS];
+            for (int j = 0; j < NS; ++j)
+                x[j] = __ldg(L + NG * j);
         }
-        __syncthreads();  // stage sb fully read: refill it with the tile two steps ahead
-        if (tid == 0 && t + 2 * static_cast<int>(gridDim.x) < ntiles)
-            issue(t + 2 * gridDim.x, sb);
-        if (inv_in)
+        if (bulk)
         {
-#pragma unroll
-            for (int j = 0; j < 32; ++j)
-                x[j] = cconj(x[j]);
-        }
-        const int fb = t / tiles_x, tx = t - fb * tiles_x;
-        const int col = tx * COLS + c;
-        const bool in_range = col < W;
-        const size_t e0 = static_cast<size_t>(g) * W + col;
-        Wp::stage_a(x, tws, g);
-        w32_col_exchange<WT_N>(x, S, c, g);
-        fftw::dft32(x);
-        float2* o = p.out + p.out_map.offset(fb) + e0;
-        if (p.mode == 2)
-        {
-            const float2* Gp = p.postmul + e0;
-#pragma unroll
-            for (int k2 = 0; k2 < 32; ++k2)
+            const bool landed = tc::mbar_wait(bar, phase);
+            if (!__all_sync(0xffffffffu, landed))
             {
-                const float2 gv = in_range ? __ldg(Gp + k2 * step) : make_float2(0.f, 0.f);
-                x[k2] = cconj(cmul(x[k2], gv));
+                tc::mbar_wait(bar, phase);  // the copy lands before the shared memory is released
+                if (lane == 0)
+                    atomicExch(&g_fft_wait_error, 1);
+                return;
             }
-            Wp::stage_a(x, tws, g);
-            w32_col_exchange<WT_N>(x, S, c, g);
-            fftw::dft32(x);
-            if (in_range)
+            phase ^= 1;
+        }
+        else
+        {
+            const uint8_t* src = source(f, y0);
+            const int n = min(Gm::RPW, p.rows - y0) * N;
+            for (int i = lane; i < n; i += 32)
             {
-#pragma unroll
-                for (int k2 = 0; k2 < 32; ++k2)
-                    o[k2 * step] = cscale(cconj(x[k2]), sc);
-            }
-            continue;
-        }
-        if (!in_range)
-            continue;
-#pragma unroll
-        for (int k2 = 0; k2 < 32; ++k2)
-        {
-            float2 v = x[k2];
-            if (inv_in)
-                v = cconj(v);
-            v = cscale(v, sc);
-            if (p.stream_out)
-                __stcs(o + k2 * step, v);
-            else
-                o[k2 * step] = v;
-        }
-    }
-    __syncthreads();
-    if (s_abort && tid == 0)
-    {
-        // a wait gave up at step k: let the (at most two) copies still in flight land before the
-        // CTA's shared memory is released (bounded waits without the abort shortcut)
-        const int t = blockIdx.x + k * gridDim.x;
-        if (t < ntiles)
-            tc::mbar_wait(&bar[k & 1], static_cast<uint32_t>((k >> 1) & 1));
-        if (t + static_cast<int>(gridDim.x) < ntiles)
-            tc::mbar_wait(&bar[(k + 1) & 1], static_cast<uint32_t>(((k + 1) >> 1) & 1));
-        atomicExch(&g_fft_wait_error, 1);
-    }
-}
-
-// Persistent row pass (N = 1024, 8-/16-bit camera input, optional premultiply): tile = 8 rows of
-// one frame (one row per warp), two CTAs per SM, CTA i takes the contiguous tile range
-// [i per, (i + 1) per) (row block major, frame minor). The raw rows of the tile two steps ahead
-// (8 or 16 KB) are loaded by TMA during the current tile; the lens rows come from L2 with their
-// loads issued before the staged pixels are used. Bounded waits as in k_fft_cols_w32_tma.
-// (Staging the lens rows in shared memory as well, one CTA per SM, measured slower.)
-constexpr int RT_ROWS = 8;
-constexpr size_t RT_RAW_MAX = static_cast<size_t>(RT_ROWS) * WT_N * 2;  // 16-bit input
-constexpr int RT_XBUF = W32Geom<WT_N>::ROW_BUF;                          // per warp (32 x 33)
-constexpr size_t RT_SMEM =
-    1024 + 2 * RT_RAW_MAX + (static_cast<size_t>(W32_WARPS) * RT_XBUF + fftw::Warp<WT_N>::TW_COUNT) * sizeof(float2) + 64;
-
-template <int ESIZE>
-__global__ void __launch_bounds__(W32_THREADS, 2) k_fft_rows_w32_tma(const __grid_constant__ CUtensorMap raw_map,
-                                                                       RowPass p, int nframes, int ntiles, int per)
-{
-    using Wp = fftw::Warp<WT_N>;
-    extern __shared__ unsigned char smem_raw[];
-    if (!ctl_active(p.ctl))
-        return;
-    unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    unsigned char* raw_st = base;  // 2 x RT_RAW_MAX
-    float2* xbuf = reinterpret_cast<float2*>(base + 2 * RT_RAW_MAX);
-    float2* tws = xbuf + W32_WARPS * RT_XBUF;
-    uint64_t* bar = reinterpret_cast<uint64_t*>(tws + Wp::TW_COUNT);
-    __shared__ int s_abort;
-    volatile int* abort = &s_abort;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    if (tid == 0)
-    {
-        tc::mbar_init(&bar[0], 1);
-        tc::mbar_init(&bar[1], 1);
-        s_abort = 0;
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    for (int e = tid; e < Wp::TW_COUNT; e += W32_THREADS)
-        tws[e] = __ldg(p.tw + e);
-    tc::fence_async_smem();
-    __syncthreads();
-
-    const int t0 = blockIdx.x * per;
-    const int t1 = min(t0 + per, ntiles);
-    constexpr uint32_t RAW_TILE = RT_ROWS * WT_N * ESIZE;
-    auto issue_raw = [&](int t, int sb) {
-        const int rb = t / nframes, f = t - rb * nframes;
-        tc::mbar_arrive_expect_tx(&bar[sb], RAW_TILE);
-#pragma unroll
-        for (int q = 0; q < WT_N / 256; ++q)
-            tc::tma_load_2d(raw_st + sb * RT_RAW_MAX + q * RT_ROWS * 256 * ESIZE, &raw_map, q * 256,
-                            f * p.rows + rb * RT_ROWS, &bar[sb]);
-    };
-    if (tid == 0 && t0 < t1)
-    {
-        issue_raw(t0, 0);
-        if (t0 + 1 < t1)
-            issue_raw(t0 + 1, 1);
-    }
-    const bool inv = p.inverse != 0;
-    const bool swap = ESIZE == 2 && p.in_kind == IN_U16_BE;
-    const float sc = p.scale;
-    int k = 0;
-    for (int t = t0; t < t1; ++t, ++k)
-    {
-        const int sb = k & 1;
-        const int rb = t / nframes, f = t - rb * nframes;
-        const size_t row = static_cast<size_t>(rb * RT_ROWS + warp) * WT_N + lane;
-        float2 x[32];
-        if (p.premul)
-        {
-#pragma unroll
-            for (int j = 0; j < 32; ++j)
-                x[j] = __ldg(p.premul + row + 32 * j);
-        }
-        const bool landed = tc::mbar_wait(&bar[sb], static_cast<uint32_t>((k >> 1) & 1), abort);
-        if (!__syncthreads_and(landed))
-        {
-            if (tid == 0)
-                s_abort = 1;
-            break;
-        }
-        // sample n = lane + 32 j of row `warp`: box j / 8 at (warp * 256 + lane + 32 (j % 8))
-        {
-            const unsigned char* rs = raw_st + sb * RT_RAW_MAX;
-#pragma unroll
-            for (int j = 0; j < 32; ++j)
-            {
-                const int off = (j >> 3) * RT_ROWS * 256 + warp * 256 + lane + 32 * (j & 7);
-                float v;
-                if constexpr (ESIZE == 1)
-                    v = static_cast<float>(rs[off]) * 257.0f;
+                if constexpr (KIND == IN_U8)
+                    reinterpret_cast<uint8_t*>(buf)[i] = src[i];
+                else if constexpr (KIND == IN_U16)
+                    reinterpret_cast<uint16_t*>(buf)[i] = reinterpret_cast<const uint16_t*>(src)[i];
+                else if constexpr (KIND == IN_F32)
+                    reinterpret_cast<float*>(buf)[i] = reinterpret_cast<const float*>(src)[i];
                 else
-                {
-                    uint16_t u = reinterpret_cast<const uint16_t*>(rs)[off];
-                    if (swap)
-                        u = static_cast<uint16_t>((u << 8) | (u >> 8));
-                    v = static_cast<float>(u);
-                }
-                x[j] = p.premul ? make_float2(v * x[j].x, v * x[j].y) : make_float2(v, 0.f);
-                if (inv)
+                    buf[i] = reinterpret_cast<const float2*>(src)[i];
+            }
+            __syncwarp();
+        }
+        {
+            const int at = (row_ok ? r : 0) * N + g;
+#pragma unroll
+            for (int j = 0; j < NS; ++j)
+            {
+                const float2 v = staged_sample<KIND>(buf, at + NG * j, swap);
+                if constexpr (PREMUL && KIND == IN_C64)
+                    x[j] = cmul_fma(v, x[j]);
+                else if constexpr (PREMUL)
+                    x[j] = make_float2(v.x * x[j].x, v.x * x[j].y);
+                else
+                    x[j] = v;
+            }
+            if (inv)
+            {
+#pragma unroll
+                for (int j = 0; j < NS; ++j)
                     x[j] = cconj(x[j]);
             }
         }
-        __syncthreads();  // raw stage sb fully read: refill it with the tile two steps ahead
-        if (tid == 0 && t + 2 < t1)
-            issue_raw(t + 2, sb);
+        __syncwarp();  // the block is rewritten by the transpose
 
-        Wp::stage_a(x, tws, lane);
-        float2* buf = xbuf + warp * RT_XBUF;
+        float2* tb = buf + r * 32 * Gm::ROW_PAD;
+        if constexpr (N == 768)
+        {
+            fftw::W768::stage_a24(x, tw, lane);
 #pragma unroll
-        for (int e = 0; e < 32; ++e)
-            buf[lane * W32Geom<WT_N>::ROW_PAD + e] = x[e];
+            for (int k1 = 0; k1 < 24; ++k1)
+                tb[lane * Gm::ROW_PAD + k1] = x[k1];
+        }
+        else
+        {
+            using Wp = fftw::Warp<N>;
+            Wp::stage_a(x, tw, g);
+            // transpose: z[n2][k1] at tb[n2 * ROW_PAD + k1]; thread g then reads z[n2][g] for every n2
+#pragma unroll
+            for (int e = 0; e < 32; ++e)
+                tb[Wp::n2_of(e, g) * Gm::ROW_PAD + Wp::k1_of(e)] = x[e];
+        }
         __syncwarp();
+        const int k1 = g < Gm::K1 ? g : 0;
 #pragma unroll
         for (int n2 = 0; n2 < 32; ++n2)
-            x[n2] = buf[n2 * W32Geom<WT_N>::ROW_PAD + lane];
-        __syncwarp();  // the block is rewritten by the next tile
+            x[n2] = tb[n2 * Gm::ROW_PAD + k1];
+        tc::fence_async_smem();
+        __syncwarp();  // the block is rewritten by the next unit's input
+        if (bulk && lane == 0 && u + du < units)
+            issue(u + du);
         fftw::dft32(x);
 
-        float2* o = p.out + p.out_map.offset(f) + row;
-#pragma unroll
-        for (int k2 = 0; k2 < 32; ++k2)
+        if (!row_ok || g >= Gm::K1)
+            continue;
+        float2* o = p.out + p.out_map.offset(f) + static_cast<size_t>(y) * N + g;
+        if (p.stream_out)
         {
-            float2 v = x[k2];
-            if (inv)
-                v = cconj(v);
-            v = cscale(v, sc);
-            if (p.stream_out)
-                __stcs(o + 32 * k2, v);
-            else
-                o[32 * k2] = v;
+#pragma unroll
+            for (int k2 = 0; k2 < 32; ++k2)
+                __stcs(o + Gm::K1 * k2, fft::pmul(x[k2], scale));
+        }
+        else
+        {
+#pragma unroll
+            for (int k2 = 0; k2 < 32; ++k2)
+                o[Gm::K1 * k2] = fft::pmul(x[k2], scale);
         }
     }
-    __syncthreads();
-    if (s_abort && tid == 0)
+}
+
+// Column pass. One tile = COLS adjacent columns of one frame; the CTA walks tiles blockIdx.x,
+// + gridDim.x, ... MODE: 0 forward, 1 inverse, 2 forward * G then inverse (the AS middle pass).
+// The tile (and, for MODE 2, the transfer function's tile) lands in the transpose block by tensor
+// copies of 256 rows each; without `bulk` (alignment, engine mode 2) the threads copy it there.
+template <int N, int MODE>
+__global__ void __launch_bounds__(W32_THREADS, 2) k_fft_cols_warp(const __grid_constant__ CUtensorMap in_map,
+                                                                  const __grid_constant__ CUtensorMap g_map, ColPass p,
+                                                                  int tiles_x, int ntiles, int bulk)
+{
+    using Gm = W32Geom<N>;
+    constexpr int NG = Gm::NG, NS = Gm::NS, K1 = Gm::K1, C = Gm::COLS;
+    extern __shared__ unsigned char smem_raw[];
+    if (!ctl_active(p.ctl))
+        return;
+    float2* S = reinterpret_cast<float2*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
+    float2* tw = S + Gm::COL_BUF;
+    uint64_t* bar = reinterpret_cast<uint64_t*>(tw + Gm::TW);
+    __shared__ int s_abort;
+    volatile int* abort = &s_abort;
+    const int tid = threadIdx.x;
+    // one tile of `map` (columns tx C .., rows fb N ..) into S
+    auto issue = [&](const CUtensorMap* map, int fb, int tx) {
+        tc::mbar_arrive_expect_tx(bar, C * N * sizeof(float2));
+#pragma unroll
+        for (int q = 0; q < N / 256; ++q)
+            tc::tma_load_2d(S + q * 256 * C, map, tx * C * 2, fb * N + q * 256, bar);
+    };
+    if (tid == 0)
     {
-        // copies still in flight at the failed step k land before the shared memory is released
-        const int t = t0 + k;
-        if (t < t1)
-            tc::mbar_wait(&bar[k & 1], static_cast<uint32_t>((k >> 1) & 1));
-        if (t + 1 < t1)
-            tc::mbar_wait(&bar[(k + 1) & 1], static_cast<uint32_t>(((k + 1) >> 1) & 1));
+        s_abort = 0;
+        tc::mbar_init(bar, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        tc::fence_async_smem();
+        if (bulk && static_cast<int>(blockIdx.x) < ntiles)
+            issue(&in_map, blockIdx.x / tiles_x, blockIdx.x % tiles_x);
+    }
+    stage_twiddles(tw, p.tw, Gm::TW, W32_THREADS);  // ends with a CTA barrier
+
+    const int c = tid % C, g = tid / C;
+    const size_t W = static_cast<size_t>(p.width);
+    const float2 scale = make_float2(p.scale, MODE != 0 ? -p.scale : p.scale);
+    const bool active_b = g < K1;  // N = 768: a quarter of the threads idle in one stage
+    uint32_t phase = 0;
+    // the tile (columns tx C .. of the N rows at src) is in S: every thread waits for the copies, and
+    // the CTA agrees on the outcome so that all of it leaves together; or the threads copy it
+    auto landed = [&](const float2* src, int tx) -> bool {
+        if (bulk)
+        {
+            const bool ok = tc::mbar_wait(bar, phase, abort);
+            phase ^= 1;
+            return __syncthreads_and(ok);
+        }
+        const int col = tx * C + c;
+#pragma unroll 4
+        for (int j = 0; j < NS; ++j)
+            S[(g + NG * j) * C + c] = col < p.width ? src[static_cast<size_t>(g + NG * j) * W + col] : make_float2(0.f, 0.f);
+        __syncthreads();
+        return true;
+    };
+    // every thread has read what it needs from S: ask for the tile of the next use
+    auto refill = [&](const CUtensorMap* map, int fb, int tx, bool any) {
+        tc::fence_async_smem();
+        __syncthreads();
+        if (bulk && any && tid == 0)
+            issue(map, fb, tx);
+    };
+    bool gave_up = false;
+    for (int t = blockIdx.x; t < ntiles; t += gridDim.x)
+    {
+        const int fb = t / tiles_x, tx = t - fb * tiles_x;
+        const int tn = t + static_cast<int>(gridDim.x);
+        const bool in_range = tx * C + c < p.width;
+        if (!landed(p.in + static_cast<size_t>(fb) * p.in_frame, tx))
+        {
+            gave_up = true;
+            break;
+        }
+        float2 x[32];
+#pragma unroll
+        for (int j = 0; j < NS; ++j)
+            x[j] = S[(g + NG * j) * C + c];
+        __syncthreads();
+        if constexpr (MODE == 1)
+        {
+#pragma unroll
+            for (int j = 0; j < NS; ++j)
+                x[j] = cconj(x[j]);
+        }
+        // forward: stage A, transpose ([k1][n2][c]), stage B; element k2 of thread g < K1 is X[g + K1 k2]
+        if constexpr (N == 768)
+        {
+            fftw::W768::stage_a24(x, tw, g);
+#pragma unroll
+            for (int k1 = 0; k1 < 24; ++k1)
+                S[k1 * Gm::COL_PAD + g * C + c] = x[k1];
+        }
+        else
+        {
+            using Wp = fftw::Warp<N>;
+            Wp::stage_a(x, tw, g);
+#pragma unroll
+            for (int e = 0; e < 32; ++e)
+                S[Wp::k1_of(e) * Gm::COL_PAD + Wp::n2_of(e, g) * C + c] = x[e];
+        }
+        __syncthreads();
+        if (active_b)
+        {
+#pragma unroll
+            for (int n2 = 0; n2 < 32; ++n2)
+                x[n2] = S[g * Gm::COL_PAD + n2 * C + c];
+        }
+        float2* o = p.out + p.out_map.offset(fb) + static_cast<size_t>(g) * W + (tx * C + c);
+        if constexpr (MODE != 2)
+        {
+            refill(&in_map, tn / tiles_x, tn % tiles_x, tn < ntiles);
+            if (!active_b)
+                continue;
+            fftw::dft32(x);
+            if (!in_range)
+                continue;
+            const size_t step = static_cast<size_t>(K1) * W;
+            if (p.stream_out)
+            {
+#pragma unroll
+                for (int k2 = 0; k2 < 32; ++k2, o += step)
+                    __stcs(o, fft::pmul(x[k2], scale));
+            }
+            else
+            {
+#pragma unroll
+                for (int k2 = 0; k2 < 32; ++k2, o += step)
+                    *o = fft::pmul(x[k2], scale);
+            }
+        }
+        else
+        {
+            // * G, conjugate, inverse transform: stage B's output has stage A's input shape (for
+            // N = 768 that of the DFT32-first order)
+            refill(&g_map, 0, tx, true);
+            if (active_b)
+                fftw::dft32(x);
+            if (!landed(p.postmul, tx))
+            {
+                gave_up = true;
+                break;
+            }
+            if (active_b)
+            {
+#pragma unroll
+                for (int k2 = 0; k2 < 32; ++k2)
+                    x[k2] = cconj(cmul_fma(x[k2], S[(g + K1 * k2) * C + c]));
+            }
+            __syncthreads();
+            if constexpr (N == 768)
+            {
+                if (active_b)
+                {
+                    fftw::W768::stage_a32(x, tw, g);
+#pragma unroll
+                    for (int k1 = 0; k1 < 32; ++k1)
+                        S[k1 * Gm::COL_PAD + g * C + c] = x[k1];
+                }
+            }
+            else
+            {
+                using Wp = fftw::Warp<N>;
+                Wp::stage_a(x, tw, g);
+#pragma unroll
+                for (int e = 0; e < 32; ++e)
+                    S[Wp::k1_of(e) * Gm::COL_PAD + Wp::n2_of(e, g) * C + c] = x[e];
+            }
+            __syncthreads();
+#pragma unroll
+            for (int n2 = 0; n2 < NS; ++n2)
+                x[n2] = S[g * Gm::COL_PAD + n2 * C + c];
+            refill(&in_map, tn / tiles_x, tn % tiles_x, tn < ntiles);
+            if constexpr (N == 768)
+                fftw::dft24(x);
+            else
+                fftw::dft32(x);
+            if (!in_range)
+                continue;
+            const size_t step = static_cast<size_t>(NG) * W;
+#pragma unroll
+            for (int k2 = 0; k2 < NS; ++k2, o += step)
+                *o = fft::pmul(x[k2], scale);
+        }
+    }
+    if (gave_up && tid == 0)
+    {
+        // the copy still in flight lands before the CTA's shared memory is released
+        tc::mbar_wait(bar, phase ^ 1);
         atomicExch(&g_fft_wait_error, 1);
     }
-}
-
-// ------------------------------------------------------------------ warp engine, N = 768
-// Rows: one warp per row (V24: 32 lanes load and run DFT24, lanes 0..23 run the DFT32 and store).
-// Columns: 8 columns per CTA, thread (c, g) = (t & 7, t >> 3); forward = V24 (warps 6-7 idle in
-// stage B), the AS middle pass continues with V32 (warps 6-7 idle in its stage A).
-constexpr int W768_ROWS = 8;
-constexpr int W768_ROW_PAD = 25;
-constexpr int W768_COLS = 8;
-constexpr int W768_COL_PAD = 32 * W768_COLS + 8;
-constexpr size_t W768_ROW_SMEM =
-    (fftw::W768::TW_COUNT + static_cast<size_t>(W768_ROWS) * 32 * W768_ROW_PAD) * sizeof(float2);
-constexpr size_t W768_COL_SMEM = (fftw::W768::TW_COUNT + static_cast<size_t>(32) * W768_COL_PAD) * sizeof(float2);
-
-__global__ void __launch_bounds__(W32_THREADS, 2) k_fft_rows_w768(RowPass p)
-{
-    using W = fftw::W768;
-    extern __shared__ float2 smem[];
-    if (!ctl_active(p.ctl))
-        return;
-    const float2* tw = stage_twiddles(smem, p.tw, W::TW_COUNT, W32_THREADS);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int y = blockIdx.x * W768_ROWS + warp;
-    if (y >= p.rows)
-        return;
-    float2* buf = smem + W::TW_COUNT + warp * 32 * W768_ROW_PAD;
-    const int b = blockIdx.y;
-    const void* p_in = p.raw_from_ctl ? static_cast<const void*>(static_cast<const uint8_t*>(p.in) + p.ctl->raw_offset)
-                                      : p.in;
-    const size_t l0 = static_cast<size_t>(y) * W::N + lane;
-    float2 x[32];
-    load_row_samples<24, 32>(p, p_in, static_cast<size_t>(b) * p.in_frame + l0, l0, x);
-    W::stage_a24(x, tw, lane);
-#pragma unroll
-    for (int k1 = 0; k1 < 24; ++k1)
-        buf[lane * W768_ROW_PAD + k1] = x[k1];
-    __syncwarp();
-    if (lane >= 24)
-        return;
-#pragma unroll
-    for (int n2 = 0; n2 < 32; ++n2)
-        x[n2] = buf[n2 * W768_ROW_PAD + lane];
-    fftw::dft32(x);
-    const bool inv = p.inverse != 0;
-    float2* o = p.out + p.out_map.offset(b) + l0;
-    const float sc = p.scale;
-#pragma unroll
-    for (int k2 = 0; k2 < 32; ++k2)
-    {
-        float2 v = x[k2];
-        if (inv)
-            v = cconj(v);
-        v = cscale(v, sc);
-        if (p.stream_out)
-            __stcs(o + 24 * k2, v);
-        else
-            o[24 * k2] = v;
-    }
-}
-
-__global__ void __launch_bounds__(W32_THREADS, 2) k_fft_cols_w768(ColPass p)
-{
-    using W7 = fftw::W768;
-    extern __shared__ float2 smem[];
-    if (!ctl_active(p.ctl))
-        return;
-    const float2* tw = stage_twiddles(smem, p.tw, W7::TW_COUNT, W32_THREADS);
-    float2* S = smem + W7::TW_COUNT;
-    const int c = threadIdx.x & (W768_COLS - 1), g = threadIdx.x / W768_COLS;
-    const int W = p.width;
-    const int col = blockIdx.x * W768_COLS + c;
-    const bool in_range = col < W;
-    const int b = blockIdx.y;
-    const size_t Ws = static_cast<size_t>(W);
-    const float2* in = p.in + static_cast<size_t>(b) * p.in_frame + col;
-    float2* o = p.out + p.out_map.offset(b) + col;
-    const bool inv_in = p.mode == 1;
-    const bool active_b = g < 24;  // stage B of V24 / stage A of V32
-
-    // V24 forward: samples g + 32 i (i < 24)
-    float2 x[32];
-#pragma unroll
-    for (int i = 0; i < 24; ++i)
-        x[i] = in_range ? in[(static_cast<size_t>(g) + 32 * i) * Ws] : make_float2(0.f, 0.f);
-    if (inv_in)
-    {
-#pragma unroll
-        for (int i = 0; i < 24; ++i)
-            x[i] = cconj(x[i]);
-    }
-    W7::stage_a24(x, tw, g);
-#pragma unroll
-    for (int k1 = 0; k1 < 24; ++k1)
-        S[k1 * W768_COL_PAD + g * W768_COLS + c] = x[k1];
-    __syncthreads();
-    if (active_b)
-    {
-#pragma unroll
-        for (int n2 = 0; n2 < 32; ++n2)
-            x[n2] = S[g * W768_COL_PAD + n2 * W768_COLS + c];
-        fftw::dft32(x);  // X[g + 24 k2], k2 < 32
-    }
-    __syncthreads();
-    const float sc = p.scale;
-    if (p.mode != 2)
-    {
-        if (!active_b || !in_range)
-            return;
-#pragma unroll
-        for (int k2 = 0; k2 < 32; ++k2)
-        {
-            float2 v = x[k2];
-            if (inv_in)
-                v = cconj(v);
-            v = cscale(v, sc);
-            float2* d = o + (static_cast<size_t>(g) + 24 * k2) * Ws;
-            if (p.stream_out)
-                __stcs(d, v);
-            else
-                *d = v;
-        }
-        return;
-    }
-    // * G, conjugate, V32 inverse (samples g + 24 i, i < 32, g < 24)
-    if (active_b)
-    {
-        const float2* Gp = p.postmul + col;
-#pragma unroll
-        for (int k2 = 0; k2 < 32; ++k2)
-        {
-            const float2 gv = in_range ? __ldg(Gp + (static_cast<size_t>(g) + 24 * k2) * Ws) : make_float2(0.f, 0.f);
-            x[k2] = cconj(cmul(x[k2], gv));
-        }
-        W7::stage_a32(x, tw, g);
-#pragma unroll
-        for (int k1 = 0; k1 < 32; ++k1)
-            S[k1 * W768_COL_PAD + g * W768_COLS + c] = x[k1];
-    }
-    __syncthreads();
-#pragma unroll
-    for (int n2 = 0; n2 < 24; ++n2)
-        x[n2] = S[g * W768_COL_PAD + n2 * W768_COLS + c];
-    fftw::dft24(x);  // X[g + 32 k2], k2 < 24
-    if (!in_range)
-        return;
-#pragma unroll
-    for (int k2 = 0; k2 < 24; ++k2)
-        o[(static_cast<size_t>(g) + 32 * k2) * Ws] = cscale(cconj(x[k2]), sc);
 }
 
 // Raw -> complex into ring slots (space transformation NONE), 8 pixels of one frame per thread
@@ -1278,17 +999,12 @@ const float2* twiddles()
     return base ? base + g_tw_offset[N] : nullptr;
 }
 
-const float2* twiddles_w768()
-{
-    const float2* base = twiddle_base();
-    return base ? base + g_tw_w768_offset : nullptr;
-}
-
+// the warp engine's tables (N = 512, 768, 1024)
 template <int N>
-const float2* twiddles_w32()
+const float2* twiddles_warp()
 {
     const float2* base = twiddle_base();
-    return base ? base + g_tw_w32_offset[N == 1024 ? 1 : 0] : nullptr;
+    return base ? base + (N == 768 ? g_tw_w768_offset : g_tw_w32_offset[N == 1024 ? 1 : 0]) : nullptr;
 }
 
 }  // namespace
@@ -1317,7 +1033,7 @@ constexpr int col_lanes()
 
 std::atomic<int> g_fft_engine{0};  // 0 automatic (warp engine for 512-, 768- and 1024-point transforms), 1 tile engine only
 
-std::atomic<int> g_fft_tma{1};  // 1: TMA-fed persistent row / column passes where they apply
+std::atomic<int> g_fft_bulk{1};  // 1: the warp engine's passes are fed by bulk copies where they apply
 
 int device_sms()
 {
@@ -1330,177 +1046,77 @@ int device_sms()
     return sms;
 }
 
-// Persistent TMA-fed row pass for N = 1024 (8-/16-bit input outside served cycles); false when it
-// does not apply (the caller then launches the register-loading kernel).
-bool launch_rows_w32_tma(const RowPass& p, int nframes, cudaStream_t st, hv_status* status)
+constexpr size_t kL2Bytes = size_t(128) << 20;
+
+// CTAs of a persistent pass: two per SM, less the SMs left to other streams, at most one per tile.
+int warp_grid(int tiles, int reserve_sms)
 {
-    const int esize = p.in_kind == IN_U8 ? 1 : (p.in_kind == IN_U16 || p.in_kind == IN_U16_BE) ? 2 : 0;
-    if (!g_fft_tma.load() || esize == 0 || p.raw_from_ctl || (p.rows % RT_ROWS) != 0 ||
-        p.in_frame != static_cast<size_t>(p.rows) * WT_N)
-        return false;
     const int sms = device_sms();
-    if (sms <= 0)
-        return false;
-    CUtensorMap raw_map;
-    if (!tc::encode_tmap_2d(&raw_map, esize == 1 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_UINT16,
-                            p.in, WT_N, static_cast<uint64_t>(nframes) * p.rows, static_cast<uint64_t>(WT_N) * esize,
-                            256, RT_ROWS))
-        return false;
-    *status = HV_OK;
-    const int ntiles = (p.rows / RT_ROWS) * nframes;
-    const int use = sms - p.reserve_sms > 0 ? sms - p.reserve_sms : 1;
-    const int per = (ntiles + 2 * use - 1) / (2 * use);  // two CTAs per SM
-    const int grid = (ntiles + per - 1) / per;
-    RowPass q = p;
-    if ((q.tw = twiddles_w32<WT_N>()) == nullptr)
-    {
-        *status = HV_ERR_CUDA;
-        return true;
-    }
-    q.tw_count = fftw::Warp<WT_N>::TW_COUNT;
-    cudaError_t e;
-    if (esize == 1)
-    {
-        e = cudaFuncSetAttribute(k_fft_rows_w32_tma<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(RT_SMEM));
-        if (e == cudaSuccess)
-            k_fft_rows_w32_tma<1><<<grid, W32_THREADS, RT_SMEM, st>>>(raw_map, q, nframes, ntiles, per);
-    }
-    else
-    {
-        e = cudaFuncSetAttribute(k_fft_rows_w32_tma<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(RT_SMEM));
-        if (e == cudaSuccess)
-            k_fft_rows_w32_tma<2><<<grid, W32_THREADS, RT_SMEM, st>>>(raw_map, q, nframes, ntiles, per);
-    }
-    if (e == cudaSuccess)
-        e = cudaGetLastError();
-    if (e != cudaSuccess)
-    {
-        set_last_error_msg(cudaGetErrorString(e));
-        *status = HV_ERR_CUDA;
-        return true;
-    }
-    count_launch();
-    return true;
+    const int use = 2 * (sms - reserve_sms > 0 ? sms - reserve_sms : 1);
+    return tiles < use ? tiles : use;
 }
 
 template <int N>
-hv_status launch_rows_w32(const RowPass& p, int nframes, cudaStream_t st)
+hv_status launch_rows_warp(const RowPass& p, int nframes, cudaStream_t st)
 {
-    if constexpr (N == WT_N)
-    {
-        hv_status r;
-        if (launch_rows_w32_tma(p, nframes, st, &r))
-            return r;
-    }
     using Gm = W32Geom<N>;
-    HV_CUDA_TRY(cudaFuncSetAttribute(k_fft_rows_w32<N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     static_cast<int>(Gm::ROW_SMEM)));
     RowPass q = p;
-    if ((q.tw = twiddles_w32<N>()) == nullptr)
+    if ((q.tw = twiddles_warp<N>()) == nullptr)
         return HV_ERR_CUDA;
     q.tw_count = Gm::TW;
-    dim3 grid((p.rows + Gm::ROWS - 1) / Gm::ROWS, nframes);
-    k_fft_rows_w32<N><<<grid, W32_THREADS, Gm::ROW_SMEM, st>>>(q);
+    const int per_frame = (p.rows + Gm::RPW - 1) / Gm::RPW;
+    const int units = per_frame * nframes;
+    int grid = warp_grid((units + W32_WARPS - 1) / W32_WARPS, p.reserve_sms);
+    // Complex input (the inverse rows of the angular spectrum) whose input and output exceed L2 is
+    // bound by DRAM: two units per warp instead of a persistent grid read and write it faster
+    // (inverse rows of 64 frames of 768 x 768: 110.4 -> 94.7 us, 32 of 1024 x 1024: 95.2 -> 85.0 us),
+    // and below that size slower (12 frames of 768 x 768: 22.9 -> 24.5 us).
+    if (p.in_kind == IN_C64 && p.reserve_sms == 0 && 16 * p.in_frame * static_cast<size_t>(nframes) > kL2Bytes)
+        grid = (units + 2 * W32_WARPS - 1) / (2 * W32_WARPS);
+    // bulk copies start on 16 bytes (rows of every input kind are a multiple of 16 bytes long)
+    const bool bulk = g_fft_bulk.load() && (reinterpret_cast<uintptr_t>(p.in) & 15) == 0 &&
+                      (p.in_frame * static_cast<size_t>(in_kind_bytes(p.in_kind))) % 16 == 0;
+    void (*kern)(RowPass, int, int, int) = nullptr;
+    const bool pre = p.premul != nullptr;
+    switch (p.in_kind)
+    {
+    case IN_U8: kern = pre ? k_fft_rows_warp<N, IN_U8, true> : k_fft_rows_warp<N, IN_U8, false>; break;
+    case IN_U16:
+    case IN_U16_BE: kern = pre ? k_fft_rows_warp<N, IN_U16, true> : k_fft_rows_warp<N, IN_U16, false>; break;
+    case IN_F32: kern = pre ? k_fft_rows_warp<N, IN_F32, true> : k_fft_rows_warp<N, IN_F32, false>; break;
+    default: kern = pre ? k_fft_rows_warp<N, IN_C64, true> : k_fft_rows_warp<N, IN_C64, false>; break;
+    }
+    HV_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(Gm::ROW_SMEM)));
+    kern<<<grid, W32_THREADS, Gm::ROW_SMEM, st>>>(q, per_frame, nframes, bulk ? 1 : 0);
     HV_LAUNCH_CHECK();
     count_launch();
     return HV_OK;
 }
 
-// Persistent TMA-fed column pass for N = 1024; false when it does not apply (the caller then
-// launches the register-loading kernel).
-bool launch_cols_w32_tma(const ColPass& p, int nframes, cudaStream_t st, hv_status* status)
+template <int N>
+hv_status launch_cols_warp(const ColPass& p, int nframes, cudaStream_t st)
 {
-    // forward / inverse passes only: the AS middle pass (two transforms per tile) is compute-bound
-    // at one CTA of 8 warps per SM and stays on the register-loading kernel (2 CTAs per SM)
-    if (!g_fft_tma.load() || p.mode == 2 || p.in_frame != static_cast<size_t>(p.width) * WT_N ||
-        (p.width % WT_COLS) != 0)
-        return false;
-    CUtensorMap map;
-    if (!tc::encode_tmap_2d_f32(&map, p.in, static_cast<uint64_t>(p.width) * 2, static_cast<uint64_t>(nframes) * WT_N,
-                                static_cast<uint64_t>(p.width) * sizeof(float2), WT_COLS * 2, 256))
-        return false;
-    const int sms = device_sms();
-    if (sms <= 0)
-        return false;
-    *status = HV_OK;
-    const cudaError_t e = cudaFuncSetAttribute(k_fft_cols_w32_tma, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               static_cast<int>(WT_SMEM));
-    if (e != cudaSuccess)
-    {
-        *status = HV_ERR_CUDA;
-        return true;
-    }
+    using Gm = W32Geom<N>;
     ColPass q = p;
-    if ((q.tw = twiddles_w32<WT_N>()) == nullptr)
-    {
-        *status = HV_ERR_CUDA;
-        return true;
-    }
-    q.tw_count = fftw::Warp<WT_N>::TW_COUNT;
-    const int tiles_x = p.width / WT_COLS;
+    if ((q.tw = twiddles_warp<N>()) == nullptr)
+        return HV_ERR_CUDA;
+    q.tw_count = Gm::TW;
+    const int tiles_x = (p.width + Gm::COLS - 1) / Gm::COLS;
     const int ntiles = tiles_x * nframes;
-    const int use = sms - p.reserve_sms > 0 ? sms - p.reserve_sms : 1;
-    const int grid = ntiles < use ? ntiles : use;
-    k_fft_cols_w32_tma<<<grid, W32_THREADS, WT_SMEM, st>>>(map, q, tiles_x, ntiles);
-    const cudaError_t le = cudaGetLastError();
-    if (le != cudaSuccess)
-    {
-        set_last_error_msg(cudaGetErrorString(le));
-        *status = HV_ERR_CUDA;
-        return true;
-    }
-    count_launch();
-    return true;
-}
-
-template <int N>
-hv_status launch_cols_w32(const ColPass& p, int nframes, cudaStream_t st)
-{
-    if constexpr (N == WT_N)
-    {
-        hv_status r;
-        if (launch_cols_w32_tma(p, nframes, st, &r))
-            return r;
-    }
-    using Gm = W32Geom<N>;
-    HV_CUDA_TRY(cudaFuncSetAttribute(k_fft_cols_w32<N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     static_cast<int>(Gm::COL_SMEM)));
-    ColPass q = p;
-    if ((q.tw = twiddles_w32<N>()) == nullptr)
-        return HV_ERR_CUDA;
-    q.tw_count = Gm::TW;
-    dim3 grid((p.width + Gm::COLS - 1) / Gm::COLS, nframes);
-    k_fft_cols_w32<N><<<grid, W32_THREADS, Gm::COL_SMEM, st>>>(q);
-    HV_LAUNCH_CHECK();
-    count_launch();
-    return HV_OK;
-}
-
-hv_status launch_rows_w768(const RowPass& p, int nframes, cudaStream_t st)
-{
-    HV_CUDA_TRY(cudaFuncSetAttribute(k_fft_rows_w768, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     static_cast<int>(W768_ROW_SMEM)));
-    RowPass q = p;
-    if ((q.tw = twiddles_w768()) == nullptr)
-        return HV_ERR_CUDA;
-    q.tw_count = fftw::W768::TW_COUNT;
-    dim3 grid((p.rows + W768_ROWS - 1) / W768_ROWS, nframes);
-    k_fft_rows_w768<<<grid, W32_THREADS, W768_ROW_SMEM, st>>>(q);
-    HV_LAUNCH_CHECK();
-    count_launch();
-    return HV_OK;
-}
-
-hv_status launch_cols_w768(const ColPass& p, int nframes, cudaStream_t st)
-{
-    HV_CUDA_TRY(cudaFuncSetAttribute(k_fft_cols_w768, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     static_cast<int>(W768_COL_SMEM)));
-    ColPass q = p;
-    if ((q.tw = twiddles_w768()) == nullptr)
-        return HV_ERR_CUDA;
-    q.tw_count = fftw::W768::TW_COUNT;
-    dim3 grid((p.width + W768_COLS - 1) / W768_COLS, nframes);
-    k_fft_cols_w768<<<grid, W32_THREADS, W768_COL_SMEM, st>>>(q);
+    const int grid = warp_grid(ntiles, p.reserve_sms);
+    // tensor copies: 16-byte aligned base and row pitch, contiguous frames
+    const uint64_t pitch = static_cast<uint64_t>(p.width) * sizeof(float2);
+    CUtensorMap in_map{}, g_map{};
+    bool bulk = g_fft_bulk.load() && p.in_frame == static_cast<size_t>(p.width) * N && pitch % 16 == 0 &&
+                (reinterpret_cast<uintptr_t>(p.in) & 15) == 0 &&
+                tc::encode_tmap_2d_f32(&in_map, p.in, static_cast<uint64_t>(p.width) * 2,
+                                       static_cast<uint64_t>(nframes) * N, pitch, Gm::COLS * 2, 256);
+    if (bulk && p.mode == 2)
+        bulk = (reinterpret_cast<uintptr_t>(p.postmul) & 15) == 0 &&
+               tc::encode_tmap_2d_f32(&g_map, p.postmul, static_cast<uint64_t>(p.width) * 2, N, pitch, Gm::COLS * 2, 256);
+    auto kern = p.mode == 2 ? k_fft_cols_warp<N, 2> : p.mode == 1 ? k_fft_cols_warp<N, 1> : k_fft_cols_warp<N, 0>;
+    HV_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(Gm::COL_SMEM)));
+    kern<<<grid, W32_THREADS, Gm::COL_SMEM, st>>>(in_map, g_map, q, tiles_x, ntiles, bulk ? 1 : 0);
     HV_LAUNCH_CHECK();
     count_launch();
     return HV_OK;
@@ -1509,12 +1125,9 @@ hv_status launch_cols_w768(const ColPass& p, int nframes, cudaStream_t st)
 template <int N>
 hv_status launch_rows(const RowPass& p, int nframes, cudaStream_t st)
 {
-    if constexpr (N == 768)
+    if constexpr (N == 512 || N == 768 || N == 1024)
         if (g_fft_engine.load() == 0)
-            return launch_rows_w768(p, nframes, st);
-    if constexpr (N == 512 || N == 1024)
-        if (g_fft_engine.load() == 0)
-            return launch_rows_w32<N>(p, nframes, st);
+            return launch_rows_warp<N>(p, nframes, st);
     constexpr int F = row_lanes<N>();
     using Tl = fft::Tile<N, F, false>;
     const int tw_count = fft::twiddle_count(typename fft::Plan<N>::List{});
@@ -1536,12 +1149,9 @@ hv_status launch_rows(const RowPass& p, int nframes, cudaStream_t st)
 template <int N>
 hv_status launch_cols(const ColPass& p, int nframes, cudaStream_t st)
 {
-    if constexpr (N == 768)
+    if constexpr (N == 512 || N == 768 || N == 1024)
         if (g_fft_engine.load() == 0)
-            return launch_cols_w768(p, nframes, st);
-    if constexpr (N == 512 || N == 1024)
-        if (g_fft_engine.load() == 0)
-            return launch_cols_w32<N>(p, nframes, st);
+            return launch_cols_warp<N>(p, nframes, st);
     constexpr int F = col_lanes<N>();
     using Tl = fft::Tile<N, F, true>;
     const int tw_count = fft::twiddle_count(typename fft::Plan<N>::List{});
@@ -1565,7 +1175,7 @@ hv_status launch_cols(const ColPass& p, int nframes, cudaStream_t st)
 void set_fft_engine(int mode)
 {
     g_fft_engine = mode == 2 ? 0 : mode;
-    g_fft_tma = mode == 2 ? 0 : 1;
+    g_fft_bulk = mode == 2 ? 0 : 1;
 }
 
 hv_status fft_status()
