@@ -374,12 +374,12 @@ hv_status hv_renormalize(float* frame, size_t n, int renorm_constant, const doub
 {
     if (!frame || !work || n == 0)
         return HV_INVALID_VALUE;
-    float* factors = reinterpret_cast<float*>(static_cast<char*>(work) + reduce_workspace(n));
-    hv_status r = renorm_factors(frame, n, renorm_constant, partials_f64, npartials, factors, work, S(stream));
+    RenormSum sum;
+    hv_status r = renorm_sum(frame, n, renorm_constant, partials_f64, npartials, work, S(stream), &sum);
     if (r != HV_OK)
         return r;
     // one-row frame: renormalise in place, no shift, no accumulation
-    return renorm_shift_accumulate(frame, frame, static_cast<int>(n), 1, factors, 0, nullptr, 0, 0, 0, 0, 0, S(stream));
+    return renorm_shift_accumulate(frame, frame, static_cast<int>(n), 1, &sum, 0, nullptr, 0, 0, 0, 0, 0, S(stream));
 }
 
 size_t hv_reduce_workspace(size_t n) { return reduce_workspace(n) + 64; }

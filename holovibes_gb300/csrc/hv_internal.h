@@ -155,9 +155,19 @@ hv_status view_tc(const float2* ring, int T, int W, int H, int K, int img_type, 
 size_t unwrap_workspace(int W, int H);
 hv_status unwrap_2d(const float* in, float* out, int W, int H, void* work, cudaStream_t st);
 size_t reduce_workspace(size_t n);
-hv_status renorm_factors(const float* frame, size_t n, int renorm_constant, const double* partials, int npartials,
-                         float* factors, void* work, cudaStream_t st, const CycleCtl* ctl = nullptr);
-hv_status renorm_shift_accumulate(const float* in, float* out, int W, int H, const float* factors, int shift,
+// The sum behind the renormalisation of a frame of n pixels (postprocessing.cc:135-155): partial sums
+// whose total the renormalising kernel takes itself, and the renormalisation constant.
+struct RenormSum
+{
+    const double* partials = nullptr;
+    int np = 0;
+    size_t n = 0;
+    int c = 0;
+};
+// Partial sums of `frame` into `work` (reduce_workspace bytes), or the given ones.
+hv_status renorm_sum(const float* frame, size_t n, int renorm_constant, const double* partials, int npartials,
+                     void* work, cudaStream_t st, RenormSum* sum, const CycleCtl* ctl = nullptr);
+hv_status renorm_shift_accumulate(const float* in, float* out, int W, int H, const RenormSum* sum, int shift,
                                   float* acc_ring, int A, int slot, int start, int count, int log_enabled,
                                   cudaStream_t st, float prescale = 1.0f, const CycleCtl* ctl = nullptr);
 hv_status shift_corners(float* frame, int W, int H, cudaStream_t st);

@@ -188,7 +188,6 @@ size_t footprint(const hv_frame_desc& fd, const hv_settings& s, bool served = fa
             z.add(view_tc_workspace(K, T));
         z.add(static_cast<size_t>(time_view_partials(fd.width, fd.height)) * 8);
         z.add(reduce_workspace(HW));
-        z.add(64);
     }
     z.add(static_cast<size_t>(K > 0 ? K : 1) * T * 8);                 // weights
     if (uses_eig(s))
@@ -238,7 +237,6 @@ size_t footprint(const hv_frame_desc& fd, const hv_settings& s, bool served = fa
     }
     z.add(static_cast<size_t>(time_view_partials(fd.width, fd.height)) * 8);
     z.add(reduce_workspace(HW));
-    z.add(64);
     if (s.accumulation > 1)
         z.add(HW * 4 * s.accumulation);
     z.add(64);
@@ -352,7 +350,6 @@ hv_status build(hv_pipe* p)
     p->npartials = time_view_partials(p->W, p->H);
     HV_ALLOC(p->partials, static_cast<size_t>(p->npartials) * sizeof(double));
     HV_ALLOC(p->reduce_work, reduce_workspace(HW));
-    HV_ALLOC(p->factors, 4 * sizeof(float));
     if (p->A > 0)
     {
         HV_ALLOC(p->acc_ring, HW * p->A * sizeof(float));
@@ -372,7 +369,6 @@ hv_status build(hv_pipe* p)
         L0.post = p->post;
         L0.partials = p->partials;
         L0.reduce_work = p->reduce_work;
-        L0.factors = p->factors;
         L0.view_tc_work = p->view_tc_work;
         for (int l = 1; l < p->nrender; ++l)
         {
@@ -388,7 +384,6 @@ hv_status build(hv_pipe* p)
             HV_ALLOC(L.post, HW * sizeof(float));
             HV_ALLOC(L.partials, static_cast<size_t>(p->npartials) * sizeof(double));
             HV_ALLOC(L.reduce_work, reduce_workspace(HW));
-            HV_ALLOC(L.factors, 4 * sizeof(float));
             if (p->view_on_tc)
             {
                 HV_ALLOC(L.view_tc_work, view_tc_workspace(p->K, p->T));
@@ -591,7 +586,7 @@ hv_status build(hv_pipe* p)
     return HV_OK;
 }
 
-// Time transform and view of one full ring, up to the renormalisation factors
+// Time transform and view of one full ring, up to the renormalisation sum
 // (fourier_transform.cc:194-242,340-460, converts.cc:19-62,251-300, postprocessing.cc:135-155):
 // sets *frame to the float frame that the fused renorm / shift / accumulation pass reads and
 // *shift_after when that pass applies the fftshift (the view kernels apply it themselves
@@ -773,8 +768,7 @@ hv_status render_view(hv_pipe* p, cudaStream_t st, const CycleCtl* ctl, const fl
             return r;
         *frame = p->unwrapped;
         *shift_after = s.fft_shift ? 1 : 0;
-        if (renorm && (r = renorm_factors(*frame, p->HW, s.renorm_constant, nullptr, 0, p->factors, p->reduce_work, st,
-                                          ctl)) != HV_OK)
+        if (renorm && (r = renorm_sum(*frame, p->HW, s.renorm_constant, nullptr, 0, p->reduce_work, st, &p->renorm, ctl)) != HV_OK)
             return r;
         return HV_OK;
     }
@@ -786,8 +780,8 @@ hv_status render_view(hv_pipe* p, cudaStream_t st, const CycleCtl* ctl, const fl
                                : ring_view(p, st, scale, shift_in_view, renorm ? p->partials : nullptr, ctl)) !=
             HV_OK)
             return r;
-        if (renorm && (r = renorm_factors(p->view, p->HW, s.renorm_constant, p->partials, p->npartials, p->factors,
-                                          p->reduce_work, st, ctl)) != HV_OK)
+        if (renorm && (r = renorm_sum(p->view, p->HW, s.renorm_constant, p->partials, p->npartials,
+                                      p->reduce_work, st, &p->renorm, ctl)) != HV_OK)
             return r;
         return HV_OK;
     }
@@ -803,8 +797,7 @@ hv_status render_view(hv_pipe* p, cudaStream_t st, const CycleCtl* ctl, const fl
         return r;
     *frame = p->unwrapped;
     *shift_after = s.fft_shift ? 1 : 0;
-    if (renorm && (r = renorm_factors(*frame, p->HW, s.renorm_constant, nullptr, 0, p->factors, p->reduce_work, st,
-                                      ctl)) != HV_OK)
+    if (renorm && (r = renorm_sum(*frame, p->HW, s.renorm_constant, nullptr, 0, p->reduce_work, st, &p->renorm, ctl)) != HV_OK)
         return r;
     return HV_OK;
 }
@@ -959,7 +952,7 @@ hv_status render(hv_pipe* p)
         start = p->acc_start;
         count = p->acc_size;
     }
-    if ((r = renorm_shift_accumulate(frame, p->post, p->W, p->H, renorm ? p->factors : nullptr, shift_after,
+    if ((r = renorm_shift_accumulate(frame, p->post, p->W, p->H, renorm ? &p->renorm : nullptr, shift_after,
                                      p->A > 0 ? p->acc_ring : nullptr, p->A, slot, start, count, s.log_enabled, st,
                                      1.0f)) != HV_OK)
         return r;
@@ -1076,7 +1069,6 @@ hv_status process_batch(hv_pipe* p, const uint8_t* raw)
             p->post = L.post;
             p->partials = L.partials;
             p->reduce_work = L.reduce_work;
-            p->factors = L.factors;
             p->view_tc_work = L.view_tc_work;
             // the contrast range of the last autocontrast (computed on another lane)
             if (p->range_ev_set)
@@ -1409,7 +1401,7 @@ hv_status served_record(hv_pipe* p, const CycleCtl* ctl, const ServedCycle& c, b
     int shift_after = 0;
     if ((r = render_view(p, st, ctl, &frame, &shift_after)) != HV_OK)
         return r;
-    if ((r = renorm_shift_accumulate(frame, p->post, p->W, p->H, renorm ? p->factors : nullptr, shift_after,
+    if ((r = renorm_shift_accumulate(frame, p->post, p->W, p->H, renorm ? &p->renorm : nullptr, shift_after,
                                      p->A > 0 ? p->acc_ring : nullptr, p->A, 0, 0, 0, s.log_enabled, st, 1.0f, ctl)) !=
         HV_OK)
         return r;

@@ -55,7 +55,6 @@ struct hv_pipe
         float* post = nullptr;
         double* partials = nullptr;
         void* reduce_work = nullptr;
-        float* factors = nullptr;
         void* view_tc_work = nullptr;
     };
     bool fast = false;
@@ -100,7 +99,7 @@ struct hv_pipe
     double* partials = nullptr;
     int npartials = 0;
     void* reduce_work = nullptr;
-    float* factors = nullptr;
+    hv::RenormSum renorm;  // of the window being rendered
     float* post = nullptr;
     float* acc_ring = nullptr;
     float* range = nullptr;

@@ -17,6 +17,7 @@
 #include <float.h>
 #include <math.h>
 
+#include <initializer_list>
 #include <mutex>
 #include <string>
 
@@ -309,34 +310,8 @@ __global__ void k_partial_sums(const float* in, size_t n, double* partials, cons
     }
 }
 
-// factors[0] = 2^c, factors[1] = (float)N / (float)sum; x' = (x * factors[0]) * factors[1]
-__global__ void k_renorm_factors(const double* partials, int np, size_t n, int c, float* factors,
-                                 const CycleCtl* ctl)
-{
-    if (!ctl_render(ctl))
-        return;
-    __shared__ double red[32];
-    double s = 0.0;
-    for (int i = threadIdx.x; i < np; i += blockDim.x)
-        s += partials[i];
-    for (int o = 16; o > 0; o >>= 1)
-        s += __shfl_down_sync(0xffffffffu, s, o);
-    if ((threadIdx.x & 31) == 0)
-        red[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if (threadIdx.x == 0)
-    {
-        double t = 0.0;
-        for (int i = 0; i < (blockDim.x + 31) / 32; ++i)
-            t += red[i];
-        factors[0] = static_cast<float>(1 << c);
-        // a zero-sum frame (all zero) stays zero instead of the reference's N / 0 = inf, 0 * inf = NaN
-        factors[1] = t != 0.0 ? __fdiv_rn(static_cast<float>(n), static_cast<float>(t)) : 0.0f;
-    }
-}
-
-hv_status renorm_factors(const float* frame, size_t n, int renorm_constant, const double* partials, int npartials,
-                         float* factors, void* work, cudaStream_t st, const CycleCtl* ctl)
+hv_status renorm_sum(const float* frame, size_t n, int renorm_constant, const double* partials, int npartials,
+                     void* work, cudaStream_t st, RenormSum* sum, const CycleCtl* ctl)
 {
     if (!partials)
     {
@@ -348,18 +323,99 @@ hv_status renorm_factors(const float* frame, size_t n, int renorm_constant, cons
         partials = p;
         npartials = grid;
     }
-    k_renorm_factors<<<1, 1024, 0, st>>>(partials, npartials, n, renorm_constant, factors, ctl);
-    HV_LAUNCH_CHECK();
-    count_launch();
+    *sum = RenormSum{partials, npartials, n, renorm_constant};
     return HV_OK;
 }
 
-// Fused: renormalise (factors may be null), optional quadrant swap (out of place), optional
-// accumulation into an A-frame ring (write slot, mean of `count` frames from `start`), optional log10.
-__global__ void k_renorm_shift_acc(const float* __restrict__ in, float* __restrict__ out, int W, int H,
-                                   const float* __restrict__ factors, int shift, float* __restrict__ acc, int A,
-                                   int slot, int start, int count, int log_enabled, float prescale,
-                                   const CycleCtl* ctl)
+// The renormalisation factors x' = (x * f[0]) * f[1], f[0] = 2^c and f[1] = (float)N / (float)sum of
+// the partial sums, for every thread of a CTA of RN_THREADS. FP64 additions run at a few per clock
+// and SM here, so the tree adds each pair once (47 warp additions; every lane of a shuffle tree adds
+// in 160). The order of the additions is fixed: thread i sums entries i, i + 1024, ..., then each
+// warp's 32 sums as a tree, then the warps in order.
+constexpr int RN_THREADS = 1024;
+
+__device__ __forceinline__ void renorm_factors(const RenormSum& r, float& f0, float& f1)
+{
+    __shared__ double a[RN_THREADS], b[RN_THREADS / 2];
+    __shared__ float f[2];
+    const int tid = threadIdx.x;
+    double s = 0.0;
+    int i = tid;
+    for (; i + 7 * RN_THREADS < r.np; i += 8 * RN_THREADS)
+    {
+        double v[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            v[k] = r.partials[i + k * RN_THREADS];
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            s += v[k];
+    }
+    for (; i < r.np; i += RN_THREADS)
+        s += r.partials[i];
+    a[tid] = s;
+    __syncthreads();
+    if (tid < RN_THREADS / 2)  // lanes l and l + 16 of warp w
+        b[tid] = a[(tid >> 4) * 32 + (tid & 15)] + a[(tid >> 4) * 32 + (tid & 15) + 16];
+    __syncthreads();
+    if (tid < RN_THREADS / 4)  // eight lanes per warp's tree
+    {
+        double t = b[(tid >> 3) * 16 + (tid & 7)] + b[(tid >> 3) * 16 + (tid & 7) + 8];
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1)
+            t += __shfl_down_sync(0xffffffffu, t, o, 8);
+        if ((tid & 7) == 0)
+            a[tid >> 3] = t;
+    }
+    __syncthreads();
+    if (tid == 0)
+    {
+        double t = 0.0;
+#pragma unroll
+        for (int w = 0; w < RN_THREADS / 32; ++w)
+            t += a[w];
+        f[0] = static_cast<float>(1 << r.c);
+        // a zero-sum frame (all zero) stays zero instead of the reference's N / 0 = inf, 0 * inf = NaN
+        f[1] = t != 0.0 ? __fdiv_rn(static_cast<float>(r.n), static_cast<float>(t)) : 0.0f;
+    }
+    __syncthreads();
+    f0 = f[0];
+    f1 = f[1];
+}
+
+// V consecutive floats (V = 4: one 16-byte access).
+template <int V>
+__device__ __forceinline__ void load_v(const float* p, float (&v)[V])
+{
+    if constexpr (V == 4)
+    {
+        const float4 f = *reinterpret_cast<const float4*>(p);
+        v[0] = f.x, v[1] = f.y, v[2] = f.z, v[3] = f.w;
+    }
+    else
+        v[0] = *p;
+}
+template <int V>
+__device__ __forceinline__ void store_v(float* p, const float (&v)[V])
+{
+    if constexpr (V == 4)
+        *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+    else
+        *p = v[0];
+}
+
+// Fused: renormalise (sum.partials null: not), optional quadrant swap (out of place), optional
+// accumulation into an A-frame ring (write slot, mean of `count` frames from `start`), optional
+// log10. V pixels per thread and step. Bound by latency (a few MB from L2): the factors without a
+// launch of their own and 16-byte accesses take the renormalisation of 1024 x 1024 from 8.8 + 10.2 to
+// 9.8 us, log10 from 5.3 to 4.0 us and the contrast map below from 6.1 to 3.8 us (serialised launch
+// times, cold caches); the mean of 8 frames, whose loads go out together, stays at 10.4 us (its 38 MB
+// come from DRAM there).
+template <int V>
+__global__ void __launch_bounds__(RN_THREADS) k_renorm_shift_acc(const float* in, float* out, int W, int H,
+                                                                 RenormSum sum, int shift, float* acc, int A, int slot,
+                                                                 int start, int count, int log_enabled, float prescale,
+                                                                 const CycleCtl* ctl)
 {
     if (!ctl_render(ctl))
         return;
@@ -371,44 +427,109 @@ __global__ void k_renorm_shift_acc(const float* __restrict__ in, float* __restri
     }
     const size_t n = static_cast<size_t>(W) * H;
     float m0 = 1.f, m1 = 1.f;
-    if (factors)
-    {
-        m0 = factors[0];
-        m1 = factors[1];
-    }
-    for (size_t e = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; e < n;
-         e += static_cast<size_t>(gridDim.x) * blockDim.x)
+    if (sum.partials)
+        renorm_factors(sum, m0, m1);
+    for (size_t e = (blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x) * V; e < n;
+         e += static_cast<size_t>(gridDim.x) * blockDim.x * V)
     {
         size_t src = e;
-        if (shift)
+        if (shift)  // V = 4: W a multiple of 8, so the four pixels stay together
         {
             const int x = static_cast<int>(e % W), y = static_cast<int>(e / W);
             src = static_cast<size_t>((y + H / 2) % H) * W + (x + W / 2) % W;
         }
-        float v = in[src];
-        if (prescale != 1.0f)
-            v = v * prescale;
-        if (factors)
-            v = (v * m0) * m1;
+        float v[V];
+        load_v<V>(in + src, v);
+#pragma unroll
+        for (int k = 0; k < V; ++k)
+        {
+            if (prescale != 1.0f)
+                v[k] = v[k] * prescale;
+            if (sum.partials)
+                v[k] = (v[k] * m0) * m1;
+        }
         if (acc)
         {
-            acc[static_cast<size_t>(slot) * n + e] = v;
-            float s = 0.f;
+            store_v<V>(acc + static_cast<size_t>(slot) * n + e, v);
+            float s[V];
+#pragma unroll
+            for (int k = 0; k < V; ++k)
+                s[k] = 0.f;
+            constexpr int D = 8;  // frames whose loads are issued together
             int pos = start;
-            for (int i = 0; i < count; ++i)
+            for (int i = 0; i < count; i += D)
             {
-                s += (pos == slot) ? v : acc[static_cast<size_t>(pos) * n + e];
-                pos = (pos + 1) % A;
+                float q[D][V];
+                int at = pos;
+#pragma unroll
+                for (int d = 0; d < D; ++d)
+                {
+                    if (i + d < count && at != slot)
+                        load_v<V>(acc + static_cast<size_t>(at) * n + e, q[d]);
+                    if (++at == A)
+                        at = 0;
+                }
+#pragma unroll
+                for (int d = 0; d < D; ++d)
+                {
+                    if (i + d < count)
+                    {
+#pragma unroll
+                        for (int k = 0; k < V; ++k)
+                            s[k] += pos == slot ? v[k] : q[d][k];
+                    }
+                    if (++pos == A)
+                        pos = 0;
+                }
             }
-            v = s / static_cast<float>(count);
+#pragma unroll
+            for (int k = 0; k < V; ++k)
+                v[k] = s[k] / static_cast<float>(count);
         }
         if (log_enabled)
-            v = log10f(v);
-        out[e] = v;
+        {
+#pragma unroll
+            for (int k = 0; k < V; ++k)
+                v[k] = log10f(v[k]);
+        }
+        store_v<V>(out + e, v);
     }
 }
 
-hv_status renorm_shift_accumulate(const float* in, float* out, int W, int H, const float* factors, int shift,
+// 16-byte accesses: every buffer aligned, a multiple of 4 pixels (and, with the quadrant swap, rows
+// whose halves are a multiple of 4).
+static bool vec4_ok(size_t n, std::initializer_list<const void*> buffers)
+{
+    uintptr_t bits = n % 4 ? 1 : 0;
+    for (const void* p : buffers)
+        bits |= reinterpret_cast<uintptr_t>(p) & 15;
+    return bits == 0;
+}
+
+static hv_status launch_renorm_shift_acc(const float* in, float* out, int W, int H, const RenormSum& sum, int shift,
+                                         float* acc, int A, int slot, int start, int count, int log_enabled,
+                                         float prescale, const CycleCtl* ctl, cudaStream_t st)
+{
+    const size_t n = static_cast<size_t>(W) * H;
+    const bool v4 = vec4_ok(n, {in, out, acc}) && (!shift || W % 8 == 0);
+    // with the factors: CTAs of 1024 threads, one per SM (each sums the partials: the SM's FP64 rate
+    // bounds that, so a second CTA would double it)
+    const int block = sum.partials ? RN_THREADS : EW_THREADS;
+    const size_t per = static_cast<size_t>(block) * (v4 ? 4 : 1);
+    const size_t want = (n + per - 1) / per, cap = sum.partials ? 152 : 152 * 32;
+    const int grid = static_cast<int>(want < cap ? (want > 0 ? want : 1) : cap);
+    if (v4)
+        k_renorm_shift_acc<4><<<grid, block, 0, st>>>(in, out, W, H, sum, shift, acc, A, slot, start, count,
+                                                      log_enabled, prescale, ctl);
+    else
+        k_renorm_shift_acc<1><<<grid, block, 0, st>>>(in, out, W, H, sum, shift, acc, A, slot, start, count,
+                                                      log_enabled, prescale, ctl);
+    HV_LAUNCH_CHECK();
+    count_launch();
+    return HV_OK;
+}
+
+hv_status renorm_shift_accumulate(const float* in, float* out, int W, int H, const RenormSum* sum, int shift,
                                   float* acc_ring, int A, int slot, int start, int count, int log_enabled,
                                   cudaStream_t st, float prescale, const CycleCtl* ctl)
 {
@@ -422,12 +543,8 @@ hv_status renorm_shift_accumulate(const float* in, float* out, int W, int H, con
         set_last_error_msg("renorm_shift_accumulate: shift must be out of place");
         return HV_INVALID_VALUE;
     }
-    const size_t n = static_cast<size_t>(W) * H;
-    k_renorm_shift_acc<<<ew_grid(n), EW_THREADS, 0, st>>>(in, out, W, H, factors, shift, acc_ring, A, slot, start,
-                                                          count, log_enabled, prescale, ctl);
-    HV_LAUNCH_CHECK();
-    count_launch();
-    return HV_OK;
+    return launch_renorm_shift_acc(in, out, W, H, sum ? *sum : RenormSum{}, shift, acc_ring, A, slot, start, count,
+                                   log_enabled, prescale, ctl, st);
 }
 
 // In-place quadrant swap: thread owns pixel (x, y) of the top half and swaps it with its partner.
@@ -466,23 +583,31 @@ hv_status accumulate(const float* frame, float* acc_ring, int A, int slot, int s
     if (A <= 0 || slot < 0 || slot >= A || start < 0 || start >= A || count <= 0 || count > A)
         return HV_INVALID_VALUE;
     // 1-row frame of n pixels: no shift, no renorm
-    k_renorm_shift_acc<<<ew_grid(n), EW_THREADS, 0, st>>>(frame, out, static_cast<int>(n), 1, nullptr, 0, acc_ring, A,
-                                                          slot, start, count, 0, 1.0f, nullptr);
-    HV_LAUNCH_CHECK();
-    count_launch();
-    return HV_OK;
+    return launch_renorm_shift_acc(frame, out, static_cast<int>(n), 1, RenormSum{}, 0, acc_ring, A, slot, start, count, 0,
+                                   1.0f, nullptr, st);
 }
 
+template <int V>
 __global__ void k_log10(float* f, size_t n)
 {
-    for (size_t e = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; e < n;
-         e += static_cast<size_t>(gridDim.x) * blockDim.x)
-        f[e] = log10f(f[e]);
+    for (size_t e = (blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x) * V; e < n;
+         e += static_cast<size_t>(gridDim.x) * blockDim.x * V)
+    {
+        float v[V];
+        load_v<V>(f + e, v);
+#pragma unroll
+        for (int k = 0; k < V; ++k)
+            v[k] = log10f(v[k]);
+        store_v<V>(f + e, v);
+    }
 }
 
 hv_status log10_map(float* frame, size_t n, cudaStream_t st)
 {
-    k_log10<<<ew_grid(n), EW_THREADS, 0, st>>>(frame, n);
+    if (vec4_ok(n, {frame}))
+        k_log10<4><<<ew_grid(n / 4), EW_THREADS, 0, st>>>(frame, n);
+    else
+        k_log10<1><<<ew_grid(n), EW_THREADS, 0, st>>>(frame, n);
     HV_LAUNCH_CHECK();
     count_launch();
     return HV_OK;
@@ -491,8 +616,12 @@ hv_status log10_map(float* frame, size_t n, cudaStream_t st)
 // ====================================================================================== percentile
 // Exact k-th smallest selection for two ranks at once. Pass d (d = 0, 1, 2) histograms the
 // digit d of the order-preserving key of the elements whose higher digits match the prefix
-// selected so far for that rank; a single-CTA scan then picks the digit holding the rank.
-// Digits: bits [31:21] (2048 bins), [20:10] (2048 bins), [9:0] (1024 bins).
+// selected so far for that rank; the CTA that finishes the pass last then picks the digit holding
+// the rank. Digits: bits [31:21] (2048 bins), [20:10] (2048 bins), [9:0] (1024 bins).
+// Bound by latency and by shared-memory atomics on few addresses (a frame's values share a handful
+// of first digits): 16 pixels per thread are loaded together, equal digits of a warp are counted by
+// one atomic, and the scan rides on the pass. 1024 x 1024: 3 x (9.0 + 5.1) us as separate histogram and
+// scan launches, 3 x 10.4 us here (serialised launch times, cold caches).
 
 constexpr int PCT_BINS = 2048;
 
@@ -501,6 +630,7 @@ struct PctState
     unsigned int prefix[2];  // selected high bits per rank
     unsigned int rank[2];    // remaining rank inside the prefix
     unsigned int count;      // number of candidate elements (frame or reticle disc)
+    unsigned int done[3];    // CTAs that finished each pass
 };
 
 __device__ __forceinline__ int digit_shift(int d) { return d == 0 ? 21 : (d == 1 ? 10 : 0); }
@@ -516,134 +646,191 @@ __device__ __forceinline__ bool in_reticle(size_t e, int W, int H, unsigned int 
     return static_cast<unsigned int>(dx * dx + dy * dy) <= r2;
 }
 
-__global__ void k_pct_hist(const float* __restrict__ f, int W, int H, int pitch, unsigned int r2, int use_reticle,
-                           const PctState* __restrict__ st, int d, unsigned int* __restrict__ hist,
-                           const CycleCtl* ctl)
+// Digit of rank r (0 or 1) after pass d from the histogram hh, by a CTA of EW_THREADS (PCT_BINS / 8).
+__device__ void pct_select(const unsigned int* hh, PctState* st, int r, int d, float pct, float* range)
+{
+    constexpr int PER = PCT_BINS / EW_THREADS;
+    __shared__ unsigned int warp_tot[EW_THREADS / 32];
+    const int nb = (d == 2) ? 1024 : PCT_BINS;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    unsigned int c[PER], v = 0;
+#pragma unroll
+    for (int i = 0; i < PER; ++i)
+    {
+        const int bin = threadIdx.x * PER + i;
+        c[i] = bin < nb ? __ldcg(hh + bin) : 0u;
+        v += c[i];
+    }
+    unsigned int incl = v;
+    for (int o = 1; o < 32; o <<= 1)
+    {
+        const unsigned int t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o)
+            incl += t;
+    }
+    __syncthreads();  // warp_tot of the previous rank is read
+    if (lane == 31)
+        warp_tot[w] = incl;
+    __syncthreads();
+    unsigned int before = incl - v, total = 0;
+#pragma unroll
+    for (int i = 0; i < EW_THREADS / 32; ++i)
+    {
+        before += i < w ? warp_tot[i] : 0u;
+        total += warp_tot[i];
+    }
+    unsigned int rank, candidates;
+    if (d == 0)
+    {
+        // total candidates and the percentile index, float32 as percentile.cu:85, clamped
+        candidates = total;
+        rank = static_cast<unsigned int>(__fmul_rn(__fdiv_rn(pct, 100.0f), static_cast<float>(total)));
+        if (total == 0)
+            rank = 0;
+        else if (rank >= total)
+            rank = total - 1;
+    }
+    else
+    {
+        candidates = __ldcg(&st->count);
+        rank = __ldcg(&st->rank[r]);
+    }
+    __syncthreads();  // every thread has the state that one of them replaces
+    // first bin whose inclusive count exceeds rank (the last bin when none does)
+    const bool mine = rank >= before && rank < before + v;
+    const bool last = rank >= total && threadIdx.x == (nb - 1) / PER;
+    if (mine || last)
+    {
+        int bin = threadIdx.x * PER;
+        unsigned int below = before;
+        if (mine)
+        {
+            int i = 0;
+#pragma unroll
+            for (int k = 0; k < PER; ++k)
+                if (k == i && rank >= below + c[k])
+                {
+                    below += c[k];
+                    ++i;
+                }
+            bin += i;
+        }
+        else
+        {
+            bin = nb - 1;
+            below = total - c[(nb - 1) % PER];
+        }
+        const unsigned int prefix = (d == 0 ? 0u : st->prefix[r]) | (static_cast<unsigned int>(bin) << digit_shift(d));
+        if (d == 0)
+            st->count = candidates;
+        st->rank[r] = rank - below;
+        st->prefix[r] = prefix;
+        if (d == 2)
+        {
+            const float val = candidates ? key_float(prefix) : 0.f;
+            // ContrastApi::update_contrast clamps both ends to >= 1
+            range[r] = val > 1.0f ? val : 1.0f;
+        }
+    }
+}
+
+// VEC: rows without gaps, no reticle, 16-byte aligned, a multiple of 4 pixels.
+template <bool VEC>
+__global__ void __launch_bounds__(EW_THREADS) k_pct_pass(const float* __restrict__ f, int W, int H, int pitch,
+                                                         unsigned int r2, int use_reticle, PctState* st, int d,
+                                                         unsigned int* hist, float lower, float upper, float* range,
+                                                         const CycleCtl* ctl)
 {
     if (ctl && !(ctl->render && ctl->pct_enable))
         return;
     __shared__ unsigned int sh[2][PCT_BINS];
-    for (int i = threadIdx.x; i < 2 * PCT_BINS; i += blockDim.x)
+    __shared__ bool s_last;
+    const int nh = d == 0 ? 1 : 2;
+    for (int i = threadIdx.x; i < nh * PCT_BINS; i += EW_THREADS)
         (&sh[0][0])[i] = 0u;
-    __syncthreads();
     const size_t n = static_cast<size_t>(W) * H;
     const int sft = digit_shift(d);
     const unsigned int dm = digit_mask(d), hm = high_mask(d);
     const unsigned int pre0 = (d == 0) ? 0u : st->prefix[0];
     const unsigned int pre1 = (d == 0) ? 0u : st->prefix[1];
-    for (size_t e = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; e < n;
-         e += static_cast<size_t>(gridDim.x) * blockDim.x)
+    __syncthreads();
+    // one atomic per distinct digit among the warp's lanes that count one
+    auto count = [&](unsigned int* h, unsigned int dig, bool on) {
+        const unsigned int active = __ballot_sync(0xffffffffu, on);
+        if (!active)
+            return;
+        if (on)
+        {
+            const unsigned int same = __match_any_sync(active, dig);
+            if ((threadIdx.x & 31) == __ffs(same) - 1)
+                atomicAdd(&h[dig], static_cast<unsigned int>(__popc(same)));
+        }
+    };
+    auto take = [&](float x, bool on) {
+        const unsigned int k = float_key(x), dig = (k >> sft) & dm;
+        if (d == 0)
+            count(sh[0], dig, on);
+        else
+        {
+            if (on && (k & hm) == pre0)
+                atomicAdd(&sh[0][dig], 1u);
+            if (on && (k & hm) == pre1)
+                atomicAdd(&sh[1][dig], 1u);
+        }
+    };
+    if constexpr (VEC)
     {
-        if (!in_reticle(e, W, H, r2, use_reticle))
-            continue;
-        const size_t a = pitch == W ? e : (e / W) * static_cast<size_t>(pitch) + e % W;
-        const unsigned int k = float_key(f[a]);
-        const unsigned int dig = (k >> sft) & dm;
-        if ((k & hm) == pre0)
-            atomicAdd(&sh[0][dig], 1u);
-        if (d > 0 && (k & hm) == pre1)
-            atomicAdd(&sh[1][dig], 1u);
+        constexpr int Q = 4;
+        const size_t n4 = n / 4, step = static_cast<size_t>(gridDim.x) * EW_THREADS;
+        const float4* f4 = reinterpret_cast<const float4*>(f);
+        // uniform trip count: every lane of a warp takes part in the votes
+        const size_t first = blockIdx.x * static_cast<size_t>(EW_THREADS) + threadIdx.x;
+        for (size_t base = 0; base < n4; base += Q * step)
+        {
+            float4 v[Q];
+#pragma unroll
+            for (int q = 0; q < Q; ++q)
+            {
+                const size_t e = base + first + q * step;
+                v[q] = e < n4 ? f4[e] : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+#pragma unroll
+            for (int q = 0; q < Q; ++q)
+            {
+                const bool on = base + first + q * step < n4;
+                take(v[q].x, on);
+                take(v[q].y, on);
+                take(v[q].z, on);
+                take(v[q].w, on);
+            }
+        }
+    }
+    else
+    {
+        const size_t step = static_cast<size_t>(gridDim.x) * EW_THREADS;
+        for (size_t base = blockIdx.x * static_cast<size_t>(EW_THREADS); base < n; base += step)
+        {
+            const size_t e = base + threadIdx.x;
+            const bool on = e < n && in_reticle(e, W, H, r2, use_reticle);
+            const size_t a = pitch == W ? e : (e / W) * static_cast<size_t>(pitch) + e % W;
+            take(on ? f[a] : 0.f, on);
+        }
     }
     __syncthreads();
-    const int nh = d == 0 ? 1 : 2;
     for (int h = 0; h < nh; ++h)
-        for (int i = threadIdx.x; i < PCT_BINS; i += blockDim.x)
+        for (int i = threadIdx.x; i < PCT_BINS; i += EW_THREADS)
             if (sh[h][i])
                 atomicAdd(&hist[h * PCT_BINS + i], sh[h][i]);
-}
-
-// One CTA of 1024 threads: prefix scan of the histogram(s), choose the digit for each rank.
-__global__ void k_pct_select(unsigned int* __restrict__ hist, PctState* __restrict__ st, int d, float lower,
-                             float upper, float* __restrict__ range, const CycleCtl* ctl)
-{
-    if (ctl && !(ctl->render && ctl->pct_enable))
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0)
+        s_last = atomicAdd(&st->done[d], 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!s_last)
         return;
-    __shared__ unsigned int scan[PCT_BINS];
-    __shared__ unsigned int warp_tot[32];
-    const int nb = (d == 2) ? 1024 : PCT_BINS;
-    const int sft = digit_shift(d);
-    for (int r = 0; r < 2; ++r)
-    {
-        const unsigned int* hh = hist + ((d == 0) ? 0 : r) * PCT_BINS;
-        // inclusive scan of nb bins, two bins per thread
-        const int i0 = threadIdx.x * 2;
-        unsigned int a = (i0 < nb) ? hh[i0] : 0u, b = (i0 + 1 < nb) ? hh[i0 + 1] : 0u;
-        unsigned int v = a + b;
-        const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-        for (int o = 1; o < 32; o <<= 1)
-        {
-            const unsigned int t = __shfl_up_sync(0xffffffffu, v, o);
-            if (lane >= o)
-                v += t;
-        }
-        if (lane == 31)
-            warp_tot[w] = v;
-        __syncthreads();
-        if (w == 0)
-        {
-            unsigned int t = warp_tot[lane];
-            for (int o = 1; o < 32; o <<= 1)
-            {
-                const unsigned int u = __shfl_up_sync(0xffffffffu, t, o);
-                if (lane >= o)
-                    t += u;
-            }
-            warp_tot[lane] = t;
-        }
-        __syncthreads();
-        const unsigned int before = (w > 0 ? warp_tot[w - 1] : 0u) + v - (a + b);
-        if (i0 < nb)
-            scan[i0] = before + a;
-        if (i0 + 1 < nb)
-            scan[i0 + 1] = before + a + b;
-        __syncthreads();
-        if (threadIdx.x == 0)
-        {
-            unsigned int rank;
-            if (d == 0)
-            {
-                // total candidates and the percentile index, float32 as percentile.cu:85, clamped
-                const unsigned int total = scan[nb - 1];
-                st->count = total;
-                const float pct = r == 0 ? lower : upper;
-                unsigned int idx = static_cast<unsigned int>(__fmul_rn(__fdiv_rn(pct, 100.0f), static_cast<float>(total)));
-                if (total == 0)
-                    idx = 0;
-                else if (idx >= total)
-                    idx = total - 1;
-                rank = idx;
-                st->prefix[r] = 0u;
-            }
-            else
-            {
-                rank = st->rank[r];
-            }
-            // first bin whose inclusive count exceeds rank
-            int lo = 0, hi = nb - 1;
-            while (lo < hi)
-            {
-                const int mid = (lo + hi) >> 1;
-                if (scan[mid] > rank)
-                    hi = mid;
-                else
-                    lo = mid + 1;
-            }
-            const unsigned int below = lo > 0 ? scan[lo - 1] : 0u;
-            st->rank[r] = rank - below;
-            st->prefix[r] |= static_cast<unsigned int>(lo) << sft;
-            if (d == 2)
-            {
-                float val = st->count ? key_float(st->prefix[r]) : 0.f;
-                // ContrastApi::update_contrast clamps both ends to >= 1
-                range[r] = val > 1.0f ? val : 1.0f;
-            }
-        }
-        __syncthreads();
-        if (d == 0)
-        {
-            // both ranks use the same histogram in pass 0
-        }
-    }
+    __threadfence();
+    pct_select(hist, st, 0, d, lower, range);
+    pct_select(hist + (d == 0 ? 0 : PCT_BINS), st, 1, d, upper, range);
 }
 
 size_t percentile_workspace(size_t n)
@@ -668,7 +855,8 @@ hv_status percentile_pitched(const float* frame, int W, int H, int pitch, float 
         return HV_INVALID_VALUE;
     unsigned int* hist = static_cast<unsigned int*>(work);  // 3 passes x 2 ranks x PCT_BINS
     PctState* state = reinterpret_cast<PctState*>(hist + 3 * 2 * PCT_BINS);
-    HV_CUDA_TRY(cudaMemsetAsync(hist, 0, 3 * 2 * PCT_BINS * sizeof(unsigned int), st));
+    static_assert(sizeof(PctState) <= sizeof(unsigned int) * 8, "the state fits behind the histograms");
+    HV_CUDA_TRY(cudaMemsetAsync(hist, 0, 3 * 2 * PCT_BINS * sizeof(unsigned int) + sizeof(PctState), st));
     int use_reticle = 0;
     unsigned int r2 = 0;
     if (reticle_scale > 0.f)
@@ -681,18 +869,21 @@ hv_status percentile_pitched(const float* frame, int W, int H, int pitch, float 
             r2 = radius * radius;
         }
     }
-    int grid = ew_grid(n);
-    if (grid > 152 * 4)
-        grid = 152 * 4;
+    const bool vec = pitch == W && !use_reticle && vec4_ok(n, {frame});
+    // 16 pixels per thread: up to two CTAs per SM
+    const size_t want = (n + 16 * EW_THREADS - 1) / (16 * EW_THREADS);
+    const int grid = static_cast<int>(want < 152 * 2 ? want : 152 * 2);
     for (int d = 0; d < 3; ++d)
     {
-        k_pct_hist<<<grid, EW_THREADS, 0, st>>>(frame, W, H, pitch, r2, use_reticle, state, d, hist + d * 2 * PCT_BINS,
-                                                ctl);
-        HV_LAUNCH_CHECK();
-        k_pct_select<<<1, 1024, 0, st>>>(hist + d * 2 * PCT_BINS, state, d, lower, upper, range, ctl);
+        if (vec)
+            k_pct_pass<true><<<grid, EW_THREADS, 0, st>>>(frame, W, H, pitch, r2, use_reticle, state, d,
+                                                          hist + d * 2 * PCT_BINS, lower, upper, range, ctl);
+        else
+            k_pct_pass<false><<<grid, EW_THREADS, 0, st>>>(frame, W, H, pitch, r2, use_reticle, state, d,
+                                                           hist + d * 2 * PCT_BINS, lower, upper, range, ctl);
         HV_LAUNCH_CHECK();
     }
-    count_launch(6);
+    count_launch(3);
     return HV_OK;
 }
 
@@ -708,6 +899,7 @@ __device__ __forceinline__ uint16_t to_ushort(float x)
     return static_cast<uint16_t>(u);
 }
 
+template <int V>
 __global__ void k_contrast_ushort(const float* __restrict__ in, const float* __restrict__ range, int invert, int apply,
                                   uint16_t* __restrict__ out, size_t n, const CycleCtl* ctl)
 {
@@ -728,13 +920,19 @@ __global__ void k_contrast_ushort(const float* __restrict__ in, const float* __r
         mn = lo;
         factor = __fdiv_rn(65535.0f, __fadd_rn(__fsub_rn(hi, lo), FLT_EPSILON));
     }
-    for (size_t e = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; e < n;
-         e += static_cast<size_t>(gridDim.x) * blockDim.x)
+    for (size_t e = (blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x) * V; e < n;
+         e += static_cast<size_t>(gridDim.x) * blockDim.x * V)
     {
-        float v = in[e];
-        if (apply)
-            v = __fmul_rn(factor, __fsub_rn(v, mn));
-        out[e] = to_ushort(v);
+        float v[V];
+        load_v<V>(in + e, v);
+        uint16_t u[V];
+#pragma unroll
+        for (int k = 0; k < V; ++k)
+            u[k] = to_ushort(apply ? __fmul_rn(factor, __fsub_rn(v[k], mn)) : v[k]);
+        if constexpr (V == 4)
+            *reinterpret_cast<ushort4*>(out + e) = make_ushort4(u[0], u[1], u[2], u[3]);
+        else
+            out[e] = u[0];
     }
 }
 
@@ -808,7 +1006,11 @@ hv_status contrast_to_ushort_normalized(const float* frame, const float* range, 
 hv_status contrast_to_ushort(const float* frame, const float* range, int invert, int apply, uint16_t* out, size_t n,
                              cudaStream_t st, const CycleCtl* ctl)
 {
-    k_contrast_ushort<<<ew_grid(n), EW_THREADS, 0, st>>>(frame, range, invert, apply, out, n, ctl);
+    // (an output slot is n pixels of 2 bytes: a multiple of 8 bytes when n is one of 4)
+    if (vec4_ok(n, {frame}) && (reinterpret_cast<uintptr_t>(out) & 7) == 0)
+        k_contrast_ushort<4><<<ew_grid(n / 4), EW_THREADS, 0, st>>>(frame, range, invert, apply, out, n, ctl);
+    else
+        k_contrast_ushort<1><<<ew_grid(n), EW_THREADS, 0, st>>>(frame, range, invert, apply, out, n, ctl);
     HV_LAUNCH_CHECK();
     count_launch();
     return HV_OK;
