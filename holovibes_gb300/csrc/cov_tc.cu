@@ -64,6 +64,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) k_cov_tc(const __grid_constant_
                                                           int raw_stages, int packed, float* __restrict__ part,
                                                           int* __restrict__ err)
 {
+    wait_prior_kernels();
     // packed (2T <= 64): one 128-row tile per stage, Yh in rows 0..63 and Yl in rows 64..127, and
     // one 128 x 128 MMA per K step gives [[Yh Yh^T, Yh Yl^T], [Yl Yh^T, Yl Yl^T]];
     // otherwise two tiles (Yh, Yl) and three MMAs into three accumulators
@@ -305,6 +306,7 @@ __device__ __forceinline__ float cov_g(const float* P, int R, int packed, int a,
 __global__ void k_cov_tc_reduce(const float* __restrict__ part, int T, int nparts, int per_slice, int packed,
                                 double2* __restrict__ cov)
 {
+    wait_prior_kernels();
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= T * T)
         return;
@@ -378,6 +380,7 @@ __global__ void __launch_bounds__(TR_ENTRIES * TR_GROUPS) k_cov_tc_tiled_reduce(
                                                                                int nsplit, int real,
                                                                                double2* __restrict__ cov)
 {
+    wait_prior_kernels();
     __shared__ double red[TR_GROUPS - 1][4][TR_ENTRIES];
     const int q = threadIdx.x / TR_ENTRIES, el = threadIdx.x % TR_ENTRIES;
     const int e = blockIdx.x * TR_ENTRIES + el;
@@ -445,6 +448,7 @@ __global__ void __launch_bounds__(TR_ENTRIES * TR_GROUPS) k_cov_tc_tiled_reduce(
 __global__ void k_ring_split(const float2* __restrict__ ring, int T, size_t npix, int slot0, int n, int real,
                              uint16_t* __restrict__ planes)
 {
+    wait_prior_kernels();
     const size_t groups = npix / 8;
     const size_t total = static_cast<size_t>(n) * groups;
     const size_t plane = (real ? 1 : 2) * static_cast<size_t>(T) * npix;
@@ -489,6 +493,7 @@ __global__ void __launch_bounds__(TP_THREADS, 1) k_cov_tc_tiled(const __grid_con
                                                                 size_t chunks_per_split, float* __restrict__ part,
                                                                 int* __restrict__ err)
 {
+    wait_prior_kernels();
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t* stages = smem + ((1024u - (smem_u32(smem) & 1023u)) & 1023u);
     __shared__ __align__(8) uint64_t full[TP_STAGES], empty[TP_STAGES];
@@ -790,8 +795,7 @@ hv_status cov_split_planes(const float2* ring, int T, size_t npix, int slot0, in
     const size_t total = static_cast<size_t>(n) * (npix / 8);
     const size_t cap = static_cast<size_t>(sm_count()) * 8;
     const int grid = static_cast<int>(std::min((total + 255) / 256, cap));
-    k_ring_split<<<grid, 256, 0, st>>>(ring, T, npix, slot0, n, real ? 1 : 0, planes);
-    HV_LAUNCH_CHECK();
+    HV_LAUNCH(k_ring_split, grid, 256, 0, st, ring, T, npix, slot0, n, real ? 1 : 0, planes);
     count_launch();
     return HV_OK;
 }
@@ -827,12 +831,9 @@ hv_status cov_tc_planes(const uint16_t* planes, int T, size_t npix, double2* cov
                                                          static_cast<int>(smem));
     HV_CUDA_TRY(attr);
     float* tpart = static_cast<float*>(work);
-    k_cov_tc_tiled<<<q.nsplit * tl.n, TP_THREADS, smem, st>>>(tmap, npix, tl, q.chunks_per_split, tpart, err);
-    HV_LAUNCH_CHECK();
-    k_cov_tc_tiled_reduce<<<(T * T + TR_ENTRIES - 1) / TR_ENTRIES, TR_ENTRIES * TR_GROUPS, 0, st>>>(tpart, T, tl,
-                                                                                                  q.nsplit, real ? 1 : 0,
-                                                                                                  cov);
-    HV_LAUNCH_CHECK();
+    HV_LAUNCH(k_cov_tc_tiled, q.nsplit * tl.n, TP_THREADS, smem, st, tmap, npix, tl, q.chunks_per_split, tpart, err);
+    HV_LAUNCH(k_cov_tc_tiled_reduce, (T * T + TR_ENTRIES - 1) / TR_ENTRIES, TR_ENTRIES * TR_GROUPS, 0, st, tpart, T, tl,
+              q.nsplit, real ? 1 : 0, cov);
     count_launch(2);
     return HV_OK;
 }
@@ -877,13 +878,12 @@ hv_status cov_tc(const float2* ring, int T, size_t npix, double2* cov, void* wor
     }
     HV_CUDA_TRY(cudaFuncSetAttribute(k_cov_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
     float* part = static_cast<float*>(work);
-    k_cov_tc<<<p.ctas, TC_THREADS, smem, st>>>(map, T, npix, p.chunks_per_cta, p.N, p.cols, raw, p.packed, part, err);
-    HV_LAUNCH_CHECK();
+    HV_LAUNCH(k_cov_tc, p.ctas, TC_THREADS, smem, st, map, T, npix, p.chunks_per_cta, p.N, p.cols, raw, p.packed, part,
+              err);
     // four partials per thread (independent loads), the slices combined by FP64 atomics
     const int per = p.ctas < 4 ? p.ctas : 4;
-    k_cov_tc_reduce<<<dim3((T * T + 255) / 256, (p.ctas + per - 1) / per), 256, 0, st>>>(part, T, p.ctas, per,
-                                                                                       p.packed, cov);
-    HV_LAUNCH_CHECK();
+    HV_LAUNCH(k_cov_tc_reduce, dim3((T * T + 255) / 256, (p.ctas + per - 1) / per), 256, 0, st, part, T, p.ctas, per,
+              p.packed, cov);
     count_launch(2);
     return HV_OK;
 }

@@ -63,6 +63,7 @@ __device__ __forceinline__ float cut_view(float re, float im, int img_type)
 __global__ void __launch_bounds__(CUT_THREADS) k_cut_values(const float2* __restrict__ ring, const float2* __restrict__ w,
                                                             CutGeom g, int img_type, float* __restrict__ vals)
 {
+    wait_prior_kernels();
     extern __shared__ float2 s_x[];  // [T][CUT_PX]
     const long long p0 = static_cast<long long>(blockIdx.x) * CUT_PX;
     const int T = g.T;
@@ -95,6 +96,7 @@ __global__ void __launch_bounds__(CUT_THREADS) k_cut_values(const float2* __rest
 // XZ[t][x] = (sum_{j < ny} vals[j W + x][t]) / ny, YZ[y][t] = (sum_{i < nx} vals[n_xz + y nx + i][t]) / nx
 __global__ void k_cut_reduce(const float* __restrict__ vals, CutGeom g, float* __restrict__ xz, float* __restrict__ yz)
 {
+    wait_prior_kernels();
     const int T = g.T;
     const long long e = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
     const long long n_xz_out = static_cast<long long>(T) * g.W;
@@ -120,6 +122,7 @@ __global__ void k_cut_reduce(const float* __restrict__ vals, CutGeom g, float* _
 // PCA: the p_acc components are the eigenvector columns, evecs[j T + s] (complex128) -> w[j][s].
 __global__ void k_c128_to_c64(const double2* __restrict__ in, float2* __restrict__ out, size_t n)
 {
+    wait_prior_kernels();
     for (size_t e = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; e < n;
          e += static_cast<size_t>(gridDim.x) * blockDim.x)
         out[e] = make_float2(static_cast<float>(in[e].x), static_cast<float>(in[e].y));
@@ -129,8 +132,7 @@ hv_status evecs_to_weights(const double2* evecs, int T, float2* w, cudaStream_t 
 {
     const size_t n = static_cast<size_t>(T) * T;
     const int grid = static_cast<int>((n + 255) / 256 < 1024 ? (n + 255) / 256 : 1024);
-    k_c128_to_c64<<<grid, 256, 0, st>>>(evecs, w, n);
-    HV_LAUNCH_CHECK();
+    HV_LAUNCH(k_c128_to_c64, grid, 256, 0, st, evecs, w, n);
     count_launch();
     return HV_OK;
 }
@@ -176,11 +178,9 @@ hv_status time_cuts(const float2* ring, int T, int W, int H, const float2* weigh
         HV_CUDA_TRY(cudaFuncSetAttribute(k_cut_values, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          static_cast<int>(smem)));
     const long long blocks = (g.npix + CUT_PX - 1) / CUT_PX;
-    k_cut_values<<<static_cast<unsigned>(blocks), CUT_THREADS, smem, st>>>(ring, weights_all, g, img_type, vals);
-    HV_LAUNCH_CHECK();
+    HV_LAUNCH(k_cut_values, static_cast<unsigned>(blocks), CUT_THREADS, smem, st, ring, weights_all, g, img_type, vals);
     const long long outs = static_cast<long long>(T) * W + static_cast<long long>(H) * T;
-    k_cut_reduce<<<static_cast<unsigned>((outs + 255) / 256), 256, 0, st>>>(vals, g, xz, yz);
-    HV_LAUNCH_CHECK();
+    HV_LAUNCH(k_cut_reduce, static_cast<unsigned>((outs + 255) / 256), 256, 0, st, vals, g, xz, yz);
     count_launch(2);
     return HV_OK;
 }

@@ -32,6 +32,57 @@ __device__ __forceinline__ bool ctl_active(const CycleCtl* c) { return !c || c->
 __device__ __forceinline__ bool ctl_render(const CycleCtl* c) { return !c || c->render; }
 #endif
 
+#ifdef __CUDACC__
+// First statement of every kernel of this library: launch_kernel lets a kernel be scheduled while
+// its stream's previous kernel drains, and this waits until that one has ended and its writes are
+// visible (at once for a kernel launched in the ordinary way). Every kernel waits before it does
+// anything else or returns, so that a kernel's end implies the end of all before it in its stream.
+__device__ __forceinline__ void wait_prior_kernels() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Launches `kernel` on `st` with programmatic stream serialisation: ordered after the stream's
+// previous work like an ordinary launch (wait_prior_kernels), without the launch gap. Measured back to back on one
+// stream: a 1 us kernel takes 4.1 us per ordinary launch and 1.5 us so, a 5.9 us one 8.2 and 6.6 us (ordinary
+// completions are seen at ticks of about 2 us). Stream captures take the ordinary launch: a graph's
+// kernels already follow one another within 0.6 us.
+template <class... P, class... A>
+inline cudaError_t launch_kernel(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args)
+{
+    cudaLaunchConfig_t c{};
+    c.gridDim = grid;
+    c.blockDim = block;
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone)
+    {
+        c.attrs = at;
+        c.numAttrs = 1;
+    }
+    return cudaLaunchKernelEx(&c, kernel, P(args)...);
+}
+
+// Zeroes `words` 32-bit words: a kernel, so that the launches around it keep following one another
+// closely (a memset between them is waited for in the ordinary way).
+static __global__ void k_zero_words(unsigned int* p, size_t words)
+{
+    wait_prior_kernels();
+    for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < words;
+         i += static_cast<size_t>(gridDim.x) * blockDim.x)
+        p[i] = 0u;
+}
+
+inline cudaError_t launch_zero(void* p, size_t bytes, cudaStream_t st)
+{
+    const size_t words = bytes / sizeof(unsigned int);
+    const int grid = static_cast<int>(words < 152 * 1024 ? (words + 1023) / 1024 : 152);
+    return launch_kernel(k_zero_words, grid, words < 1024 ? 32 * ((words + 31) / 32) : 1024, 0, st,
+                         static_cast<unsigned int*>(p), words);
+}
+#endif
+
 void set_last_error(const char* msg, const char* file, int line);
 void set_last_error_msg(const char* msg);
 void count_launch(uint64_t n = 1);
@@ -206,4 +257,7 @@ hv_status contrast_to_ushort_normalized(const float* frame, const float* range, 
         }                                                                                                              \
     } while (0)
 
-#define HV_LAUNCH_CHECK() HV_CUDA_TRY(cudaGetLastError())
+// One kernel launch: kernel, grid, block, dynamic shared memory, stream, arguments.
+#define HV_LAUNCH(...) HV_CUDA_TRY(hv::launch_kernel(__VA_ARGS__))
+// Zeroes device memory in stream order (a multiple of 4 bytes).
+#define HV_LAUNCH_ZERO(ptr, bytes, st) HV_CUDA_TRY(hv::launch_zero(ptr, bytes, st))

@@ -18,6 +18,7 @@ namespace {
 __global__ void k_unpack12(const uint8_t* __restrict__ in, size_t in_bytes, uint16_t* __restrict__ out,
                            size_t out_count)
 {
+    wait_prior_kernels();
     const size_t groups = (out_count + 1) / 2;
     for (size_t g = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; g < groups;
          g += static_cast<size_t>(gridDim.x) * blockDim.x)
@@ -33,6 +34,7 @@ __global__ void k_unpack12(const uint8_t* __restrict__ in, size_t in_bytes, uint
 __global__ void k_unpack10(const uint8_t* __restrict__ in, size_t in_bytes, uint16_t* __restrict__ out,
                            size_t out_count)
 {
+    wait_prior_kernels();
     const size_t groups = (out_count + 3) / 4;
     for (size_t g = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; g < groups;
          g += static_cast<size_t>(gridDim.x) * blockDim.x)
@@ -64,14 +66,13 @@ hv_status unpack_packed(int bits, const void* in, size_t in_bytes, uint16_t* out
     if (out_count == 0)
         return HV_OK;
     if (bits == 12)
-        k_unpack12<<<unpack_grid((out_count + 1) / 2), 256, 0, st>>>(static_cast<const uint8_t*>(in), in_bytes, out,
-                                                                      out_count);
+        HV_LAUNCH(k_unpack12, unpack_grid((out_count + 1) / 2), 256, 0, st, static_cast<const uint8_t*>(in), in_bytes,
+                  out, out_count);
     else if (bits == 10)
-        k_unpack10<<<unpack_grid((out_count + 3) / 4), 256, 0, st>>>(static_cast<const uint8_t*>(in), in_bytes, out,
-                                                                      out_count);
+        HV_LAUNCH(k_unpack10, unpack_grid((out_count + 3) / 4), 256, 0, st, static_cast<const uint8_t*>(in), in_bytes,
+                  out, out_count);
     else
         return HV_INVALID_VALUE;
-    HV_LAUNCH_CHECK();
     count_launch();
     return HV_OK;
 }

@@ -40,6 +40,7 @@ static int ew_grid(size_t n)
 // z = exp(i*phase) (kernel_init_unwrap_2d)
 __global__ void k_unwrap_init(const float* in, float2* z, size_t n)
 {
+    wait_prior_kernels();
     for (size_t e = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; e < n;
          e += static_cast<size_t>(gridDim.x) * blockDim.x)
     {
@@ -61,6 +62,7 @@ __device__ __forceinline__ void shifted_freqs(size_t e, int W, int H, float& fx,
 // gx = Z * sfx, gy = Z * sfy (kernel_multiply_complexes_by_floats_)
 __global__ void k_unwrap_grad_freq(const float2* Z, float2* gx, float2* gy, int W, int H)
 {
+    wait_prior_kernels();
     const size_t n = static_cast<size_t>(W) * H;
     for (size_t e = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; e < n;
          e += static_cast<size_t>(gridDim.x) * blockDim.x)
@@ -76,6 +78,7 @@ __global__ void k_unwrap_grad_freq(const float2* Z, float2* gx, float2* gy, int 
 // g *= (i * 2pi) then g *= conj(i z) (kernel_multiply_complexes_by_single_complex, eq_unwrap_2d)
 __global__ void k_unwrap_eq(float2* gx, float2* gy, const float2* z, size_t n, float two_pi)
 {
+    wait_prior_kernels();
     const float2 i2pi = make_float2(0.f, two_pi);
     for (size_t e = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; e < n;
          e += static_cast<size_t>(gridDim.x) * blockDim.x)
@@ -89,6 +92,7 @@ __global__ void k_unwrap_eq(float2* gx, float2* gy, const float2* z, size_t n, f
 // acc = gx * sfx/(sfx^2+sfy^2) + gy * sfy/(...) (kernel_norm_ratio + kernel_add_complex_frames)
 __global__ void k_unwrap_ratio(const float2* gx, const float2* gy, float2* acc, int W, int H)
 {
+    wait_prior_kernels();
     const size_t n = static_cast<size_t>(W) * H;
     for (size_t e = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; e < n;
          e += static_cast<size_t>(gridDim.x) * blockDim.x)
@@ -120,6 +124,7 @@ __device__ __forceinline__ float key_float(unsigned int k)
 
 __global__ void k_unwrap_last(const float2* acc, float* out, size_t n, float two_pi, unsigned int* minmax)
 {
+    wait_prior_kernels();
     unsigned int kmin = 0xffffffffu, kmax = 0u;
     for (size_t e = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; e < n;
          e += static_cast<size_t>(gridDim.x) * blockDim.x)
@@ -144,6 +149,7 @@ __global__ void k_unwrap_last(const float2* acc, float* out, size_t n, float two
 
 __global__ void k_init_minmax(unsigned int* minmax)
 {
+    wait_prior_kernels();
     minmax[0] = 0xffffffffu;
     minmax[1] = 0u;
 }
@@ -151,6 +157,7 @@ __global__ void k_init_minmax(unsigned int* minmax)
 // rescale_float_unwrap2d: (in + |min|)/(|min| + max)*65535 if min < 0 else (in - min)/(max - min)*65535
 __global__ void k_unwrap_rescale(float* io, size_t n, const unsigned int* minmax)
 {
+    wait_prior_kernels();
     const float mn = key_float(minmax[0]), mx = key_float(minmax[1]);
     for (size_t e = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; e < n;
          e += static_cast<size_t>(gridDim.x) * blockDim.x)
@@ -193,29 +200,22 @@ hv_status unwrap_2d(const float* in, float* out, int W, int H, void* work, cudaS
     unsigned int* minmax = reinterpret_cast<unsigned int*>(Z + n);
     const float two_pi = 6.28318530717959f;  // M_2PI of common.cuh:29
     const int grid = ew_grid(n);
-    k_unwrap_init<<<grid, EW_THREADS, 0, st>>>(in, z, n);
-    HV_LAUNCH_CHECK();
+    HV_LAUNCH(k_unwrap_init, grid, EW_THREADS, 0, st, in, z, n);
     hv_status s = fft2d(z, Z, n0, n1, 1, 0, 1.0f, st);
     if (s != HV_OK)
         return s;
-    k_unwrap_grad_freq<<<grid, EW_THREADS, 0, st>>>(Z, gx, gy, W, H);
-    HV_LAUNCH_CHECK();
+    HV_LAUNCH(k_unwrap_grad_freq, grid, EW_THREADS, 0, st, Z, gx, gy, W, H);
     if ((s = fft2d(g, g, n0, n1, 2, 1, 1.0f, st)) != HV_OK)
         return s;
-    k_unwrap_eq<<<grid, EW_THREADS, 0, st>>>(gx, gy, z, n, two_pi);
-    HV_LAUNCH_CHECK();
+    HV_LAUNCH(k_unwrap_eq, grid, EW_THREADS, 0, st, gx, gy, z, n, two_pi);
     if ((s = fft2d(g, g, n0, n1, 2, 0, 1.0f, st)) != HV_OK)
         return s;
-    k_unwrap_ratio<<<grid, EW_THREADS, 0, st>>>(gx, gy, Z, W, H);
-    HV_LAUNCH_CHECK();
+    HV_LAUNCH(k_unwrap_ratio, grid, EW_THREADS, 0, st, gx, gy, Z, W, H);
     if ((s = fft2d(Z, Z, n0, n1, 1, 1, 1.0f, st)) != HV_OK)
         return s;
-    k_init_minmax<<<1, 1, 0, st>>>(minmax);
-    HV_LAUNCH_CHECK();
-    k_unwrap_last<<<grid, EW_THREADS, 0, st>>>(Z, out, n, two_pi, minmax);
-    HV_LAUNCH_CHECK();
-    k_unwrap_rescale<<<grid, EW_THREADS, 0, st>>>(out, n, minmax);
-    HV_LAUNCH_CHECK();
+    HV_LAUNCH(k_init_minmax, 1, 1, 0, st, minmax);
+    HV_LAUNCH(k_unwrap_last, grid, EW_THREADS, 0, st, Z, out, n, two_pi, minmax);
+    HV_LAUNCH(k_unwrap_rescale, grid, EW_THREADS, 0, st, out, n, minmax);
     count_launch(7);
     return HV_OK;
 }
@@ -289,6 +289,7 @@ size_t reduce_workspace(size_t n)
 
 __global__ void k_partial_sums(const float* in, size_t n, double* partials, const CycleCtl* ctl)
 {
+    wait_prior_kernels();
     if (!ctl_render(ctl))
         return;
     __shared__ double red[EW_THREADS / 32];
@@ -317,8 +318,7 @@ hv_status renorm_sum(const float* frame, size_t n, int renorm_constant, const do
     {
         double* p = static_cast<double*>(work);
         const int grid = ew_grid(n);
-        k_partial_sums<<<grid, EW_THREADS, 0, st>>>(frame, n, p, ctl);
-        HV_LAUNCH_CHECK();
+        HV_LAUNCH(k_partial_sums, grid, EW_THREADS, 0, st, frame, n, p, ctl);
         count_launch();
         partials = p;
         npartials = grid;
@@ -417,6 +417,7 @@ __global__ void __launch_bounds__(RN_THREADS) k_renorm_shift_acc(const float* in
                                                                  int start, int count, int log_enabled, float prescale,
                                                                  const CycleCtl* ctl)
 {
+    wait_prior_kernels();
     if (!ctl_render(ctl))
         return;
     if (ctl)
@@ -519,12 +520,11 @@ static hv_status launch_renorm_shift_acc(const float* in, float* out, int W, int
     const size_t want = (n + per - 1) / per, cap = sum.partials ? 152 : 152 * 32;
     const int grid = static_cast<int>(want < cap ? (want > 0 ? want : 1) : cap);
     if (v4)
-        k_renorm_shift_acc<4><<<grid, block, 0, st>>>(in, out, W, H, sum, shift, acc, A, slot, start, count,
-                                                      log_enabled, prescale, ctl);
+        HV_LAUNCH(k_renorm_shift_acc<4>, grid, block, 0, st, in, out, W, H, sum, shift, acc, A, slot, start, count,
+                  log_enabled, prescale, ctl);
     else
-        k_renorm_shift_acc<1><<<grid, block, 0, st>>>(in, out, W, H, sum, shift, acc, A, slot, start, count,
-                                                      log_enabled, prescale, ctl);
-    HV_LAUNCH_CHECK();
+        HV_LAUNCH(k_renorm_shift_acc<1>, grid, block, 0, st, in, out, W, H, sum, shift, acc, A, slot, start, count,
+                  log_enabled, prescale, ctl);
     count_launch();
     return HV_OK;
 }
@@ -550,6 +550,7 @@ hv_status renorm_shift_accumulate(const float* in, float* out, int W, int H, con
 // In-place quadrant swap: thread owns pixel (x, y) of the top half and swaps it with its partner.
 __global__ void k_shift_corners(float* f, int W, int H)
 {
+    wait_prior_kernels();
     const size_t half = static_cast<size_t>(W) * (H / 2);
     for (size_t e = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; e < half;
          e += static_cast<size_t>(gridDim.x) * blockDim.x)
@@ -571,8 +572,7 @@ hv_status shift_corners(float* frame, int W, int H, cudaStream_t st)
         set_last_error_msg("shift_corners needs even width and height");
         return HV_INVALID_VALUE;
     }
-    k_shift_corners<<<ew_grid(static_cast<size_t>(W) * H / 2), EW_THREADS, 0, st>>>(frame, W, H);
-    HV_LAUNCH_CHECK();
+    HV_LAUNCH(k_shift_corners, ew_grid(static_cast<size_t>(W) * H / 2), EW_THREADS, 0, st, frame, W, H);
     count_launch();
     return HV_OK;
 }
@@ -590,6 +590,7 @@ hv_status accumulate(const float* frame, float* acc_ring, int A, int slot, int s
 template <int V>
 __global__ void k_log10(float* f, size_t n)
 {
+    wait_prior_kernels();
     for (size_t e = (blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x) * V; e < n;
          e += static_cast<size_t>(gridDim.x) * blockDim.x * V)
     {
@@ -605,10 +606,9 @@ __global__ void k_log10(float* f, size_t n)
 hv_status log10_map(float* frame, size_t n, cudaStream_t st)
 {
     if (vec4_ok(n, {frame}))
-        k_log10<4><<<ew_grid(n / 4), EW_THREADS, 0, st>>>(frame, n);
+        HV_LAUNCH(k_log10<4>, ew_grid(n / 4), EW_THREADS, 0, st, frame, n);
     else
-        k_log10<1><<<ew_grid(n), EW_THREADS, 0, st>>>(frame, n);
-    HV_LAUNCH_CHECK();
+        HV_LAUNCH(k_log10<1>, ew_grid(n), EW_THREADS, 0, st, frame, n);
     count_launch();
     return HV_OK;
 }
@@ -741,6 +741,7 @@ __global__ void __launch_bounds__(EW_THREADS) k_pct_pass(const float* __restrict
                                                          unsigned int* hist, float lower, float upper, float* range,
                                                          const CycleCtl* ctl)
 {
+    wait_prior_kernels();
     if (ctl && !(ctl->render && ctl->pct_enable))
         return;
     __shared__ unsigned int sh[2][PCT_BINS];
@@ -856,7 +857,7 @@ hv_status percentile_pitched(const float* frame, int W, int H, int pitch, float 
     unsigned int* hist = static_cast<unsigned int*>(work);  // 3 passes x 2 ranks x PCT_BINS
     PctState* state = reinterpret_cast<PctState*>(hist + 3 * 2 * PCT_BINS);
     static_assert(sizeof(PctState) <= sizeof(unsigned int) * 8, "the state fits behind the histograms");
-    HV_CUDA_TRY(cudaMemsetAsync(hist, 0, 3 * 2 * PCT_BINS * sizeof(unsigned int) + sizeof(PctState), st));
+    HV_LAUNCH_ZERO(hist, 3 * 2 * PCT_BINS * sizeof(unsigned int) + sizeof(PctState), st);
     int use_reticle = 0;
     unsigned int r2 = 0;
     if (reticle_scale > 0.f)
@@ -876,12 +877,11 @@ hv_status percentile_pitched(const float* frame, int W, int H, int pitch, float 
     for (int d = 0; d < 3; ++d)
     {
         if (vec)
-            k_pct_pass<true><<<grid, EW_THREADS, 0, st>>>(frame, W, H, pitch, r2, use_reticle, state, d,
-                                                          hist + d * 2 * PCT_BINS, lower, upper, range, ctl);
+            HV_LAUNCH(k_pct_pass<true>, grid, EW_THREADS, 0, st, frame, W, H, pitch, r2, use_reticle, state, d,
+                      hist + d * 2 * PCT_BINS, lower, upper, range, ctl);
         else
-            k_pct_pass<false><<<grid, EW_THREADS, 0, st>>>(frame, W, H, pitch, r2, use_reticle, state, d,
-                                                           hist + d * 2 * PCT_BINS, lower, upper, range, ctl);
-        HV_LAUNCH_CHECK();
+            HV_LAUNCH(k_pct_pass<false>, grid, EW_THREADS, 0, st, frame, W, H, pitch, r2, use_reticle, state, d,
+                      hist + d * 2 * PCT_BINS, lower, upper, range, ctl);
     }
     count_launch(3);
     return HV_OK;
@@ -903,6 +903,7 @@ template <int V>
 __global__ void k_contrast_ushort(const float* __restrict__ in, const float* __restrict__ range, int invert, int apply,
                                   uint16_t* __restrict__ out, size_t n, const CycleCtl* ctl)
 {
+    wait_prior_kernels();
     if (!ctl_render(ctl))
         return;
     if (ctl)
@@ -944,6 +945,7 @@ __global__ void k_contrast_ushort(const float* __restrict__ in, const float* __r
 __global__ void k_f2d_view(const float2* __restrict__ spec, const float2* __restrict__ mult, int W, int H,
                            float* __restrict__ out)
 {
+    wait_prior_kernels();
     const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
     if (x >= W)
         return;
@@ -958,8 +960,7 @@ hv_status filter2d_view_frame(const float2* spec, const float2* mult, int W, int
     if ((W & 1) || (H & 1))
         return HV_INVALID_VALUE;
     dim3 block(128), grid((W + 127) / 128, H);
-    k_f2d_view<<<grid, block, 0, st>>>(spec, mult, W, H, out);
-    HV_LAUNCH_CHECK();
+    HV_LAUNCH(k_f2d_view, grid, block, 0, st, spec, mult, W, H, out);
     count_launch();
     return HV_OK;
 }
@@ -970,6 +971,7 @@ hv_status filter2d_view_frame(const float2* spec, const float2* mult, int W, int
 __global__ void k_contrast_ushort_normalized(const float* __restrict__ in, const float* __restrict__ range, int invert,
                                              int apply, uint16_t* __restrict__ out, size_t n)
 {
+    wait_prior_kernels();
     float mn = 0.f, factor = 1.f;
     if (apply)
     {
@@ -997,8 +999,7 @@ __global__ void k_contrast_ushort_normalized(const float* __restrict__ in, const
 hv_status contrast_to_ushort_normalized(const float* frame, const float* range, int invert, int apply, uint16_t* out,
                                         size_t n, cudaStream_t st)
 {
-    k_contrast_ushort_normalized<<<ew_grid(n), EW_THREADS, 0, st>>>(frame, range, invert, apply, out, n);
-    HV_LAUNCH_CHECK();
+    HV_LAUNCH(k_contrast_ushort_normalized, ew_grid(n), EW_THREADS, 0, st, frame, range, invert, apply, out, n);
     count_launch();
     return HV_OK;
 }
@@ -1008,10 +1009,9 @@ hv_status contrast_to_ushort(const float* frame, const float* range, int invert,
 {
     // (an output slot is n pixels of 2 bytes: a multiple of 8 bytes when n is one of 4)
     if (vec4_ok(n, {frame}) && (reinterpret_cast<uintptr_t>(out) & 7) == 0)
-        k_contrast_ushort<4><<<ew_grid(n / 4), EW_THREADS, 0, st>>>(frame, range, invert, apply, out, n, ctl);
+        HV_LAUNCH(k_contrast_ushort<4>, ew_grid(n / 4), EW_THREADS, 0, st, frame, range, invert, apply, out, n, ctl);
     else
-        k_contrast_ushort<1><<<ew_grid(n), EW_THREADS, 0, st>>>(frame, range, invert, apply, out, n, ctl);
-    HV_LAUNCH_CHECK();
+        HV_LAUNCH(k_contrast_ushort<1>, ew_grid(n), EW_THREADS, 0, st, frame, range, invert, apply, out, n, ctl);
     count_launch();
     return HV_OK;
 }

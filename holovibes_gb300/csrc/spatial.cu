@@ -37,6 +37,7 @@ namespace hv {
 
 __global__ void k_fresnel_lens(float2* out, int W, int H, double lam, double z, double pixel_size_um, int mode)
 {
+    wait_prior_kernels();
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = blockIdx.y;
     if (x >= W || y >= H)
@@ -73,6 +74,7 @@ __global__ void k_fresnel_lens(float2* out, int W, int H, double lam, double z, 
 
 __global__ void k_spectral_lens(float2* out, int W, int H, double lam, double z, double pixel_size_um, int mode)
 {
+    wait_prior_kernels();
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = blockIdx.y;
     if (x >= W || y >= H)
@@ -152,6 +154,7 @@ __device__ __forceinline__ const float2* stage_twiddles(float2* dst, const float
 template <int N, int F>
 __global__ void __launch_bounds__(fft::Tile<N, F, false>::NT) k_fft_rows(RowPass p)
 {
+    wait_prior_kernels();
     using Tl = fft::Tile<N, F, false>;
     extern __shared__ float2 smem[];
     if (!ctl_active(p.ctl))
@@ -292,6 +295,7 @@ struct ColPass
 template <int N, int F>
 __global__ void __launch_bounds__(fft::Tile<N, F, true>::NT) k_fft_cols(ColPass p)
 {
+    wait_prior_kernels();
     using Tl = fft::Tile<N, F, true>;
     extern __shared__ float2 smem[];
     if (!ctl_active(p.ctl))
@@ -439,6 +443,7 @@ __device__ __forceinline__ float2 staged_sample(const void* row, int at, bool sw
 template <int N, int KIND, bool PREMUL>
 __global__ void __launch_bounds__(W32_THREADS, 2) k_fft_rows_warp(RowPass p, int per_frame, int nframes, int bulk)
 {
+    wait_prior_kernels();
     using Gm = W32Geom<N>;
     constexpr int NG = Gm::NG, NS = Gm::NS;
     constexpr int ESIZE = KIND == IN_U8 ? 1 : KIND == IN_U16 ? 2 : KIND == IN_F32 ? 4 : 8;
@@ -610,6 +615,7 @@ __global__ void __launch_bounds__(W32_THREADS, 2) k_fft_cols_warp(const __grid_c
                                                                   const __grid_constant__ CUtensorMap g_map, ColPass p,
                                                                   int tiles_x, int ntiles, int bulk)
 {
+    wait_prior_kernels();
     using Gm = W32Geom<N>;
     constexpr int NG = Gm::NG, NS = Gm::NS, K1 = Gm::K1, C = Gm::COLS;
     extern __shared__ unsigned char smem_raw[];
@@ -804,6 +810,7 @@ __global__ void __launch_bounds__(W32_THREADS, 2) k_fft_cols_warp(const __grid_c
 __global__ void k_convert8(const void* in, int kind, size_t frame_px, int batch, float2* ring, FrameMap map,
                            const CycleCtl* ctl, uint16_t* planes)
 {
+    wait_prior_kernels();
     if (!ctl_active(ctl))
         return;
     if (ctl)
@@ -875,6 +882,7 @@ __global__ void k_convert8(const void* in, int kind, size_t frame_px, int batch,
 __global__ void k_ring_from_planes(const uint16_t* __restrict__ planes, int T, size_t frame_px, int slot0, int n,
                                    float2* __restrict__ ring)
 {
+    wait_prior_kernels();
     const size_t groups = frame_px / 8;
     const size_t total = groups * n;
     const size_t plane = static_cast<size_t>(T) * frame_px;
@@ -903,6 +911,7 @@ __global__ void k_ring_from_planes(const uint16_t* __restrict__ planes, int T, s
 __global__ void k_convert(const void* in, int kind, size_t frame_px, int batch, float2* ring, FrameMap map,
                           const CycleCtl* ctl)
 {
+    wait_prior_kernels();
     if (!ctl_active(ctl))
         return;
     if (ctl)
@@ -1087,8 +1096,7 @@ hv_status launch_rows_warp(const RowPass& p, int nframes, cudaStream_t st)
     default: kern = pre ? k_fft_rows_warp<N, IN_C64, true> : k_fft_rows_warp<N, IN_C64, false>; break;
     }
     HV_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(Gm::ROW_SMEM)));
-    kern<<<grid, W32_THREADS, Gm::ROW_SMEM, st>>>(q, per_frame, nframes, bulk ? 1 : 0);
-    HV_LAUNCH_CHECK();
+    HV_LAUNCH(kern, grid, W32_THREADS, Gm::ROW_SMEM, st, q, per_frame, nframes, bulk ? 1 : 0);
     count_launch();
     return HV_OK;
 }
@@ -1116,8 +1124,7 @@ hv_status launch_cols_warp(const ColPass& p, int nframes, cudaStream_t st)
                tc::encode_tmap_2d_f32(&g_map, p.postmul, static_cast<uint64_t>(p.width) * 2, N, pitch, Gm::COLS * 2, 256);
     auto kern = p.mode == 2 ? k_fft_cols_warp<N, 2> : p.mode == 1 ? k_fft_cols_warp<N, 1> : k_fft_cols_warp<N, 0>;
     HV_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(Gm::COL_SMEM)));
-    kern<<<grid, W32_THREADS, Gm::COL_SMEM, st>>>(in_map, g_map, q, tiles_x, ntiles, bulk ? 1 : 0);
-    HV_LAUNCH_CHECK();
+    HV_LAUNCH(kern, grid, W32_THREADS, Gm::COL_SMEM, st, in_map, g_map, q, tiles_x, ntiles, bulk ? 1 : 0);
     count_launch();
     return HV_OK;
 }
@@ -1140,8 +1147,7 @@ hv_status launch_rows(const RowPass& p, int nframes, cudaStream_t st)
         return HV_ERR_CUDA;
     q.tw_count = tw_count;
     dim3 grid((p.rows + F - 1) / F, nframes);
-    k_fft_rows<N, F><<<grid, Tl::NT, smem, st>>>(q);
-    HV_LAUNCH_CHECK();
+    HV_LAUNCH((k_fft_rows<N, F>), grid, Tl::NT, smem, st, q);
     count_launch();
     return HV_OK;
 }
@@ -1164,8 +1170,7 @@ hv_status launch_cols(const ColPass& p, int nframes, cudaStream_t st)
         return HV_ERR_CUDA;
     q.tw_count = tw_count;
     dim3 grid((p.width + F - 1) / F, nframes);
-    k_fft_cols<N, F><<<grid, Tl::NT, smem, st>>>(q);
-    HV_LAUNCH_CHECK();
+    HV_LAUNCH((k_fft_cols<N, F>), grid, Tl::NT, smem, st, q);
     count_launch();
     return HV_OK;
 }
@@ -1224,8 +1229,7 @@ hv_status fft_cols(const ColPass& p, int N, int nframes, cudaStream_t st)
 hv_status make_fresnel_lens(float2* lens, int W, int H, float lam, float z, float ps, int mode, cudaStream_t st)
 {
     dim3 block(128), grid((W + 127) / 128, H);
-    k_fresnel_lens<<<grid, block, 0, st>>>(lens, W, H, lam, z, ps, mode);
-    HV_LAUNCH_CHECK();
+    HV_LAUNCH(k_fresnel_lens, grid, block, 0, st, lens, W, H, lam, z, ps, mode);
     count_launch();
     return HV_OK;
 }
@@ -1233,8 +1237,7 @@ hv_status make_fresnel_lens(float2* lens, int W, int H, float lam, float z, floa
 hv_status make_spectral_lens(float2* lens, int W, int H, float lam, float z, float ps, int mode, cudaStream_t st)
 {
     dim3 block(128), grid((W + 127) / 128, H);
-    k_spectral_lens<<<grid, block, 0, st>>>(lens, W, H, lam, z, ps, mode);
-    HV_LAUNCH_CHECK();
+    HV_LAUNCH(k_spectral_lens, grid, block, 0, st, lens, W, H, lam, z, ps, mode);
     count_launch();
     return HV_OK;
 }
@@ -1248,6 +1251,7 @@ hv_status make_spectral_lens(float2* lens, int W, int H, float lam, float z, flo
 // FFT-layout complex array in place (multiply = 1: the AS transfer function, fourier_transform.cc:134-137).
 __global__ void k_filter2d_mask(float2* dst, int W, int H, int n1, int n2, int sl, int sh, int multiply)
 {
+    wait_prior_kernels();
     const int X = blockIdx.x * blockDim.x + threadIdx.x, Y = blockIdx.y;
     if (X >= W || Y >= H)
         return;
@@ -1283,8 +1287,7 @@ hv_status filter2d_mask(float2* dst, int W, int H, int n1, int n2, int smooth_lo
     if (!dst || W <= 0 || H <= 0 || (W & 1) || (H & 1) || n1 < 0 || n2 <= n1 || smooth_low < 0 || smooth_high < 0)
         return HV_INVALID_VALUE;
     dim3 block(128), grid((W + 127) / 128, H);
-    k_filter2d_mask<<<grid, block, 0, st>>>(dst, W, H, n1, n2, smooth_low, smooth_high, multiply);
-    HV_LAUNCH_CHECK();
+    HV_LAUNCH(k_filter2d_mask, grid, block, 0, st, dst, W, H, n1, n2, smooth_low, smooth_high, multiply);
     count_launch();
     return HV_OK;
 }
@@ -1331,8 +1334,7 @@ hv_status spatial_transform(const void* raw, int kind, int W, int H, int batch, 
         {
             const size_t total = HW / 8 * batch;
             const int grid = static_cast<int>((total + block - 1) / block < 152 * 8 ? (total + block - 1) / block : 152 * 8);
-            k_convert8<<<grid, block, 0, st>>>(raw, kind, HW, batch, ring, ring_map, ctl, real_planes);
-            HV_LAUNCH_CHECK();
+            HV_LAUNCH(k_convert8, grid, block, 0, st, raw, kind, HW, batch, ring, ring_map, ctl, real_planes);
             count_launch();
             return HV_OK;
         }
@@ -1343,8 +1345,7 @@ hv_status spatial_transform(const void* raw, int kind, int W, int H, int batch, 
         }
         const size_t total = HW * batch;
         const int grid = static_cast<int>((total + block - 1) / block < 152 * 16 ? (total + block - 1) / block : 152 * 16);
-        k_convert<<<grid, block, 0, st>>>(raw, kind, HW, batch, ring, ring_map, ctl);
-        HV_LAUNCH_CHECK();
+        HV_LAUNCH(k_convert, grid, block, 0, st, raw, kind, HW, batch, ring, ring_map, ctl);
         count_launch();
         return HV_OK;
     }
@@ -1467,8 +1468,7 @@ hv_status convert_to_planes(const void* raw, int kind, size_t HW, int batch, int
     // stream) find room beside this pass
     const int cap = device_sms() * 6;
     const int grid = static_cast<int>((total + block - 1) / block < static_cast<size_t>(cap) ? (total + block - 1) / block : cap);
-    k_convert8<<<grid, block, 0, st>>>(raw, kind, HW, batch, nullptr, map, nullptr, planes);
-    HV_LAUNCH_CHECK();
+    HV_LAUNCH(k_convert8, grid, block, 0, st, raw, kind, HW, batch, nullptr, map, nullptr, planes);
     count_launch();
     return HV_OK;
 }
@@ -1481,8 +1481,7 @@ hv_status ring_from_planes(const uint16_t* planes, int T, size_t HW, int slot0, 
     const int block = 256;
     const int cap = device_sms() * 6;  // as convert_to_planes: room for the eigensolve stream's kernels
     const int grid = static_cast<int>((total + block - 1) / block < static_cast<size_t>(cap) ? (total + block - 1) / block : cap);
-    k_ring_from_planes<<<grid, block, 0, st>>>(planes, T, HW, slot0, n, ring);
-    HV_LAUNCH_CHECK();
+    HV_LAUNCH(k_ring_from_planes, grid, block, 0, st, planes, T, HW, slot0, n, ring);
     count_launch();
     return HV_OK;
 }

@@ -53,6 +53,7 @@ __global__ void __launch_bounds__(TV_THREADS) k_time_view(const float2* __restri
                                                            double* __restrict__ partials, const CycleCtl* ctl,
                                                            const float* __restrict__ bin_w)
 {
+    wait_prior_kernels();
     // bin_w (moments): out = sum_k |X_k|^2 bin_w[k] instead of the mean of the view over the bins
     if (!ctl_render(ctl))
         return;
@@ -151,6 +152,7 @@ __global__ void __launch_bounds__(TV_THREADS) k_time_view2(const float2* __restr
                                                             double* __restrict__ partials, int npartials,
                                                             const CycleCtl* ctl, const float* __restrict__ bin_w)
 {
+    wait_prior_kernels();
     if (!ctl_render(ctl))
         return;
     extern __shared__ __align__(16) float2 wsm[];  // [T][KC]
@@ -337,6 +339,7 @@ __global__ void __launch_bounds__(TV_THREADS, 8) k_time_view_planes(const uint16
                                                                  int npartials, const CycleCtl* ctl,
                                                                  const float* __restrict__ bin_w)
 {
+    wait_prior_kernels();
     if (!ctl_render(ctl))
         return;
     extern __shared__ __align__(16) float2 wsm[];  // [T][KC]
@@ -474,16 +477,14 @@ static hv_status launch_time_view(const float2* ring, int T, int W, int H, const
             HV_CUDA_TRY(cudaFuncSetAttribute(k_time_view2<KC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              static_cast<int>(smem)));
         const int grid2 = static_cast<int>((HW + 2 * TV_THREADS - 1) / (2 * TV_THREADS));
-        k_time_view2<KC><<<grid2, TV_THREADS, smem, st>>>(ring, T, W, H, weights, K, img_type, scale, shift, out,
-                                                          partials, np, ctl, bin_w);
-        HV_LAUNCH_CHECK();
+        HV_LAUNCH(k_time_view2<KC>, grid2, TV_THREADS, smem, st, ring, T, W, H, weights, K, img_type, scale, shift, out,
+                  partials, np, ctl, bin_w);
         count_launch();
         return HV_OK;
     }
     const int grid = np;
-    k_time_view<KC><<<grid, TV_THREADS, smem, st>>>(ring, T, W, H, weights, K, img_type, scale, shift, out, partials,
-                                                    ctl, bin_w);
-    HV_LAUNCH_CHECK();
+    HV_LAUNCH(k_time_view<KC>, grid, TV_THREADS, smem, st, ring, T, W, H, weights, K, img_type, scale, shift, out,
+              partials, ctl, bin_w);
     count_launch();
     return HV_OK;
 }
@@ -536,10 +537,8 @@ static hv_status launch_time_view_planes(const uint16_t* planes, const float2* r
                                          static_cast<int>(smem)));
     const size_t HW = static_cast<size_t>(W) * H;
     const int grid = static_cast<int>((HW + 2 * TV_THREADS - 1) / (2 * TV_THREADS));
-    k_time_view_planes<KC><<<grid, TV_THREADS, smem, st>>>(planes, ring, r0, rn, T, W, H, weights, K, img_type, scale,
-                                                           shift, out, partials, time_view_partials(W, H), ctl,
-                                                           bin_w);
-    HV_LAUNCH_CHECK();
+    HV_LAUNCH(k_time_view_planes<KC>, grid, TV_THREADS, smem, st, planes, ring, r0, rn, T, W, H, weights, K, img_type,
+              scale, shift, out, partials, time_view_partials(W, H), ctl, bin_w);
     count_launch();
     return HV_OK;
 }
@@ -580,6 +579,7 @@ hv_status time_view_planes(const uint16_t* planes, const float2* ring, int ring_
 
 __global__ void k_stft_weights(float2* w, int T, int pmin, int K)
 {
+    wait_prior_kernels();
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= K * T)
         return;
@@ -592,6 +592,7 @@ __global__ void k_stft_weights(float2* w, int T, int pmin, int K)
 
 __global__ void k_delta_weights(float2* w, int T, int pmin, int K)
 {
+    wait_prior_kernels();
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= K * T)
         return;
@@ -632,8 +633,7 @@ hv_status stft_weights(float2* weights, int T, int pmin, int pmax, cudaStream_t 
     const int K = pmax - pmin + 1;
     if (K <= 0 || T <= 0)
         return HV_INVALID_VALUE;
-    k_stft_weights<<<(K * T + 255) / 256, 256, 0, st>>>(weights, T, pmin, K);
-    HV_LAUNCH_CHECK();
+    HV_LAUNCH(k_stft_weights, (K * T + 255) / 256, 256, 0, st, weights, T, pmin, K);
     count_launch();
     return HV_OK;
 }
@@ -643,8 +643,7 @@ hv_status delta_weights(float2* weights, int T, int pmin, int pmax, cudaStream_t
     const int K = pmax - pmin + 1;
     if (K <= 0 || T <= 0)
         return HV_INVALID_VALUE;
-    k_delta_weights<<<(K * T + 255) / 256, 256, 0, st>>>(weights, T, pmin, K);
-    HV_LAUNCH_CHECK();
+    HV_LAUNCH(k_delta_weights, (K * T + 255) / 256, 256, 0, st, weights, T, pmin, K);
     count_launch();
     return HV_OK;
 }
@@ -683,6 +682,7 @@ static CovPlan cov_plan(int T, size_t npix)
 __global__ void __launch_bounds__(COV_THREADS) k_cov_partial(const float2* __restrict__ ring, int T, size_t npix,
                                                               int tiles1d, size_t chunk_px, float2* __restrict__ part)
 {
+    wait_prior_kernels();
     __shared__ float2 A[COV_PX][COV_TILE + 1];
     __shared__ float2 B[COV_PX][COV_TILE + 1];
     // tile index -> (ti, tj) with ti <= tj
@@ -746,6 +746,7 @@ __global__ void __launch_bounds__(COV_THREADS) k_cov_partial(const float2* __res
 __global__ void k_cov_reduce(const float2* __restrict__ part, int T, int tiles1d, int ntiles, int chunks,
                              int chunks_per_slice, double2* __restrict__ cov)
 {
+    wait_prior_kernels();
     const int e = blockIdx.x * blockDim.x + threadIdx.x;  // over T*T
     if (e >= T * T)
         return;
@@ -808,8 +809,8 @@ hv_status pca_covariance(const float2* ring, int T, size_t npix, double2* cov, v
         return HV_INVALID_VALUE;
     int* err = static_cast<int*>(work);
     char* ws = static_cast<char*>(work) + COV_FLAGS;
-    HV_CUDA_TRY(cudaMemsetAsync(cov, 0, static_cast<size_t>(T) * T * sizeof(double2), st));
-    HV_CUDA_TRY(cudaMemsetAsync(err, 0, sizeof(int), st));
+    HV_LAUNCH_ZERO(cov, static_cast<size_t>(T) * T * sizeof(double2), st);
+    HV_LAUNCH_ZERO(err, sizeof(int), st);
     const bool tc_ok = cov_tc_supported(T) && npix % 8 == 0 && (reinterpret_cast<uintptr_t>(ring) & 15) == 0;
     const int mode = g_cov_mode.load();
     if ((mode == 0 && tc_ok) || mode == 2)
@@ -824,13 +825,11 @@ hv_status pca_covariance(const float2* ring, int T, size_t npix, double2* cov, v
     const CovPlan p = cov_plan(T, npix);
     float2* part = reinterpret_cast<float2*>(ws);
     dim3 grid(p.ntiles, p.chunks);
-    k_cov_partial<<<grid, COV_THREADS, 0, st>>>(ring, T, npix, p.tiles1d, p.chunk_px, part);
-    HV_LAUNCH_CHECK();
+    HV_LAUNCH(k_cov_partial, grid, COV_THREADS, 0, st, ring, T, npix, p.tiles1d, p.chunk_px, part);
     const int slices = p.chunks < 32 ? p.chunks : 32;
     const int per = (p.chunks + slices - 1) / slices;
     dim3 rgrid((T * T + 255) / 256, (p.chunks + per - 1) / per);
-    k_cov_reduce<<<rgrid, 256, 0, st>>>(part, T, p.tiles1d, p.ntiles, p.chunks, per, cov);
-    HV_LAUNCH_CHECK();
+    HV_LAUNCH(k_cov_reduce, rgrid, 256, 0, st, part, T, p.tiles1d, p.ntiles, p.chunks, per, cov);
     count_launch(2);
     return HV_OK;
 }
@@ -844,7 +843,7 @@ hv_status pca_covariance_planes(const uint16_t* planes, int T, size_t npix, doub
         return HV_ERR_UNSUPPORTED;
     int* err = static_cast<int*>(work);
     char* ws = static_cast<char*>(work) + COV_FLAGS;
-    HV_CUDA_TRY(cudaMemsetAsync(err, 0, sizeof(int), st));
+    HV_LAUNCH_ZERO(err, sizeof(int), st);
     return cov_tc_planes(planes, T, npix, cov, ws, err, blocks, real, st);
 }
 
@@ -879,6 +878,7 @@ __device__ __forceinline__ double2 zmul(double2 a, double2 b)
 __global__ void __launch_bounds__(JAC_THREADS) k_jacobi(double2* A, double2* V, int T, int Tp, double* evals,
                                                          int* pair_buf, double* rot_buf)
 {
+    wait_prior_kernels();
     // pair_buf: 2*(Tp/2) ints; rot_buf: 4*(Tp/2) doubles (c, s, cos phi, sin phi)
     __shared__ double red[JAC_THREADS / 32];
     __shared__ double s_off, s_norm;
@@ -1321,6 +1321,7 @@ __global__ void __launch_bounds__(JS_THREADS) k_jacobi_smem(const double2* __res
                                                             int T, int Tp, double* __restrict__ evals, int warm,
                                                             float floor_rel)
 {
+    wait_prior_kernels();
     extern __shared__ __align__(16) unsigned char js_raw[];
     Cx<R>* js = reinterpret_cast<Cx<R>*>(js_raw);
     const int LD = T + 1;
@@ -1581,6 +1582,7 @@ __global__ void __launch_bounds__(BJ_THREADS) k_jacobi_block(const double2* __re
                                                              double2* __restrict__ Vout,
                                                              double* __restrict__ evals, double floor_rel)
 {
+    wait_prior_kernels();
     using R = float;
     extern __shared__ __align__(16) unsigned char bj_raw[];
     Cx<R>* sm0 = reinterpret_cast<Cx<R>*>(bj_raw);
@@ -1791,6 +1793,7 @@ __global__ void __launch_bounds__(BJ_THREADS) k_jacobi_block(const double2* __re
 template <class Acc>
 __global__ void k_eig_refine(const double2* __restrict__ A, double2* __restrict__ V, int T, double* __restrict__ evals)
 {
+    wait_prior_kernels();
     __shared__ double2 v[JC_MAX_T];
     __shared__ double red[4];
     __shared__ Acc redl[4];
@@ -1844,6 +1847,7 @@ __global__ void k_eig_refine(const double2* __restrict__ A, double2* __restrict_
 __global__ void k_eig_sort(const double* evals_in, const double2* V, int T, double* evals, double2* evecs, int pmin,
                            int pmax, float2* weights)
 {
+    wait_prior_kernels();
     __shared__ int s_rank;
     const int i = blockIdx.x;
     const double ei = evals_in[i];
@@ -1912,6 +1916,7 @@ __device__ __forceinline__ double2 warp_sum2(double2 v)
 __global__ void k_eigref_matvec(const double2* __restrict__ C, const double2* __restrict__ evecs, int T, int r0,
                                 double2* __restrict__ Y)
 {
+    wait_prior_kernels();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int t = blockIdx.x * 8 + warp, j = blockIdx.y;
     if (t >= T)
@@ -1939,6 +1944,7 @@ __global__ void __launch_bounds__(ER_PROJ_THREADS) k_eigref_project(const double
                                                                    int b0, double2* __restrict__ D,
                                                                    double2* __restrict__ G)
 {
+    wait_prior_kernels();
     __shared__ double2 sd[ER_PROJ_THREADS / 32], sg[ER_PROJ_THREADS / 32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int i = b0 + blockIdx.x, j = blockIdx.y;
@@ -1997,6 +2003,7 @@ __global__ void __launch_bounds__(32 * ER_UPD_WARPS) k_eigref_update(const doubl
                                                                     const double2* __restrict__ Y, int T, int r0,
                                                                     int K, int b0, double2* __restrict__ Vn)
 {
+    wait_prior_kernels();
     __shared__ double2 coef[JC_MAX_T];
     __shared__ double2 comp[JC_MAX_T];
     __shared__ double2 pacc[ER_UPD_WARPS][32], pproj[ER_UPD_WARPS][32];
@@ -2071,6 +2078,7 @@ __global__ void k_eigref_finish(double2* __restrict__ evecs, double* __restrict_
                                 const double2* __restrict__ D, const double2* __restrict__ G, int T, int r0, int pmin,
                                 int pmax, float2* __restrict__ weights)
 {
+    wait_prior_kernels();
     __shared__ double red[4];
     const int j = blockIdx.x, tid = threadIdx.x, rj = r0 + j;
     const double2* v = Vn + static_cast<size_t>(j) * T;
@@ -2127,6 +2135,7 @@ static size_t ts_bytes(int T)
 // 0 also stores it
 __global__ void k_ts_convert(const double2* __restrict__ C, int T, float2* __restrict__ C32, double* __restrict__ scale)
 {
+    wait_prior_kernels();
     __shared__ double s_scale;
     if (threadIdx.x < 32)
     {
@@ -2156,6 +2165,7 @@ __global__ void k_ts_convert(const double2* __restrict__ C, int T, float2* __res
 // cold start: Y[t][k] = C32[t][k T / TS_P] (columns of C span its dominant eigenvectors)
 __global__ void k_ts_init(const float2* __restrict__ C32, int T, float2* __restrict__ Y)
 {
+    wait_prior_kernels();
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= T * TS_P)
         return;
@@ -2169,6 +2179,7 @@ __global__ void k_ts_init(const float2* __restrict__ C32, int T, float2* __restr
 __global__ void __launch_bounds__(TS_MM_ROWS * TS_MM_SPLIT * 32)
     k_ts_matmul(const float2* __restrict__ C32, const float2* __restrict__ V, int T, float2* __restrict__ Y)
 {
+    wait_prior_kernels();
     __shared__ float2 part[TS_MM_ROWS * TS_MM_SPLIT][TS_P];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int t = blockIdx.x * TS_MM_ROWS + warp / TS_MM_SPLIT, q = warp % TS_MM_SPLIT;
@@ -2309,6 +2320,7 @@ __device__ __forceinline__ float ts_project(float2 (&y)[TS_ORTH_RPT][TS_P], floa
 __global__ void __launch_bounds__(TS_ORTH_THREADS) k_ts_orth(const float2* __restrict__ Y, int T, float2* __restrict__ V,
                                                               const int* __restrict__ only_if = nullptr)
 {
+    wait_prior_kernels();
     if (only_if && *only_if == 0)  // the Cholesky-QR of the warm iteration succeeded
         return;
     __shared__ float2 red[2][TS_ORTH_THREADS / 32][TS_P];
@@ -2390,6 +2402,7 @@ __global__ void __launch_bounds__(TS_ORTH_THREADS) k_ts_orth(const float2* __res
 __global__ void __launch_bounds__(32) k_ts_cholqr(const float2* __restrict__ G, float2* __restrict__ M,
                                                   int* __restrict__ fail)
 {
+    wait_prior_kernels();
     __shared__ float2 L[TS_P][TS_P + 1];  // index a = TS_P - 1 - (column of Y); lower triangle = L
     __shared__ float2 X[TS_P][TS_P + 1];  // L^-1
     __shared__ float d[TS_P];
@@ -2466,6 +2479,7 @@ __global__ void __launch_bounds__(TS_GRAM_WARPS * 32) k_ts_gram(const float2* __
                                                                const float2* __restrict__ Y, int T,
                                                                float2* __restrict__ H)
 {
+    wait_prior_kernels();
     __shared__ float2 part[TS_GRAM_WARPS][TS_P];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, i = blockIdx.x;
     float r0 = 0.f, i0 = 0.f, r1 = 0.f, i1 = 0.f;
@@ -2508,6 +2522,7 @@ __global__ void __launch_bounds__(JS_THREADS) k_ts_rr(const float2* __restrict__
                                                      const double* __restrict__ scale, double* __restrict__ evals,
                                                      float2* __restrict__ Qo)
 {
+    wait_prior_kernels();
     constexpr int NW = JS_THREADS / 32;
     __shared__ Cx<float> Hs[TS_P * TS_LD], Qs[TS_P * TS_LD];
     __shared__ JacScratch<float> sc;
@@ -2565,6 +2580,7 @@ __global__ void __launch_bounds__(JS_THREADS) k_ts_rr(const float2* __restrict__
 __global__ void __launch_bounds__(256) k_ts_ritz(const float2* __restrict__ V, const float2* __restrict__ Qo, int T,
                                                  double2* __restrict__ evecs, float2* __restrict__ Vw)
 {
+    wait_prior_kernels();
     __shared__ float2 q[TS_P][TS_P];
     __shared__ float2 u[TS_P][TS_P + 1];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -2674,14 +2690,10 @@ hv_status pca_eigh(double2* cov, int T, double* evals, double2* evecs, int pmin,
         const dim3 gw((T + 7) / 8, Kr), gp(T - b0, Kr), gt((T + 31) / 32, Kr);
         for (int iter = 0; iter < iters; ++iter)
         {
-            k_eigref_matvec<<<gw, 256, 0, st>>>(cov, evecs, T, refine_lo, Y);
-            HV_LAUNCH_CHECK();
-            k_eigref_project<<<gp, ER_PROJ_THREADS, 0, st>>>(evecs, Y, T, refine_lo, b0, D, G);
-            HV_LAUNCH_CHECK();
-            k_eigref_update<<<gt, 32 * ER_UPD_WARPS, 0, st>>>(evecs, evals, D, G, Y, T, refine_lo, Kr, b0, Vn);
-            HV_LAUNCH_CHECK();
-            k_eigref_finish<<<Kr, 128, 0, st>>>(evecs, evals, Vn, D, G, T, refine_lo, pmin, pmax, weights);
-            HV_LAUNCH_CHECK();
+            HV_LAUNCH(k_eigref_matvec, gw, 256, 0, st, cov, evecs, T, refine_lo, Y);
+            HV_LAUNCH(k_eigref_project, gp, ER_PROJ_THREADS, 0, st, evecs, Y, T, refine_lo, b0, D, G);
+            HV_LAUNCH(k_eigref_update, gt, 32 * ER_UPD_WARPS, 0, st, evecs, evals, D, G, Y, T, refine_lo, Kr, b0, Vn);
+            HV_LAUNCH(k_eigref_finish, Kr, 128, 0, st, evecs, evals, Vn, D, G, T, refine_lo, pmin, pmax, weights);
             count_launch(4);
         }
         return HV_OK;
@@ -2699,51 +2711,38 @@ hv_status pca_eigh(double2* cov, int T, double* evals, double2* evecs, int pmin,
         const int gb = (T * TS_P + 255) / 256;
         const int gm = (T + TS_MM_ROWS - 1) / TS_MM_ROWS;
         constexpr int mm_threads = TS_MM_ROWS * TS_MM_SPLIT * 32;
-        k_ts_convert<<<std::min(512, (T * T + 1023) / 1024), 256, 0, st>>>(cov, T, C32, scale);
-        HV_LAUNCH_CHECK();
+        HV_LAUNCH(k_ts_convert, std::min(512, (T * T + 1023) / 1024), 256, 0, st, cov, T, C32, scale);
         // warm: the previous window's Ritz vectors are orthonormal (V Q with V orthonormal, Q unitary)
         // and start the iteration as they are
         if (!warm)
         {
-            k_ts_init<<<gb, 256, 0, st>>>(C32, T, Ys);
-            HV_LAUNCH_CHECK();
-            k_ts_orth<<<1, TS_ORTH_THREADS, 0, st>>>(Ys, T, Vs);
-            HV_LAUNCH_CHECK();
+            HV_LAUNCH(k_ts_init, gb, 256, 0, st, C32, T, Ys);
+            HV_LAUNCH(k_ts_orth, 1, TS_ORTH_THREADS, 0, st, Ys, T, Vs, nullptr);
         }
         const int iters = warm ? TS_ITERS_WARM : TS_ITERS_COLD;
         int* chol_fail = reinterpret_cast<int*>(scale + 1);
         int extra = 0;
         for (int it = 0; it < iters; ++it)
         {
-            k_ts_matmul<<<gm, mm_threads, 0, st>>>(C32, it == 0 && warm ? Vw : Vs, T, Ys);
-            HV_LAUNCH_CHECK();
+            HV_LAUNCH(k_ts_matmul, gm, mm_threads, 0, st, C32, it == 0 && warm ? Vw : Vs, T, Ys);
             if (warm && cholqr_enabled())
             {
                 // Cholesky-QR (Gram, 32 x 32 factorisation, V = Y M), Gram-Schmidt only if it failed
-                k_ts_gram<<<TS_P, TS_GRAM_WARPS * 32, 0, st>>>(Ys, Ys, T, Hm);
-                HV_LAUNCH_CHECK();
-                k_ts_cholqr<<<1, 32, 0, st>>>(Hm, Qo, chol_fail);
-                HV_LAUNCH_CHECK();
-                k_ts_ritz<<<(T + TS_P - 1) / TS_P, 256, 0, st>>>(Ys, Qo, T, nullptr, Vs);
-                HV_LAUNCH_CHECK();
-                k_ts_orth<<<1, TS_ORTH_THREADS, 0, st>>>(Ys, T, Vs, chol_fail);
-                HV_LAUNCH_CHECK();
+                HV_LAUNCH(k_ts_gram, TS_P, TS_GRAM_WARPS * 32, 0, st, Ys, Ys, T, Hm);
+                HV_LAUNCH(k_ts_cholqr, 1, 32, 0, st, Hm, Qo, chol_fail);
+                HV_LAUNCH(k_ts_ritz, (T + TS_P - 1) / TS_P, 256, 0, st, Ys, Qo, T, nullptr, Vs);
+                HV_LAUNCH(k_ts_orth, 1, TS_ORTH_THREADS, 0, st, Ys, T, Vs, chol_fail);
                 extra += 3;
             }
             else
             {
-                k_ts_orth<<<1, TS_ORTH_THREADS, 0, st>>>(Ys, T, Vs);
-                HV_LAUNCH_CHECK();
+                HV_LAUNCH(k_ts_orth, 1, TS_ORTH_THREADS, 0, st, Ys, T, Vs, nullptr);
             }
         }
-        k_ts_matmul<<<gm, mm_threads, 0, st>>>(C32, Vs, T, Ys);
-        HV_LAUNCH_CHECK();
-        k_ts_gram<<<TS_P, TS_GRAM_WARPS * 32, 0, st>>>(Vs, Ys, T, Hm);
-        HV_LAUNCH_CHECK();
-        k_ts_rr<<<1, JS_THREADS, 0, st>>>(Hm, T, scale, evals, Qo);
-        HV_LAUNCH_CHECK();
-        k_ts_ritz<<<(T + TS_P - 1) / TS_P, 256, 0, st>>>(Vs, Qo, T, evecs, Vw);
-        HV_LAUNCH_CHECK();
+        HV_LAUNCH(k_ts_matmul, gm, mm_threads, 0, st, C32, Vs, T, Ys);
+        HV_LAUNCH(k_ts_gram, TS_P, TS_GRAM_WARPS * 32, 0, st, Vs, Ys, T, Hm);
+        HV_LAUNCH(k_ts_rr, 1, JS_THREADS, 0, st, Hm, T, scale, evals, Qo);
+        HV_LAUNCH(k_ts_ritz, (T + TS_P - 1) / TS_P, 256, 0, st, Vs, Qo, T, evecs, Vw);
         count_launch(5 + 2 * iters + extra + (warm ? 0 : 2));
         // two corrections: on 512 x 512 frames with T = 512 and stride 64, one warm iteration and two
         // corrections reach the view error of three and three (3.5e-7 .. 1.9e-6 from FP64)
@@ -2755,7 +2754,7 @@ hv_status pca_eigh(double2* cov, int T, double* evals, double2* evecs, int pmin,
         if (smem > 48 * 1024)
             HV_CUDA_TRY(cudaFuncSetAttribute(k_jacobi_smem<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              static_cast<int>(jacobi_smem_bytes<float>(JS_MAX_T, true))));
-        k_jacobi_smem<float><<<1, JS_THREADS, smem, st>>>(cov, V, T, Tp, ev_unsorted, warm ? 1 : 0, floor_rel);
+        HV_LAUNCH(k_jacobi_smem<float>, 1, JS_THREADS, smem, st, cov, V, T, Tp, ev_unsorted, warm ? 1 : 0, floor_rel);
     }
     else if (T <= JS_MAX_T)
     {
@@ -2763,7 +2762,7 @@ hv_status pca_eigh(double2* cov, int T, double* evals, double2* evecs, int pmin,
         if (smem > 48 * 1024)
             HV_CUDA_TRY(cudaFuncSetAttribute(k_jacobi_smem<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              static_cast<int>(smem)));
-        k_jacobi_smem<double><<<1, JS_THREADS, smem, st>>>(cov, V, T, Tp, ev_unsorted, 0, 0.0f);
+        HV_LAUNCH(k_jacobi_smem<double>, 1, JS_THREADS, smem, st, cov, V, T, Tp, ev_unsorted, 0, 0.0f);
     }
     else if (T <= JC_MAX_T && prec == HV_EIG_FP32)
     {
@@ -2782,7 +2781,7 @@ hv_status pca_eigh(double2* cov, int T, double* evals, double2* evecs, int pmin,
         int* flags = reinterpret_cast<int*>(base + off2);  // three sweep flags (zeroed by the kernel)
         double* fro2 = reinterpret_cast<double*>(base + off2 + 32);
         GridBarrier* bar = reinterpret_cast<GridBarrier*>(base + off2 + 64);
-        HV_CUDA_TRY(cudaMemsetAsync(base + off2, 0, 128, st));
+        HV_LAUNCH_ZERO(base + off2, 128, st);
         HV_CUDA_TRY(cudaFuncSetAttribute(k_jacobi_block, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          static_cast<int>(BJ_SMEM)));
         // co-resident CTAs per SM (the cooperative grid must fit); thread-safe one-time query
@@ -2808,22 +2807,19 @@ hv_status pca_eigh(double2* cov, int T, double* evals, double2* evecs, int pmin,
     }
     if (T <= JS_MAX_T || (T <= JC_MAX_T && prec == HV_EIG_FP32))
     {
-        HV_LAUNCH_CHECK();
         if (loose)
-            k_eig_refine<float><<<T, 128, 0, st>>>(cov, V, T, ev_unsorted);
+            HV_LAUNCH(k_eig_refine<float>, T, 128, 0, st, cov, V, T, ev_unsorted);
         else
-            k_eig_refine<double><<<T, 128, 0, st>>>(cov, V, T, ev_unsorted);
+            HV_LAUNCH(k_eig_refine<double>, T, 128, 0, st, cov, V, T, ev_unsorted);
         count_launch();
     }
     else
     {
-        k_jacobi<<<1, JAC_THREADS, 0, st>>>(cov, V, T, Tp, ev_unsorted, pairs, rot);  // FP64 sweeps, in place
+        HV_LAUNCH(k_jacobi, 1, JAC_THREADS, 0, st, cov, V, T, Tp, ev_unsorted, pairs, rot);  // FP64 sweeps, in place
         if (cov_kept)
             *cov_kept = false;
     }
-    HV_LAUNCH_CHECK();
-    k_eig_sort<<<T, 128, 0, st>>>(ev_unsorted, V, T, evals, evecs, pmin, pmax, weights);
-    HV_LAUNCH_CHECK();
+    HV_LAUNCH(k_eig_sort, T, 128, 0, st, ev_unsorted, V, T, evals, evecs, pmin, pmax, weights);
     count_launch(2);
     // FP32 sweeps: the kept eigenvectors are corrected in FP64 (FP64 sweeps need no correction)
     const bool fp32_sweeps = T <= JS_MAX_T ? prec == HV_EIG_FP32 : (T <= JC_MAX_T && prec == HV_EIG_FP32);
@@ -2843,6 +2839,7 @@ hv_status pca_eigh(double2* cov, int T, double* evals, double2* evecs, int pmin,
 // computed in FP64 from the FP64 eigenvectors (column-major, evecs[j*T + t]); one CTA per bin.
 __global__ void k_ssa_weights(const double2* __restrict__ evecs, int T, int qmin, int qn, int pmin, float2* w)
 {
+    wait_prior_kernels();
     extern __shared__ double2 s_c[];  // qn coefficients of this bin
     const int k = blockIdx.x;
     const long long p = pmin + k;
@@ -2886,8 +2883,7 @@ hv_status ssa_weights(const double2* evecs, int T, int qmin, int qn, int pmin, i
         set_last_error_msg("ssa_weights: more than 3072 eigenvectors kept");
         return HV_ERR_UNSUPPORTED;
     }
-    k_ssa_weights<<<K, 256, static_cast<size_t>(qn) * sizeof(double2), st>>>(evecs, T, qmin, qn, pmin, weights);
-    HV_LAUNCH_CHECK();
+    HV_LAUNCH(k_ssa_weights, K, 256, static_cast<size_t>(qn) * sizeof(double2), st, evecs, T, qmin, qn, pmin, weights);
     count_launch();
     return HV_OK;
 }
@@ -2904,6 +2900,7 @@ __global__ void __launch_bounds__(PI_THREADS) k_phase_increase(const float2* __r
                                                                const float2* __restrict__ w, float2* pred, float* hist,
                                                                int first, int use_hist, float* out, float2* mm)
 {
+    wait_prior_kernels();
     extern __shared__ float2 s_w[];
     __shared__ float s_mn[PI_THREADS / 32], s_mx[PI_THREADS / 32];
     for (int t = threadIdx.x; t < T; t += blockDim.x)
@@ -2967,6 +2964,7 @@ __global__ void __launch_bounds__(PI_THREADS) k_phase_increase(const float2* __r
 __global__ void k_rescale_float(const float* __restrict__ in, size_t HW, const float2* __restrict__ mm, int nmm,
                                 float post_scale, float* __restrict__ out)
 {
+    wait_prior_kernels();
     __shared__ float s_mn, s_mx;
     if (threadIdx.x < 32)
     {
@@ -3016,9 +3014,8 @@ hv_status phase_increase(const float2* ring, int T, size_t HW, const float2* w, 
         set_last_error_msg("phase_increase: time window above 5120 frames");
         return HV_ERR_UNSUPPORTED;
     }
-    k_phase_increase<<<static_cast<unsigned>(grid), PI_THREADS, static_cast<size_t>(T) * sizeof(float2), st>>>(
-        ring, T, HW, w, pred, hist, first, use_hist, out, mm);
-    HV_LAUNCH_CHECK();
+    HV_LAUNCH(k_phase_increase, static_cast<unsigned>(grid), PI_THREADS, static_cast<size_t>(T) * sizeof(float2), st,
+              ring, T, HW, w, pred, hist, first, use_hist, out, mm);
     count_launch();
     return HV_OK;
 }
@@ -3031,8 +3028,7 @@ hv_status rescale_float(const float* in, size_t HW, const float2* mm, float post
     const int nmm = static_cast<int>((prefix + PI_THREADS - 1) / PI_THREADS);
     size_t grid = (HW + 255) / 256;
     grid = grid < 152 * 16 ? grid : 152 * 16;
-    k_rescale_float<<<static_cast<unsigned>(grid), 256, 0, st>>>(in, HW, mm, nmm, post_scale, out);
-    HV_LAUNCH_CHECK();
+    HV_LAUNCH(k_rescale_float, static_cast<unsigned>(grid), 256, 0, st, in, HW, mm, nmm, post_scale, out);
     count_launch();
     return HV_OK;
 }

@@ -81,6 +81,7 @@ struct ViewTcArgs
 template <bool MOM>
 __global__ void __launch_bounds__(V_THREADS, 1) k_view_tc(const __grid_constant__ CUtensorMap ring_map, ViewTcArgs a)
 {
+    wait_prior_kernels();
     if (!ctl_render(a.ctl))
         return;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -362,6 +363,7 @@ __global__ void __launch_bounds__(V_THREADS, 1) k_view_tc(const __grid_constant_
 // rows >= 2K and samples >= T are zero. Split into BF16 hi / lo in the swizzled layout.
 __global__ void k_view_tc_weights(const float2* __restrict__ W, int K, int T, int N, int nchunks, uint8_t* bimg)
 {
+    wait_prior_kernels();
     const int e = blockIdx.x * blockDim.x + threadIdx.x;  // over nchunks * N * 8 chunks of 8 K values
     if (e >= nchunks * N * 8)
         return;
@@ -438,8 +440,7 @@ hv_status view_tc_prepare(const float2* weights, int K, int T, void* work, cudaS
     const int nchunks = (T + V_TC - 1) / V_TC;
     uint8_t* bimg = static_cast<uint8_t*>(work) + 256;  // [0, 256): error flag
     const int total = nchunks * N * 8;
-    k_view_tc_weights<<<(total + 255) / 256, 256, 0, st>>>(weights, K, T, N, nchunks, bimg);
-    HV_LAUNCH_CHECK();
+    HV_LAUNCH(k_view_tc_weights, (total + 255) / 256, 256, 0, st, weights, K, T, N, nchunks, bimg);
     count_launch();
     return HV_OK;
 }
@@ -504,9 +505,8 @@ hv_status view_tc(const float2* ring, int T, int W, int H, int K, int img_type, 
     int grid = a.ntiles < sms ? a.ntiles : sms;
     if (grid < 1)
         grid = 1;
-    HV_CUDA_TRY(cudaMemsetAsync(a.err, 0, sizeof(int), st));
-    kern<<<grid, V_THREADS, smem, st>>>(map, a);
-    HV_LAUNCH_CHECK();
+    HV_LAUNCH_ZERO(a.err, sizeof(int), st);
+    HV_LAUNCH(kern, grid, V_THREADS, smem, st, map, a);
     count_launch();
     return HV_OK;
 }
