@@ -22,6 +22,7 @@
 #include <math.h>
 
 #include <atomic>
+#include <type_traits>
 #include <vector>
 
 #include "hv_common.cuh"
@@ -42,6 +43,77 @@ __device__ __forceinline__ float view_value(float2 X, int img_type)
         return t * t;
     }
     return atan2f(X.y, X.x);
+}
+
+// Position of pixel `pix` after the quadrant swap (even W and H), or itself; 32-bit divisions where
+// the index allows (the 64-bit ones cost a 1024 x 1024 view 1.8 us).
+__device__ __forceinline__ size_t view_target(size_t pix, int W, int H, int shift)
+{
+    if (!shift)
+        return pix;
+    if (pix >> 32)
+        return static_cast<size_t>((static_cast<int>(pix / W) + H / 2) % H) * W + (static_cast<int>(pix % W) + W / 2) % W;
+    const unsigned int p = static_cast<unsigned int>(pix), w = static_cast<unsigned int>(W);
+    const unsigned int y = p / w, x = p - y * w, h = static_cast<unsigned int>(H);
+    const unsigned int ys = y >= h / 2 ? y - h / 2 : y + h / 2, xs = x >= w / 2 ? x - w / 2 : x + w / 2;
+    return static_cast<size_t>(ys) * w + xs;
+}
+
+// Sum of the warp's values a and b (0 where a lane has none) as a double. An FP64 instruction
+// occupies a scheduler's FP64 unit for 64 to 76 clocks per warp here (measured), conversions from FP32
+// included, so the sum is taken in 64-bit integers: each value as a multiple of 2^(emax - 181)
+// (emax: the largest biased exponent in the warp; values within 2^31 of it lose nothing, smaller
+// ones less than 2^-54 of it), summed by three 24-bit limbs, and rounded to a double once. A warp
+// that holds an infinity or a NaN takes the FP64 tree. The partials of a 1024 x 1024 view cost
+// 3.7 us as FP64 shuffle trees.
+__device__ __forceinline__ long long sum_term(float v, int emax)
+{
+    const unsigned int u = __float_as_uint(v);
+    const int e = static_cast<int>((u >> 23) & 255u);
+    const long long m = e ? (u & 0x7fffffu) | 0x800000u : u & 0x7fffffu;
+    const int right = emax - (e ? e : 1);  // 0 .. 253
+    const long long f = right < 56 ? (m << 31) >> right : 0;
+    return (u >> 31) ? -f : f;
+}
+
+__device__ __forceinline__ double warp_sum(float a, float b)
+{
+    const unsigned int full = 0xffffffffu;
+    const unsigned int ua = __float_as_uint(a) & 0x7fffffffu, ub = __float_as_uint(b) & 0x7fffffffu;
+    const int emax = static_cast<int>(__reduce_max_sync(full, ua > ub ? ua : ub) >> 23);
+    if (emax == 255)
+    {
+        double d = static_cast<double>(a) + static_cast<double>(b);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+            d += __shfl_down_sync(full, d, o);
+        return d;  // lane 0
+    }
+    const int em = emax ? emax : 1;
+    const long long s = sum_term(a, em) + sum_term(b, em);
+    const unsigned int l0 = __reduce_add_sync(full, static_cast<unsigned int>(s) & 0xffffffu);
+    const unsigned int l1 = __reduce_add_sync(full, static_cast<unsigned int>(s >> 24) & 0xffffffu);
+    const int l2 = __reduce_add_sync(full, static_cast<int>(s >> 48));
+    const long long t = (static_cast<long long>(l2) << 48) + (static_cast<long long>(l1) << 24) + l0;
+    // t * 2^(em - 181) to the nearest double (ties to even), in integers
+    unsigned long long mag = t < 0 ? static_cast<unsigned long long>(-t) : static_cast<unsigned long long>(t);
+    if (mag == 0)
+        return 0.0;
+    int top = 63 - __clzll(mag);  // t has top + 1 bits
+    if (top > 52)
+    {
+        const int drop = top - 52;
+        const unsigned long long rest = mag & ((1ull << drop) - 1), tie = 1ull << (drop - 1);
+        mag >>= drop;
+        if (rest > tie || (rest == tie && (mag & 1)))
+            ++mag;
+    }
+    else
+        mag <<= 52 - top;
+    // mag: 53 bits (or 2^53 after rounding up, which carries into the exponent)
+    const unsigned long long ex = static_cast<unsigned long long>(top + em - 181 + 1023 - 1);
+    const unsigned long long bits = (ex << 52) + mag;
+    return __longlong_as_double(static_cast<long long>(bits | (t < 0 ? 1ull << 63 : 0ull)));
 }
 
 // ring: [T][HW] complex; weights: [K][T] complex. One pixel per thread; the K bins are done in
@@ -116,19 +188,11 @@ __global__ void __launch_bounds__(TV_THREADS) k_time_view(const float2* __restri
         v = bin_w ? acc_view : acc_view / static_cast<float>(K);
         if (scale != 1.0f)
             v = v * scale;
-        const int x = static_cast<int>(pix % W);
-        const int y = static_cast<int>(pix / W);
-        size_t dst = pix;
-        if (shift)
-            dst = static_cast<size_t>((y + H / 2) % H) * W + (x + W / 2) % W;
-        out[dst] = v;
+        out[view_target(pix, W, H, shift)] = v;
     }
     if (partials)
     {
-        double d = valid ? static_cast<double>(v) : 0.0;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-            d += __shfl_down_sync(0xffffffffu, d, o);
+        const double d = warp_sum(valid ? v : 0.f, 0.f);
         if ((threadIdx.x & 31) == 0)
             red[threadIdx.x >> 5] = d;
         __syncthreads();
@@ -144,7 +208,11 @@ __global__ void __launch_bounds__(TV_THREADS) k_time_view(const float2* __restri
 
 // Two adjacent pixels per thread (16-byte ring loads: 512 contiguous bytes per warp and frame;
 // HW even). 128 threads cover 256 pixels and write the two 128-pixel renormalisation partials of
-// their CTA, the same partials as k_time_view.
+// their CTA, the same partials as k_time_view. Bound by DRAM. One bin (two accumulators per pixel)
+// has little to do between loads: it takes 16 frames per batch of loads and asks for the first
+// frames in L2 before it stages the weights (512 x 512 with the partials: T = 16 8.8 -> 7.9 us, 32 14.4
+// -> 12.8, 64 26.4 -> 23.6, 0.84 of the copy bandwidth); more bins take 8 in a plain unrolled loop (the
+// same batches slow a K = 4, T = 128 view from 44.2 to 50.3 us).
 template <int KC>
 __global__ void __launch_bounds__(TV_THREADS) k_time_view2(const float2* __restrict__ ring, int T, int W, int H,
                                                             const float2* __restrict__ weights, int K, int img_type,
@@ -160,6 +228,14 @@ __global__ void __launch_bounds__(TV_THREADS) k_time_view2(const float2* __restr
     const size_t HW = static_cast<size_t>(W) * H;
     const size_t pix0 = 2 * (blockIdx.x * static_cast<size_t>(TV_THREADS) + threadIdx.x);
     const bool valid = pix0 < HW;
+    // one bin: the first frames are asked for before the weights are staged
+    if constexpr (KC == 1)
+    {
+#pragma unroll
+        for (int f = 0; f < 8; ++f)
+            if (valid && f < T)
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(ring + pix0 + static_cast<size_t>(f) * HW));
+    }
     float view0 = 0.f, view1 = 0.f;
     for (int k0 = 0; k0 < K; k0 += KC)
     {
@@ -179,10 +255,7 @@ __global__ void __launch_bounds__(TV_THREADS) k_time_view2(const float2* __restr
         {
             const float4* src = reinterpret_cast<const float4*>(ring + pix0);
             const size_t step = HW / 2;
-#pragma unroll 8
-            for (int t = 0; t < T; ++t)
-            {
-                const float4 x = __ldg(src + static_cast<size_t>(t) * step);
+            auto accumulate = [&](const float4& x, int t) {
                 const float2* wt = wsm + t * KC;
 #pragma unroll
                 for (int kk = 0; kk < KC; ++kk)
@@ -193,6 +266,36 @@ __global__ void __launch_bounds__(TV_THREADS) k_time_view2(const float2* __restr
                     a1[kk].x = fmaf(x.z, w.x, fmaf(-x.w, w.y, a1[kk].x));
                     a1[kk].y = fmaf(x.z, w.y, fmaf(x.w, w.x, a1[kk].y));
                 }
+            };
+            if constexpr (KC == 1)
+            {
+                int t = 0;
+                // frames t .. t + N - 1: their loads go out together
+                auto frames = [&](auto n) {
+                    constexpr int N = decltype(n)::value;
+                    float4 x[N];
+#pragma unroll
+                    for (int i = 0; i < N; ++i)
+                        x[i] = __ldg(src + static_cast<size_t>(t + i) * step);
+#pragma unroll
+                    for (int i = 0; i < N; ++i)
+                        accumulate(x[i], t + i);
+                    t += N;
+                };
+                while (t + 16 <= T)
+                    frames(std::integral_constant<int, 16>{});
+                while (t + 8 <= T)
+                    frames(std::integral_constant<int, 8>{});
+                while (t + 2 <= T)
+                    frames(std::integral_constant<int, 2>{});
+                if (t < T)
+                    frames(std::integral_constant<int, 1>{});
+            }
+            else
+            {
+#pragma unroll 8
+                for (int t = 0; t < T; ++t)
+                    accumulate(__ldg(src + static_cast<size_t>(t) * step), t);
             }
             const int kn = (K - k0) < KC ? (K - k0) : KC;
 #pragma unroll
@@ -223,24 +326,17 @@ __global__ void __launch_bounds__(TV_THREADS) k_time_view2(const float2* __restr
             v0 = v0 * scale;
             v1 = v1 * scale;
         }
-#pragma unroll
-        for (int q = 0; q < 2; ++q)
+        if (W % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 7) == 0)  // the pair stays together
+            *reinterpret_cast<float2*>(out + view_target(pix0, W, H, shift)) = make_float2(v0, v1);
+        else
         {
-            const size_t pix = pix0 + q;
-            const int x = static_cast<int>(pix % W);
-            const int y = static_cast<int>(pix / W);
-            size_t dst = pix;
-            if (shift)
-                dst = static_cast<size_t>((y + H / 2) % H) * W + (x + W / 2) % W;
-            out[dst] = q ? v1 : v0;
+            out[view_target(pix0, W, H, shift)] = v0;
+            out[view_target(pix0 + 1, W, H, shift)] = v1;
         }
     }
     if (partials)
     {
-        double d = valid ? static_cast<double>(v0) + static_cast<double>(v1) : 0.0;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-            d += __shfl_down_sync(0xffffffffu, d, o);
+        const double d = warp_sum(valid ? v0 : 0.f, valid ? v1 : 0.f);
         if ((threadIdx.x & 31) == 0)
             red[threadIdx.x >> 5] = d;
         __syncthreads();
@@ -418,24 +514,17 @@ __global__ void __launch_bounds__(TV_THREADS, 8) k_time_view_planes(const uint16
             v0 = v0 * scale;
             v1 = v1 * scale;
         }
-#pragma unroll
-        for (int q = 0; q < 2; ++q)
+        if (W % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 7) == 0)  // the pair stays together
+            *reinterpret_cast<float2*>(out + view_target(pix0, W, H, shift)) = make_float2(v0, v1);
+        else
         {
-            const size_t pix = pix0 + q;
-            const int x = static_cast<int>(pix % W);
-            const int y = static_cast<int>(pix / W);
-            size_t dst = pix;
-            if (shift)
-                dst = static_cast<size_t>((y + H / 2) % H) * W + (x + W / 2) % W;
-            out[dst] = q ? v1 : v0;
+            out[view_target(pix0, W, H, shift)] = v0;
+            out[view_target(pix0 + 1, W, H, shift)] = v1;
         }
     }
     if (partials)
     {
-        double d = valid ? static_cast<double>(v0) + static_cast<double>(v1) : 0.0;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-            d += __shfl_down_sync(0xffffffffu, d, o);
+        const double d = warp_sum(valid ? v0 : 0.f, valid ? v1 : 0.f);
         if ((threadIdx.x & 31) == 0)
             red[threadIdx.x >> 5] = d;
         __syncthreads();
