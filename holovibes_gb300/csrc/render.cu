@@ -35,82 +35,178 @@ static int ew_grid(size_t n)
     return static_cast<int>(g < cap ? (g > 0 ? g : 1) : cap);
 }
 
+// V consecutive floats (V = 4: one 16-byte access).
+template <int V>
+__device__ __forceinline__ void load_v(const float* p, float (&v)[V])
+{
+    if constexpr (V == 4)
+    {
+        const float4 f = *reinterpret_cast<const float4*>(p);
+        v[0] = f.x, v[1] = f.y, v[2] = f.z, v[3] = f.w;
+    }
+    else
+        v[0] = *p;
+}
+template <int V>
+__device__ __forceinline__ void store_v(float* p, const float (&v)[V])
+{
+    if constexpr (V == 4)
+        *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+    else
+        *p = v[0];
+}
+
+// 16-byte accesses: every buffer aligned, a multiple of 4 pixels (and, with the quadrant swap, rows
+// whose halves are a multiple of 4).
+static bool vec4_ok(size_t n, std::initializer_list<const void*> buffers)
+{
+    uintptr_t bits = n % 4 ? 1 : 0;
+    for (const void* p : buffers)
+        bits |= reinterpret_cast<uintptr_t>(p) & 15;
+    return bits == 0;
+}
+
 // ====================================================================================== unwrap
 
-// z = exp(i*phase) (kernel_init_unwrap_2d)
-__global__ void k_unwrap_init(const float* in, float2* z, size_t n)
+// The element-wise steps run on V consecutive elements per thread (V = 4: 16-byte accesses). Between
+// the eight FFT passes of one frame they are bound by latency; 32-bit index divisions, and one
+// atomic pair per CTA for the extremes (one per warp held k_unwrap_last at 26 us for 768 x 768).
+
+// V consecutive complex values (V = 1 or 4).
+template <int V>
+__device__ __forceinline__ void load_c(const float2* p, float2 (&v)[V])
+{
+    if constexpr (V == 4)
+    {
+        const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
+        v[0] = make_float2(a.x, a.y), v[1] = make_float2(a.z, a.w);
+        v[2] = make_float2(b.x, b.y), v[3] = make_float2(b.z, b.w);
+    }
+    else
+        v[0] = *p;
+}
+template <int V>
+__device__ __forceinline__ void store_c(float2* p, const float2 (&v)[V])
+{
+    if constexpr (V == 4)
+    {
+        reinterpret_cast<float4*>(p)[0] = make_float4(v[0].x, v[0].y, v[1].x, v[1].y);
+        reinterpret_cast<float4*>(p)[1] = make_float4(v[2].x, v[2].y, v[3].x, v[3].y);
+    }
+    else
+        *p = v[0];
+}
+
+// z = exp(i*phase) (kernel_init_unwrap_2d); the extremes' keys start empty
+template <int V>
+__global__ void k_unwrap_init(const float* in, float2* z, unsigned int n, unsigned int* minmax)
 {
     wait_prior_kernels();
-    for (size_t e = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; e < n;
-         e += static_cast<size_t>(gridDim.x) * blockDim.x)
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+    {
+        minmax[0] = 0xffffffffu;
+        minmax[1] = 0u;
+    }
+    const unsigned int e = (blockIdx.x * blockDim.x + threadIdx.x) * V;
+    if (e >= n)
+        return;
+    float v[V];
+    load_v<V>(in + e, v);
+    float2 o[V];
+#pragma unroll
+    for (int k = 0; k < V; ++k)
     {
         float s, c;
-        sincosf(in[e], &s, &c);
-        z[e] = make_float2(c, s);
+        sincosf(v[k], &s, &c);
+        o[k] = make_float2(c, s);
     }
+    store_c<V>(z + e, o);
 }
 
 // Frequency index of flat element e after circ_shift(-W/2, -H/2) of the fx / fy grids:
 // sfx[y][x] = ((x + W/2) % W) - W/2, sfy[y][x] = ((y + H/2) % H) - H/2.
-__device__ __forceinline__ void shifted_freqs(size_t e, int W, int H, float& fx, float& fy)
+__device__ __forceinline__ void shifted_freqs(unsigned int e, int W, int H, float& fx, float& fy)
 {
-    const int x = static_cast<int>(e % W), y = static_cast<int>(e / W);
+    const int y = static_cast<int>(e / static_cast<unsigned int>(W));
+    const int x = static_cast<int>(e - static_cast<unsigned int>(y) * static_cast<unsigned int>(W));
     fx = static_cast<float>((x + (W >> 1)) % W - (W >> 1));
     fy = static_cast<float>((y + (H >> 1)) % H - (H >> 1));
 }
 
 // gx = Z * sfx, gy = Z * sfy (kernel_multiply_complexes_by_floats_)
+template <int V>
 __global__ void k_unwrap_grad_freq(const float2* Z, float2* gx, float2* gy, int W, int H)
 {
     wait_prior_kernels();
-    const size_t n = static_cast<size_t>(W) * H;
-    for (size_t e = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; e < n;
-         e += static_cast<size_t>(gridDim.x) * blockDim.x)
+    const unsigned int n = static_cast<unsigned int>(W) * H, e = (blockIdx.x * blockDim.x + threadIdx.x) * V;
+    if (e >= n)
+        return;
+    float2 v[V], ox[V], oy[V];
+    load_c<V>(Z + e, v);
+#pragma unroll
+    for (int k = 0; k < V; ++k)
     {
         float fx, fy;
-        shifted_freqs(e, W, H, fx, fy);
-        const float2 v = Z[e];
-        gx[e] = cscale(v, fx);
-        gy[e] = cscale(v, fy);
+        shifted_freqs(e + k, W, H, fx, fy);
+        ox[k] = cscale(v[k], fx);
+        oy[k] = cscale(v[k], fy);
     }
+    store_c<V>(gx + e, ox);
+    store_c<V>(gy + e, oy);
 }
 
 // g *= (i * 2pi) then g *= conj(i z) (kernel_multiply_complexes_by_single_complex, eq_unwrap_2d)
-__global__ void k_unwrap_eq(float2* gx, float2* gy, const float2* z, size_t n, float two_pi)
+template <int V>
+__global__ void k_unwrap_eq(float2* gx, float2* gy, const float2* z, unsigned int n, float two_pi)
 {
     wait_prior_kernels();
     const float2 i2pi = make_float2(0.f, two_pi);
-    for (size_t e = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; e < n;
-         e += static_cast<size_t>(gridDim.x) * blockDim.x)
+    const unsigned int e = (blockIdx.x * blockDim.x + threadIdx.x) * V;
+    if (e >= n)
+        return;
+    float2 vz[V], vx[V], vy[V];
+    load_c<V>(z + e, vz);
+    load_c<V>(gx + e, vx);
+    load_c<V>(gy + e, vy);
+#pragma unroll
+    for (int k = 0; k < V; ++k)
     {
-        const float2 zc = cconj(cmul(z[e], make_float2(0.f, 1.f)));
-        gx[e] = cmul(cmul(gx[e], i2pi), zc);
-        gy[e] = cmul(cmul(gy[e], i2pi), zc);
+        const float2 zc = cconj(cmul(vz[k], make_float2(0.f, 1.f)));
+        vx[k] = cmul(cmul(vx[k], i2pi), zc);
+        vy[k] = cmul(cmul(vy[k], i2pi), zc);
     }
+    store_c<V>(gx + e, vx);
+    store_c<V>(gy + e, vy);
 }
 
 // acc = gx * sfx/(sfx^2+sfy^2) + gy * sfy/(...) (kernel_norm_ratio + kernel_add_complex_frames)
+template <int V>
 __global__ void k_unwrap_ratio(const float2* gx, const float2* gy, float2* acc, int W, int H)
 {
     wait_prior_kernels();
-    const size_t n = static_cast<size_t>(W) * H;
-    for (size_t e = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; e < n;
-         e += static_cast<size_t>(gridDim.x) * blockDim.x)
+    const unsigned int n = static_cast<unsigned int>(W) * H, e = (blockIdx.x * blockDim.x + threadIdx.x) * V;
+    if (e >= n)
+        return;
+    float2 vx[V], vy[V], r[V];
+    load_c<V>(gx + e, vx);
+    load_c<V>(gy + e, vy);
+#pragma unroll
+    for (int k = 0; k < V; ++k)
     {
         float fx, fy;
-        shifted_freqs(e, W, H, fx, fy);
+        shifted_freqs(e + k, W, H, fx, fy);
         const float norm = fx * fx + fy * fy;
-        float2 r = make_float2(0.f, 0.f);
+        r[k] = make_float2(0.f, 0.f);
         if (norm != 0.f)
         {
             const float cx = fx / norm, cy = fy / norm;
-            r = cadd(cscale(gx[e], cx), cscale(gy[e], cy));
+            r[k] = cadd(cscale(vx[k], cx), cscale(vy[k], cy));
         }
-        acc[e] = r;
     }
+    store_c<V>(acc + e, r);
 }
 
-// out = Im(acc) / -2pi (kernel_unwrap2d_last_step), plus FP64-free min/max via ordered keys
+// order-preserving keys of floats
 __device__ __forceinline__ unsigned int float_key(float f)
 {
     const unsigned int u = __float_as_uint(f);
@@ -122,57 +218,74 @@ __device__ __forceinline__ float key_float(unsigned int k)
     return __uint_as_float(u);
 }
 
-__global__ void k_unwrap_last(const float2* acc, float* out, size_t n, float two_pi, unsigned int* minmax)
+// out = Im(acc) / -2pi (kernel_unwrap2d_last_step) and the frame's extremes
+template <int V>
+__global__ void __launch_bounds__(EW_THREADS) k_unwrap_last(const float2* acc, float* out, unsigned int n,
+                                                            float two_pi, unsigned int* minmax)
 {
     wait_prior_kernels();
+    __shared__ unsigned int lo[EW_THREADS / 32], hi[EW_THREADS / 32];
     unsigned int kmin = 0xffffffffu, kmax = 0u;
-    for (size_t e = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; e < n;
-         e += static_cast<size_t>(gridDim.x) * blockDim.x)
+    const unsigned int e = (blockIdx.x * blockDim.x + threadIdx.x) * V;
+    if (e < n)
     {
-        const float v = acc[e].y / -two_pi;
-        out[e] = v;
-        const unsigned int k = float_key(v);
-        kmin = min(kmin, k);
-        kmax = max(kmax, k);
+        float2 a[V];
+        float v[V];
+        load_c<V>(acc + e, a);
+#pragma unroll
+        for (int k = 0; k < V; ++k)
+        {
+            v[k] = a[k].y / -two_pi;
+            const unsigned int key = float_key(v[k]);
+            kmin = min(kmin, key);
+            kmax = max(kmax, key);
+        }
+        store_v<V>(out + e, v);
     }
-    for (int o = 16; o > 0; o >>= 1)
-    {
-        kmin = min(kmin, __shfl_down_sync(0xffffffffu, kmin, o));
-        kmax = max(kmax, __shfl_down_sync(0xffffffffu, kmax, o));
-    }
+    kmin = __reduce_min_sync(0xffffffffu, kmin);
+    kmax = __reduce_max_sync(0xffffffffu, kmax);
     if ((threadIdx.x & 31) == 0)
     {
+        lo[threadIdx.x >> 5] = kmin;
+        hi[threadIdx.x >> 5] = kmax;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0)
+    {
+#pragma unroll
+        for (int w = 1; w < EW_THREADS / 32; ++w)
+        {
+            kmin = min(kmin, lo[w]);
+            kmax = max(kmax, hi[w]);
+        }
         atomicMin(minmax, kmin);
         atomicMax(minmax + 1, kmax);
     }
 }
 
-__global__ void k_init_minmax(unsigned int* minmax)
-{
-    wait_prior_kernels();
-    minmax[0] = 0xffffffffu;
-    minmax[1] = 0u;
-}
-
 // rescale_float_unwrap2d: (in + |min|)/(|min| + max)*65535 if min < 0 else (in - min)/(max - min)*65535
-__global__ void k_unwrap_rescale(float* io, size_t n, const unsigned int* minmax)
+template <int V>
+__global__ void k_unwrap_rescale(float* io, unsigned int n, const unsigned int* minmax)
 {
     wait_prior_kernels();
     const float mn = key_float(minmax[0]), mx = key_float(minmax[1]);
-    for (size_t e = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; e < n;
-         e += static_cast<size_t>(gridDim.x) * blockDim.x)
+    const unsigned int e = (blockIdx.x * blockDim.x + threadIdx.x) * V;
+    if (e >= n)
+        return;
+    float v[V];
+    load_v<V>(io + e, v);
+#pragma unroll
+    for (int k = 0; k < V; ++k)
     {
-        const float in = io[e];
-        float r;
         // a constant frame maps to 0 (the reference divides 0 by 0 there)
         if (mx == mn)
-            r = 0.0f;
+            v[k] = 0.0f;
         else if (mn < 0.f)
-            r = __fdiv_rn(__fadd_rn(in, fabsf(mn)), __fadd_rn(fabsf(mn), mx)) * 65535.0f;
+            v[k] = __fdiv_rn(__fadd_rn(v[k], fabsf(mn)), __fadd_rn(fabsf(mn), mx)) * 65535.0f;
         else
-            r = __fdiv_rn(__fsub_rn(in, mn), __fsub_rn(mx, mn)) * 65535.0f;
-        io[e] = r;
+            v[k] = __fdiv_rn(__fsub_rn(v[k], mn), __fsub_rn(mx, mn)) * 65535.0f;
     }
+    store_v<V>(io + e, v);
 }
 
 size_t unwrap_workspace(int W, int H)
@@ -181,43 +294,50 @@ size_t unwrap_workspace(int W, int H)
     return 4 * n * sizeof(float2) + 256;
 }
 
-hv_status unwrap_2d(const float* in, float* out, int W, int H, void* work, cudaStream_t st)
+template <int V>
+static hv_status unwrap_steps(const float* in, float* out, int W, int H, void* work, cudaStream_t st)
 {
-    const size_t n = static_cast<size_t>(W) * H;
+    const unsigned int n = static_cast<unsigned int>(W) * H;
     // The reference plans its unwrap FFT with plan(width, height) (icompute.hh:140): the
     // row-major buffer is transformed as `width` rows of `height` samples.
     const int n0 = W, n1 = H;
-    if (!fft_size_supported(n0) || !fft_size_supported(n1))
-    {
-        set_last_error_msg("unwrap_2d: frame size not supported by the shared-memory FFT");
-        return HV_ERR_UNSUPPORTED;
-    }
     float2* z = static_cast<float2*>(work);
     float2* g = z + n;  // gx, gy contiguous (batch of 2)
     float2* gx = g;
     float2* gy = g + n;
-    float2* Z = g + 2 * n;
+    float2* Z = g + 2 * static_cast<size_t>(n);
     unsigned int* minmax = reinterpret_cast<unsigned int*>(Z + n);
     const float two_pi = 6.28318530717959f;  // M_2PI of common.cuh:29
-    const int grid = ew_grid(n);
-    HV_LAUNCH(k_unwrap_init, grid, EW_THREADS, 0, st, in, z, n);
-    hv_status s = fft2d(z, Z, n0, n1, 1, 0, 1.0f, st);
-    if (s != HV_OK)
+    const int grid = static_cast<int>((n / V + EW_THREADS - 1) / EW_THREADS);
+    hv_status s;
+    HV_LAUNCH(k_unwrap_init<V>, grid, EW_THREADS, 0, st, in, z, n, minmax);
+    if ((s = fft2d(z, Z, n0, n1, 1, 0, 1.0f, st)) != HV_OK)
         return s;
-    HV_LAUNCH(k_unwrap_grad_freq, grid, EW_THREADS, 0, st, Z, gx, gy, W, H);
+    HV_LAUNCH(k_unwrap_grad_freq<V>, grid, EW_THREADS, 0, st, Z, gx, gy, W, H);
     if ((s = fft2d(g, g, n0, n1, 2, 1, 1.0f, st)) != HV_OK)
         return s;
-    HV_LAUNCH(k_unwrap_eq, grid, EW_THREADS, 0, st, gx, gy, z, n, two_pi);
+    HV_LAUNCH(k_unwrap_eq<V>, grid, EW_THREADS, 0, st, gx, gy, z, n, two_pi);
     if ((s = fft2d(g, g, n0, n1, 2, 0, 1.0f, st)) != HV_OK)
         return s;
-    HV_LAUNCH(k_unwrap_ratio, grid, EW_THREADS, 0, st, gx, gy, Z, W, H);
+    HV_LAUNCH(k_unwrap_ratio<V>, grid, EW_THREADS, 0, st, gx, gy, Z, W, H);
     if ((s = fft2d(Z, Z, n0, n1, 1, 1, 1.0f, st)) != HV_OK)
         return s;
-    HV_LAUNCH(k_init_minmax, 1, 1, 0, st, minmax);
-    HV_LAUNCH(k_unwrap_last, grid, EW_THREADS, 0, st, Z, out, n, two_pi, minmax);
-    HV_LAUNCH(k_unwrap_rescale, grid, EW_THREADS, 0, st, out, n, minmax);
-    count_launch(7);
+    HV_LAUNCH(k_unwrap_last<V>, grid, EW_THREADS, 0, st, Z, out, n, two_pi, minmax);
+    HV_LAUNCH(k_unwrap_rescale<V>, grid, EW_THREADS, 0, st, out, n, minmax);
+    count_launch(6);
     return HV_OK;
+}
+
+hv_status unwrap_2d(const float* in, float* out, int W, int H, void* work, cudaStream_t st)
+{
+    if (!fft_size_supported(W) || !fft_size_supported(H))
+    {
+        set_last_error_msg("unwrap_2d: frame size not supported by the shared-memory FFT");
+        return HV_ERR_UNSUPPORTED;
+    }
+    // transform lengths are multiples of 16, so only the buffers' alignment decides
+    return vec4_ok(static_cast<size_t>(W) * H, {in, out, work}) ? unwrap_steps<4>(in, out, W, H, work, st)
+                                                                : unwrap_steps<1>(in, out, W, H, work, st);
 }
 
 // ---------------------------------------------------------------------- unwrap without allocation
@@ -383,27 +503,6 @@ __device__ __forceinline__ void renorm_factors(const RenormSum& r, float& f0, fl
     f1 = f[1];
 }
 
-// V consecutive floats (V = 4: one 16-byte access).
-template <int V>
-__device__ __forceinline__ void load_v(const float* p, float (&v)[V])
-{
-    if constexpr (V == 4)
-    {
-        const float4 f = *reinterpret_cast<const float4*>(p);
-        v[0] = f.x, v[1] = f.y, v[2] = f.z, v[3] = f.w;
-    }
-    else
-        v[0] = *p;
-}
-template <int V>
-__device__ __forceinline__ void store_v(float* p, const float (&v)[V])
-{
-    if constexpr (V == 4)
-        *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
-    else
-        *p = v[0];
-}
-
 // Fused: renormalise (sum.partials null: not), optional quadrant swap (out of place), optional
 // accumulation into an A-frame ring (write slot, mean of `count` frames from `start`), optional
 // log10. V pixels per thread and step. Bound by latency (a few MB from L2): the factors without a
@@ -495,16 +594,6 @@ __global__ void __launch_bounds__(RN_THREADS) k_renorm_shift_acc(const float* in
         }
         store_v<V>(out + e, v);
     }
-}
-
-// 16-byte accesses: every buffer aligned, a multiple of 4 pixels (and, with the quadrant swap, rows
-// whose halves are a multiple of 4).
-static bool vec4_ok(size_t n, std::initializer_list<const void*> buffers)
-{
-    uintptr_t bits = n % 4 ? 1 : 0;
-    for (const void* p : buffers)
-        bits |= reinterpret_cast<uintptr_t>(p) & 15;
-    return bits == 0;
 }
 
 static hv_status launch_renorm_shift_acc(const float* in, float* out, int W, int H, const RenormSum& sum, int shift,

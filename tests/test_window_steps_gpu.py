@@ -149,3 +149,19 @@ def test_contrast_and_log_maps(cuda, n, off):
     ref = np.log10(y.astype(np.float64))
     # log10f: 2 ulp of the result, or of 1 near log10(1) = 0
     assert np.all(np.abs(host(yd, np.float32, (n,)) - ref) <= 2.0 ** -22 * np.maximum(np.abs(ref), 0.1))
+
+
+@pytest.mark.parametrize("W,H", [(16, 16), (48, 64), (512, 16), (768, 64)])
+def test_unwrap_alignment(cuda, W, H):
+    """Buffers off 16-byte alignment take the element-wise steps one value at a time: the same bits."""
+    rng = np.random.default_rng(W)
+    phase = rng.uniform(-np.pi, np.pi, (H, W)).astype(np.float32)
+    n = W * H
+    nw = hv.lib().hv_unwrap_workspace(W, H)
+    got = []
+    for off in (0, 1):
+        out, work = zeros(n * 4 + 4), zeros(nw + 8)
+        call("hv_unwrap_2d", _offset(phase, off), ptr(out) + 4 * off, W, H, ptr(work) + 8 * off, None)
+        got.append(host(out, np.float32, (n + off,))[off:])
+    assert np.all(np.isfinite(got[0]))
+    assert np.array_equal(got[0], got[1])
