@@ -1122,6 +1122,7 @@ __global__ void __launch_bounds__(JAC_THREADS) k_jacobi(double2* A, double2* V, 
 // identities are skipped and the sweeps stop after a sweep without rotation. The skip threshold is
 // a few units of the working precision relative to sqrt(|a_pp a_qq|).
 constexpr int JS_THREADS = 256;
+constexpr int JS_WIDE = 1024, JS_MID = 512;  // one-CTA FP32 sweeps of T > 32 and T <= 32: a warp per pair
 constexpr int JS_MAX_T = 64;
 
 template <class R>
@@ -1371,6 +1372,197 @@ __device__ bool smem_sweeps(Cx<R>* A, Cx<R>* V, int T_, int Tp_, int LD_, JacScr
     return any;
 }
 
+// The same sweeps (round-robin order, whole sweeps) for the one-CTA eigensolvers in FP32, bit for
+// bit, arranged for the latency and the issue slots of a step (on the way to convergence only some
+// pairs rotate: 11 of 32 on average at T = 64, and a third of the steps have none):
+//   * A <- J^H A J: one warp per rotating pair, a lane per other pair (a block of two rotating pairs
+//     belongs to the larger index);
+//   * then warp 0 computes the next step's rotations, which need only A, while the other warps apply
+//     the current ones to V, 32 rows of one rotating pair per warp;
+//   * after a step without rotations the warps look ahead, one step each, to the next that has any.
+// A holds Tp x Tp entries (Tp even; row and column T of an odd matrix are 0 and stay so: nothing
+// rotates them), with the odd leading dimension LD.
+// One CTA of 256 threads took 2 x 2 blocks and V rows in turn, phase after phase: k_jacobi_smem of a 512 x
+// 512, T = 64 ring 531 -> 245 us (212 steps with rotations of about 1 us each, bound by the latency of
+// the block update and of the rotation's square roots and division), the warm T = 32 one of 1024 x
+// 1024 frames 91 -> 65 us (cold caches). Not kept: V's rows in registers, moved from lane to lane
+// with the pairing (589 against 504 us for the whole eigensolve at T = 64: every row pays every step).
+struct JacScratchWarps
+{
+    JacRot<float> rot[32][JS_MAX_T / 2];     // slot: a step looked at
+    unsigned int mask[32];                   // its rotating pairs
+    unsigned char list[32][JS_MAX_T / 2];    // and their indices
+};
+
+template <int NT, int LD, int N = 0>
+__device__ void smem_sweeps_warps(Cx<float>* A, Cx<float>* V, int T_, int Tp_, JacScratchWarps& sc, float floor,
+                                  int max_sweeps)
+{
+    constexpr int NW = NT / 32;
+    const int T = N > 0 ? N : T_, Tp = N > 0 ? N : Tp_;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int h = Tp / 2, n1 = Tp - 1;
+    const int row_blocks = (T + 31) / 32;
+    const float thr = jac_threshold<float>();
+    // sweep_pair without its divisions (step < n1, k < h)
+    auto pair_of = [&](int step, int k, int& p, int& q) {
+        int a = step + k, b = step - k;
+        a = k == 0 ? n1 : (a >= n1 ? a - n1 : a);
+        b = b < 0 ? b + n1 : b;
+        p = min(a, b);
+        q = max(a, b);
+    };
+    // rotations of a step into a slot (a whole warp)
+    auto look_at = [&](int step, int slot) {
+        bool active = false;
+        JacRot<float> r = {1, 0, 1, 0};
+        if (lane < h)
+        {
+            int p, q;
+            pair_of(step, lane, p, q);
+            active = jac_rotation(A[p * LD + q], A[p * LD + p].x, A[q * LD + q].x, thr, floor, r);
+            sc.rot[slot][lane] = r;
+        }
+        const unsigned int m = __ballot_sync(0xffffffffu, active);
+        if (active)
+            sc.list[slot][__popc(m & ((1u << lane) - 1u))] = static_cast<unsigned char>(lane);
+        if (lane == 0)
+            sc.mask[slot] = m;
+    };
+    if (warp == 0)
+        look_at(0, 0);
+    __syncthreads();
+    int sweep = 0, step = 0;   // slots base .. base + count - 1 hold steps step .. step + count - 1
+    int base = 0, count = 1;
+    bool sweep_active = false;
+    for (;;)
+    {
+        int first = 0;
+        unsigned int mask = sc.mask[base];
+        if (count > 1)
+        {
+            const unsigned int mine = lane < count ? sc.mask[base + lane] : 0u;
+            const unsigned int some = __ballot_sync(0xffffffffu, mine != 0u);
+            first = some ? __ffs(some) - 1 : 0;
+            mask = __shfl_sync(0xffffffffu, mine, first);
+        }
+        if (!mask)
+        {
+            step += count;
+            if (step == n1)
+            {
+                if (!sweep_active || ++sweep >= max_sweeps)
+                    break;
+                sweep_active = false;
+                step = 0;
+            }
+            __syncthreads();  // every warp has read the masks
+            base = 0;
+            count = min(NW, n1 - step);
+            if (warp < count)
+                look_at(step + warp, warp);
+            __syncthreads();
+            continue;
+        }
+        const int slot = base + first;
+        const int nact = __popc(mask);
+        step += first;
+        sweep_active = true;
+        for (int i = warp; i < nact; i += NW)
+        {
+            const int ka = sc.list[slot][i], kb = lane;
+            if (kb >= h || (kb > ka && ((mask >> kb) & 1u)))
+                continue;
+            const int k1 = max(ka, kb), k2 = min(ka, kb);
+            int r0, r1, c0, c1;
+            pair_of(step, k1, r0, r1);
+            pair_of(step, k2, c0, c1);
+            const Cx<float> z = {0, 0};
+            Cx<float> B[2][2];
+            B[0][0] = A[r0 * LD + c0];
+            B[0][1] = A[r0 * LD + c1];
+            B[1][0] = A[r1 * LD + c0];
+            B[1][1] = A[r1 * LD + c1];
+            // X = B J2, J2 = [[c, s], [-s e^{-i phi}, c e^{-i phi}]]
+            const JacRot<float> J1 = sc.rot[slot][k1], J2 = sc.rot[slot][k2];
+            const float cr2 = J2.c, s2 = J2.s;
+            const Cx<float> em2 = {J2.cph, -J2.sph};
+            Cx<float> X[2][2];
+#pragma unroll
+            for (int r = 0; r < 2; ++r)
+            {
+                const Cx<float> y1 = cxmul(B[r][1], em2);
+                X[r][0] = {cr2 * B[r][0].x - s2 * y1.x, cr2 * B[r][0].y - s2 * y1.y};
+                X[r][1] = {s2 * B[r][0].x + cr2 * y1.x, s2 * B[r][0].y + cr2 * y1.y};
+            }
+            // Y = J1^H X: row0 = c X0 - s e^{i phi} X1, row1 = s X0 + c e^{i phi} X1
+            const float cr1 = J1.c, s1 = J1.s;
+            const Cx<float> ep1 = {J1.cph, J1.sph};
+            Cx<float> Y[2][2];
+#pragma unroll
+            for (int cc = 0; cc < 2; ++cc)
+            {
+                const Cx<float> x1 = cxmul(X[1][cc], ep1);
+                Y[0][cc] = {cr1 * X[0][cc].x - s1 * x1.x, cr1 * X[0][cc].y - s1 * x1.y};
+                Y[1][cc] = {s1 * X[0][cc].x + cr1 * x1.x, s1 * X[0][cc].y + cr1 * x1.y};
+            }
+            if (k1 == k2)
+            {
+                Y[0][1] = z;
+                Y[1][0] = z;
+                Y[0][0].y = 0;
+                Y[1][1].y = 0;
+            }
+            A[r0 * LD + c0] = Y[0][0];
+            A[r0 * LD + c1] = Y[0][1];
+            A[r1 * LD + c0] = Y[1][0];
+            A[r1 * LD + c1] = Y[1][1];
+            if (k1 != k2)
+            {
+                A[c0 * LD + r0] = {Y[0][0].x, -Y[0][0].y};
+                A[c1 * LD + r0] = {Y[0][1].x, -Y[0][1].y};
+                A[c0 * LD + r1] = {Y[1][0].x, -Y[1][0].y};
+                A[c1 * LD + r1] = {Y[1][1].x, -Y[1][1].y};
+            }
+        }
+        __syncthreads();
+        const bool wrap = step + 1 == n1;
+        const int next_slot = slot == 0 ? 1 : 0;
+        if (warp == 0)
+            look_at(wrap ? 0 : step + 1, next_slot);
+        else
+        {
+            // V <- V J for the rotating pairs
+            for (int i = warp - 1; i < nact * row_blocks; i += NW - 1)
+            {
+                const int j = row_blocks == 1 ? i : i >> 1, r = (row_blocks == 1 ? 0 : (i & 1) * 32) + lane;
+                if (r >= T)
+                    continue;
+                const int k = sc.list[slot][j];
+                int p, q;
+                pair_of(step, k, p, q);
+                const JacRot<float> J = sc.rot[slot][k];
+                const float c = J.c, s = J.s;
+                const Cx<float> em = {J.cph, -J.sph};
+                const Cx<float> vp = V[r * LD + p], vq = cxmul(V[r * LD + q], em);
+                V[r * LD + p] = {c * vp.x - s * vq.x, c * vp.y - s * vq.y};
+                V[r * LD + q] = {s * vp.x + c * vq.x, s * vp.y + c * vq.y};
+            }
+        }
+        __syncthreads();
+        base = next_slot;
+        count = 1;
+        step = wrap ? 0 : step + 1;
+        if (wrap)
+        {
+            if (++sweep >= max_sweeps)
+                break;
+            sweep_active = false;
+        }
+    }
+    __syncthreads();
+}
+
 // C = op(X) Y for T x T shared-memory matrices (leading dimension LD), op(X) = X or X^H; every
 // thread of the block takes output elements in turn.
 template <class R, int NT>
@@ -1393,11 +1585,45 @@ __device__ void smem_cgemm(const Cx<R>* X, const Cx<R>* Y, Cx<R>* C, int T, int 
     }
 }
 
+// Leading dimension of k_jacobi_smem's matrices: odd (no bank conflicts along rows or columns) and, in
+// FP32, fixed for T <= 32 and above.
+template <class R>
+constexpr int jacobi_ld(int T)
+{
+    return sizeof(R) == sizeof(float) ? (T > 32 ? JS_MAX_T + 1 : 33) : T | 1;
+}
+
 // Shared-memory bytes of k_jacobi_smem: A and V, plus two work matrices for a warm start.
 template <class R>
 size_t jacobi_smem_bytes(int T, bool warm)
 {
-    return (warm ? 4 : 2) * static_cast<size_t>(T) * (T + 1) * sizeof(Cx<R>);
+    return (warm ? 4 : 2) * static_cast<size_t>(T + (T & 1)) * jacobi_ld<R>(T) * sizeof(Cx<R>);
+}
+
+// FP64 instructions, conversions included, take 64 clocks of a scheduler here: a one-CTA kernel
+// converts its matrices in integers instead.
+// a * 2^k as a float, rounded to nearest (ties to even).
+__device__ __forceinline__ float scaled_float(double a, int k)
+{
+    const unsigned long long u = static_cast<unsigned long long>(__double_as_longlong(a));
+    const int ex = static_cast<int>((u >> 52) & 2047u), e = ex - 1023 + 127 + k;
+    if ((u << 1) == 0)
+        return __uint_as_float(static_cast<unsigned int>(u >> 32));  // +-0
+    if (ex == 0 || ex == 2047 || e < 1 || e > 253)
+        return static_cast<float>(scalbn(a, k));
+    const unsigned int m = static_cast<unsigned int>(u >> 29) & 0x7fffffu, rest = static_cast<unsigned int>(u) & 0x1fffffffu;
+    const unsigned int up = rest > 0x10000000u || (rest == 0x10000000u && (m & 1u)) ? 1u : 0u;
+    return __uint_as_float((static_cast<unsigned int>(u >> 32) & 0x80000000u) | ((static_cast<unsigned int>(e) << 23) + m + up));
+}
+
+// The float as a double.
+__device__ __forceinline__ double widened(float f)
+{
+    const unsigned int u = __float_as_uint(f), ex = (u >> 23) & 255u;
+    if (ex == 255u || (ex == 0u && (u << 1) != 0u))
+        return static_cast<double>(f);
+    const unsigned long long mag = ex ? (static_cast<unsigned long long>(u & 0x7fffffffu) << 29) + (896ull << 52) : 0ull;
+    return __longlong_as_double(static_cast<long long>((static_cast<unsigned long long>(u & 0x80000000u) << 32) | mag));
 }
 
 // `warm` (FP32 only): Vout holds the orthonormal eigenvector basis of the previous call on this
@@ -1405,20 +1631,21 @@ size_t jacobi_smem_bytes(int T, bool warm)
 // is nearly diagonal when consecutive windows share their temporal modes, so one or two sweeps
 // finish it. V0 is first re-orthonormalised by one Newton-Schulz step V0 (3 I - V0^H V0) / 2, so
 // rounding does not accumulate from window to window.
-template <class R>
-__global__ void __launch_bounds__(JS_THREADS) k_jacobi_smem(const double2* __restrict__ Ain, double2* __restrict__ Vout,
+template <class R, int NT>
+__global__ void __launch_bounds__(NT) k_jacobi_smem(const double2* __restrict__ Ain, double2* __restrict__ Vout,
                                                             int T, int Tp, double* __restrict__ evals, int warm,
                                                             float floor_rel)
 {
     wait_prior_kernels();
     extern __shared__ __align__(16) unsigned char js_raw[];
     Cx<R>* js = reinterpret_cast<Cx<R>*>(js_raw);
-    const int LD = T + 1;
+    // FP32: the instance of NT threads serves one leading dimension
+    const int LD = sizeof(R) == sizeof(float) ? (NT == JS_WIDE ? JS_MAX_T + 1 : 33) : T | 1;
     Cx<R>* A = js;
-    Cx<R>* V = js + T * LD;
-    Cx<R>* X = V + T * LD;  // warm start only
-    Cx<R>* N = X + T * LD;
-    __shared__ JacScratch<R> sc;
+    Cx<R>* V = js + Tp * LD;
+    Cx<R>* X = V + Tp * LD;  // warm start only
+    Cx<R>* N = X + Tp * LD;
+    __shared__ std::conditional_t<sizeof(R) == sizeof(float), JacScratchWarps, JacScratch<R>> sc;
     __shared__ double s_scale;
     const int tid = threadIdx.x;
     if (tid < 32)
@@ -1432,17 +1659,28 @@ __global__ void __launch_bounds__(JS_THREADS) k_jacobi_smem(const double2* __res
             s_scale = jac_scale(m);
     }
     __syncthreads();
+    // the row and column that make Tp even
+    if (T < Tp)
+        for (int e = tid; e < Tp; e += NT)
+            A[T * LD + e] = A[e * LD + T] = {0, 0};
     // the sweeps run on 2^-e A (exact scaling): the squares of the entries stay finite in FP32
     const double scale = s_scale;
-    for (int e = tid; e < T * T; e += JS_THREADS)
+    const int scale_k = static_cast<int>((static_cast<unsigned long long>(__double_as_longlong(scale)) >> 52) & 2047u) - 1023;
+    for (int e = tid; e < T * T; e += NT)
     {
         const int i = e / T, j = e % T;
         const double2 a = Ain[e];
-        A[i * LD + j] = {static_cast<R>(a.x * scale), static_cast<R>(i == j ? 0.0 : a.y * scale)};
+        if constexpr (sizeof(R) == sizeof(float))
+            A[i * LD + j] = {scaled_float(a.x, scale_k), i == j ? 0.0f : scaled_float(a.y, scale_k)};
+        else
+            A[i * LD + j] = {a.x * scale, i == j ? 0.0 : a.y * scale};
         if (warm)
         {
             const double2 v = Vout[e];
-            N[i * LD + j] = {static_cast<R>(v.x), static_cast<R>(v.y)};
+            if constexpr (sizeof(R) == sizeof(float))
+                N[i * LD + j] = {scaled_float(v.x, 0), scaled_float(v.y, 0)};
+            else
+                N[i * LD + j] = {v.x, v.y};
         }
         else
             V[i * LD + j] = {static_cast<R>(i == j ? 1 : 0), static_cast<R>(0)};
@@ -1451,22 +1689,22 @@ __global__ void __launch_bounds__(JS_THREADS) k_jacobi_smem(const double2* __res
     if (warm)
     {
         // V = V0 (3 I - V0^H V0) / 2 (V0 in N), then A <- V^H A V
-        smem_cgemm<R, JS_THREADS>(N, N, X, T, LD, true);
+        smem_cgemm<R, NT>(N, N, X, T, LD, true);
         __syncthreads();
-        for (int e = tid; e < T * T; e += JS_THREADS)
+        for (int e = tid; e < T * T; e += NT)
         {
             const int i = e / T, j = e % T;
             const Cx<R> x = X[i * LD + j];
             X[i * LD + j] = {R(-0.5) * x.x + (i == j ? R(1.5) : R(0)), R(-0.5) * x.y};
         }
         __syncthreads();
-        smem_cgemm<R, JS_THREADS>(N, X, V, T, LD, false);
+        smem_cgemm<R, NT>(N, X, V, T, LD, false);
         __syncthreads();
-        smem_cgemm<R, JS_THREADS>(A, V, X, T, LD, false);
+        smem_cgemm<R, NT>(A, V, X, T, LD, false);
         __syncthreads();
-        smem_cgemm<R, JS_THREADS>(V, X, N, T, LD, true);
+        smem_cgemm<R, NT>(V, X, N, T, LD, true);
         __syncthreads();
-        for (int e = tid; e < T * T; e += JS_THREADS)
+        for (int e = tid; e < T * T; e += NT)
         {
             const int i = e / T, j = e % T;
             const Cx<R> a = N[i * LD + j], b = N[j * LD + i];
@@ -1478,35 +1716,62 @@ __global__ void __launch_bounds__(JS_THREADS) k_jacobi_smem(const double2* __res
     // the round-off level of the FP32 updates, below which they keep regenerating off-diagonal
     // entries of the small eigenvalues and the sweeps would run to their limit; 2e-5 when only the
     // kept eigenvectors are used, which are refined in FP64 afterwards).
-    __shared__ double s_fro[JS_THREADS / 32];
     R floor = R(0);
     if constexpr (sizeof(R) == sizeof(float))
     {
-        double f2 = 0.0;
-        for (int e = tid; e < T * T; e += JS_THREADS)
+        // the squares' sum in pairs of floats (hi + lo, 46 bits or more)
+        __shared__ float s_hi[NT / 32], s_lo[NT / 32];
+        float hi = 0.f, lo = 0.f;
+        auto add = [&](float x) {
+            const float s = hi + x, bb = s - hi;
+            lo += (hi - (s - bb)) + (x - bb);
+            hi = s;
+        };
+        for (int e = tid; e < T * T; e += NT)
         {
             const Cx<R> a = A[(e / T) * LD + e % T];
-            f2 += static_cast<double>(a.x) * a.x + static_cast<double>(a.y) * a.y;
+            const float px = __fmul_rn(a.x, a.x), py = __fmul_rn(a.y, a.y);
+            lo += __fmaf_rn(a.x, a.x, -px) + __fmaf_rn(a.y, a.y, -py);
+            add(px);
+            add(py);
         }
         for (int o = 16; o > 0; o >>= 1)
-            f2 += __shfl_xor_sync(0xffffffffu, f2, o);
+        {
+            const float oh = __shfl_xor_sync(0xffffffffu, hi, o), ol = __shfl_xor_sync(0xffffffffu, lo, o);
+            add(oh);
+            lo += ol;
+        }
         if ((tid & 31) == 0)
-            s_fro[tid >> 5] = f2;
+        {
+            s_hi[tid >> 5] = hi;
+            s_lo[tid >> 5] = lo;
+        }
         __syncthreads();
-        double t2 = 0.0;
-        for (int w = 0; w < JS_THREADS / 32; ++w)
-            t2 += s_fro[w];
-        floor = static_cast<R>(static_cast<double>(floor_rel) * sqrt(t2));
+        if (tid == 0)
+        {
+            double t2 = 0.0;
+            for (int w = 0; w < NT / 32; ++w)
+                t2 += static_cast<double>(s_hi[w]) + static_cast<double>(s_lo[w]);
+            s_hi[0] = static_cast<float>(static_cast<double>(floor_rel) * sqrt(t2));
+        }
+        __syncthreads();
+        floor = s_hi[0];
     }
-    smem_sweeps<R, JS_THREADS>(A, V, T, Tp, LD, sc, floor, JAC_MAX_SWEEPS);
+    if constexpr (sizeof(R) == sizeof(float))
+        smem_sweeps_warps<NT, NT == JS_WIDE ? JS_MAX_T + 1 : 33>(A, V, T, Tp, sc, floor, JAC_MAX_SWEEPS);
+    else
+        smem_sweeps<R, NT>(A, V, T, Tp, LD, sc, floor, JAC_MAX_SWEEPS);
     __syncthreads();
-    for (int e = tid; e < T * T; e += JS_THREADS)
+    for (int e = tid; e < T * T; e += NT)
     {
         const int i = e / T, j = e % T;
-        Vout[e] = make_double2(static_cast<double>(V[i * LD + j].x), static_cast<double>(V[i * LD + j].y));
+        if constexpr (sizeof(R) == sizeof(float))
+            Vout[e] = make_double2(widened(V[i * LD + j].x), widened(V[i * LD + j].y));
+        else
+            Vout[e] = make_double2(V[i * LD + j].x, V[i * LD + j].y);
     }
-    for (int i = tid; i < T; i += JS_THREADS)
-        evals[i] = static_cast<double>(A[i * LD + i].x) / scale;
+    for (int i = tid; i < T; i += NT)
+        evals[i] = scalbn(static_cast<double>(A[i * LD + i].x), -scale_k);
 }
 
 // Grid-wide kernels (64 < T <= JC_MAX_T) synchronise through a bounded sense-reversal barrier: a
@@ -2607,20 +2872,20 @@ __global__ void __launch_bounds__(TS_GRAM_WARPS * 32) k_ts_gram(const float2* __
 // k_ts_rr: H Q = Q diag(theta) by FP32 Jacobi on the Hermitian part of H (one CTA); the Ritz values
 // (scaled back) into evals[T - TS_P ..] in ascending order, evals below set to 0, and Qo = the columns
 // of Q in that order.
-__global__ void __launch_bounds__(JS_THREADS) k_ts_rr(const float2* __restrict__ H, int T,
+__global__ void __launch_bounds__(JS_MID) k_ts_rr(const float2* __restrict__ H, int T,
                                                      const double* __restrict__ scale, double* __restrict__ evals,
                                                      float2* __restrict__ Qo)
 {
     wait_prior_kernels();
-    constexpr int NW = JS_THREADS / 32;
+    constexpr int NW = JS_MID / 32;
     __shared__ Cx<float> Hs[TS_P * TS_LD], Qs[TS_P * TS_LD];
-    __shared__ JacScratch<float> sc;
+    __shared__ JacScratchWarps sc;
     __shared__ int order[TS_P];
     __shared__ float s_fro[NW];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     // Hermitian part, real diagonal; round-off floor as in the other FP32 sweeps
     float f2 = 0.f;
-    for (int e = tid; e < TS_P * TS_P; e += JS_THREADS)
+    for (int e = tid; e < TS_P * TS_P; e += JS_MID)
     {
         const int i = e / TS_P, k = e % TS_P;
         const float2 a = H[i * TS_P + k], b = H[k * TS_P + i];
@@ -2637,7 +2902,7 @@ __global__ void __launch_bounds__(JS_THREADS) k_ts_rr(const float2* __restrict__
     float tot = 0.f;
     for (int w = 0; w < NW; ++w)
         tot += s_fro[w];
-    smem_sweeps<float, JS_THREADS>(Hs, Qs, TS_P, TS_P, TS_LD, sc, 5e-7f * sqrtf(tot), JAC_MAX_SWEEPS);
+    smem_sweeps_warps<JS_MID, TS_LD, TS_P>(Hs, Qs, TS_P, TS_P, sc, 5e-7f * sqrtf(tot), JAC_MAX_SWEEPS);
     __syncthreads();
     if (tid < TS_P)
     {
@@ -2651,10 +2916,10 @@ __global__ void __launch_bounds__(JS_THREADS) k_ts_rr(const float2* __restrict__
         order[rank] = tid;
         evals[T - TS_P + rank] = static_cast<double>(th) / *scale;
     }
-    for (int i = tid; i < T - TS_P; i += JS_THREADS)
+    for (int i = tid; i < T - TS_P; i += JS_MID)
         evals[i] = 0.0;
     __syncthreads();
-    for (int e = tid; e < TS_P * TS_P; e += JS_THREADS)
+    for (int e = tid; e < TS_P * TS_P; e += JS_MID)
     {
         const int k = e / TS_P, r = e % TS_P;
         const Cx<float> q = Qs[k * TS_LD + order[r]];
@@ -2830,7 +3095,7 @@ hv_status pca_eigh(double2* cov, int T, double* evals, double2* evecs, int pmin,
         }
         HV_LAUNCH(k_ts_matmul, gm, mm_threads, 0, st, C32, Vs, T, Ys);
         HV_LAUNCH(k_ts_gram, TS_P, TS_GRAM_WARPS * 32, 0, st, Vs, Ys, T, Hm);
-        HV_LAUNCH(k_ts_rr, 1, JS_THREADS, 0, st, Hm, T, scale, evals, Qo);
+        HV_LAUNCH(k_ts_rr, 1, JS_MID, 0, st, Hm, T, scale, evals, Qo);
         HV_LAUNCH(k_ts_ritz, (T + TS_P - 1) / TS_P, 256, 0, st, Vs, Qo, T, evecs, Vw);
         count_launch(5 + 2 * iters + extra + (warm ? 0 : 2));
         // two corrections: on 512 x 512 frames with T = 512 and stride 64, one warm iteration and two
@@ -2840,18 +3105,18 @@ hv_status pca_eigh(double2* cov, int T, double* evals, double2* evecs, int pmin,
     if (T <= JS_MAX_T && prec == HV_EIG_FP32)
     {
         const size_t smem = jacobi_smem_bytes<float>(T, warm);
-        if (smem > 48 * 1024)
-            HV_CUDA_TRY(cudaFuncSetAttribute(k_jacobi_smem<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             static_cast<int>(jacobi_smem_bytes<float>(JS_MAX_T, true))));
-        HV_LAUNCH(k_jacobi_smem<float>, 1, JS_THREADS, smem, st, cov, V, T, Tp, ev_unsorted, warm ? 1 : 0, floor_rel);
+        auto kern = T > 32 ? k_jacobi_smem<float, JS_WIDE> : k_jacobi_smem<float, JS_MID>;
+        const int threads = T > 32 ? JS_WIDE : JS_MID;
+        HV_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+        HV_LAUNCH(kern, 1, threads, smem, st, cov, V, T, Tp, ev_unsorted, warm ? 1 : 0, floor_rel);
     }
     else if (T <= JS_MAX_T)
     {
         const size_t smem = jacobi_smem_bytes<double>(T, false);
         if (smem > 48 * 1024)
-            HV_CUDA_TRY(cudaFuncSetAttribute(k_jacobi_smem<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            HV_CUDA_TRY(cudaFuncSetAttribute((k_jacobi_smem<double, JS_THREADS>), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              static_cast<int>(smem)));
-        HV_LAUNCH(k_jacobi_smem<double>, 1, JS_THREADS, smem, st, cov, V, T, Tp, ev_unsorted, 0, 0.0f);
+        HV_LAUNCH((k_jacobi_smem<double, JS_THREADS>), 1, JS_THREADS, smem, st, cov, V, T, Tp, ev_unsorted, 0, 0.0f);
     }
     else if (T <= JC_MAX_T && prec == HV_EIG_FP32)
     {
