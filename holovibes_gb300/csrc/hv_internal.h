@@ -101,10 +101,11 @@ hv_status spatial_transform(const void* raw, int kind, int W, int H, int batch, 
                             float2* work, float2* ring, int slot0, int nslots, cudaStream_t st,
                             const CycleCtl* ctl = nullptr, const float2* f2d_mask = nullptr,
                             float2* work2 = nullptr, uint16_t* real_planes = nullptr, int reserve_sms = 0);
-// Raw 8/16-bit frames (no spatial transform) -> the real split-BF16 planes of ring slots slot0 ..
-// (mod T) only; and the ring slots back from those planes (exact for integer pixels below 2^16).
-hv_status convert_to_planes(const void* raw, int kind, size_t HW, int batch, int slot0, int T, uint16_t* planes,
-                            cudaStream_t st);
+// Raw 8/16-bit frames (no spatial transform, frames of a multiple of 8 pixels) -> the real split-BF16
+// planes of ring slots slot0 .. (mod T) and frames sample0 .. (mod cap) of a ring of 16-bit samples
+// (the converted integers); and ring slots from those planes (exact for integer pixels below 2^16).
+hv_status convert_window(const void* raw, int kind, size_t HW, int batch, int slot0, int T, uint16_t* planes,
+                         int sample0, int cap, uint16_t* samples, cudaStream_t st);
 hv_status ring_from_planes(const uint16_t* planes, int T, size_t HW, int slot0, int n, float2* ring, cudaStream_t st);
 // filter2D band-pass mask in FFT layout: written as complex (multiply = 0) or multiplied into dst.
 hv_status filter2d_mask(float2* dst, int W, int H, int n1, int n2, int smooth_low, int smooth_high, int multiply,
@@ -129,6 +130,12 @@ hv_status time_view_planes(const uint16_t* planes, const float2* ring, int ring_
                            const float2* weights, int K, int img_type, float scale, int shift, float* out,
                            double* partials, cudaStream_t st, const CycleCtl* ctl = nullptr,
                            const float* bin_w = nullptr);
+// time_view on a real ring held as 16-bit integer samples ([cap][HW], HW % 8 == 0): the window's frames
+// are first .. first + T - 1 (mod cap), the oldest in ring slot slot0 (the weights follow the slots).
+hv_status time_view_samples(const uint16_t* samples, int cap, int first, int slot0, int T, int W, int H,
+                            const float2* weights, int K, int img_type, float scale, int shift, float* out,
+                            double* partials, cudaStream_t st, const CycleCtl* ctl = nullptr,
+                            const float* bin_w = nullptr);
 hv_status moment_bin_weights(float* bin_w, int T, int pmin, int pmax, int order, float camera_fps, cudaStream_t st);
 inline bool is_moment(int img_type) { return img_type >= HV_IMG_MOMENTS_0 && img_type <= HV_IMG_MOMENTS_2; }
 hv_status stft_weights(float2* weights, int T, int pmin, int pmax, cudaStream_t st);

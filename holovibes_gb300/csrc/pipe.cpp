@@ -70,8 +70,8 @@ void free_buffers(hv_pipe* p)
         L = hv_pipe::Lane{};
     }
     for (cudaEvent_t* e : {&p->join_ev, &p->range_ev, &p->pp_cov_ev[0], &p->pp_cov_ev[1], &p->pp_eig_ev[0],
-                           &p->pp_eig_ev[1], &p->pp_view_ev[0], &p->pp_view_ev[1], &p->pp_main_ev, &p->pp_ring_ev[0],
-                           &p->pp_ring_ev[1], &p->pp_ring_ev[2], &p->pp_ring_ev[3]})
+                           &p->pp_eig_ev[1], &p->pp_view_ev[0], &p->pp_view_ev[1], &p->pp_view_ev[2],
+                           &p->pp_view_ev[3]})
         if (*e)
         {
             cudaEventDestroy(*e);
@@ -143,10 +143,11 @@ int planes_real(const hv_settings& s)
 bool uses_planes(const hv_frame_desc& fd, const hv_settings& s, bool served);
 
 // PCA on the converted integer frames (no spatial transform) with sliding windows: the windows are
-// pipelined over three streams (process_batch, render_view). The ring is rebuilt from the real
-// split planes (exact for integer pixels), so only the conversion into the planes reads the input
-// batch; a window's eigensolve then overlaps the next batch's conversion and covariance update and
-// the previous window's view.
+// pipelined over three streams (process_batch, render_view). The covariance reads the split planes, the views
+// a ring of 16-bit samples with room for two more batches than the window, so a window's eigensolve
+// overlaps the next batch's conversion and covariance update and the previous window's view. (With views
+// that read planes and complex slots, and a ring rebuild behind each view that the next conversion had to wait
+// for, the streams hardly overlapped: 512 frames of 512 x 512, stride 64, 406 us a window; so 315 us.)
 bool uses_pca_pipeline(const hv_frame_desc& fd, const hv_settings& s, bool served)
 {
     const int T = s.time_transformation_size, B = s.batch_size;
@@ -198,8 +199,11 @@ size_t footprint(const hv_frame_desc& fd, const hv_settings& s, bool served = fa
     }
     if (uses_planes(fd, s, served))
         z.add(cov_planes_bytes(T, HW, planes_real(s)));
-    if (uses_pca_pipeline(fd, s, served))  // the second covariance and weights buffers
+    if (uses_pca_pipeline(fd, s, served))  // the second covariance and weights buffers, the sample ring
+    {
         z.add(static_cast<size_t>(T) * T * 16 + static_cast<size_t>(K > 0 ? K : 1) * T * 8);
+        z.add(HW * 2 * (static_cast<size_t>(T) + 2 * B));
+    }
     z.add(HW * 4 * 2);  // view + post
     if (is_moment(s.image_type))
         z.add(static_cast<size_t>(K > 0 ? K : 1) * sizeof(float));
@@ -486,9 +490,12 @@ hv_status build(hv_pipe* p)
     p->windows = 0;
     // PCA windows over three streams (the tensor-core view's prepared weights are not double-buffered)
     p->pp = uses_pca_pipeline(p->fd, s, p->served) && p->planes_ok && !p->view_on_tc && !p->fast;
-    p->pp_w = p->pp_b = 0;
+    p->pp_w = p->pp_head = p->ring_stale = 0;
     if (p->pp)
     {
+        p->pp_cap = p->T + 2 * p->B;
+        if ((st = dalloc(p, p->pp_samples, HW * 2 * static_cast<size_t>(p->pp_cap))) != HV_OK)
+            return st;
         p->render_stream = p->render_stream_owned;
         p->pp_cov[0] = p->cov;
         if ((st = dalloc(p, p->pp_cov[1], static_cast<size_t>(p->T) * p->T * sizeof(double2))) != HV_OK)
@@ -497,8 +504,7 @@ hv_status build(hv_pipe* p)
         if ((st = dalloc(p, p->pp_weights[1], static_cast<size_t>(p->K) * p->T * sizeof(float2))) != HV_OK)
             return st;
         for (cudaEvent_t* e : {&p->pp_cov_ev[0], &p->pp_cov_ev[1], &p->pp_eig_ev[0], &p->pp_eig_ev[1],
-                               &p->pp_view_ev[0], &p->pp_view_ev[1], &p->pp_main_ev, &p->pp_ring_ev[0],
-                               &p->pp_ring_ev[1], &p->pp_ring_ev[2], &p->pp_ring_ev[3]})
+                               &p->pp_view_ev[0], &p->pp_view_ev[1], &p->pp_view_ev[2], &p->pp_view_ev[3]})
             HV_CUDA_TRY(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
     }
     // lens (computed once per refresh, fourier_transform.cc:93-137)
@@ -593,6 +599,17 @@ hv_status build(hv_pipe* p)
 // otherwise). `ctl` gates the kernels of a served cycle (null for the plain pipe).
 hv_status render_view(hv_pipe* p, cudaStream_t st, const CycleCtl* ctl, const float** frame, int* shift_after);
 
+// The pipelined PCA windows leave the ring behind; this rebuilds the slots written since it was last
+// asked for, on the pipe stream (which writes the planes).
+hv_status refresh_ring(hv_pipe* p)
+{
+    const int end = (p->ring_start + p->ring_size) % p->T, n = p->ring_stale;
+    const hv_status r = ring_from_planes(p->planes, p->T, p->HW, (end - n + p->T) % p->T, n, p->ring, p->stream);
+    if (r == HV_OK)
+        p->ring_stale = 0;
+    return r;
+}
+
 // The covariance and eigensolve of a PCA window of the three-stream pipeline (p->pp): the update
 // of covariance buffer w % 2 on the pipe stream (from the other buffer, the previous window's),
 // the eigensolve into weights buffer w % 2 on the eigensolve stream, then the view on the render
@@ -622,12 +639,8 @@ hv_status render_view_pp(hv_pipe* p, cudaStream_t st, uint32_t dirty, uint32_t a
             blocks = b2;
         }
         r = pca_covariance_planes(p->planes, p->T, p->HW, cov, p->cov_work, blocks, 1, p->stream);
-        if (r == HV_ERR_UNSUPPORTED)  // the SIMT engine mode: from the ring, which the render stream writes
-        {
-            HV_CUDA_TRY(cudaEventRecord(p->pp_main_ev, st));
-            HV_CUDA_TRY(cudaStreamWaitEvent(p->stream, p->pp_main_ev, 0));
+        if (r == HV_ERR_UNSUPPORTED && (r = refresh_ring(p)) == HV_OK)  // the SIMT engine mode: from the ring
             r = pca_covariance(p->ring, p->T, p->HW, cov, p->cov_work, p->stream);
-        }
         if (r != HV_OK)
             return r;
     }
@@ -636,7 +649,7 @@ hv_status render_view_pp(hv_pipe* p, cudaStream_t st, uint32_t dirty, uint32_t a
     HV_CUDA_TRY(cudaEventRecord(p->pp_cov_ev[i], p->stream));
     HV_CUDA_TRY(cudaStreamWaitEvent(es, p->pp_cov_ev[i], 0));
     if (w >= 2)  // window w - 2's view read this weights buffer
-        HV_CUDA_TRY(cudaStreamWaitEvent(es, p->pp_view_ev[i], 0));
+        HV_CUDA_TRY(cudaStreamWaitEvent(es, p->pp_view_ev[(w - 2) & 3], 0));
     bool kept = false;
     if ((r = pca_eigh(cov, p->T, p->evals, p->evecs, p->pmin, p->pmax, p->pp_weights[i], p->eig_work, es, p->pmin,
                       p->pmax, p->eig_warm, true, &kept)) != HV_OK)
@@ -651,23 +664,21 @@ hv_status render_view_pp(hv_pipe* p, cudaStream_t st, uint32_t dirty, uint32_t a
     p->pp_nested = false;
     if (r != HV_OK)
         return r;
-    HV_CUDA_TRY(cudaEventRecord(p->pp_view_ev[i], st));
+    HV_CUDA_TRY(cudaEventRecord(p->pp_view_ev[w & 3], st));
     return HV_OK;
 }
 
-// The FP32 SIMT time view of the ring into p->view. The pipelined PCA windows (p->pp: a real
-// ring) read the real split planes instead, half the bytes; the slots that the next batch's
-// planes overwrite while this view may still run (the next batch waits only for the views
-// enqueued before the previous batch) are read from the ring, which holds every slot.
+// The FP32 SIMT time view of the ring into p->view. The pipelined PCA windows (p->pp) read the
+// 16-bit samples instead, a quarter of the bytes.
 hv_status ring_view(hv_pipe* p, cudaStream_t st, float scale, int shift, double* partials, const CycleCtl* ctl,
                     bool bins = true)
 {
     const hv_settings& s = p->s;
     const float* bin_w = bins ? p->bin_w : nullptr;
     if (p->pp)
-        return time_view_planes(p->planes, p->ring, (p->ring_start + p->ring_size) % p->T, std::min(p->B, p->T),
-                                p->T, p->W, p->H, p->weights, p->K, s.image_type, scale, shift, p->view, partials, st,
-                                ctl, bin_w);
+        return time_view_samples(p->pp_samples, p->pp_cap, (p->pp_head + p->pp_cap - p->T) % p->pp_cap, p->ring_start,
+                                 p->T, p->W, p->H, p->weights, p->K, s.image_type, scale, shift, p->view, partials, st,
+                                 ctl, bin_w);
     return time_view(p->ring, p->T, p->W, p->H, p->weights, p->K, s.image_type, scale, shift, p->view, partials, st,
                      ctl, bin_w);
 }
@@ -1100,39 +1111,17 @@ hv_status process_batch(hv_pipe* p, const uint8_t* raw)
     hv_status r = HV_OK;
     if (p->pp)
     {
-        // the batch is read once, into its slots' planes (pipe stream: the covariance update reads
-        // them next); the render stream writes the ring slots from the planes after the previous
-        // window's view. The views read the planes: batch b waits for the ring copy of batch b - 1,
-        // which the render stream runs after every view enqueued before batch b - 1. A view
-        // enqueued since (it may run while batch b is converted) reads the slots of batch b from
-        // the ring (ring_view).
-        const int b = p->pp_b++;
-        if (b >= 1)
-            HV_CUDA_TRY(cudaStreamWaitEvent(p->stream, p->pp_ring_ev[(b - 1) & 3], 0));
-        r = convert_to_planes(raw, p->kind, p->HW, nb, begin, T, p->planes, p->stream);
-        if (r == HV_OK)
-        {
-            HV_CUDA_TRY(cudaEventRecord(p->pp_main_ev, p->stream));
-            HV_CUDA_TRY(cudaStreamWaitEvent(p->render_stream, p->pp_main_ev, 0));
-            if ((r = ring_from_planes(p->planes, T, p->HW, begin, nb, p->ring, p->render_stream)) != HV_OK)
-                return r;
-        }
-        else if (r == HV_ERR_UNSUPPORTED)
-        {
-            // a batch off 16-byte alignment: converted into the ring on the pipe stream once the
-            // render stream is idle, then split
-            HV_CUDA_TRY(cudaEventRecord(p->pp_main_ev, p->render_stream));
-            HV_CUDA_TRY(cudaStreamWaitEvent(p->stream, p->pp_main_ev, 0));
-            if ((r = spatial_transform(raw, p->kind, p->W, p->H, nb, p->s.space_transformation, p->lens, p->spatial,
-                                       p->ring, begin, T, p->stream, nullptr, p->f2d_mask, p->work2)) != HV_OK ||
-                (r = cov_split_planes(p->ring, T, p->HW, begin, nb, p->planes, 1, p->stream)) != HV_OK)
-                return r;
-            HV_CUDA_TRY(cudaEventRecord(p->pp_main_ev, p->stream));
-            HV_CUDA_TRY(cudaStreamWaitEvent(p->render_stream, p->pp_main_ev, 0));
-        }
-        else
+        // the batch is read once, into its slots' planes (which the covariance update reads next, on the
+        // same stream) and into the sample ring. The frames overwritten there are older than the
+        // window of three renders ago (pp_cap = T + 2 B): its view has to be through, the two
+        // views enqueued since may still run.
+        if (p->pp_w >= 3)
+            HV_CUDA_TRY(cudaStreamWaitEvent(p->stream, p->pp_view_ev[(p->pp_w - 3) & 3], 0));
+        if ((r = convert_window(raw, p->kind, p->HW, nb, begin, T, p->planes, p->pp_head, p->pp_cap, p->pp_samples,
+                                p->stream)) != HV_OK)
             return r;
-        HV_CUDA_TRY(cudaEventRecord(p->pp_ring_ev[b & 3], p->render_stream));
+        p->pp_head = (p->pp_head + nb) % p->pp_cap;
+        p->ring_stale = std::min(T, p->ring_stale + nb);
     }
     // real planes (no spatial transform) come out of the conversion pass itself
     const bool fused_split = !p->pp && p->planes_ok && p->planes_real && p->HW % 8 == 0 &&
@@ -1841,6 +1830,13 @@ hv_status hv_pipe_get_ring(hv_pipe* p, void* dst_host, int32_t* start, int32_t* 
         const hv_status rs = sync_render(p);
         if (rs != HV_OK)
             return rs;
+    }
+    if (dst_host && p->pp)
+    {
+        const hv_status rs = refresh_ring(p);
+        if (rs != HV_OK)
+            return rs;
+        HV_CUDA_TRY(cudaStreamSynchronize(p->stream));
     }
     if (dst_host)
         HV_CUDA_TRY(cudaMemcpy(dst_host, p->ring, p->HW * p->T * sizeof(float2), cudaMemcpyDeviceToHost));

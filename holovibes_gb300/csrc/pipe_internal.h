@@ -83,16 +83,18 @@ struct hv_pipe
     bool planes_ok = false;
     int planes_real = 0;  // the ring's imaginary parts are 0: real rows only
     // PCA windows pipelined over three streams (pipe.cpp, `pp`): the pipe stream converts each
-    // batch into the split planes and updates the covariance, the eigensolve stream solves it,
-    // the render stream writes the ring from the planes and renders; covariance and weights
-    // alternate between two buffers by window parity
+    // batch into the split planes and a ring of 16-bit samples and updates the covariance, the
+    // eigensolve stream solves it, the render stream views the samples and renders; covariance and
+    // weights alternate between two buffers by window parity. The sample ring holds pp_cap = T + 2 B
+    // frames, the next one goes to pp_head. `ring` is not written on the way: its newest ring_stale
+    // slots are rebuilt from the planes when they are asked for (refresh_ring).
     bool pp = false, pp_nested = false;
-    int pp_w = 0, pp_b = 0;
+    int pp_w = 0, pp_cap = 0, pp_head = 0, ring_stale = 0;
+    uint16_t* pp_samples = nullptr;
     double2* pp_cov[2] = {nullptr, nullptr};
     float2* pp_weights[2] = {nullptr, nullptr};
     cudaEvent_t pp_cov_ev[2] = {nullptr, nullptr}, pp_eig_ev[2] = {nullptr, nullptr};
-    cudaEvent_t pp_view_ev[2] = {nullptr, nullptr}, pp_main_ev = nullptr;
-    cudaEvent_t pp_ring_ev[4] = {nullptr, nullptr, nullptr, nullptr};
+    cudaEvent_t pp_view_ev[4] = {nullptr, nullptr, nullptr, nullptr};
     float* view = nullptr;
     float* unwrapped = nullptr;
     void* unwrap_work = nullptr;

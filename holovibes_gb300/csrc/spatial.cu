@@ -856,13 +856,10 @@ __global__ void k_convert8(const void* in, int kind, size_t frame_px, int batch,
             v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = c.x, v[5] = c.y, v[6] = c.z, v[7] = c.w;
         }
         const size_t off = map.offset(b);
-        if (ring)
-        {
-            float4* o = reinterpret_cast<float4*>(ring + off + px);
+        float4* o = reinterpret_cast<float4*>(ring + off + px);
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
-                __stcs(o + i, make_float4(v[2 * i], 0.f, v[2 * i + 1], 0.f));
-        }
+        for (int i = 0; i < 4; ++i)
+            __stcs(o + i, make_float4(v[2 * i], 0.f, v[2 * i + 1], 0.f));
         if (planes)
         {
             uint4 hi, lo;
@@ -874,6 +871,81 @@ __global__ void k_convert8(const void* in, int kind, size_t frame_px, int batch,
             *reinterpret_cast<uint4*>(planes + slot_px) = hi;
             *reinterpret_cast<uint4*>(planes + plane + slot_px) = lo;
         }
+    }
+}
+
+// Raw 8/16-bit frames (no spatial transform) -> the real split planes of ring slots slot0 .. (mod T)
+// and, as 16-bit integers, frames sample0 .. (mod cap) of the sample ring: what the pipelined PCA
+// windows' covariance and views read. 8 pixels per thread; without VEC (a batch off 16-byte
+// alignment) the pixels are loaded one by one. DRAM-bound: 64 16-bit frames of 512 x 512 (33.6 MB read,
+// 100.7 MB written).
+template <int KIND, bool VEC>
+__global__ void k_convert_window(const void* __restrict__ in, int swap, size_t frame_px, int batch, int slot0, int T,
+                                 uint16_t* __restrict__ planes, int sample0, int cap, uint16_t* __restrict__ samples)
+{
+    wait_prior_kernels();
+    const size_t groups = frame_px / 8;
+    const size_t total = groups * batch;
+    const size_t plane = static_cast<size_t>(T) * frame_px;
+    for (size_t e = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; e < total;
+         e += static_cast<size_t>(gridDim.x) * blockDim.x)
+    {
+        const int b = static_cast<int>(e / groups);
+        const size_t px = (e - static_cast<size_t>(b) * groups) * 8;
+        const size_t src = static_cast<size_t>(b) * frame_px + px;
+        uint32_t x[4];  // pixel pairs
+        if constexpr (KIND == IN_U8)
+        {
+            const uint8_t* p = static_cast<const uint8_t*>(in) + src;
+            uint32_t w[2];
+            if constexpr (VEC)
+            {
+                const uint2 v = *reinterpret_cast<const uint2*>(p);
+                w[0] = v.x, w[1] = v.y;
+            }
+            else
+            {
+#pragma unroll
+                for (int i = 0; i < 2; ++i)
+                    w[i] = p[4 * i] | (p[4 * i + 1] << 8) | (p[4 * i + 2] << 16) | (static_cast<uint32_t>(p[4 * i + 3]) << 24);
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+            {
+                const uint32_t h = w[i / 2] >> (16 * (i % 2));
+                x[i] = ((h & 0xffu) | ((h & 0xff00u) << 8)) * 257u;
+            }
+        }
+        else
+        {
+            const uint16_t* p = static_cast<const uint16_t*>(in) + src;
+            if constexpr (VEC)
+            {
+                const uint4 v = *reinterpret_cast<const uint4*>(p);
+                x[0] = v.x, x[1] = v.y, x[2] = v.z, x[3] = v.w;
+            }
+            else
+            {
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    x[i] = p[2 * i] | (static_cast<uint32_t>(p[2 * i + 1]) << 16);
+            }
+            if (swap)
+            {
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    x[i] = ((x[i] & 0x00ff00ffu) << 8) | ((x[i] >> 8) & 0x00ff00ffu);
+            }
+        }
+        uint32_t hi[4], lo[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            tc::split2(static_cast<float>(x[i] & 0xffffu), static_cast<float>(x[i] >> 16), hi[i], lo[i]);
+        uint16_t* o = planes + static_cast<size_t>((slot0 + b) % T) * frame_px + px;
+        *reinterpret_cast<uint4*>(o) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+        *reinterpret_cast<uint4*>(o + plane) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+        *reinterpret_cast<uint4*>(samples + static_cast<size_t>((sample0 + b) % cap) * frame_px + px) =
+            make_uint4(x[0], x[1], x[2], x[3]);
     }
 }
 
@@ -1456,19 +1528,21 @@ hv_status spatial_transform(const void* raw, int kind, int W, int H, int batch, 
     return HV_INVALID_VALUE;
 }
 
-hv_status convert_to_planes(const void* raw, int kind, size_t HW, int batch, int slot0, int T, uint16_t* planes,
-                            cudaStream_t st)
+hv_status convert_window(const void* raw, int kind, size_t HW, int batch, int slot0, int T, uint16_t* planes,
+                         int sample0, int cap, uint16_t* samples, cudaStream_t st)
 {
-    if (HW % 8 != 0 || kind == IN_C64 || (reinterpret_cast<uintptr_t>(raw) & 15) != 0 || batch <= 0)
+    if (HW % 8 != 0 || (kind != IN_U8 && kind != IN_U16 && kind != IN_U16_BE) || batch <= 0)
         return HV_ERR_UNSUPPORTED;
-    const FrameMap map{HW, slot0, T};
     const size_t total = HW / 8 * batch;
     const int block = 256;
     // three quarters of the SMs' thread slots: the pipelined windows' eigensolve kernels (another
     // stream) find room beside this pass
-    const int cap = device_sms() * 6;
-    const int grid = static_cast<int>((total + block - 1) / block < static_cast<size_t>(cap) ? (total + block - 1) / block : cap);
-    HV_LAUNCH(k_convert8, grid, block, 0, st, raw, kind, HW, batch, nullptr, map, nullptr, planes);
+    const int cap_ctas = device_sms() * 6;
+    const int grid = static_cast<int>((total + block - 1) / block < static_cast<size_t>(cap_ctas) ? (total + block - 1) / block : cap_ctas);
+    const bool vec = (reinterpret_cast<uintptr_t>(raw) & 15) == 0;
+    auto kern = kind == IN_U8 ? (vec ? k_convert_window<IN_U8, true> : k_convert_window<IN_U8, false>)
+                              : (vec ? k_convert_window<IN_U16, true> : k_convert_window<IN_U16, false>);
+    HV_LAUNCH(kern, grid, block, 0, st, raw, kind == IN_U16_BE ? 1 : 0, HW, batch, slot0, T, planes, sample0, cap, samples);
     count_launch();
     return HV_OK;
 }
@@ -1479,7 +1553,7 @@ hv_status ring_from_planes(const uint16_t* planes, int T, size_t HW, int slot0, 
         return n <= 0 ? HV_OK : HV_ERR_UNSUPPORTED;
     const size_t total = HW / 8 * n;
     const int block = 256;
-    const int cap = device_sms() * 6;  // as convert_to_planes: room for the eigensolve stream's kernels
+    const int cap = device_sms() * 6;  // as convert_window: room for the eigensolve stream's kernels
     const int grid = static_cast<int>((total + block - 1) / block < static_cast<size_t>(cap) ? (total + block - 1) / block : cap);
     HV_LAUNCH(k_ring_from_planes, grid, block, 0, st, planes, T, HW, slot0, n, ring);
     count_launch();

@@ -25,6 +25,7 @@
 #include <type_traits>
 #include <vector>
 
+#include "fft_smem.cuh"
 #include "hv_common.cuh"
 #include "hv_internal.h"
 
@@ -419,21 +420,101 @@ __device__ __forceinline__ void tvp_ring(float2 (&a)[2][KC], const float4* __res
     }
 }
 
-// The view of a real ring (zero imaginary parts) read from its split-BF16 planes ([2][T][HW] bf16,
-// hi then lo): 4 bytes per sample instead of the 8 of the complex ring. The ring slots
-// [r0, r0 + rn) mod T are read from the complex ring instead (the slots that the next batch's
-// planes overwrite while this view may still run). Two adjacent pixels per thread, 128 threads
-// cover 256 pixels and write their two 128-pixel renormalisation partials (those of k_time_view).
-// The view values equal k_time_view's on the same ring. 64 registers: the grid leaves a CTA slot
-// free on most SMs for the pipelined windows' eigensolve kernels (another stream).
+// The window's real samples from 16-bit integers, 2 bytes per sample (512 frames of 512 x 512, 4 bins: 268 MB
+// and the instructions of 1.1 G multiply-adds; from the planes and the ring the same view moved 604 MB). The integer becomes a float in the
+// mantissa of 2^23 (exact, no conversion unit); the multiply-adds, those of the other sources, go two
+// to an instruction.
 template <int KC>
-__global__ void __launch_bounds__(TV_THREADS, 8) k_time_view_planes(const uint16_t* __restrict__ planes,
-                                                                 const float2* __restrict__ ring, int r0, int rn, int T,
-                                                                 int W, int H, const float2* __restrict__ weights,
-                                                                 int K, int img_type, float scale, int shift,
-                                                                 float* __restrict__ out, double* __restrict__ partials,
-                                                                 int npartials, const CycleCtl* ctl,
-                                                                 const float* __restrict__ bin_w)
+__device__ __forceinline__ void tvp_samples(float2 (&a)[2][KC], const uint32_t* __restrict__ x, size_t step, int t0,
+                                            int n, const float2* wsm)
+{
+    auto add = [&](uint32_t v, int t) {
+        const float x0 = __uint_as_float(0x4b000000u | (v & 0xffffu)) - 8388608.0f;
+        const float x1 = __uint_as_float(0x4b000000u | (v >> 16)) - 8388608.0f;
+        const float2* wt = wsm + t * KC;
+#pragma unroll
+        for (int kk = 0; kk < KC; ++kk)
+        {
+            a[0][kk] = fft::pfma(make_float2(x0, x0), wt[kk], a[0][kk]);
+            a[1][kk] = fft::pfma(make_float2(x1, x1), wt[kk], a[1][kk]);
+        }
+    };
+    constexpr int D = 16;  // frames whose loads are issued before the first is used
+    int i = 0;
+    for (; i + D <= n; i += D)
+    {
+        uint32_t v[D];
+#pragma unroll
+        for (int j = 0; j < D; ++j)
+            v[j] = __ldcs(x + static_cast<size_t>(i + j) * step);
+#pragma unroll
+        for (int j = 0; j < D; ++j)
+            add(v[j], t0 + i + j);
+    }
+    for (; i < n; ++i)
+        add(__ldcs(x + static_cast<size_t>(i) * step), t0 + i);
+}
+
+// Where k_time_view_real reads the window from; accumulate adds the slots 0 .. T - 1 in order.
+// Planes: split-BF16 planes ([2][T][HW] bf16, hi then lo), except the ring slots [r0, r0 + rn) mod T,
+// which come from the complex ring (slots whose planes are being overwritten).
+struct PlanesSource
+{
+    const uint16_t* planes;
+    const float2* ring;
+    int r0, rn;
+    template <int KC>
+    __device__ __forceinline__ void accumulate(float2 (&a)[2][KC], size_t pix0, size_t HW, int T, const float2* wsm) const
+    {
+        for (int t = 0; t < T;)
+        {
+            // slots t .. of one run, all from one source
+            const int d = t < r0 ? t - r0 + T : t - r0;
+            const int n = min((d < rn ? rn : T) - d, T - t);
+            if (d < rn)
+                tvp_ring<KC>(a, reinterpret_cast<const float4*>(ring + pix0), HW / 2, t, t + n, wsm);
+            else
+                tvp_planes<KC>(a, reinterpret_cast<const uint32_t*>(planes + pix0),
+                               reinterpret_cast<const uint32_t*>(planes + static_cast<size_t>(T) * HW + pix0), HW / 2, t,
+                               t + n, wsm);
+            t += n;
+        }
+    }
+};
+
+// Samples: frames first .. first + T - 1 (mod cap) of a ring of 16-bit integers, the oldest in slot slot0.
+struct SamplesSource
+{
+    const uint16_t* samples;
+    int cap, first, slot0;
+    template <int KC>
+    __device__ __forceinline__ void accumulate(float2 (&a)[2][KC], size_t pix0, size_t HW, int T, const float2* wsm) const
+    {
+        for (int t = 0; t < T;)
+        {
+            // slots t .. of one run: to the end of the window's order, of the slots or of the sample ring
+            const int age = t < slot0 ? t + T - slot0 : t - slot0;
+            int frame = first + age;
+            frame -= frame >= cap ? cap : 0;
+            const int n = min((t < slot0 ? slot0 : T) - t, cap - frame);
+            tvp_samples<KC>(a, reinterpret_cast<const uint32_t*>(samples + static_cast<size_t>(frame) * HW + pix0), HW / 2,
+                            t, n, wsm);
+            t += n;
+        }
+    }
+};
+
+// The view of a real ring (zero imaginary parts) read from its split-BF16 planes (4 bytes per sample
+// instead of the 8 of the complex ring) or from 16-bit samples (2 bytes). Two adjacent pixels per
+// thread, 128 threads cover 256 pixels and write their two 128-pixel renormalisation partials (those of
+// k_time_view). The view values equal k_time_view's on the same ring. 64 registers: the grid leaves a
+// CTA slot free on most SMs for the pipelined windows' eigensolve kernels (another stream).
+template <int KC, class Source>
+__global__ void __launch_bounds__(TV_THREADS, 8) k_time_view_real(const __grid_constant__ Source source, int T, int W, int H,
+                                                                  const float2* __restrict__ weights, int K, int img_type,
+                                                                  float scale, int shift, float* __restrict__ out,
+                                                                  double* __restrict__ partials, int npartials,
+                                                                  const CycleCtl* ctl, const float* __restrict__ bin_w)
 {
     wait_prior_kernels();
     if (!ctl_render(ctl))
@@ -443,22 +524,6 @@ __global__ void __launch_bounds__(TV_THREADS, 8) k_time_view_planes(const uint16
     const size_t HW = static_cast<size_t>(W) * H;
     const size_t pix0 = 2 * (blockIdx.x * static_cast<size_t>(TV_THREADS) + threadIdx.x);
     const bool valid = pix0 < HW;  // HW even: both pixels or none
-    // slot order [0, T) cut into at most three runs, each from one source
-    int cut[4], src[3], nrun;
-    if (rn <= 0)
-    {
-        cut[0] = 0, cut[1] = T, src[0] = 0, nrun = 1;
-    }
-    else if (r0 + rn <= T)
-    {
-        cut[0] = 0, cut[1] = r0, cut[2] = r0 + rn, cut[3] = T;
-        src[0] = 0, src[1] = 1, src[2] = 0, nrun = 3;
-    }
-    else
-    {
-        cut[0] = 0, cut[1] = r0 + rn - T, cut[2] = r0, cut[3] = T;
-        src[0] = 1, src[1] = 0, src[2] = 1, nrun = 3;
-    }
     float view0 = 0.f, view1 = 0.f;
     for (int k0 = 0; k0 < K; k0 += KC)
     {
@@ -476,15 +541,7 @@ __global__ void __launch_bounds__(TV_THREADS, 8) k_time_view_planes(const uint16
             a[0][kk] = a[1][kk] = make_float2(0.f, 0.f);
         if (valid)
         {
-            for (int r = 0; r < nrun; ++r)
-            {
-                if (src[r])
-                    tvp_ring<KC>(a, reinterpret_cast<const float4*>(ring + pix0), HW / 2, cut[r], cut[r + 1], wsm);
-                else
-                    tvp_planes<KC>(a, reinterpret_cast<const uint32_t*>(planes + pix0),
-                                   reinterpret_cast<const uint32_t*>(planes + static_cast<size_t>(T) * HW + pix0),
-                                   HW / 2, cut[r], cut[r + 1], wsm);
-            }
+            source.accumulate(a, pix0, HW, T, wsm);
             const int kn = (K - k0) < KC ? (K - k0) : KC;
 #pragma unroll
             for (int kk = 0; kk < KC; ++kk)
@@ -609,11 +666,10 @@ hv_status time_view(const float2* ring, int T, int W, int H, const float2* weigh
     return launch_time_view<16>(ring, T, W, H, weights, K, img_type, scale, shift, out, partials, st, ctl, bin_w);
 }
 
-template <int KC>
-static hv_status launch_time_view_planes(const uint16_t* planes, const float2* ring, int r0, int rn, int T, int W,
-                                         int H, const float2* weights, int K, int img_type, float scale, int shift,
-                                         float* out, double* partials, cudaStream_t st, const CycleCtl* ctl,
-                                         const float* bin_w)
+template <int KC, class Source>
+static hv_status launch_time_view_real(const Source& source, int T, int W, int H, const float2* weights, int K,
+                                       int img_type, float scale, int shift, float* out, double* partials,
+                                       cudaStream_t st, const CycleCtl* ctl, const float* bin_w)
 {
     const size_t smem = static_cast<size_t>(T) * KC * sizeof(float2);
     if (smem > 200 * 1024)
@@ -621,15 +677,27 @@ static hv_status launch_time_view_planes(const uint16_t* planes, const float2* r
         set_last_error_msg("time window too large for the time-view kernel");
         return HV_ERR_UNSUPPORTED;
     }
+    auto kern = k_time_view_real<KC, Source>;
     if (smem > 48 * 1024)
-        HV_CUDA_TRY(cudaFuncSetAttribute(k_time_view_planes<KC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(smem)));
+        HV_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
     const size_t HW = static_cast<size_t>(W) * H;
     const int grid = static_cast<int>((HW + 2 * TV_THREADS - 1) / (2 * TV_THREADS));
-    HV_LAUNCH(k_time_view_planes<KC>, grid, TV_THREADS, smem, st, planes, ring, r0, rn, T, W, H, weights, K, img_type,
-              scale, shift, out, partials, time_view_partials(W, H), ctl, bin_w);
+    HV_LAUNCH(kern, grid, TV_THREADS, smem, st, source, T, W, H, weights, K, img_type, scale, shift, out, partials,
+              time_view_partials(W, H), ctl, bin_w);
     count_launch();
     return HV_OK;
+}
+
+// chunks of up to 4 bins (2 KC complex accumulators per thread)
+template <class Source>
+static hv_status time_view_real(const Source& source, int T, int W, int H, const float2* weights, int K, int img_type,
+                                float scale, int shift, float* out, double* partials, cudaStream_t st,
+                                const CycleCtl* ctl, const float* bin_w)
+{
+    auto launch = K == 1   ? launch_time_view_real<1, Source>
+                  : K == 2 ? launch_time_view_real<2, Source>
+                           : launch_time_view_real<4, Source>;
+    return launch(source, T, W, H, weights, K, img_type, scale, shift, out, partials, st, ctl, bin_w);
 }
 
 hv_status time_view_planes(const uint16_t* planes, const float2* ring, int ring_slot0, int ring_n, int T, int W, int H,
@@ -653,15 +721,23 @@ hv_status time_view_planes(const uint16_t* planes, const float2* ring, int ring_
         set_last_error_msg("time_view_planes: W x H must be a multiple of 8 and the planes and ring 16-byte aligned");
         return HV_ERR_UNSUPPORTED;
     }
-    // chunks of up to 4 bins (2 KC complex accumulators per thread)
-    if (K == 1)
-        return launch_time_view_planes<1>(planes, ring, ring_slot0, ring_n, T, W, H, weights, K, img_type, scale, shift,
-                                          out, partials, st, ctl, bin_w);
-    if (K == 2)
-        return launch_time_view_planes<2>(planes, ring, ring_slot0, ring_n, T, W, H, weights, K, img_type, scale, shift,
-                                          out, partials, st, ctl, bin_w);
-    return launch_time_view_planes<4>(planes, ring, ring_slot0, ring_n, T, W, H, weights, K, img_type, scale, shift,
-                                      out, partials, st, ctl, bin_w);
+    return time_view_real(PlanesSource{planes, ring, ring_slot0, ring_n}, T, W, H, weights, K, img_type, scale, shift, out,
+                          partials, st, ctl, bin_w);
+}
+
+hv_status time_view_samples(const uint16_t* samples, int cap, int first, int slot0, int T, int W, int H,
+                            const float2* weights, int K, int img_type, float scale, int shift, float* out,
+                            double* partials, cudaStream_t st, const CycleCtl* ctl, const float* bin_w)
+{
+    const size_t HW = static_cast<size_t>(W) * H;
+    if (T <= 0 || K <= 0 || W <= 0 || H <= 0 || cap < T || first < 0 || first >= cap || slot0 < 0 || slot0 >= T ||
+        HW % 8 != 0 || (shift && ((W & 1) || (H & 1))))
+    {
+        set_last_error_msg("time_view_samples: bad sizes");
+        return HV_INVALID_VALUE;
+    }
+    return time_view_real(SamplesSource{samples, cap, first, slot0}, T, W, H, weights, K, img_type, scale, shift, out,
+                          partials, st, ctl, bin_w);
 }
 
 // ------------------------------------------------------------------------------ weights
