@@ -137,6 +137,23 @@ __device__ __forceinline__ void tma_load_3d(void* dst_smem, const void* tmap, in
         : "memory");
 }
 
+// tma_load_3d of data that is read once: its lines are the first to leave L2.
+__device__ __forceinline__ uint64_t evict_first_policy()
+{
+    uint64_t p;
+    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
+    return p;
+}
+__device__ __forceinline__ void tma_load_3d_streaming(void* dst_smem, const void* tmap, int x, int y, int z,
+                                                      uint64_t* bar, uint64_t policy)
+{
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint [%0], "
+        "[%1, {%2, %3, %4}], [%5], %6;" ::"r"(smem_u32(dst_smem)),
+        "l"(tmap), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar)), "l"(policy)
+        : "memory");
+}
+
 __device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                          uint32_t accumulate)
 {

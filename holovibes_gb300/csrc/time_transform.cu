@@ -420,51 +420,79 @@ __device__ __forceinline__ void tvp_ring(float2 (&a)[2][KC], const float4* __res
     }
 }
 
-// The window's real samples from 16-bit integers, 2 bytes per sample (512 frames of 512 x 512, 4 bins: 268 MB
-// and the instructions of 1.1 G multiply-adds; from the planes and the ring the same view moved 604 MB). The integer becomes a float in the
-// mantissa of 2^23 (exact, no conversion unit); the multiply-adds, those of the other sources, go two
-// to an instruction.
-template <int KC>
-__device__ __forceinline__ void tvp_samples(float2 (&a)[2][KC], const uint32_t* __restrict__ x, size_t step, int t0,
-                                            int n, const float2* wsm)
+// Pixel pairs 64 pixels apart (GROUPS of them per thread) of the window's real samples from 16-bit integers.
+// The integer becomes a float in the mantissa of 2^23 (exact, no conversion unit); the multiply-adds, those
+// of the other sources, go two to an instruction.
+template <int KC, int GROUPS>
+__device__ __forceinline__ void tvp_samples(float2 (&a)[GROUPS][2][KC], const uint32_t* const (&x)[GROUPS], size_t at,
+                                            size_t step, int t0, int n, const float2* wsm)
 {
-    auto add = [&](uint32_t v, int t) {
-        const float x0 = __uint_as_float(0x4b000000u | (v & 0xffffu)) - 8388608.0f;
-        const float x1 = __uint_as_float(0x4b000000u | (v >> 16)) - 8388608.0f;
-        const float2* wt = wsm + t * KC;
+    auto add = [&](const uint32_t (&v)[GROUPS], int t) {
+        float2 w[KC];
 #pragma unroll
         for (int kk = 0; kk < KC; ++kk)
+            w[kk] = wsm[t * KC + kk];
+#pragma unroll
+        for (int g = 0; g < GROUPS; ++g)
         {
-            a[0][kk] = fft::pfma(make_float2(x0, x0), wt[kk], a[0][kk]);
-            a[1][kk] = fft::pfma(make_float2(x1, x1), wt[kk], a[1][kk]);
+            const float x0 = __uint_as_float(__byte_perm(v[g], 0x4b000000u, 0x7610)) - 8388608.0f;
+            const float x1 = __uint_as_float(__byte_perm(v[g], 0x4b000000u, 0x7632)) - 8388608.0f;
+#pragma unroll
+            for (int kk = 0; kk < KC; ++kk)
+            {
+                a[g][0][kk] = fft::pfma(make_float2(x0, x0), w[kk], a[g][0][kk]);
+                a[g][1][kk] = fft::pfma(make_float2(x1, x1), w[kk], a[g][1][kk]);
+            }
         }
     };
-    constexpr int D = 16;  // frames whose loads are issued before the first is used
+    constexpr int D = 8;  // frames per batch of loads; the next batch is on its way while one is summed
     int i = 0;
-    for (; i + D <= n; i += D)
+    if (n >= D)
     {
-        uint32_t v[D];
+        uint32_t v[2][D][GROUPS];
+        auto load = [&](uint32_t (&b)[D][GROUPS], int i0) {
 #pragma unroll
-        for (int j = 0; j < D; ++j)
-            v[j] = __ldcs(x + static_cast<size_t>(i + j) * step);
+            for (int j = 0; j < D; ++j)
 #pragma unroll
-        for (int j = 0; j < D; ++j)
-            add(v[j], t0 + i + j);
+                for (int g = 0; g < GROUPS; ++g)
+                    b[j][g] = __ldcs(x[g] + at + static_cast<size_t>(i0 + j) * step);
+        };
+        load(v[0], 0);
+        int cur = 0;
+#pragma unroll 2
+        for (; i + D <= n; i += D)
+        {
+            if (i + 2 * D <= n)
+                load(v[cur ^ 1], i + D);
+#pragma unroll
+            for (int j = 0; j < D; ++j)
+                add(v[cur][j], t0 + i + j);
+            cur ^= 1;
+        }
     }
     for (; i < n; ++i)
-        add(__ldcs(x + static_cast<size_t>(i) * step), t0 + i);
+    {
+        uint32_t v[GROUPS];
+#pragma unroll
+        for (int g = 0; g < GROUPS; ++g)
+            v[g] = __ldcs(x[g] + at + static_cast<size_t>(i) * step);
+        add(v, t0 + i);
+    }
 }
 
-// Where k_time_view_real reads the window from; accumulate adds the slots 0 .. T - 1 in order.
+// Where k_time_view_real reads the window from; accumulate adds the slots 0 .. T - 1 in order for the
+// pixel pairs pix[g].
 // Planes: split-BF16 planes ([2][T][HW] bf16, hi then lo), except the ring slots [r0, r0 + rn) mod T,
 // which come from the complex ring (slots whose planes are being overwritten).
 struct PlanesSource
 {
+    static constexpr int GROUPS = 1, CTAS = 8;
     const uint16_t* planes;
     const float2* ring;
     int r0, rn;
     template <int KC>
-    __device__ __forceinline__ void accumulate(float2 (&a)[2][KC], size_t pix0, size_t HW, int T, const float2* wsm) const
+    __device__ __forceinline__ void accumulate(float2 (&a)[GROUPS][2][KC], const size_t (&pix)[GROUPS], size_t HW, int T,
+                                               const float2* wsm) const
     {
         for (int t = 0; t < T;)
         {
@@ -472,24 +500,31 @@ struct PlanesSource
             const int d = t < r0 ? t - r0 + T : t - r0;
             const int n = min((d < rn ? rn : T) - d, T - t);
             if (d < rn)
-                tvp_ring<KC>(a, reinterpret_cast<const float4*>(ring + pix0), HW / 2, t, t + n, wsm);
+                tvp_ring<KC>(a[0], reinterpret_cast<const float4*>(ring + pix[0]), HW / 2, t, t + n, wsm);
             else
-                tvp_planes<KC>(a, reinterpret_cast<const uint32_t*>(planes + pix0),
-                               reinterpret_cast<const uint32_t*>(planes + static_cast<size_t>(T) * HW + pix0), HW / 2, t,
-                               t + n, wsm);
+                tvp_planes<KC>(a[0], reinterpret_cast<const uint32_t*>(planes + pix[0]),
+                               reinterpret_cast<const uint32_t*>(planes + static_cast<size_t>(T) * HW + pix[0]), HW / 2,
+                               t, t + n, wsm);
             t += n;
         }
     }
 };
 
 // Samples: frames first .. first + T - 1 (mod cap) of a ring of 16-bit integers, the oldest in slot slot0.
+// Two pixel pairs per thread share the weights' loads.
 struct SamplesSource
 {
+    static constexpr int GROUPS = 2, CTAS = 8;
     const uint16_t* samples;
     int cap, first, slot0;
     template <int KC>
-    __device__ __forceinline__ void accumulate(float2 (&a)[2][KC], size_t pix0, size_t HW, int T, const float2* wsm) const
+    __device__ __forceinline__ void accumulate(float2 (&a)[GROUPS][2][KC], const size_t (&pix)[GROUPS], size_t HW, int T,
+                                               const float2* wsm) const
     {
+        const uint32_t* x[GROUPS];
+#pragma unroll
+        for (int g = 0; g < GROUPS; ++g)
+            x[g] = reinterpret_cast<const uint32_t*>(samples + pix[g]);
         for (int t = 0; t < T;)
         {
             // slots t .. of one run: to the end of the window's order, of the slots or of the sample ring
@@ -497,52 +532,62 @@ struct SamplesSource
             int frame = first + age;
             frame -= frame >= cap ? cap : 0;
             const int n = min((t < slot0 ? slot0 : T) - t, cap - frame);
-            tvp_samples<KC>(a, reinterpret_cast<const uint32_t*>(samples + static_cast<size_t>(frame) * HW + pix0), HW / 2,
-                            t, n, wsm);
+            tvp_samples<KC, GROUPS>(a, x, static_cast<size_t>(frame) * (HW / 2), HW / 2, t, n, wsm);
             t += n;
         }
     }
 };
 
 // The view of a real ring (zero imaginary parts) read from its split-BF16 planes (4 bytes per sample
-// instead of the 8 of the complex ring) or from 16-bit samples (2 bytes). Two adjacent pixels per
-// thread, 128 threads cover 256 pixels and write their two 128-pixel renormalisation partials (those of
-// k_time_view). The view values equal k_time_view's on the same ring. 64 registers: the grid leaves a
-// CTA slot free on most SMs for the pipelined windows' eigensolve kernels (another stream).
+// instead of the 8 of the complex ring) or from 16-bit samples (2 bytes). A CTA covers 256 pixels in four
+// units of 64, lane l of a warp the pixels 2 l and 2 l + 1 of its GROUPS units, and writes their two
+// 128-pixel renormalisation partials (those of k_time_view). The view values equal k_time_view's on the same
+// ring.
 template <int KC, class Source>
-__global__ void __launch_bounds__(TV_THREADS, 8) k_time_view_real(const __grid_constant__ Source source, int T, int W, int H,
-                                                                  const float2* __restrict__ weights, int K, int img_type,
-                                                                  float scale, int shift, float* __restrict__ out,
-                                                                  double* __restrict__ partials, int npartials,
-                                                                  const CycleCtl* ctl, const float* __restrict__ bin_w)
+__global__ void __launch_bounds__(TV_THREADS / Source::GROUPS, Source::CTAS)
+    k_time_view_real(const __grid_constant__ Source source, int T, int W, int H, const float2* __restrict__ weights, int K,
+                     int img_type, float scale, int shift, float* __restrict__ out, double* __restrict__ partials,
+                     int npartials, const CycleCtl* ctl, const float* __restrict__ bin_w)
 {
     wait_prior_kernels();
     if (!ctl_render(ctl))
         return;
+    constexpr int GROUPS = Source::GROUPS, THREADS = TV_THREADS / GROUPS;
     extern __shared__ __align__(16) float2 wsm[];  // [T][KC]
-    __shared__ double red[TV_THREADS / 32];
+    __shared__ double red[4];
     const size_t HW = static_cast<size_t>(W) * H;
-    const size_t pix0 = 2 * (blockIdx.x * static_cast<size_t>(TV_THREADS) + threadIdx.x);
-    const bool valid = pix0 < HW;  // HW even: both pixels or none
-    float view0 = 0.f, view1 = 0.f;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    size_t pix[GROUPS];     // (a pair beyond the frame repeats the last one; HW is even)
+    bool valid[GROUPS];
+    float view[GROUPS][2];
+#pragma unroll
+    for (int g = 0; g < GROUPS; ++g)
+    {
+        pix[g] = blockIdx.x * static_cast<size_t>(2 * TV_THREADS) + 64 * (warp * GROUPS + g) + 2 * lane;
+        valid[g] = pix[g] < HW;
+        pix[g] = valid[g] ? pix[g] : HW - 2;
+        view[g][0] = view[g][1] = 0.f;
+    }
     for (int k0 = 0; k0 < K; k0 += KC)
     {
         __syncthreads();
-        for (int e = threadIdx.x; e < T * KC; e += TV_THREADS)
+        for (int e = threadIdx.x; e < T * KC; e += THREADS)
         {
             const int t = e / KC, kk = e - t * KC;
             const int k = k0 + kk;
             wsm[e] = (k < K) ? weights[static_cast<size_t>(k) * T + t] : make_float2(0.f, 0.f);
         }
         __syncthreads();
-        float2 a[2][KC];
+        float2 a[GROUPS][2][KC];
 #pragma unroll
-        for (int kk = 0; kk < KC; ++kk)
-            a[0][kk] = a[1][kk] = make_float2(0.f, 0.f);
-        if (valid)
-        {
-            source.accumulate(a, pix0, HW, T, wsm);
-            const int kn = (K - k0) < KC ? (K - k0) : KC;
+        for (int g = 0; g < GROUPS; ++g)
+#pragma unroll
+            for (int kk = 0; kk < KC; ++kk)
+                a[g][0][kk] = a[g][1][kk] = make_float2(0.f, 0.f);
+        source.accumulate(a, pix, HW, T, wsm);
+        const int kn = (K - k0) < KC ? (K - k0) : KC;
+#pragma unroll
+        for (int g = 0; g < GROUPS; ++g)
 #pragma unroll
             for (int kk = 0; kk < KC; ++kk)
                 if (kk < kn)
@@ -550,48 +595,52 @@ __global__ void __launch_bounds__(TV_THREADS, 8) k_time_view_real(const __grid_c
                     if (bin_w)
                     {
                         const float bw = __ldg(bin_w + k0 + kk);
-                        view0 += (a[0][kk].x * a[0][kk].x + a[0][kk].y * a[0][kk].y) * bw;
-                        view1 += (a[1][kk].x * a[1][kk].x + a[1][kk].y * a[1][kk].y) * bw;
+                        view[g][0] += (a[g][0][kk].x * a[g][0][kk].x + a[g][0][kk].y * a[g][0][kk].y) * bw;
+                        view[g][1] += (a[g][1][kk].x * a[g][1][kk].x + a[g][1][kk].y * a[g][1][kk].y) * bw;
                     }
                     else
                     {
-                        view0 += view_value(a[0][kk], img_type);
-                        view1 += view_value(a[1][kk], img_type);
+                        view[g][0] += view_value(a[g][0][kk], img_type);
+                        view[g][1] += view_value(a[g][1][kk], img_type);
                     }
                 }
+    }
+#pragma unroll
+    for (int g = 0; g < GROUPS; ++g)
+    {
+        float v0 = 0.f, v1 = 0.f;
+        if (valid[g])
+        {
+            v0 = bin_w ? view[g][0] : view[g][0] / static_cast<float>(K);
+            v1 = bin_w ? view[g][1] : view[g][1] / static_cast<float>(K);
+            if (scale != 1.0f)
+            {
+                v0 = v0 * scale;
+                v1 = v1 * scale;
+            }
+            if (W % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 7) == 0)  // the pair stays together
+                *reinterpret_cast<float2*>(out + view_target(pix[g], W, H, shift)) = make_float2(v0, v1);
+            else
+            {
+                out[view_target(pix[g], W, H, shift)] = v0;
+                out[view_target(pix[g] + 1, W, H, shift)] = v1;
+            }
+        }
+        if (partials)
+        {
+            const double d = warp_sum(v0, v1);
+            if (lane == 0)
+                red[warp * GROUPS + g] = d;
         }
     }
-    float v0 = 0.f, v1 = 0.f;
-    if (valid)
+    if (!partials)
+        return;
+    __syncthreads();
+    if (threadIdx.x < 2)
     {
-        v0 = bin_w ? view0 : view0 / static_cast<float>(K);
-        v1 = bin_w ? view1 : view1 / static_cast<float>(K);
-        if (scale != 1.0f)
-        {
-            v0 = v0 * scale;
-            v1 = v1 * scale;
-        }
-        if (W % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 7) == 0)  // the pair stays together
-            *reinterpret_cast<float2*>(out + view_target(pix0, W, H, shift)) = make_float2(v0, v1);
-        else
-        {
-            out[view_target(pix0, W, H, shift)] = v0;
-            out[view_target(pix0 + 1, W, H, shift)] = v1;
-        }
-    }
-    if (partials)
-    {
-        const double d = warp_sum(valid ? v0 : 0.f, valid ? v1 : 0.f);
-        if ((threadIdx.x & 31) == 0)
-            red[threadIdx.x >> 5] = d;
-        __syncthreads();
-        // warps 0-1: pixels 0..127 of the CTA, warps 2-3: 128..255
-        if (threadIdx.x < 2)
-        {
-            const int pi = 2 * blockIdx.x + threadIdx.x;
-            if (pi < npartials)
-                partials[pi] = red[2 * threadIdx.x] + red[2 * threadIdx.x + 1];
-        }
+        const int pi = 2 * blockIdx.x + threadIdx.x;
+        if (pi < npartials)
+            partials[pi] = red[2 * threadIdx.x] + red[2 * threadIdx.x + 1];
     }
 }
 
@@ -682,7 +731,7 @@ static hv_status launch_time_view_real(const Source& source, int T, int W, int H
         HV_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
     const size_t HW = static_cast<size_t>(W) * H;
     const int grid = static_cast<int>((HW + 2 * TV_THREADS - 1) / (2 * TV_THREADS));
-    HV_LAUNCH(kern, grid, TV_THREADS, smem, st, source, T, W, H, weights, K, img_type, scale, shift, out, partials,
+    HV_LAUNCH(kern, grid, TV_THREADS / Source::GROUPS, smem, st, source, T, W, H, weights, K, img_type, scale, shift, out, partials,
               time_view_partials(W, H), ctl, bin_w);
     count_launch();
     return HV_OK;
@@ -1463,15 +1512,16 @@ __device__ bool smem_sweeps(Cx<R>* A, Cx<R>* V, int T_, int Tp_, int LD_, JacScr
 // the block update and of the rotation's square roots and division), the warm T = 32 one of 1024 x
 // 1024 frames 91 -> 65 us (cold caches). Not kept: V's rows in registers, moved from lane to lane
 // with the pairing (589 against 504 us for the whole eigensolve at T = 64: every row pays every step).
+template <int PAIRS = JS_MAX_T / 2>
 struct JacScratchWarps
 {
-    JacRot<float> rot[32][JS_MAX_T / 2];     // slot: a step looked at
-    unsigned int mask[32];                   // its rotating pairs
-    unsigned char list[32][JS_MAX_T / 2];    // and their indices
+    JacRot<float> rot[32][PAIRS];     // slot: a step looked at
+    unsigned int mask[32];            // its rotating pairs
+    unsigned char list[32][PAIRS];    // and their indices
 };
 
-template <int NT, int LD, int N = 0>
-__device__ void smem_sweeps_warps(Cx<float>* A, Cx<float>* V, int T_, int Tp_, JacScratchWarps& sc, float floor,
+template <int NT, int LD, int N = 0, class Scratch>
+__device__ void smem_sweeps_warps(Cx<float>* A, Cx<float>* V, int T_, int Tp_, Scratch& sc, float floor,
                                   int max_sweeps)
 {
     constexpr int NW = NT / 32;
@@ -1721,7 +1771,7 @@ __global__ void __launch_bounds__(NT) k_jacobi_smem(const double2* __restrict__ 
     Cx<R>* V = js + Tp * LD;
     Cx<R>* X = V + Tp * LD;  // warm start only
     Cx<R>* N = X + Tp * LD;
-    __shared__ std::conditional_t<sizeof(R) == sizeof(float), JacScratchWarps, JacScratch<R>> sc;
+    __shared__ std::conditional_t<sizeof(R) == sizeof(float), JacScratchWarps<>, JacScratch<R>> sc;
     __shared__ double s_scale;
     const int tid = threadIdx.x;
     if (tid < 32)
@@ -2342,6 +2392,29 @@ __device__ __forceinline__ double2 warp_sum2(double2 v)
     return v;
 }
 
+// FP64 products are what these kernels pay for (two lanes per clock and SM), and the eigenvectors of real
+// frames have imaginary parts that are exactly 0. Where the imaginary parts of a whole warp's operands are 0 and
+// the real parts finite, the complex multiply-add is its real product and sum, to the bit (the terms left
+// out are +-0), and the imaginary accumulator is not touched: 2 FP64 operations instead of 6.
+__device__ __forceinline__ bool real_finite(double2 v)
+{
+    return (__double_as_longlong(v.y) << 1) == 0 && (__double2hiint(v.x) & 0x7ff00000) != 0x7ff00000;
+}
+__device__ __forceinline__ double add_product(double acc, double a, double b)
+{
+    return __dadd_rn(acc, __dmul_rn(a, b));
+}
+// warp_sum2 of sums whose imaginary parts are 0 in most calls
+__device__ __forceinline__ double2 warp_sum2_real(double2 v)
+{
+    if (__any_sync(0xffffffffu, (__double_as_longlong(v.y) << 1) != 0))
+        return warp_sum2(v);
+    for (int o = 16; o > 0; o >>= 1)
+        v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
+    v.y = 0.0;
+    return v;
+}
+
 // Y[j][t] = sum_s C[t][s] v_{r0+j}[s]; grid (ceil(T / 8), K), 256 threads
 __global__ void k_eigref_matvec(const double2* __restrict__ C, const double2* __restrict__ evecs, int T, int r0,
                                 double2* __restrict__ Y)
@@ -2354,13 +2427,32 @@ __global__ void k_eigref_matvec(const double2* __restrict__ C, const double2* __
     const double2* v = evecs + static_cast<size_t>(r0 + j) * T;
     const double2* c = C + static_cast<size_t>(t) * T;
     double2 acc = make_double2(0.0, 0.0);
-    for (int s2 = lane; s2 < T; s2 += 32)
+    constexpr int D = 4;  // terms per lane whose loads are issued together
+    for (int s0 = 0; s0 < T; s0 += 32 * D)
     {
-        const double2 a = c[s2], x = v[s2];
-        acc.x += a.x * x.x - a.y * x.y;
-        acc.y += a.x * x.y + a.y * x.x;
+        double2 a[D], x[D];
+#pragma unroll
+        for (int d = 0; d < D; ++d)
+        {
+            const int s2 = s0 + 32 * d + lane;
+            a[d] = s2 < T ? c[s2] : make_double2(0.0, 0.0);
+            x[d] = s2 < T ? v[s2] : make_double2(0.0, 0.0);
+        }
+#pragma unroll
+        for (int d = 0; d < D; ++d)
+        {
+            if (s0 + 32 * d >= T)
+                break;
+            if (__all_sync(0xffffffffu, real_finite(a[d]) && real_finite(x[d])))
+                acc.x = add_product(acc.x, a[d].x, x[d].x);
+            else if (s0 + 32 * d + lane < T)
+            {
+                acc.x += a[d].x * x[d].x - a[d].y * x[d].y;
+                acc.y += a[d].x * x[d].y + a[d].y * x[d].x;
+            }
+        }
     }
-    acc = warp_sum2(acc);
+    acc = warp_sum2_real(acc);
     if (lane == 0)
         Y[static_cast<size_t>(j) * T + t] = acc;
 }
@@ -2747,8 +2839,9 @@ __device__ __forceinline__ float ts_project(float2 (&y)[TS_ORTH_RPT][TS_P], floa
 // always register slot 0 and the slots rotate by one after every column, so that registers are
 // indexed by constants only. A column left without norm (Y of rank < TS_P) becomes the unit vector
 // e_k, made orthogonal at the next iteration.
-__global__ void __launch_bounds__(TS_ORTH_THREADS) k_ts_orth(const float2* __restrict__ Y, int T, float2* __restrict__ V,
-                                                              const int* __restrict__ only_if = nullptr)
+template <int CTAS>
+__global__ void __launch_bounds__(TS_ORTH_THREADS, CTAS) k_ts_orth(const float2* __restrict__ Y, int T,
+                                                                   float2* __restrict__ V, const int* __restrict__ only_if)
 {
     wait_prior_kernels();
     if (only_if && *only_if == 0)  // the Cholesky-QR of the warm iteration succeeded
@@ -2828,78 +2921,81 @@ __global__ void __launch_bounds__(TS_ORTH_THREADS) k_ts_orth(const float2* __res
 // j .. TS_P - 1 of Y. The warm start's C V has near-orthogonal columns (the previous window's Ritz
 // vectors times a covariance that changed by one stride), so G' is near the identity and the FP32
 // factorisation is well conditioned. A pivot below 1e-6 (Y of rank < TS_P, or columns too close to
-// dependent) sets *fail and k_ts_orth recomputes V by Gram-Schmidt. One warp.
-__global__ void __launch_bounds__(32) k_ts_cholqr(const float2* __restrict__ G, float2* __restrict__ M,
-                                                  int* __restrict__ fail)
+// dependent) sets *fail and k_ts_orth recomputes V by Gram-Schmidt. One CTA.
+//
+// Column m of L and row m of L^-1 sit in the registers of warp m mod TS_CHOL_WARPS (lane = row of L, column
+// of L^-1). Step j finishes column j and row j and every later column and row takes its term of them, in the
+// order in which a left-looking factorisation adds them: one barrier per step.
+constexpr int TS_CHOL_WARPS = 16;
+__global__ void __launch_bounds__(TS_CHOL_WARPS * 32, 4) k_ts_cholqr(const float2* __restrict__ G, float2* __restrict__ M,
+                                                                  int* __restrict__ fail)
 {
     wait_prior_kernels();
-    __shared__ float2 L[TS_P][TS_P + 1];  // index a = TS_P - 1 - (column of Y); lower triangle = L
-    __shared__ float2 X[TS_P][TS_P + 1];  // L^-1
-    __shared__ float d[TS_P];
-    const int lane = threadIdx.x;
+    __shared__ float2 s_col[2][TS_P], s_row[2][TS_P];
+    constexpr int SLOTS = TS_P / TS_CHOL_WARPS;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    float d;  // of index a = lane (a = TS_P - 1 - column of Y)
     {
         const float g = G[(TS_P - 1 - lane) * TS_P + (TS_P - 1 - lane)].x;
-        d[lane] = (g > 0.f && isfinite(g)) ? rsqrtf(g) : 0.f;
+        d = (g > 0.f && isfinite(g)) ? rsqrtf(g) : 0.f;
     }
-    __syncwarp();
-    for (int a = 0; a < TS_P; ++a)
+    float2 l[SLOTS], x[SLOTS];
+#pragma unroll
+    for (int s = 0; s < SLOTS; ++s)
     {
-        const float2 v = G[(TS_P - 1 - a) * TS_P + (TS_P - 1 - lane)];
-        const float sc = d[a] * d[lane];
-        L[a][lane] = make_float2(v.x * sc, v.y * sc);
+        const int m = warp + s * TS_CHOL_WARPS;
+        const float2 v = G[(TS_P - 1 - lane) * TS_P + (TS_P - 1 - m)];  // G'(lane, m)
+        const float sc = d * __shfl_sync(0xffffffffu, d, m);
+        l[s] = make_float2(v.x * sc, v.y * sc);
+        x[s] = make_float2(m == lane ? 1.f : 0.f, 0.f);
     }
-    __syncwarp();
-    bool ok = true;
-    for (int j = 0; j < TS_P; ++j)
-    {
-        // every lane forms the same pivot from the same (broadcast) values
-        float p = L[j][j].x;
-        for (int k = 0; k < j; ++k)
+    bool ok = true;  // of the steps that this warp finished
+#pragma unroll
+    for (int s = 0; s < SLOTS; ++s)
+        for (int w = 0; w < TS_CHOL_WARPS; ++w)
         {
-            const float2 l = L[j][k];
-            p -= l.x * l.x + l.y * l.y;
-        }
-        ok = ok && p > 1e-6f && isfinite(p);
-        const float ljj = sqrtf(fmaxf(p, 1e-6f));
-        __syncwarp();
-        if (lane > j)
-        {
-            float2 a = L[lane][j];
-            for (int k = 0; k < j; ++k)
+            const int j = w + s * TS_CHOL_WARPS, buf = j & 1;
+            if (warp == w)
             {
-                const float2 li = L[lane][k], lj = L[j][k];  // a -= li conj(lj)
-                a.x -= li.x * lj.x + li.y * lj.y;
-                a.y -= li.y * lj.x - li.x * lj.y;
+                const float p = __shfl_sync(0xffffffffu, l[s].x, j);
+                ok = ok && p > 1e-6f && isfinite(p);
+                const float ljj = sqrtf(fmaxf(p, 1e-6f));
+                const float inv = 1.f / ljj;
+                l[s] = lane == j ? make_float2(ljj, 0.f) : make_float2(l[s].x / ljj, l[s].y / ljj);
+                x[s] = make_float2(x[s].x * inv, x[s].y * inv);
+                s_col[buf][lane] = l[s];
+                s_row[buf][lane] = x[s];
             }
-            L[lane][j] = make_float2(a.x / ljj, a.y / ljj);
+            __syncthreads();  // (step j + 1 writes the other buffer; step j + 2 comes after its barrier)
+            const float2 li = s_col[buf][lane], xr = s_row[buf][lane];
+#pragma unroll
+            for (int u = 0; u < SLOTS; ++u)
+            {
+                const int m = warp + u * TS_CHOL_WARPS;
+                if (m <= j)
+                    continue;
+                const float2 lj = s_col[buf][m];
+                if (lane >= m)
+                {
+                    // l -= li conj(lj)
+                    l[u].x -= fmaf(li.x, lj.x, li.y * lj.y);
+                    l[u].y -= fmaf(li.y, lj.x, -(li.x * lj.y));
+                }
+                x[u].x -= fmaf(lj.x, xr.x, -(lj.y * xr.y));
+                x[u].y -= fmaf(lj.y, xr.x, lj.x * xr.y);
+            }
         }
-        if (lane == 0)
-            L[j][j] = make_float2(ljj, 0.f);
-        __syncwarp();
-    }
-    // X = L^-1 by forward substitution, lane = column
-    for (int i = 0; i < TS_P; ++i)
-    {
-        float2 a = make_float2(i == lane ? 1.f : 0.f, 0.f);
-        for (int k = 0; k < i; ++k)
-        {
-            const float2 l = L[i][k], x = X[k][lane];
-            a.x -= l.x * x.x - l.y * x.y;
-            a.y -= l.x * x.y + l.y * x.x;
-        }
-        const float inv = 1.f / L[i][i].x;
-        X[i][lane] = make_float2(a.x * inv, a.y * inv);
-    }
-    __syncwarp();
     // M[k][r] (Y column k into V column r) = d_k conj(X[b][a]) with a = TS_P-1-k, b = TS_P-1-r, a <= b
-    for (int k = 0; k < TS_P; ++k)
+#pragma unroll
+    for (int s = 0; s < SLOTS; ++s)
     {
-        const int a = TS_P - 1 - k, b = TS_P - 1 - lane;
-        const float2 x = X[b][a];
-        M[k * TS_P + lane] = a <= b ? make_float2(d[a] * x.x, -d[a] * x.y) : make_float2(0.f, 0.f);
+        const int b = warp + s * TS_CHOL_WARPS;
+        M[(TS_P - 1 - lane) * TS_P + (TS_P - 1 - b)] =
+            lane <= b ? make_float2(d * x[s].x, -d * x[s].y) : make_float2(0.f, 0.f);
     }
-    if (lane == 0)
-        *fail = ok ? 0 : 1;
+    const int all_ok = __syncthreads_and(ok);
+    if (threadIdx.x == 0)
+        *fail = all_ok ? 0 : 1;
 }
 
 // Rayleigh-Ritz in three launches. k_ts_gram: H = V^H Y (Y = C32 V), one CTA per row i of H, warp w
@@ -2914,23 +3010,38 @@ __global__ void __launch_bounds__(TS_GRAM_WARPS * 32) k_ts_gram(const float2* __
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, i = blockIdx.x;
     float r0 = 0.f, i0 = 0.f, r1 = 0.f, i1 = 0.f;
     int t = warp;
-#pragma unroll 4
-    for (; t + TS_GRAM_WARPS < T; t += 2 * TS_GRAM_WARPS)
-    {
-        const float2 a0 = V[static_cast<size_t>(t) * TS_P + i], b0 = Y[static_cast<size_t>(t) * TS_P + lane];
-        const float2 a1 = V[static_cast<size_t>(t + TS_GRAM_WARPS) * TS_P + i];
-        const float2 b1 = Y[static_cast<size_t>(t + TS_GRAM_WARPS) * TS_P + lane];
+    auto term0 = [&](float2 a0, float2 b0) {
         r0 = fmaf(a0.x, b0.x, fmaf(a0.y, b0.y, r0));
         i0 = fmaf(a0.x, b0.y, fmaf(-a0.y, b0.x, i0));
+    };
+    auto term1 = [&](float2 a1, float2 b1) {
         r1 = fmaf(a1.x, b1.x, fmaf(a1.y, b1.y, r1));
         i1 = fmaf(a1.x, b1.y, fmaf(-a1.y, b1.x, i1));
+    };
+    constexpr int D = 16;  // rows whose loads are issued together
+    for (; t + (D - 1) * TS_GRAM_WARPS < T; t += D * TS_GRAM_WARPS)
+    {
+        float2 a[D], b[D];
+#pragma unroll
+        for (int k = 0; k < D; ++k)
+        {
+            a[k] = V[static_cast<size_t>(t + k * TS_GRAM_WARPS) * TS_P + i];
+            b[k] = Y[static_cast<size_t>(t + k * TS_GRAM_WARPS) * TS_P + lane];
+        }
+#pragma unroll
+        for (int k = 0; k < D; k += 2)
+        {
+            term0(a[k], b[k]);
+            term1(a[k + 1], b[k + 1]);
+        }
+    }
+    for (; t + TS_GRAM_WARPS < T; t += 2 * TS_GRAM_WARPS)
+    {
+        term0(V[static_cast<size_t>(t) * TS_P + i], Y[static_cast<size_t>(t) * TS_P + lane]);
+        term1(V[static_cast<size_t>(t + TS_GRAM_WARPS) * TS_P + i], Y[static_cast<size_t>(t + TS_GRAM_WARPS) * TS_P + lane]);
     }
     if (t < T)
-    {
-        const float2 a0 = V[static_cast<size_t>(t) * TS_P + i], b0 = Y[static_cast<size_t>(t) * TS_P + lane];
-        r0 = fmaf(a0.x, b0.x, fmaf(a0.y, b0.y, r0));
-        i0 = fmaf(a0.x, b0.y, fmaf(-a0.y, b0.x, i0));
-    }
+        term0(V[static_cast<size_t>(t) * TS_P + i], Y[static_cast<size_t>(t) * TS_P + lane]);
     part[warp][lane] = make_float2(r0 + r1, i0 + i1);
     __syncthreads();
     if (warp == 0)
@@ -2948,14 +3059,14 @@ __global__ void __launch_bounds__(TS_GRAM_WARPS * 32) k_ts_gram(const float2* __
 // k_ts_rr: H Q = Q diag(theta) by FP32 Jacobi on the Hermitian part of H (one CTA); the Ritz values
 // (scaled back) into evals[T - TS_P ..] in ascending order, evals below set to 0, and Qo = the columns
 // of Q in that order.
-__global__ void __launch_bounds__(JS_MID) k_ts_rr(const float2* __restrict__ H, int T,
+__global__ void __launch_bounds__(JS_MID, 4) k_ts_rr(const float2* __restrict__ H, int T,
                                                      const double* __restrict__ scale, double* __restrict__ evals,
                                                      float2* __restrict__ Qo)
 {
     wait_prior_kernels();
     constexpr int NW = JS_MID / 32;
     __shared__ Cx<float> Hs[TS_P * TS_LD], Qs[TS_P * TS_LD];
-    __shared__ JacScratchWarps sc;
+    __shared__ JacScratchWarps<TS_P / 2> sc;
     __shared__ int order[TS_P];
     __shared__ float s_fro[NW];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -3003,47 +3114,46 @@ __global__ void __launch_bounds__(JS_MID) k_ts_rr(const float2* __restrict__ H, 
     }
 }
 
-// k_ts_ritz: the Ritz vectors U = V Qo, TS_P rows of U per CTA (warp w: rows w, w + 8, ..., lane =
-// column r): into the warm start Vw (row-major) and, when evecs is not null, evecs columns
-// T - TS_P + r (FP64, through a shared-memory transpose so that each eigenvector's rows are written
-// contiguously). Also the Cholesky-QR's V = Y M (evecs null).
-__global__ void __launch_bounds__(256) k_ts_ritz(const float2* __restrict__ V, const float2* __restrict__ Qo, int T,
-                                                 double2* __restrict__ evecs, float2* __restrict__ Vw)
+// k_ts_ritz: the Ritz vectors U = V Qo, TS_RITZ_ROWS rows of U per CTA (a warp each, lane = column r): into
+// the warm start Vw (row-major) and, when evecs is not null, evecs columns T - TS_P + r (FP64, through a
+// shared-memory transpose so that the rows of an eigenvector are written contiguously). Also the
+// Cholesky-QR's V = Y M (evecs null).
+constexpr int TS_RITZ_ROWS = 8;
+__global__ void __launch_bounds__(32 * TS_RITZ_ROWS) k_ts_ritz(const float2* __restrict__ V, const float2* __restrict__ Qo,
+                                                              int T, double2* __restrict__ evecs, float2* __restrict__ Vw)
 {
     wait_prior_kernels();
     __shared__ float2 q[TS_P][TS_P];
-    __shared__ float2 u[TS_P][TS_P + 1];
+    __shared__ float2 u[TS_RITZ_ROWS][TS_P + 1];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int t0 = blockIdx.x * TS_P;
-    for (int e = tid; e < TS_P * TS_P; e += 256)
+    const int t0 = blockIdx.x * TS_RITZ_ROWS, t = t0 + warp;
+    const float2 v = t < T ? V[static_cast<size_t>(t) * TS_P + lane] : make_float2(0.f, 0.f);
+    for (int e = tid; e < TS_P * TS_P; e += 32 * TS_RITZ_ROWS)
         q[e / TS_P][e % TS_P] = Qo[e];
     __syncthreads();
-    for (int rr = warp; rr < TS_P; rr += 8)
-    {
-        const int t = t0 + rr;
-        if (t >= T)
-            break;
-        const float2 v = V[static_cast<size_t>(t) * TS_P + lane];
-        float re = 0.f, im = 0.f;
+    float re = 0.f, im = 0.f;
 #pragma unroll
-        for (int k = 0; k < TS_P; ++k)
-        {
-            const float vx = __shfl_sync(0xffffffffu, v.x, k), vy = __shfl_sync(0xffffffffu, v.y, k);
-            const float2 qq = q[k][lane];
-            re += vx * qq.x - vy * qq.y;
-            im += vx * qq.y + vy * qq.x;
-        }
-        u[rr][lane] = make_float2(re, im);
-        Vw[static_cast<size_t>(t) * TS_P + lane] = make_float2(re, im);
+    for (int k = 0; k < TS_P; ++k)
+    {
+        const float vx = __shfl_sync(0xffffffffu, v.x, k), vy = __shfl_sync(0xffffffffu, v.y, k);
+        const float2 qq = q[k][lane];
+        re += vx * qq.x - vy * qq.y;
+        im += vx * qq.y + vy * qq.x;
     }
+    if (t < T)
+        Vw[static_cast<size_t>(t) * TS_P + lane] = make_float2(re, im);
+    if (!evecs)
+        return;
+    u[warp][lane] = make_float2(re, im);
     __syncthreads();
-    if (evecs && t0 + lane < T)
-        for (int r = warp; r < TS_P; r += 8)
-        {
-            const float2 x = u[lane][r];
-            evecs[static_cast<size_t>(T - TS_P + r) * T + t0 + lane] = make_double2(x.x, x.y);
-        }
+    const int row = tid % TS_RITZ_ROWS, r = tid / TS_RITZ_ROWS;
+    if (t0 + row < T)
+    {
+        const float2 x = u[row][r];
+        evecs[static_cast<size_t>(T - TS_P + r) * T + t0 + row] = make_double2(x.x, x.y);
+    }
 }
+static_assert(TS_RITZ_ROWS == 8, "a thread per row and column of the transpose");
 
 static std::atomic<int> g_eig_precision{HV_EIG_FP32};
 static std::atomic<int> g_cholqr{1};
@@ -3147,7 +3257,7 @@ hv_status pca_eigh(double2* cov, int T, double* evals, double2* evecs, int pmin,
         if (!warm)
         {
             HV_LAUNCH(k_ts_init, gb, 256, 0, st, C32, T, Ys);
-            HV_LAUNCH(k_ts_orth, 1, TS_ORTH_THREADS, 0, st, Ys, T, Vs, nullptr);
+            HV_LAUNCH(k_ts_orth<1>, 1, TS_ORTH_THREADS, 0, st, Ys, T, Vs, nullptr);
         }
         const int iters = warm ? TS_ITERS_WARM : TS_ITERS_COLD;
         int* chol_fail = reinterpret_cast<int*>(scale + 1);
@@ -3159,20 +3269,20 @@ hv_status pca_eigh(double2* cov, int T, double* evals, double2* evecs, int pmin,
             {
                 // Cholesky-QR (Gram, 32 x 32 factorisation, V = Y M), Gram-Schmidt only if it failed
                 HV_LAUNCH(k_ts_gram, TS_P, TS_GRAM_WARPS * 32, 0, st, Ys, Ys, T, Hm);
-                HV_LAUNCH(k_ts_cholqr, 1, 32, 0, st, Hm, Qo, chol_fail);
-                HV_LAUNCH(k_ts_ritz, (T + TS_P - 1) / TS_P, 256, 0, st, Ys, Qo, T, nullptr, Vs);
-                HV_LAUNCH(k_ts_orth, 1, TS_ORTH_THREADS, 0, st, Ys, T, Vs, chol_fail);
+                HV_LAUNCH(k_ts_cholqr, 1, TS_CHOL_WARPS * 32, 0, st, Hm, Qo, chol_fail);
+                HV_LAUNCH(k_ts_ritz, (T + TS_RITZ_ROWS - 1) / TS_RITZ_ROWS, 32 * TS_RITZ_ROWS, 0, st, Ys, Qo, T, nullptr, Vs);
+                HV_LAUNCH(k_ts_orth<4>, 1, TS_ORTH_THREADS, 0, st, Ys, T, Vs, chol_fail);
                 extra += 3;
             }
             else
             {
-                HV_LAUNCH(k_ts_orth, 1, TS_ORTH_THREADS, 0, st, Ys, T, Vs, nullptr);
+                HV_LAUNCH(k_ts_orth<1>, 1, TS_ORTH_THREADS, 0, st, Ys, T, Vs, nullptr);
             }
         }
         HV_LAUNCH(k_ts_matmul, gm, mm_threads, 0, st, C32, Vs, T, Ys);
         HV_LAUNCH(k_ts_gram, TS_P, TS_GRAM_WARPS * 32, 0, st, Vs, Ys, T, Hm);
         HV_LAUNCH(k_ts_rr, 1, JS_MID, 0, st, Hm, T, scale, evals, Qo);
-        HV_LAUNCH(k_ts_ritz, (T + TS_P - 1) / TS_P, 256, 0, st, Vs, Qo, T, evecs, Vw);
+        HV_LAUNCH(k_ts_ritz, (T + TS_RITZ_ROWS - 1) / TS_RITZ_ROWS, 32 * TS_RITZ_ROWS, 0, st, Vs, Qo, T, evecs, Vw);
         count_launch(5 + 2 * iters + extra + (warm ? 0 : 2));
         // two corrections: on 512 x 512 frames with T = 512 and stride 64, one warm iteration and two
         // corrections reach the view error of three and three (3.5e-7 .. 1.9e-6 from FP64)
