@@ -836,8 +836,8 @@ hv_status cov_tc_planes(const uint16_t* planes, int T, size_t npix, double2* cov
                                                          static_cast<int>(smem));
     HV_CUDA_TRY(attr);
     float* tpart = static_cast<float*>(work);
-    HV_LAUNCH(k_cov_tc_tiled, q.nsplit * tl.n, TP_THREADS, smem, st, tmap, npix, tl, q.chunks_per_split, tpart, err);
-    HV_LAUNCH(k_cov_tc_tiled_reduce, (T * T + TR_ENTRIES - 1) / TR_ENTRIES, TR_ENTRIES * TR_GROUPS, 0, st, tpart, T, tl,
+    HV_LAUNCH_BESIDE(k_cov_tc_tiled, q.nsplit * tl.n, TP_THREADS, smem, st, tmap, npix, tl, q.chunks_per_split, tpart, err);
+    HV_LAUNCH_BESIDE(k_cov_tc_tiled_reduce, (T * T + TR_ENTRIES - 1) / TR_ENTRIES, TR_ENTRIES * TR_GROUPS, 0, st, tpart, T, tl,
               q.nsplit, real ? 1 : 0, cov);
     count_launch(2);
     return HV_OK;

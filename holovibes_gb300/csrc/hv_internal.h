@@ -44,7 +44,10 @@ __device__ __forceinline__ void wait_prior_kernels() { asm volatile("griddepcont
 // stream: a 1 us kernel takes 4.1 us per ordinary launch and 1.5 us so, a 5.9 us one 8.2 and 6.6 us (ordinary
 // completions are seen at ticks of about 2 us). Stream captures take the ordinary launch: a graph's
 // kernels already follow one another within 0.6 us.
-template <class... P, class... A>
+// BESIDE: for the kernels of the pipelined PCA windows, which run beside the covariance of another window: they
+// ask for its split of L1 and shared memory (the largest share of shared memory), because an SM changes its
+// split only when it is empty.
+template <bool BESIDE = false, class... P, class... A>
 inline cudaError_t launch_kernel(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args)
 {
     cudaLaunchConfig_t c{};
@@ -52,14 +55,16 @@ inline cudaError_t launch_kernel(void (*kernel)(P...), dim3 grid, dim3 block, si
     c.blockDim = block;
     c.dynamicSmemBytes = smem;
     c.stream = st;
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    at[1].val.sharedMemCarveout = cudaSharedmemCarveoutMaxShared;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone)
     {
         c.attrs = at;
-        c.numAttrs = 1;
+        c.numAttrs = BESIDE ? 2 : 1;
     }
     return cudaLaunchKernelEx(&c, kernel, P(args)...);
 }
@@ -191,10 +196,18 @@ void set_eig_cholqr(int on);
 // which the FP32 sweeps start (T <= 64). `kept_only`: the caller uses only the refined
 // eigenvectors and the order of the eigenvalues (coarser sweeps, FP32 Rayleigh quotients for the
 // others). `cov_kept` (optional): false when the eigensolve overwrote `cov` (the FP64 sweeps in
-// global memory).
+// global memory). `corr` (optional): the FP64 corrections run on its stream (everything is finished
+// there), so that the next call's sweeps can start on `st` beside them, with other evals, evecs and
+// cov; `weights` are not written before its event weights_free.
+struct EigCorrections
+{
+    cudaStream_t st;
+    cudaEvent_t sweeps_done;   // recorded and waited for by the call
+    cudaEvent_t weights_free;  // null: free
+};
 hv_status pca_eigh(double2* cov, int T, double* evals, double2* evecs, int pmin, int pmax, float2* weights, void* work,
                    cudaStream_t st, int refine_lo, int refine_hi, bool warm = false, bool kept_only = false,
-                   bool* cov_kept = nullptr);
+                   bool* cov_kept = nullptr, const EigCorrections* corr = nullptr);
 
 // view_tc.cu
 bool view_tc_supported(int K);
@@ -266,5 +279,6 @@ hv_status contrast_to_ushort_normalized(const float* frame, const float* range, 
 
 // One kernel launch: kernel, grid, block, dynamic shared memory, stream, arguments.
 #define HV_LAUNCH(...) HV_CUDA_TRY(hv::launch_kernel(__VA_ARGS__))
+#define HV_LAUNCH_BESIDE(...) HV_CUDA_TRY(hv::launch_kernel<true>(__VA_ARGS__))
 // Zeroes device memory in stream order (a multiple of 4 bytes).
 #define HV_LAUNCH_ZERO(ptr, bytes, st) HV_CUDA_TRY(hv::launch_zero(ptr, bytes, st))

@@ -69,9 +69,9 @@ void free_buffers(hv_pipe* p)
             }
         L = hv_pipe::Lane{};
     }
-    for (cudaEvent_t* e : {&p->join_ev, &p->range_ev, &p->pp_cov_ev[0], &p->pp_cov_ev[1], &p->pp_eig_ev[0],
-                           &p->pp_eig_ev[1], &p->pp_view_ev[0], &p->pp_view_ev[1], &p->pp_view_ev[2],
-                           &p->pp_view_ev[3]})
+    for (cudaEvent_t* e : {&p->join_ev, &p->range_ev, &p->pp_sweeps_ev, &p->pp_cov_ev[0], &p->pp_cov_ev[1], &p->pp_cov_ev[2],
+                           &p->pp_cov_ev[3], &p->pp_eig_ev[0], &p->pp_eig_ev[1], &p->pp_eig_ev[2], &p->pp_eig_ev[3],
+                           &p->pp_view_ev[0], &p->pp_view_ev[1], &p->pp_view_ev[2], &p->pp_view_ev[3]})
         if (*e)
         {
             cudaEventDestroy(*e);
@@ -147,7 +147,9 @@ bool uses_planes(const hv_frame_desc& fd, const hv_settings& s, bool served);
 // a ring of 16-bit samples with room for two more batches than the window, so a window's eigensolve
 // overlaps the next batch's conversion and covariance update and the previous window's view. (With views
 // that read planes and complex slots, and a ring rebuild behind each view that the next conversion had to wait
-// for, the streams hardly overlapped: 512 frames of 512 x 512, stride 64, 406 us a window; so 315 us.)
+// for, the streams hardly overlapped: 512 frames of 512 x 512, stride 64, 406 us a window; with the sample ring
+// 315 us, with eigensolve kernels that fit beside the covariance 294 us, with the corrections on their own stream and four
+// covariance buffers 270 us. The covariance and the view, each of which fills the SMs, bound it now.)
 bool uses_pca_pipeline(const hv_frame_desc& fd, const hv_settings& s, bool served)
 {
     const int T = s.time_transformation_size, B = s.batch_size;
@@ -199,8 +201,9 @@ size_t footprint(const hv_frame_desc& fd, const hv_settings& s, bool served = fa
     }
     if (uses_planes(fd, s, served))
         z.add(cov_planes_bytes(T, HW, planes_real(s)));
-    if (uses_pca_pipeline(fd, s, served))  // the second covariance and weights buffers, the sample ring
+    if (uses_pca_pipeline(fd, s, served))  // the second buffers of the windows in flight, the sample ring
     {
+        z.add(3 * static_cast<size_t>(T) * T * 16 + static_cast<size_t>(T) * 8);
         z.add(static_cast<size_t>(T) * T * 16 + static_cast<size_t>(K > 0 ? K : 1) * T * 8);
         z.add(HW * 2 * (static_cast<size_t>(T) + 2 * B));
     }
@@ -498,13 +501,20 @@ hv_status build(hv_pipe* p)
             return st;
         p->render_stream = p->render_stream_owned;
         p->pp_cov[0] = p->cov;
-        if ((st = dalloc(p, p->pp_cov[1], static_cast<size_t>(p->T) * p->T * sizeof(double2))) != HV_OK)
-            return st;
+        for (int i = 1; i < 4; ++i)
+            if ((st = dalloc(p, p->pp_cov[i], static_cast<size_t>(p->T) * p->T * sizeof(double2))) != HV_OK)
+                return st;
         p->pp_weights[0] = p->weights;
+        p->pp_evecs[0] = p->evecs;
+        p->pp_evals[0] = p->evals;
+        if ((st = dalloc(p, p->pp_evecs[1], static_cast<size_t>(p->T) * p->T * sizeof(double2))) != HV_OK ||
+            (st = dalloc(p, p->pp_evals[1], static_cast<size_t>(p->T) * sizeof(double))) != HV_OK)
+            return st;
         if ((st = dalloc(p, p->pp_weights[1], static_cast<size_t>(p->K) * p->T * sizeof(float2))) != HV_OK)
             return st;
-        for (cudaEvent_t* e : {&p->pp_cov_ev[0], &p->pp_cov_ev[1], &p->pp_eig_ev[0], &p->pp_eig_ev[1],
-                               &p->pp_view_ev[0], &p->pp_view_ev[1], &p->pp_view_ev[2], &p->pp_view_ev[3]})
+        for (cudaEvent_t* e : {&p->pp_sweeps_ev, &p->pp_cov_ev[0], &p->pp_cov_ev[1], &p->pp_cov_ev[2], &p->pp_cov_ev[3],
+                               &p->pp_eig_ev[0], &p->pp_eig_ev[1], &p->pp_eig_ev[2], &p->pp_eig_ev[3], &p->pp_view_ev[0],
+                               &p->pp_view_ev[1], &p->pp_view_ev[2], &p->pp_view_ev[3]})
             HV_CUDA_TRY(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
     }
     // lens (computed once per refresh, fourier_transform.cc:93-137)
@@ -610,22 +620,22 @@ hv_status refresh_ring(hv_pipe* p)
     return r;
 }
 
-// The covariance and eigensolve of a PCA window of the three-stream pipeline (p->pp): the update
-// of covariance buffer w % 2 on the pipe stream (from the other buffer, the previous window's),
-// the eigensolve into weights buffer w % 2 on the eigensolve stream, then the view on the render
-// stream `st` (render_view's view part, with p->weights bound to the window's buffer).
+// The covariance and eigensolve of a PCA window of the pipelined windows (p->pp): the update of
+// covariance buffer w % 4 on the pipe stream (from the previous window's), the eigensolve into weights
+// buffer w % 2 on the eigensolve stream, its FP64 corrections on the corrections' stream, then the view
+// on the render stream `st` (render_view's view part, with p->weights bound to the window's buffer).
 hv_status render_view_pp(hv_pipe* p, cudaStream_t st, uint32_t dirty, uint32_t all, const float** frame,
                          int* shift_after)
 {
-    const int w = p->pp_w++, i = w & 1;
-    double2* cov = p->pp_cov[i];
+    const int w = p->pp_w++, i = w & 1, c = w & 3;
+    double2* cov = p->pp_cov[c];
     cudaStream_t es = p->eig_stream;
     hv_status r;
-    if (w >= 2)  // window w - 2's eigensolve read this buffer
-        HV_CUDA_TRY(cudaStreamWaitEvent(p->stream, p->pp_eig_ev[i], 0));
+    if (w >= 4)  // window w - 4's eigensolve read this buffer
+        HV_CUDA_TRY(cudaStreamWaitEvent(p->stream, p->pp_eig_ev[c], 0));
     const bool inc = w >= 1 && p->cov_valid && p->cov_mode == cov_mode() && dirty != all && cov_incremental();
     if (inc)
-        HV_CUDA_TRY(cudaMemcpyAsync(cov, p->pp_cov[i ^ 1], static_cast<size_t>(p->T) * p->T * sizeof(double2),
+        HV_CUDA_TRY(cudaMemcpyAsync(cov, p->pp_cov[(w - 1) & 3], static_cast<size_t>(p->T) * p->T * sizeof(double2),
                                     cudaMemcpyDeviceToDevice, p->stream));
     if (!inc || dirty)
     {
@@ -646,18 +656,21 @@ hv_status render_view_pp(hv_pipe* p, cudaStream_t st, uint32_t dirty, uint32_t a
     }
     p->cov_dirty = 0;
     p->cov_mode = cov_mode();
-    HV_CUDA_TRY(cudaEventRecord(p->pp_cov_ev[i], p->stream));
-    HV_CUDA_TRY(cudaStreamWaitEvent(es, p->pp_cov_ev[i], 0));
-    if (w >= 2)  // window w - 2's view read this weights buffer
-        HV_CUDA_TRY(cudaStreamWaitEvent(es, p->pp_view_ev[(w - 2) & 3], 0));
+    HV_CUDA_TRY(cudaEventRecord(p->pp_cov_ev[c], p->stream));
+    HV_CUDA_TRY(cudaStreamWaitEvent(es, p->pp_cov_ev[c], 0));
+    if (w >= 2)  // window w - 2's corrections read these eigenvectors
+        HV_CUDA_TRY(cudaStreamWaitEvent(es, p->pp_eig_ev[(w - 2) & 3], 0));
+    // the corrections of window w run beside the sweeps of window w + 1; window w - 2's view read this
+    // weights buffer
+    const EigCorrections corr{p->corr_stream, p->pp_sweeps_ev, w >= 2 ? p->pp_view_ev[(w - 2) & 3] : nullptr};
     bool kept = false;
-    if ((r = pca_eigh(cov, p->T, p->evals, p->evecs, p->pmin, p->pmax, p->pp_weights[i], p->eig_work, es, p->pmin,
-                      p->pmax, p->eig_warm, true, &kept)) != HV_OK)
+    if ((r = pca_eigh(cov, p->T, p->pp_evals[i], p->pp_evecs[i], p->pmin, p->pmax, p->pp_weights[i], p->eig_work, es,
+                      p->pmin, p->pmax, p->eig_warm, true, &kept, &corr)) != HV_OK)
         return r;
     p->eig_warm = true;
     p->cov_valid = kept;
-    HV_CUDA_TRY(cudaEventRecord(p->pp_eig_ev[i], es));
-    HV_CUDA_TRY(cudaStreamWaitEvent(st, p->pp_eig_ev[i], 0));
+    HV_CUDA_TRY(cudaEventRecord(p->pp_eig_ev[c], p->corr_stream));
+    HV_CUDA_TRY(cudaStreamWaitEvent(st, p->pp_eig_ev[c], 0));
     p->weights = p->pp_weights[i];
     p->pp_nested = true;
     r = render_view(p, st, nullptr, frame, shift_after);
@@ -1484,7 +1497,8 @@ hv_pipe* hv_pipe_create(const hv_frame_desc* fd, const hv_settings* settings, vo
         cudaStreamCreateWithFlags(&p->render_extra[0], cudaStreamNonBlocking) != cudaSuccess ||
         cudaStreamCreateWithFlags(&p->render_extra[1], cudaStreamNonBlocking) != cudaSuccess ||
         cudaDeviceGetStreamPriorityRange(&least_prio, &greatest_prio) != cudaSuccess ||
-        cudaStreamCreateWithPriority(&p->eig_stream, cudaStreamNonBlocking, greatest_prio) != cudaSuccess)
+        cudaStreamCreateWithPriority(&p->eig_stream, cudaStreamNonBlocking, greatest_prio) != cudaSuccess ||
+        cudaStreamCreateWithPriority(&p->corr_stream, cudaStreamNonBlocking, greatest_prio) != cudaSuccess)
     {
         out = HV_ERR_CUDA;
         hv_pipe_destroy(p);
@@ -1514,6 +1528,8 @@ void hv_pipe_destroy(hv_pipe* p)
             cudaStreamSynchronize(e);
     if (p->eig_stream)
         cudaStreamSynchronize(p->eig_stream);
+    if (p->corr_stream)
+        cudaStreamSynchronize(p->corr_stream);
     free_buffers(p);
     if (p->copy_stream)
         cudaStreamDestroy(p->copy_stream);
@@ -1524,6 +1540,8 @@ void hv_pipe_destroy(hv_pipe* p)
             cudaStreamDestroy(e);
     if (p->eig_stream)
         cudaStreamDestroy(p->eig_stream);
+    if (p->corr_stream)
+        cudaStreamDestroy(p->corr_stream);
     if (p->own_stream && p->stream)
         cudaStreamDestroy(p->stream);
     delete p;
@@ -1634,7 +1652,10 @@ static hv_status sync_render(hv_pipe* p)
 {
     HV_CUDA_TRY(cudaStreamSynchronize(p->render_stream));
     if (p->pp)
+    {
         HV_CUDA_TRY(cudaStreamSynchronize(p->eig_stream));
+        HV_CUDA_TRY(cudaStreamSynchronize(p->corr_stream));
+    }
     if (p->nrender > 1)
         for (int l = 0; l < p->nrender; ++l)
             HV_CUDA_TRY(cudaStreamSynchronize(p->lanes[l].st));

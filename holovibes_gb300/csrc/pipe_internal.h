@@ -61,7 +61,8 @@ struct hv_pipe
     Lane lanes[kMaxLanes];
     int nlanes = 0, nrender = 1;
     cudaStream_t render_extra[kMaxLanes - 1] = {nullptr, nullptr};  // render streams of lanes 1, 2
-    cudaStream_t eig_stream = nullptr;  // the pipelined PCA windows' eigensolves (greatest priority)
+    // the pipelined PCA windows' eigensolves and their FP64 corrections (greatest priority)
+    cudaStream_t eig_stream = nullptr, corr_stream = nullptr;
     cudaEvent_t range_ev = nullptr;  // after the last autocontrast (lanes with their own streams)
     bool range_ev_set = false;
     cudaEvent_t join_ev = nullptr;
@@ -84,16 +85,20 @@ struct hv_pipe
     int planes_real = 0;  // the ring's imaginary parts are 0: real rows only
     // PCA windows pipelined over three streams (pipe.cpp, `pp`): the pipe stream converts each
     // batch into the split planes and a ring of 16-bit samples and updates the covariance, the
-    // eigensolve stream solves it, the render stream views the samples and renders; covariance and
-    // weights alternate between two buffers by window parity. The sample ring holds pp_cap = T + 2 B
+    // eigensolve stream solves it, the corrections' stream corrects the kept eigenvectors, the render
+    // stream views the samples and renders; eigenvectors and weights alternate between two buffers, the
+    // covariance goes round four (its update must not wait for the corrections of the window before last). The sample ring holds pp_cap = T + 2 B
     // frames, the next one goes to pp_head. `ring` is not written on the way: its newest ring_stale
     // slots are rebuilt from the planes when they are asked for (refresh_ring).
     bool pp = false, pp_nested = false;
     int pp_w = 0, pp_cap = 0, pp_head = 0, ring_stale = 0;
     uint16_t* pp_samples = nullptr;
-    double2* pp_cov[2] = {nullptr, nullptr};
+    double2* pp_cov[4] = {nullptr, nullptr, nullptr, nullptr};
     float2* pp_weights[2] = {nullptr, nullptr};
-    cudaEvent_t pp_cov_ev[2] = {nullptr, nullptr}, pp_eig_ev[2] = {nullptr, nullptr};
+    double2* pp_evecs[2] = {nullptr, nullptr};
+    double* pp_evals[2] = {nullptr, nullptr};
+    cudaEvent_t pp_sweeps_ev = nullptr;
+    cudaEvent_t pp_cov_ev[4] = {nullptr, nullptr, nullptr, nullptr}, pp_eig_ev[4] = {nullptr, nullptr, nullptr, nullptr};
     cudaEvent_t pp_view_ev[4] = {nullptr, nullptr, nullptr, nullptr};
     float* view = nullptr;
     float* unwrapped = nullptr;

@@ -1542,7 +1542,7 @@ hv_status convert_window(const void* raw, int kind, size_t HW, int batch, int sl
     const bool vec = (reinterpret_cast<uintptr_t>(raw) & 15) == 0;
     auto kern = kind == IN_U8 ? (vec ? k_convert_window<IN_U8, true> : k_convert_window<IN_U8, false>)
                               : (vec ? k_convert_window<IN_U16, true> : k_convert_window<IN_U16, false>);
-    HV_LAUNCH(kern, grid, block, 0, st, raw, kind == IN_U16_BE ? 1 : 0, HW, batch, slot0, T, planes, sample0, cap, samples);
+    HV_LAUNCH_BESIDE(kern, grid, block, 0, st, raw, kind == IN_U16_BE ? 1 : 0, HW, batch, slot0, T, planes, sample0, cap, samples);
     count_launch();
     return HV_OK;
 }

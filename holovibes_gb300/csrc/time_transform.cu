@@ -422,7 +422,9 @@ __device__ __forceinline__ void tvp_ring(float2 (&a)[2][KC], const float4* __res
 
 // Pixel pairs 64 pixels apart (GROUPS of them per thread) of the window's real samples from 16-bit integers.
 // The integer becomes a float in the mantissa of 2^23 (exact, no conversion unit); the multiply-adds, those
-// of the other sources, go two to an instruction.
+// of the other sources, go two to an instruction. Bound by the issue of these: 512 frames of 512 x 512, 4
+// bins, 268 MB: 76 us (115 us from the planes and the ring); neither asynchronous copies into shared memory nor weights stored
+// as packed pairs nor more warps made it faster (78 to 90 us).
 template <int KC, int GROUPS>
 __device__ __forceinline__ void tvp_samples(float2 (&a)[GROUPS][2][KC], const uint32_t* const (&x)[GROUPS], size_t at,
                                             size_t step, int t0, int n, const float2* wsm)
@@ -731,7 +733,7 @@ static hv_status launch_time_view_real(const Source& source, int T, int W, int H
         HV_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
     const size_t HW = static_cast<size_t>(W) * H;
     const int grid = static_cast<int>((HW + 2 * TV_THREADS - 1) / (2 * TV_THREADS));
-    HV_LAUNCH(kern, grid, TV_THREADS / Source::GROUPS, smem, st, source, T, W, H, weights, K, img_type, scale, shift, out, partials,
+    HV_LAUNCH_BESIDE(kern, grid, TV_THREADS / Source::GROUPS, smem, st, source, T, W, H, weights, K, img_type, scale, shift, out, partials,
               time_view_partials(W, H), ctl, bin_w);
     count_launch();
     return HV_OK;
@@ -2415,13 +2417,15 @@ __device__ __forceinline__ double2 warp_sum2_real(double2 v)
     return v;
 }
 
-// Y[j][t] = sum_s C[t][s] v_{r0+j}[s]; grid (ceil(T / 8), K), 256 threads
+// Y[j][t] = sum_s C[t][s] v_{r0+j}[s]; grid (ceil(T / ER_MV_ROWS), K), a warp per row. Small CTAs: they fit
+// into what the covariance and a view leave of an SM.
+constexpr int ER_MV_ROWS = 2;
 __global__ void k_eigref_matvec(const double2* __restrict__ C, const double2* __restrict__ evecs, int T, int r0,
                                 double2* __restrict__ Y)
 {
     wait_prior_kernels();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int t = blockIdx.x * 8 + warp, j = blockIdx.y;
+    const int t = blockIdx.x * ER_MV_ROWS + warp, j = blockIdx.y;
     if (t >= T)
         return;
     const double2* v = evecs + static_cast<size_t>(r0 + j) * T;
@@ -2526,8 +2530,8 @@ __global__ void __launch_bounds__(32 * ER_UPD_WARPS) k_eigref_update(const doubl
                                                                     int K, int b0, double2* __restrict__ Vn)
 {
     wait_prior_kernels();
-    __shared__ double2 coef[JC_MAX_T];
-    __shared__ double2 comp[JC_MAX_T];
+    extern __shared__ __align__(16) double2 er_coef[];  // of the basis vectors b0 .. T - 1
+    double2 *coef = er_coef, *comp = er_coef + (T - b0);
     __shared__ double2 pacc[ER_UPD_WARPS][32], pproj[ER_UPD_WARPS][32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int t = blockIdx.x * 32 + lane, j = blockIdx.y;
@@ -2549,21 +2553,21 @@ __global__ void __launch_bounds__(32 * ER_UPD_WARPS) k_eigref_update(const doubl
             const double inv = 1.0 / gap;
             c = make_double2(cr.x * inv, cr.y * inv);
         }
-        coef[i] = c;
-        comp[i] = cr;
+        coef[i - b0] = c;
+        comp[i - b0] = cr;
     }
     __syncthreads();
     double2 acc = make_double2(0.0, 0.0), proj = make_double2(0.0, 0.0);
     if (t < T)
         for (int i = b0 + warp; i < T; i += ER_UPD_WARPS)
         {
-            const double2 c = coef[i];
+            const double2 c = coef[i - b0];
             const double2 v = evecs[static_cast<size_t>(i) * T + t];
             acc.x += v.x * c.x - v.y * c.y;
             acc.y += v.x * c.y + v.y * c.x;
             if (b0 > 0)
             {
-                const double2 cr = comp[i];
+                const double2 cr = comp[i - b0];
                 proj.x += v.x * cr.x - v.y * cr.y;
                 proj.y += v.x * cr.y + v.y * cr.x;
             }
@@ -3184,7 +3188,8 @@ size_t pca_eigh_workspace(int T)
 }
 
 hv_status pca_eigh(double2* cov, int T, double* evals, double2* evecs, int pmin, int pmax, float2* weights, void* work,
-                   cudaStream_t st, int refine_lo, int refine_hi, bool warm, bool kept_only, bool* cov_kept)
+                   cudaStream_t st, int refine_lo, int refine_hi, bool warm, bool kept_only, bool* cov_kept,
+                   const EigCorrections* corr)
 {
     if (cov_kept)
         *cov_kept = true;
@@ -3222,22 +3227,34 @@ hv_status pca_eigh(double2* cov, int T, double* evals, double2* evecs, int pmin,
     // covariance, with the eigenvectors of ranks b0 .. T-1 as the basis; `iters` corrections (the
     // first leaves O(theta^2) against the FP32 error of the basis, the next bring that to the FP64
     // level)
-    auto refine_kept = [&](int b0, int iters) -> hv_status {
+    auto refine_kept = [&](int b0, int iters, cudaStream_t st) -> hv_status {
         double2* Y = reinterpret_cast<double2*>(er_base);
         double2* D = Y + static_cast<size_t>(ER_MAX_K) * T;
         double2* G = D + static_cast<size_t>(ER_MAX_K) * T;
         double2* Vn = G + static_cast<size_t>(ER_MAX_K) * T;
-        const dim3 gw((T + 7) / 8, Kr), gp(T - b0, Kr), gt((T + 31) / 32, Kr);
+        const dim3 gw((T + ER_MV_ROWS - 1) / ER_MV_ROWS, Kr), gp(T - b0, Kr), gt((T + 31) / 32, Kr);
         for (int iter = 0; iter < iters; ++iter)
         {
-            HV_LAUNCH(k_eigref_matvec, gw, 256, 0, st, cov, evecs, T, refine_lo, Y);
-            HV_LAUNCH(k_eigref_project, gp, ER_PROJ_THREADS, 0, st, evecs, Y, T, refine_lo, b0, D, G);
-            HV_LAUNCH(k_eigref_update, gt, 32 * ER_UPD_WARPS, 0, st, evecs, evals, D, G, Y, T, refine_lo, Kr, b0, Vn);
-            HV_LAUNCH(k_eigref_finish, Kr, 128, 0, st, evecs, evals, Vn, D, G, T, refine_lo, pmin, pmax, weights);
+            HV_LAUNCH_BESIDE(k_eigref_matvec, gw, 32 * ER_MV_ROWS, 0, st, cov, evecs, T, refine_lo, Y);
+            HV_LAUNCH_BESIDE(k_eigref_project, gp, ER_PROJ_THREADS, 0, st, evecs, Y, T, refine_lo, b0, D, G);
+            HV_LAUNCH_BESIDE(k_eigref_update, gt, 32 * ER_UPD_WARPS, 2 * static_cast<size_t>(T - b0) * sizeof(double2), st,
+                             evecs, evals, D, G, Y, T, refine_lo, Kr, b0, Vn);
+            HV_LAUNCH_BESIDE(k_eigref_finish, Kr, 128, 0, st, evecs, evals, Vn, D, G, T, refine_lo, pmin, pmax, weights);
             count_launch(4);
         }
         return HV_OK;
     };
+    // the stream of the corrections, behind what `st` has done so far
+    auto corrections = [&](cudaStream_t& cs) -> hv_status {
+        cs = st;
+        if (!corr)
+            return HV_OK;
+        cs = corr->st;
+        HV_CUDA_TRY(cudaEventRecord(corr->sweeps_done, st));
+        HV_CUDA_TRY(cudaStreamWaitEvent(cs, corr->sweeps_done, 0));
+        return HV_OK;
+    };
+    cudaStream_t cs = st;
     // the largest eigenpairs only: subspace iteration instead of the block Jacobi
     if (loose && prec == HV_EIG_FP32 && T > JS_MAX_T && T <= JC_MAX_T && refine_lo >= T - TS_MAX_KEEP)
     {
@@ -3251,43 +3268,51 @@ hv_status pca_eigh(double2* cov, int T, double* evals, double2* evecs, int pmin,
         const int gb = (T * TS_P + 255) / 256;
         const int gm = (T + TS_MM_ROWS - 1) / TS_MM_ROWS;
         constexpr int mm_threads = TS_MM_ROWS * TS_MM_SPLIT * 32;
-        HV_LAUNCH(k_ts_convert, std::min(512, (T * T + 1023) / 1024), 256, 0, st, cov, T, C32, scale);
+        HV_LAUNCH_BESIDE(k_ts_convert, std::min(512, (T * T + 1023) / 1024), 256, 0, st, cov, T, C32, scale);
         // warm: the previous window's Ritz vectors are orthonormal (V Q with V orthonormal, Q unitary)
         // and start the iteration as they are
         if (!warm)
         {
-            HV_LAUNCH(k_ts_init, gb, 256, 0, st, C32, T, Ys);
-            HV_LAUNCH(k_ts_orth<1>, 1, TS_ORTH_THREADS, 0, st, Ys, T, Vs, nullptr);
+            HV_LAUNCH_BESIDE(k_ts_init, gb, 256, 0, st, C32, T, Ys);
+            HV_LAUNCH_BESIDE(k_ts_orth<1>, 1, TS_ORTH_THREADS, 0, st, Ys, T, Vs, nullptr);
         }
         const int iters = warm ? TS_ITERS_WARM : TS_ITERS_COLD;
         int* chol_fail = reinterpret_cast<int*>(scale + 1);
         int extra = 0;
         for (int it = 0; it < iters; ++it)
         {
-            HV_LAUNCH(k_ts_matmul, gm, mm_threads, 0, st, C32, it == 0 && warm ? Vw : Vs, T, Ys);
+            HV_LAUNCH_BESIDE(k_ts_matmul, gm, mm_threads, 0, st, C32, it == 0 && warm ? Vw : Vs, T, Ys);
             if (warm && cholqr_enabled())
             {
                 // Cholesky-QR (Gram, 32 x 32 factorisation, V = Y M), Gram-Schmidt only if it failed
-                HV_LAUNCH(k_ts_gram, TS_P, TS_GRAM_WARPS * 32, 0, st, Ys, Ys, T, Hm);
-                HV_LAUNCH(k_ts_cholqr, 1, TS_CHOL_WARPS * 32, 0, st, Hm, Qo, chol_fail);
-                HV_LAUNCH(k_ts_ritz, (T + TS_RITZ_ROWS - 1) / TS_RITZ_ROWS, 32 * TS_RITZ_ROWS, 0, st, Ys, Qo, T, nullptr, Vs);
-                HV_LAUNCH(k_ts_orth<4>, 1, TS_ORTH_THREADS, 0, st, Ys, T, Vs, chol_fail);
+                HV_LAUNCH_BESIDE(k_ts_gram, TS_P, TS_GRAM_WARPS * 32, 0, st, Ys, Ys, T, Hm);
+                HV_LAUNCH_BESIDE(k_ts_cholqr, 1, TS_CHOL_WARPS * 32, 0, st, Hm, Qo, chol_fail);
+                HV_LAUNCH_BESIDE(k_ts_ritz, (T + TS_RITZ_ROWS - 1) / TS_RITZ_ROWS, 32 * TS_RITZ_ROWS, 0, st, Ys, Qo, T, nullptr, Vs);
+                HV_LAUNCH_BESIDE(k_ts_orth<4>, 1, TS_ORTH_THREADS, 0, st, Ys, T, Vs, chol_fail);
                 extra += 3;
             }
             else
             {
-                HV_LAUNCH(k_ts_orth<1>, 1, TS_ORTH_THREADS, 0, st, Ys, T, Vs, nullptr);
+                HV_LAUNCH_BESIDE(k_ts_orth<1>, 1, TS_ORTH_THREADS, 0, st, Ys, T, Vs, nullptr);
             }
         }
-        HV_LAUNCH(k_ts_matmul, gm, mm_threads, 0, st, C32, Vs, T, Ys);
-        HV_LAUNCH(k_ts_gram, TS_P, TS_GRAM_WARPS * 32, 0, st, Vs, Ys, T, Hm);
-        HV_LAUNCH(k_ts_rr, 1, JS_MID, 0, st, Hm, T, scale, evals, Qo);
-        HV_LAUNCH(k_ts_ritz, (T + TS_RITZ_ROWS - 1) / TS_RITZ_ROWS, 32 * TS_RITZ_ROWS, 0, st, Vs, Qo, T, evecs, Vw);
+        HV_LAUNCH_BESIDE(k_ts_matmul, gm, mm_threads, 0, st, C32, Vs, T, Ys);
+        HV_LAUNCH_BESIDE(k_ts_gram, TS_P, TS_GRAM_WARPS * 32, 0, st, Vs, Ys, T, Hm);
+        HV_LAUNCH_BESIDE(k_ts_rr, 1, JS_MID, 0, st, Hm, T, scale, evals, Qo);
+        HV_LAUNCH_BESIDE(k_ts_ritz, (T + TS_RITZ_ROWS - 1) / TS_RITZ_ROWS, 32 * TS_RITZ_ROWS, 0, st, Vs, Qo, T, evecs, Vw);
         count_launch(5 + 2 * iters + extra + (warm ? 0 : 2));
         // two corrections: on 512 x 512 frames with T = 512 and stride 64, one warm iteration and two
         // corrections reach the view error of three and three (3.5e-7 .. 1.9e-6 from FP64)
-        return refine_kept(T - TS_P, 2);
+        // (the weights are first written there)
+        const hv_status rc = corrections(cs);
+        if (rc != HV_OK)
+            return rc;
+        if (corr && corr->weights_free)
+            HV_CUDA_TRY(cudaStreamWaitEvent(cs, corr->weights_free, 0));
+        return refine_kept(T - TS_P, 2, cs);
     }
+    if (corr && corr->weights_free)
+        HV_CUDA_TRY(cudaStreamWaitEvent(st, corr->weights_free, 0));
     if (T <= JS_MAX_T && prec == HV_EIG_FP32)
     {
         const size_t smem = jacobi_smem_bytes<float>(T, warm);
@@ -3363,9 +3388,12 @@ hv_status pca_eigh(double2* cov, int T, double* evals, double2* evecs, int pmin,
     count_launch(2);
     // FP32 sweeps: the kept eigenvectors are corrected in FP64 (FP64 sweeps need no correction)
     const bool fp32_sweeps = T <= JS_MAX_T ? prec == HV_EIG_FP32 : (T <= JC_MAX_T && prec == HV_EIG_FP32);
+    const hv_status rc = corrections(cs);
+    if (rc != HV_OK)
+        return rc;
     if (fp32_sweeps && refine_lo >= 0 && refine_hi < T && Kr >= 1 && Kr <= ER_MAX_K)
     {
-        hv_status rr = refine_kept(0, loose ? 3 : 2);
+        hv_status rr = refine_kept(0, loose ? 3 : 2, cs);
         if (rr != HV_OK)
             return rr;
     }
