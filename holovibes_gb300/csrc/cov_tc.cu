@@ -38,7 +38,6 @@ constexpr int TC_MMA_WARP = TC_CONVERTERS / 32;  // warp 8 issues the MMAs
 constexpr int TC_LOAD_WARP = TC_MMA_WARP + 1;    // warp 9 issues the tensor copies
 constexpr int TC_THREADS = TC_CONVERTERS + 64;
 constexpr int TC_A_STAGES = 2;
-constexpr int TC_A_STAGES_PACKED = 2;
 constexpr int TC_MAX_RAW = 8;
 constexpr int TC_KC = 64;           // pixels (K elements) per chunk
 constexpr int TC_ROWS = 128;        // M rows of the operand tile (2T <= 128, zero padded)
@@ -58,41 +57,44 @@ __device__ __forceinline__ uint32_t tile_offset(int r, int kgroup) { return tc::
 __device__ __forceinline__ uint64_t smem_desc(uint32_t addr) { return tc::sw128_desc(addr); }
 using tc::instr_desc;
 
-// part: [gridDim.x][2T][2T] FP32 partial G; err: set to 1 when a bounded wait gave up.
+// part: [nparts][2T][2T] FP32 partial G; err: set to 1 when a bounded wait gave up. A CTA takes the
+// parts blockIdx.x, blockIdx.x + gridDim.x, ...: the loads and conversions of the next one run beside the
+// end of the one before (above T = 40 the accumulators leave room for one CTA per SM, which was launched
+// twice). What bounds it is the conversion's latency: raw stages of one chunk, freed as soon as it is converted,
+// and four rows in flight per warp. Covariance with its reduction, 512 x 512 frames: T = 16 38 -> 25.5 us, T = 32
+// 47.6 -> 31.7, T = 64 93 -> 59; 32 frames of 1024 x 768 70 -> 58.
 __global__ void __launch_bounds__(TC_THREADS, 2) k_cov_tc(const __grid_constant__ CUtensorMap ring_map, int T,
-                                                          size_t npix, size_t chunks_per_cta, int N, uint32_t tmem_cols,
-                                                          int raw_stages, int packed, float* __restrict__ part,
-                                                          int* __restrict__ err)
+                                                          size_t npix, size_t chunks_per_part, int nparts, int N,
+                                                          uint32_t tmem_cols, int raw_stages, int packed,
+                                                          float* __restrict__ part, int* __restrict__ err)
 {
     wait_prior_kernels();
     // packed (2T <= 64): one 128-row tile per stage, Yh in rows 0..63 and Yl in rows 64..127, and
     // one 128 x 128 MMA per K step gives [[Yh Yh^T, Yh Yl^T], [Yl Yh^T, Yl Yl^T]];
     // otherwise two tiles (Yh, Yl) and three MMAs into three accumulators
-    const int A_STAGES = packed ? TC_A_STAGES_PACKED : TC_A_STAGES;
     const uint32_t a_stage_bytes = packed ? TILE_BYTES : 2 * TILE_BYTES;
     extern __shared__ __align__(1024) uint8_t smem[];
     // A stages ([hi | lo] tiles) then the raw stages, on 1024-byte boundaries; 1 KB of launch slack
     uint8_t* tiles = smem + ((1024u - (smem_u32(smem) & 1023u)) & 1023u);
-    const uint32_t raw_bytes = static_cast<uint32_t>(T) * TC_KC * 16;  // a pair of chunks: T rows of 1 KB
-    uint8_t* raw_base = tiles + A_STAGES * a_stage_bytes;
+    const uint32_t raw_bytes = static_cast<uint32_t>(T) * TC_KC * 8;  // a chunk: T rows of 512 bytes
+    uint8_t* raw_base = tiles + TC_A_STAGES * a_stage_bytes;
     __shared__ __align__(8) uint64_t raw_full[TC_MAX_RAW], raw_empty[TC_MAX_RAW];
-    __shared__ __align__(8) uint64_t a_full[TC_A_STAGES_PACKED], a_empty[TC_A_STAGES_PACKED];
-    __shared__ __align__(8) uint64_t done, drain;
+    __shared__ __align__(8) uint64_t a_full[TC_A_STAGES], a_empty[TC_A_STAGES];
+    __shared__ __align__(8) uint64_t done, acc_read, drain;
     __shared__ uint32_t tmem_base;
-    __shared__ int s_abort;
+    __shared__ int s_abort, s_issued;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int rows = 2 * T, R = raw_stages;
     const size_t nchunks = (npix + TC_KC - 1) / TC_KC;
-    const size_t c_begin = blockIdx.x * chunks_per_cta;
-    size_t c_end = c_begin + chunks_per_cta;
-    if (c_end > nchunks)
-        c_end = nchunks;
-    const int nmine = static_cast<int>(c_end > c_begin ? c_end - c_begin : 0);
     volatile int* abort = &s_abort;
+    auto chunks_of = [&](int p) -> int {
+        const size_t c0 = static_cast<size_t>(p) * chunks_per_part;
+        return c0 >= nchunks ? 0 : static_cast<int>(nchunks - c0 < chunks_per_part ? nchunks - c0 : chunks_per_part);
+    };
 
     // zero the A tiles once (rows >= 2T stay zero)
-    for (int i = tid; i < A_STAGES * static_cast<int>(a_stage_bytes) / 16; i += TC_THREADS)
+    for (int i = tid; i < TC_A_STAGES * static_cast<int>(a_stage_bytes) / 16; i += TC_THREADS)
         reinterpret_cast<uint4*>(tiles)[i] = make_uint4(0, 0, 0, 0);
     if (tid == 0)
     {
@@ -101,14 +103,16 @@ __global__ void __launch_bounds__(TC_THREADS, 2) k_cov_tc(const __grid_constant_
             mbar_init(&raw_full[i], 1);
             mbar_init(&raw_empty[i], TC_CONVERTERS / 32);
         }
-        for (int i = 0; i < A_STAGES; ++i)
+        for (int i = 0; i < TC_A_STAGES; ++i)
         {
             mbar_init(&a_full[i], TC_CONVERTERS / 32);
             mbar_init(&a_empty[i], 1);
         }
         mbar_init(&done, 1);
+        mbar_init(&acc_read, 4);
         mbar_init(&drain, 1);
         s_abort = 0;
+        s_issued = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == TC_MMA_WARP)
@@ -124,22 +128,31 @@ __global__ void __launch_bounds__(TC_THREADS, 2) k_cov_tc(const __grid_constant_
     tc_fence_after();
     const uint32_t tmem = tmem_base;
 
+    // every role walks the same chunks: it counts them over all parts, k the parts
     if (warp == TC_LOAD_WARP)
     {
         // ------------------------------------------------------------------ loader (TMA)
         if (lane == 0)
         {
             asm volatile("prefetch.tensormap [%0];" ::"l"(&ring_map) : "memory");
-            const int npairs = (nmine + 1) / 2;
-            for (int m = 0; m < npairs; ++m)
+            int it = 0;
+            for (int p = blockIdx.x; p < nparts && !*abort; p += gridDim.x)
             {
-                const int r = m % R;
-                if (m >= R)
-                    mbar_wait(&raw_empty[r], static_cast<uint32_t>(((m / R) - 1) & 1), abort);
-                tc::mbar_arrive_expect_tx(&raw_full[r], raw_bytes);
-                tc::tma_load_2d(raw_base + r * raw_bytes, &ring_map, static_cast<int>(2 * TC_KC * (c_begin + 2 * m)), 0,
-                                &raw_full[r]);
+                const int n = chunks_of(p);
+                for (int m = 0; m < n; ++m, ++it)
+                {
+                    const int r = it % R;
+                    if (it >= R)
+                        mbar_wait(&raw_empty[r], static_cast<uint32_t>(((it / R) - 1) & 1), abort);
+                    if (*abort)
+                        break;
+                    tc::mbar_arrive_expect_tx(&raw_full[r], raw_bytes);
+                    tc::tma_load_2d(raw_base + r * raw_bytes, &ring_map,
+                                    static_cast<int>(2 * TC_KC * (static_cast<size_t>(p) * chunks_per_part + m)), 0,
+                                    &raw_full[r]);
+                }
             }
+            s_issued = it;
         }
         __syncwarp();
     }
@@ -149,123 +162,174 @@ __global__ void __launch_bounds__(TC_THREADS, 2) k_cov_tc(const __grid_constant_
         // one raw row (frame t: 64 complex samples, 512 B) per warp iteration: lane l reads 16 B
         // (pixels 2l, 2l+1), splits Re and Im into BF16 hi / lo pairs and writes 32-bit words
         // j = l & 3 of chunk g = l >> 2 in rows 2t (Re) and 2t+1 (Im): conflict-free reads and writes
-        for (int it = 0; it < nmine; ++it)
+        const int g = lane >> 2;
+        const uint32_t j4 = static_cast<uint32_t>(lane & 3) * 4u;
+        const int lo_row = packed ? 64 : 0;  // Yl rows: 64.. of the same tile, or the lo tile
+        int it = 0, k = 0;
+        for (int p = blockIdx.x; p < nparts; p += gridDim.x, ++k)
         {
-            const int m = it >> 1, half = it & 1;  // chunk it is half `half` of raw pair m
-            const int r = m % R, st = it % A_STAGES;
-            if (half == 0)
-                mbar_wait(&raw_full[r], static_cast<uint32_t>((m / R) & 1), abort);
-            if (it >= A_STAGES)
-                mbar_wait(&a_empty[st], static_cast<uint32_t>(((it / A_STAGES) - 1) & 1), abort);
-            const uint8_t* raw = raw_base + r * raw_bytes + half * (TC_KC * 8);
-            uint8_t* th = tiles + st * a_stage_bytes;
-            uint8_t* tl = packed ? th : th + TILE_BYTES;
-            const int lo_row = packed ? 64 : 0;  // Yl rows: 64.. of the same tile, or the lo tile
-            const int g = lane >> 2;
-            const uint32_t j4 = static_cast<uint32_t>(lane & 3) * 4u;
-            for (int t = warp; t < T; t += TC_CONVERTERS / 32)
+            const int n = chunks_of(p);
+            for (int m = 0; m < n; ++m, ++it)
             {
-                const float4 f = reinterpret_cast<const float4*>(raw + t * (TC_KC * 16))[lane];
-                uint32_t reh, rel, imh, iml;
-                tc::split2(f.x, f.z, reh, rel);
-                tc::split2(f.y, f.w, imh, iml);
-                const uint32_t ore = tile_offset(2 * t, g) + j4, oim = tile_offset(2 * t + 1, g) + j4;
-                const uint32_t lre = tile_offset(lo_row + 2 * t, g) + j4, lim = tile_offset(lo_row + 2 * t + 1, g) + j4;
-                *reinterpret_cast<uint32_t*>(th + ore) = reh;
-                *reinterpret_cast<uint32_t*>(th + oim) = imh;
-                *reinterpret_cast<uint32_t*>(tl + lre) = rel;
-                *reinterpret_cast<uint32_t*>(tl + lim) = iml;
+                const int r = it % R, st = it % TC_A_STAGES;
+                mbar_wait(&raw_full[r], static_cast<uint32_t>((it / R) & 1), abort);
+                const uint8_t* raw = raw_base + r * raw_bytes;
+                uint8_t* th = tiles + st * a_stage_bytes;
+                uint8_t* tl = packed ? th : th + TILE_BYTES;
+                constexpr int D = 4, STEP = TC_CONVERTERS / 32;  // rows in flight per warp
+                // the tile is free: waited for once the first rows are on their way (or there are none)
+                auto wait_tile = [&] {
+                    if (it >= TC_A_STAGES)
+                        mbar_wait(&a_empty[st], static_cast<uint32_t>(((it / TC_A_STAGES) - 1) & 1), abort);
+                };
+                if (warp >= T)
+                    wait_tile();
+                for (int t0 = warp; t0 < T; t0 += D * STEP)
+                {
+                    float4 f[D];
+#pragma unroll
+                    for (int d = 0; d < D; ++d)
+                        if (t0 + d * STEP < T)
+                            f[d] = reinterpret_cast<const float4*>(raw + (t0 + d * STEP) * (TC_KC * 8))[lane];
+                    if (t0 == warp)
+                        wait_tile();
+#pragma unroll
+                    for (int d = 0; d < D; ++d)
+                    {
+                        const int t = t0 + d * STEP;
+                        if (t >= T)
+                            break;
+                        uint32_t reh, rel, imh, iml;
+                        tc::split2(f[d].x, f[d].z, reh, rel);
+                        tc::split2(f[d].y, f[d].w, imh, iml);
+                        const uint32_t ore = tile_offset(2 * t, g) + j4, oim = tile_offset(2 * t + 1, g) + j4;
+                        const uint32_t lre = tile_offset(lo_row + 2 * t, g) + j4,
+                                       lim = tile_offset(lo_row + 2 * t + 1, g) + j4;
+                        *reinterpret_cast<uint32_t*>(th + ore) = reh;
+                        *reinterpret_cast<uint32_t*>(th + oim) = imh;
+                        *reinterpret_cast<uint32_t*>(tl + lre) = rel;
+                        *reinterpret_cast<uint32_t*>(tl + lim) = iml;
+                    }
+                }
+                fence_async_smem();
+                __syncwarp();
+                if (lane == 0)
+                {
+                    mbar_arrive(&raw_empty[r]);
+                    mbar_arrive(&a_full[st]);
+                }
             }
-            fence_async_smem();
+            if (warp >= 4)
+                continue;
+            // the part's end: wait for its last MMAs, warps 0-3 read row 32w + lane of G, columns 0..N-1
+            mbar_wait(&done, static_cast<uint32_t>(k & 1), abort);
+            tc_fence_after();
+            const int row = warp * 32 + lane;
+            if (packed)
+            {
+                // partial layout [128][64]: row i < 64 holds Yh Yh^T + Yh Yl^T, row 64 + i holds
+                // Yl Yh^T + Yl Yl^T (the packed MMA computes all four blocks, so the fourth product
+                // costs nothing here: with it, samples whose hi + lo split is exact, such as integer
+                // camera values below 2^16, give exact products before the FP32 accumulation)
+                float* dst = part + static_cast<size_t>(p) * TC_ROWS * 64 + static_cast<size_t>(row) * 64;
+                const bool vec = (reinterpret_cast<uintptr_t>(part) & 15) == 0;
+                for (int c0 = 0; c0 < 64; c0 += 16)
+                {
+                    float v[16], w1[16];
+                    const uint32_t taddr = tmem + (static_cast<uint32_t>(warp * 32) << 16) + static_cast<uint32_t>(c0);
+                    tmem_ld16(taddr, v);
+                    tmem_ld16(taddr + 64u, w1);
+#pragma unroll
+                    for (int i = 0; i < 16; ++i)
+                        v[i] = n ? v[i] + w1[i] : 0.f;
+                    if (vec)
+                    {
+#pragma unroll
+                        for (int i = 0; i < 16; i += 4)
+                            *reinterpret_cast<float4*>(dst + c0 + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+                    }
+                    else
+                    {
+#pragma unroll
+                        for (int i = 0; i < 16; ++i)
+                            dst[c0 + i] = v[i];
+                    }
+                }
+            }
+            else
+            {
+                float* dst = part + static_cast<size_t>(p) * rows * rows + static_cast<size_t>(row) * rows;
+                for (int c0 = 0; c0 < N; c0 += 16)
+                {
+                    float v[16], w1[16], w2[16];
+                    const uint32_t taddr = tmem + (static_cast<uint32_t>(warp * 32) << 16) + static_cast<uint32_t>(c0);
+                    tmem_ld16(taddr, v);
+                    tmem_ld16(taddr + static_cast<uint32_t>(N), w1);
+                    tmem_ld16(taddr + static_cast<uint32_t>(2 * N), w2);
+#pragma unroll
+                    for (int i = 0; i < 16; ++i)
+                        v[i] = n ? v[i] + (w1[i] + w2[i]) : 0.f;
+                    if (row >= rows)
+                        continue;
+                    if (rows % 4 == 0 && (reinterpret_cast<uintptr_t>(part) & 15) == 0)
+                    {
+#pragma unroll
+                        for (int i = 0; i < 16; i += 4)
+                            if (c0 + i < rows)
+                                *reinterpret_cast<float4*>(dst + c0 + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+                    }
+                    else
+                    {
+#pragma unroll
+                        for (int i = 0; i < 16; ++i)
+                            if (c0 + i < rows)
+                                dst[c0 + i] = v[i];
+                    }
+                }
+            }
+            tc_fence_before();
             __syncwarp();
             if (lane == 0)
-            {
-                if (half == 1 || it == nmine - 1)
-                    mbar_arrive(&raw_empty[r]);  // both halves of the pair converted
-                mbar_arrive(&a_full[st]);
-            }
+                mbar_arrive(&acc_read);  // the next part may overwrite the accumulators
         }
     }
     else if (lane == 0)
     {
         // ------------------------------------------------------------------ MMA issuer
         const uint32_t idesc = instr_desc(TC_ROWS, packed ? TC_ROWS : N);
-        for (int it = 0; it < nmine; ++it)
+        int it = 0, k = 0;
+        for (int p = blockIdx.x; p < nparts; p += gridDim.x, ++k)
         {
-            const int st = it % A_STAGES;
-            mbar_wait(&a_full[st], static_cast<uint32_t>((it / A_STAGES) & 1), abort);
-            tc_fence_after();
-            const uint32_t ah = smem_u32(tiles + st * a_stage_bytes), al = ah + TILE_BYTES;
-            if (packed)
+            const int n = chunks_of(p);
+            if (k > 0)
             {
+                mbar_wait(&acc_read, static_cast<uint32_t>((k - 1) & 1), abort);
+                tc_fence_after();
+            }
+            for (int m = 0; m < n; ++m, ++it)
+            {
+                const int st = it % TC_A_STAGES;
+                mbar_wait(&a_full[st], static_cast<uint32_t>((it / TC_A_STAGES) & 1), abort);
+                tc_fence_after();
+                const uint32_t ah = smem_u32(tiles + st * a_stage_bytes), al = ah + TILE_BYTES;
 #pragma unroll
                 for (int s2 = 0; s2 < TC_KC / 16; ++s2)
                 {
-                    const uint64_t d = smem_desc(ah + s2 * 32);
-                    mma_bf16(tmem, d, d, idesc, (it > 0 || s2 > 0) ? 1u : 0u);  // [Yh; Yl] [Yh; Yl]^T
+                    const uint64_t dh = smem_desc(ah + s2 * 32), dl = smem_desc(al + s2 * 32);
+                    const uint32_t acc = (m > 0 || s2 > 0) ? 1u : 0u;
+                    if (packed)
+                    {
+                        mma_bf16(tmem, dh, dh, idesc, acc);  // [Yh; Yl] [Yh; Yl]^T
+                        continue;
+                    }
+                    // three independent accumulator chains (consecutive MMAs do not wait on each other)
+                    mma_bf16(tmem, dh, dh, idesc, acc);                                 // Yh Yh^T
+                    mma_bf16(tmem + static_cast<uint32_t>(N), dh, dl, idesc, acc);      // Yh Yl^T
+                    mma_bf16(tmem + static_cast<uint32_t>(2 * N), dl, dh, idesc, acc);  // Yl Yh^T
                 }
                 mma_commit(&a_empty[st]);
-                continue;
             }
-#pragma unroll
-            for (int s2 = 0; s2 < TC_KC / 16; ++s2)
-            {
-                const uint64_t dh = smem_desc(ah + s2 * 32), dl = smem_desc(al + s2 * 32);
-                const uint32_t acc = (it > 0 || s2 > 0) ? 1u : 0u;
-                // three independent accumulator chains (consecutive MMAs do not wait on each other)
-                mma_bf16(tmem, dh, dh, idesc, acc);                                      // Yh Yh^T
-                mma_bf16(tmem + static_cast<uint32_t>(N), dh, dl, idesc, acc);           // Yh Yl^T
-                mma_bf16(tmem + static_cast<uint32_t>(2 * N), dl, dh, idesc, acc);       // Yl Yh^T
-            }
-            mma_commit(&a_empty[st]);
-        }
-        mma_commit(&done);
-    }
-    // epilogue: wait for the last MMAs, warps 0-3 read row r = 32w + lane of G, columns 0..N-1
-    if (warp < 4)
-    {
-        mbar_wait(&done, 0, abort);
-        tc_fence_after();
-        const int r = warp * 32 + lane;
-        if (packed)
-        {
-            // partial layout [128][64]: row i < 64 holds Yh Yh^T + Yh Yl^T, row 64 + i holds
-            // Yl Yh^T + Yl Yl^T (the packed MMA computes all four blocks, so the fourth product
-            // costs nothing here: with it, samples whose hi + lo split is exact, such as integer
-            // camera values below 2^16, give exact products before the FP32 accumulation)
-            float* dstp = part + static_cast<size_t>(blockIdx.x) * TC_ROWS * 64 + static_cast<size_t>(r) * 64;
-            for (int c0 = 0; c0 < 64; c0 += 16)
-            {
-                float v[16], w1[16];
-                const uint32_t taddr = tmem + (static_cast<uint32_t>(warp * 32) << 16) + static_cast<uint32_t>(c0);
-                tmem_ld16(taddr, v);
-                tmem_ld16(taddr + 64u, w1);
-#pragma unroll
-                for (int i = 0; i < 16; ++i)
-                {
-                    v[i] += w1[i];
-                    dstp[c0 + i] = nmine ? v[i] : 0.f;
-                }
-            }
-        }
-        float* dst = part + static_cast<size_t>(blockIdx.x) * rows * rows;
-        for (int c0 = 0; c0 < (packed ? 0 : N); c0 += 16)
-        {
-            float v[16], w1[16], w2[16];
-            const uint32_t taddr = tmem + (static_cast<uint32_t>(warp * 32) << 16) + static_cast<uint32_t>(c0);
-            tmem_ld16(taddr, v);
-            tmem_ld16(taddr + static_cast<uint32_t>(N), w1);
-            tmem_ld16(taddr + static_cast<uint32_t>(2 * N), w2);
-#pragma unroll
-            for (int i = 0; i < 16; ++i)
-                v[i] += w1[i] + w2[i];
-            if (r < rows)
-            {
-#pragma unroll
-                for (int i = 0; i < 16; ++i)
-                    if (c0 + i < rows)
-                        dst[static_cast<size_t>(r) * rows + c0 + i] = nmine ? v[i] : 0.f;
-            }
+            mma_commit(&done);
         }
     }
     tc_fence_before();
@@ -276,8 +340,8 @@ __global__ void __launch_bounds__(TC_THREADS, 2) k_cov_tc(const __grid_constant_
         // memory are released (bounded waits)
         if (warp == TC_LOAD_WARP && lane == 0)
         {
-            const int npairs = (nmine + 1) / 2;
-            for (int m = npairs - R > 0 ? npairs - R : 0; m < npairs; ++m)
+            const int issued = s_issued;
+            for (int m = issued - R > 0 ? issued - R : 0; m < issued; ++m)
                 mbar_wait(&raw_full[m % R], static_cast<uint32_t>((m / R) & 1));
             atomicExch(err, 1);
         }
@@ -307,30 +371,39 @@ __global__ void k_cov_tc_reduce(const float* __restrict__ part, int T, int npart
                                 double2* __restrict__ cov)
 {
     wait_prior_kernels();
+    // the upper triangle is summed and mirrored, so the result is exactly Hermitian: row r and row T - 1 - r
+    // of it make T + 1 entries together (the FP64 sums are what bounds this: no idle lanes)
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= T * T)
+    const int r = e / (T + 1), c = e % (T + 1);
+    if (r >= (T + 1) / 2)
         return;
-    // the upper triangle is summed and mirrored, so the result is exactly Hermitian
-    const int ei = e / T, ej = e % T;
-    const bool mirror = ei > ej;
-    const int i = mirror ? ej : ei, j = mirror ? ei : ej;
+    const bool first = c < T - r;
+    const int i = first ? r : T - 1 - r, j = first ? r + c : i + c - (T - r);
+    if (!first && i == r)  // the middle row of an odd T
+        return;
     const int R = 2 * T;
     double g00 = 0, g11 = 0, g01 = 0, g10 = 0;
     const int c0 = blockIdx.y * per_slice;
     const int c1 = min(nparts, c0 + per_slice);
     const size_t stride = packed ? static_cast<size_t>(TC_ROWS) * 64 : static_cast<size_t>(R) * R;
 #pragma unroll 4
-    for (int c = c0; c < c1; ++c)
+    for (int k = c0; k < c1; ++k)
     {
-        const float* G = part + static_cast<size_t>(c) * stride;
+        const float* G = part + static_cast<size_t>(k) * stride;
         g00 += cov_g(G, R, packed, 2 * i, 2 * j);
         g11 += cov_g(G, R, packed, 2 * i + 1, 2 * j + 1);
         g01 += cov_g(G, R, packed, 2 * i, 2 * j + 1);
         g10 += cov_g(G, R, packed, 2 * i + 1, 2 * j);
     }
-    atomicAdd(&cov[e].x, g00 + g11);
+    double2* u = &cov[static_cast<size_t>(i) * T + j];
+    atomicAdd(&u->x, g00 + g11);
     if (i != j)
-        atomicAdd(&cov[e].y, mirror ? -(g01 - g10) : (g01 - g10));
+    {
+        double2* m = &cov[static_cast<size_t>(j) * T + i];
+        atomicAdd(&u->y, g01 - g10);
+        atomicAdd(&m->x, g00 + g11);
+        atomicAdd(&m->y, -(g01 - g10));
+    }
 }
 
 int sm_count();
@@ -733,9 +806,8 @@ TcPlan tc_plan(int T, size_t npix)
 {
     TcPlan p;
     const size_t nchunks = (npix + TC_KC - 1) / TC_KC;
-    // two persistent CTAs per SM (96 KB of shared memory each: two handoff pipelines per SM, 85.9
-    // -> 76.3 us at T = 32 on 1024 x 1024 frames against one CTA with 200 KB), or whole waves of
-    // them when a CTA's chain would exceed the limit
+    // two parts per SM (two CTAs where their accumulators fit into tensor memory side by side), or whole waves of
+    // them when a part's chain would exceed the limit
     const size_t sms = 2 * static_cast<size_t>(sm_count());
     const size_t chain = 2 * T <= 64 ? kMaxChainChunksPacked : kMaxChainChunks;
     size_t waves = (nchunks + sms * chain - 1) / (sms * chain);
@@ -867,15 +939,19 @@ hv_status cov_tc(const float2* ring, int T, size_t npix, double2* cov, void* wor
         return cov_tc_planes(planes, T, npix, cov, work, err, ~0u, 0, st);
     }
     const TcPlan p = tc_plan(T, npix);
-    // raw stages: T x 64 complex samples (T x 512 B) each, as many as fit beside the A stages in 96 KB
-    const size_t raw_bytes = static_cast<size_t>(T) * TC_KC * 16;  // pairs of 64-pixel chunks
-    const size_t a_bytes = p.packed ? static_cast<size_t>(TC_A_STAGES_PACKED) * TILE_BYTES
-                                    : static_cast<size_t>(TC_A_STAGES) * 2 * TILE_BYTES;
-    int raw = static_cast<int>((96 * 1024 - a_bytes) / raw_bytes);
+    // raw stages: T x 64 complex samples (T x 512 B) each
+    const size_t raw_bytes = static_cast<size_t>(T) * TC_KC * 8;
+    const size_t a_bytes = static_cast<size_t>(TC_A_STAGES) * (p.packed ? 1 : 2) * TILE_BYTES;
+    // two CTAs per SM where the accumulators leave room for two (the tensor memory has 512 columns), else
+    // one that takes its parts one after another
+    const bool two = p.cols <= 256;
+    const size_t budget = (two ? 108 : 216) * 1024;
+    int raw = static_cast<int>((budget - a_bytes) / raw_bytes);
     raw = raw > TC_MAX_RAW ? TC_MAX_RAW : (raw < 2 ? 2 : raw);
     const size_t smem = a_bytes + raw * raw_bytes + 1024;
+    const int grid = std::min(p.ctas, (two ? 2 : 1) * sm_count());
     CUtensorMap map;
-    if (!tc::encode_tmap_2d_f32(&map, ring, 2 * npix, static_cast<uint64_t>(T), npix * 8, 4 * TC_KC,
+    if (!tc::encode_tmap_2d_f32(&map, ring, 2 * npix, static_cast<uint64_t>(T), npix * 8, 2 * TC_KC,
                                 static_cast<uint32_t>(T)))
     {
         set_last_error_msg("tensor-core covariance: cuTensorMapEncodeTiled failed");
@@ -883,11 +959,11 @@ hv_status cov_tc(const float2* ring, int T, size_t npix, double2* cov, void* wor
     }
     HV_CUDA_TRY(cudaFuncSetAttribute(k_cov_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
     float* part = static_cast<float*>(work);
-    HV_LAUNCH(k_cov_tc, p.ctas, TC_THREADS, smem, st, map, T, npix, p.chunks_per_cta, p.N, p.cols, raw, p.packed, part,
-              err);
+    HV_LAUNCH(k_cov_tc, grid, TC_THREADS, smem, st, map, T, npix, p.chunks_per_cta, p.ctas, p.N, p.cols, raw, p.packed,
+              part, err);
     // four partials per thread (independent loads), the slices combined by FP64 atomics
     const int per = p.ctas < 4 ? p.ctas : 4;
-    HV_LAUNCH(k_cov_tc_reduce, dim3((T * T + 255) / 256, (p.ctas + per - 1) / per), 256, 0, st, part, T, p.ctas, per,
+    HV_LAUNCH(k_cov_tc_reduce, dim3(((T + 1) / 2 * (T + 1) + 255) / 256, (p.ctas + per - 1) / per), 256, 0, st, part, T, p.ctas, per,
               p.packed, cov);
     count_launch(2);
     return HV_OK;
