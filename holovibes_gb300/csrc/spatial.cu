@@ -1224,13 +1224,9 @@ hv_status launch_rows(const RowPass& p, int nframes, cudaStream_t st)
     return HV_OK;
 }
 
-template <int N>
-hv_status launch_cols(const ColPass& p, int nframes, cudaStream_t st)
+template <int N, int F>
+hv_status launch_cols_tiles(const ColPass& p, int nframes, cudaStream_t st)
 {
-    if constexpr (N == 512 || N == 768 || N == 1024)
-        if (g_fft_engine.load() == 0)
-            return launch_cols_warp<N>(p, nframes, st);
-    constexpr int F = col_lanes<N>();
     using Tl = fft::Tile<N, F, true>;
     const int tw_count = fft::twiddle_count(typename fft::Plan<N>::List{});
     const size_t smem = (static_cast<size_t>(F) * N + tw_count) * sizeof(float2);
@@ -1245,6 +1241,22 @@ hv_status launch_cols(const ColPass& p, int nframes, cudaStream_t st)
     HV_LAUNCH((k_fft_cols<N, F>), grid, Tl::NT, smem, st, q);
     count_launch();
     return HV_OK;
+}
+
+template <int N>
+hv_status launch_cols(const ColPass& p, int nframes, cudaStream_t st)
+{
+    if constexpr (N == 512 || N == 768 || N == 1024)
+        if (g_fft_engine.load() == 0)
+            return launch_cols_warp<N>(p, nframes, st);
+    constexpr int F = col_lanes<N>();
+    // While half as wide tiles still find an SM each, they are the faster ones (AS middle pass, 1 to 4 frames of
+    // 256 x 256 4.8 -> 3.7 us, 384 x 384 7.3 -> 6.2, 192 x 192 5.6 -> 5.3); beyond that both sizes take the same time
+    // (256: 8 frames 4.9 and 5.0 us) and more frames fill the wide ones better. Tiles of a quarter gained nothing more.
+    if constexpr (F == 16 && (N == 128 || N == 192 || N == 256 || N == 384))
+        if (static_cast<long long>((p.width + F - 1) / F) * nframes * 2 <= device_sms())
+            return launch_cols_tiles<N, F / 2>(p, nframes, st);
+    return launch_cols_tiles<N, F>(p, nframes, st);
 }
 
 }  // namespace
