@@ -143,7 +143,7 @@ int planes_real(const hv_settings& s)
 bool uses_planes(const hv_frame_desc& fd, const hv_settings& s, bool served);
 
 // PCA on the converted integer frames (no spatial transform) with sliding windows: the windows are
-// pipelined over three streams (process_batch, render_view). The covariance reads the split planes, the views
+// pipelined over four streams (process_batch, render_view). The covariance reads the split planes, the views
 // a ring of 16-bit samples with room for two more batches than the window, so a window's eigensolve
 // overlaps the next batch's conversion and covariance update and the previous window's view. (With views
 // that read planes and complex slots, and a ring rebuild behind each view that the next conversion had to wait
@@ -491,7 +491,7 @@ hv_status build(hv_pipe* p)
     p->range_ev_set = false;
     p->render_stream = p->fast ? p->render_stream_owned : p->stream;
     p->windows = 0;
-    // PCA windows over three streams (the tensor-core view's prepared weights are not double-buffered)
+    // PCA windows over four streams (the tensor-core view's prepared weights are not double-buffered)
     p->pp = uses_pca_pipeline(p->fd, s, p->served) && p->planes_ok && !p->view_on_tc && !p->fast;
     p->pp_w = p->pp_head = p->ring_stale = 0;
     if (p->pp)

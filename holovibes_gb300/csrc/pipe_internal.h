@@ -83,7 +83,7 @@ struct hv_pipe
     uint16_t* planes = nullptr;
     bool planes_ok = false;
     int planes_real = 0;  // the ring's imaginary parts are 0: real rows only
-    // PCA windows pipelined over three streams (pipe.cpp, `pp`): the pipe stream converts each
+    // PCA windows pipelined over four streams (pipe.cpp, `pp`): the pipe stream converts each
     // batch into the split planes and a ring of 16-bit samples and updates the covariance, the
     // eigensolve stream solves it, the corrections' stream corrects the kept eigenvectors, the render
     // stream views the samples and renders; eigenvectors and weights alternate between two buffers, the
