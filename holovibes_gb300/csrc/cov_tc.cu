@@ -60,9 +60,10 @@ using tc::instr_desc;
 // part: [nparts][2T][2T] FP32 partial G; err: set to 1 when a bounded wait gave up. A CTA takes the
 // parts blockIdx.x, blockIdx.x + gridDim.x, ...: the loads and conversions of the next one run beside the
 // end of the one before (above T = 40 the accumulators leave room for one CTA per SM, which was launched
-// twice). What bounds it is the conversion's latency: raw stages of one chunk, freed as soon as it is converted,
-// and four rows in flight per warp. Covariance with its reduction, 512 x 512 frames: T = 16 38 -> 25.5 us, T = 32
-// 47.6 -> 31.7, T = 64 93 -> 59; 32 frames of 1024 x 768 70 -> 58.
+// twice). What bounds it are the conversion's latency and instructions: raw stages of one chunk, freed as
+// soon as it is converted, four rows in flight per warp, their places in the tile a constant step apart. Covariance with
+// its reduction, 512 x 512 frames: T = 16 38 -> 24.7 us, T = 32 47.6 -> 29.7, T = 64 93 -> 54.8; 32 frames of 1024 x 768
+// 70 -> 52.9.
 __global__ void __launch_bounds__(TC_THREADS, 2) k_cov_tc(const __grid_constant__ CUtensorMap ring_map, int T,
                                                           size_t npix, size_t chunks_per_part, int nparts, int N,
                                                           uint32_t tmem_cols, int raw_stages, int packed,
@@ -162,21 +163,24 @@ __global__ void __launch_bounds__(TC_THREADS, 2) k_cov_tc(const __grid_constant_
         // one raw row (frame t: 64 complex samples, 512 B) per warp iteration: lane l reads 16 B
         // (pixels 2l, 2l+1), splits Re and Im into BF16 hi / lo pairs and writes 32-bit words
         // j = l & 3 of chunk g = l >> 2 in rows 2t (Re) and 2t+1 (Im): conflict-free reads and writes
-        const int g = lane >> 2;
         const uint32_t j4 = static_cast<uint32_t>(lane & 3) * 4u;
-        const int lo_row = packed ? 64 : 0;  // Yl rows: 64.. of the same tile, or the lo tile
-        int it = 0, k = 0;
+        // a warp's rows lie 16 tile rows apart, so their places in the swizzled tile are a constant step apart
+        constexpr int D = 4, STEP = TC_CONVERTERS / 32;  // rows in flight per warp
+        constexpr uint32_t TILE_STEP = 2 * STEP * 128;
+        static_assert(2 * STEP % 8 == 0, "whole swizzle atoms between a warp's rows");
+        const uint32_t ore = tile_offset(2 * warp, lane >> 2) + j4, oim = tile_offset(2 * warp + 1, lane >> 2) + j4;
+        const uint32_t lo = packed ? 64 * 128 : TILE_BYTES;  // Yl: rows 64.. of the same tile, or the lo tile
+        int it = 0, k = 0, r = 0;  // r: raw stage of chunk it, used for the raw_round-th time (mod 2)
+        uint32_t raw_round = 0;
         for (int p = blockIdx.x; p < nparts; p += gridDim.x, ++k)
         {
             const int n = chunks_of(p);
             for (int m = 0; m < n; ++m, ++it)
             {
-                const int r = it % R, st = it % TC_A_STAGES;
-                mbar_wait(&raw_full[r], static_cast<uint32_t>((it / R) & 1), abort);
+                const int st = it % TC_A_STAGES;
+                mbar_wait(&raw_full[r], raw_round, abort);
                 const uint8_t* raw = raw_base + r * raw_bytes;
                 uint8_t* th = tiles + st * a_stage_bytes;
-                uint8_t* tl = packed ? th : th + TILE_BYTES;
-                constexpr int D = 4, STEP = TC_CONVERTERS / 32;  // rows in flight per warp
                 // the tile is free: waited for once the first rows are on their way (or there are none)
                 auto wait_tile = [&] {
                     if (it >= TC_A_STAGES)
@@ -184,31 +188,31 @@ __global__ void __launch_bounds__(TC_THREADS, 2) k_cov_tc(const __grid_constant_
                 };
                 if (warp >= T)
                     wait_tile();
-                for (int t0 = warp; t0 < T; t0 += D * STEP)
+                const uint8_t* src = raw + warp * (TC_KC * 8) + lane * 16;
+                uint8_t* dst = th;
+                for (int t0 = warp; t0 < T; t0 += D * STEP, src += D * STEP * (TC_KC * 8), dst += D * TILE_STEP)
                 {
                     float4 f[D];
 #pragma unroll
                     for (int d = 0; d < D; ++d)
                         if (t0 + d * STEP < T)
-                            f[d] = reinterpret_cast<const float4*>(raw + (t0 + d * STEP) * (TC_KC * 8))[lane];
+                            f[d] = *reinterpret_cast<const float4*>(src + d * STEP * (TC_KC * 8));
                     if (t0 == warp)
                         wait_tile();
 #pragma unroll
                     for (int d = 0; d < D; ++d)
                     {
-                        const int t = t0 + d * STEP;
-                        if (t >= T)
+                        if (t0 + d * STEP >= T)
                             break;
                         uint32_t reh, rel, imh, iml;
                         tc::split2(f[d].x, f[d].z, reh, rel);
                         tc::split2(f[d].y, f[d].w, imh, iml);
-                        const uint32_t ore = tile_offset(2 * t, g) + j4, oim = tile_offset(2 * t + 1, g) + j4;
-                        const uint32_t lre = tile_offset(lo_row + 2 * t, g) + j4,
-                                       lim = tile_offset(lo_row + 2 * t + 1, g) + j4;
-                        *reinterpret_cast<uint32_t*>(th + ore) = reh;
-                        *reinterpret_cast<uint32_t*>(th + oim) = imh;
-                        *reinterpret_cast<uint32_t*>(tl + lre) = rel;
-                        *reinterpret_cast<uint32_t*>(tl + lim) = iml;
+                        uint8_t* re = dst + d * TILE_STEP + ore;
+                        uint8_t* im = dst + d * TILE_STEP + oim;
+                        *reinterpret_cast<uint32_t*>(re) = reh;
+                        *reinterpret_cast<uint32_t*>(im) = imh;
+                        *reinterpret_cast<uint32_t*>(re + lo) = rel;
+                        *reinterpret_cast<uint32_t*>(im + lo) = iml;
                     }
                 }
                 fence_async_smem();
@@ -217,6 +221,11 @@ __global__ void __launch_bounds__(TC_THREADS, 2) k_cov_tc(const __grid_constant_
                 {
                     mbar_arrive(&raw_empty[r]);
                     mbar_arrive(&a_full[st]);
+                }
+                if (++r == R)
+                {
+                    r = 0;
+                    raw_round ^= 1;
                 }
             }
             if (warp >= 4)

@@ -128,16 +128,7 @@ __device__ __forceinline__ void tma_load_2d(void* dst_smem, const void* tmap, in
         : "memory");
 }
 
-__device__ __forceinline__ void tma_load_3d(void* dst_smem, const void* tmap, int x, int y, int z, uint64_t* bar)
-{
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], "
-        "[%5];" ::"r"(smem_u32(dst_smem)),
-        "l"(tmap), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
-        : "memory");
-}
-
-// tma_load_3d of data that is read once: its lines are the first to leave L2.
+// 3-D tiled tensor copy of data that is read once, with a policy that makes its lines the first to leave L2.
 __device__ __forceinline__ uint64_t evict_first_policy()
 {
     uint64_t p;
