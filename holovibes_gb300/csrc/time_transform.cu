@@ -668,7 +668,8 @@ static hv_status launch_time_view(const float2* ring, int T, int W, int H, const
                                          static_cast<int>(smem)));
     const int np = time_view_partials(W, H);
     const size_t HW = static_cast<size_t>(W) * H;
-    if (KC <= 4 && HW % 2 == 0)
+    // (a ring off 16-byte alignment takes k_time_view's 8-byte loads)
+    if (KC <= 4 && HW % 2 == 0 && (reinterpret_cast<uintptr_t>(ring) & 15) == 0)
     {
         if (smem > 48 * 1024)
             HV_CUDA_TRY(cudaFuncSetAttribute(k_time_view2<KC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
