@@ -913,9 +913,8 @@ hv_status cov_tc_planes(const uint16_t* planes, int T, size_t npix, double2* cov
         return HV_ERR_CUDA;
     }
     const size_t smem = static_cast<size_t>(TP_STAGES) * TP_STAGE_BYTES + 1024;
-    static const cudaError_t attr = cudaFuncSetAttribute(k_cov_tc_tiled, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                         static_cast<int>(smem));
-    HV_CUDA_TRY(attr);
+    // at every launch: the opt-in to this much shared memory belongs to the current device
+    HV_CUDA_TRY(cudaFuncSetAttribute(k_cov_tc_tiled, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
     float* tpart = static_cast<float*>(work);
     HV_LAUNCH_BESIDE(k_cov_tc_tiled, q.nsplit * tl.n, TP_THREADS, smem, st, tmap, npix, tl, q.chunks_per_split, tpart, err);
     HV_LAUNCH_BESIDE(k_cov_tc_tiled_reduce, (T * T + TR_ENTRIES - 1) / TR_ENTRIES, TR_ENTRIES * TR_GROUPS, 0, st, tpart, T, tl,
