@@ -493,7 +493,8 @@ hv_status build(hv_pipe* p)
     p->windows = 0;
     // PCA windows over four streams (the tensor-core view's prepared weights are not double-buffered)
     p->pp = uses_pca_pipeline(p->fd, s, p->served) && p->planes_ok && !p->view_on_tc && !p->fast;
-    p->pp_w = p->pp_head = p->ring_stale = 0;
+    p->pp_w = PcaWindowCount{};
+    p->pp_head = p->ring_stale = 0;
     if (p->pp)
     {
         p->pp_cap = p->T + 2 * p->B;
@@ -627,15 +628,17 @@ hv_status refresh_ring(hv_pipe* p)
 hv_status render_view_pp(hv_pipe* p, cudaStream_t st, uint32_t dirty, uint32_t all, const float** frame,
                          int* shift_after)
 {
-    const int w = p->pp_w++, i = w & 1, c = w & 3;
+    const PcaWindowCount w = p->pp_w;  // this window's
+    ++p->pp_w.n;
+    const int i = w.slot(0, 2), c = w.slot(0, 4);
     double2* cov = p->pp_cov[c];
     cudaStream_t es = p->eig_stream;
     hv_status r;
-    if (w >= 4)  // window w - 4's eigensolve read this buffer
+    if (w.has(4))  // window w - 4's eigensolve read this buffer
         HV_CUDA_TRY(cudaStreamWaitEvent(p->stream, p->pp_eig_ev[c], 0));
-    const bool inc = w >= 1 && p->cov_valid && p->cov_mode == cov_mode() && dirty != all && cov_incremental();
+    const bool inc = w.has(1) && p->cov_valid && p->cov_mode == cov_mode() && dirty != all && cov_incremental();
     if (inc)
-        HV_CUDA_TRY(cudaMemcpyAsync(cov, p->pp_cov[(w - 1) & 3], static_cast<size_t>(p->T) * p->T * sizeof(double2),
+        HV_CUDA_TRY(cudaMemcpyAsync(cov, p->pp_cov[w.slot(1, 4)], static_cast<size_t>(p->T) * p->T * sizeof(double2),
                                     cudaMemcpyDeviceToDevice, p->stream));
     if (!inc || dirty)
     {
@@ -658,11 +661,11 @@ hv_status render_view_pp(hv_pipe* p, cudaStream_t st, uint32_t dirty, uint32_t a
     p->cov_mode = cov_mode();
     HV_CUDA_TRY(cudaEventRecord(p->pp_cov_ev[c], p->stream));
     HV_CUDA_TRY(cudaStreamWaitEvent(es, p->pp_cov_ev[c], 0));
-    if (w >= 2)  // window w - 2's corrections read these eigenvectors
-        HV_CUDA_TRY(cudaStreamWaitEvent(es, p->pp_eig_ev[(w - 2) & 3], 0));
+    if (w.has(2))  // window w - 2's corrections read these eigenvectors
+        HV_CUDA_TRY(cudaStreamWaitEvent(es, p->pp_eig_ev[w.slot(2, 4)], 0));
     // the corrections of window w run beside the sweeps of window w + 1; window w - 2's view read this
     // weights buffer
-    const EigCorrections corr{p->corr_stream, p->pp_sweeps_ev, w >= 2 ? p->pp_view_ev[(w - 2) & 3] : nullptr};
+    const EigCorrections corr{p->corr_stream, p->pp_sweeps_ev, w.has(2) ? p->pp_view_ev[w.slot(2, 4)] : nullptr};
     bool kept = false;
     if ((r = pca_eigh(cov, p->T, p->pp_evals[i], p->pp_evecs[i], p->pmin, p->pmax, p->pp_weights[i], p->eig_work, es,
                       p->pmin, p->pmax, p->eig_warm, true, &kept, &corr)) != HV_OK)
@@ -677,7 +680,7 @@ hv_status render_view_pp(hv_pipe* p, cudaStream_t st, uint32_t dirty, uint32_t a
     p->pp_nested = false;
     if (r != HV_OK)
         return r;
-    HV_CUDA_TRY(cudaEventRecord(p->pp_view_ev[w & 3], st));
+    HV_CUDA_TRY(cudaEventRecord(p->pp_view_ev[c], st));
     return HV_OK;
 }
 
@@ -1128,8 +1131,8 @@ hv_status process_batch(hv_pipe* p, const uint8_t* raw)
         // same stream) and into the sample ring. The frames overwritten there are older than the
         // window of three renders ago (pp_cap = T + 2 B): its view has to be through, the two
         // views enqueued since may still run.
-        if (p->pp_w >= 3)
-            HV_CUDA_TRY(cudaStreamWaitEvent(p->stream, p->pp_view_ev[(p->pp_w - 3) & 3], 0));
+        if (p->pp_w.has(3))
+            HV_CUDA_TRY(cudaStreamWaitEvent(p->stream, p->pp_view_ev[p->pp_w.slot(3, 4)], 0));
         if ((r = convert_window(raw, p->kind, p->HW, nb, begin, T, p->planes, p->pp_head, p->pp_cap, p->pp_samples,
                                 p->stream)) != HV_OK)
             return r;

@@ -8,6 +8,21 @@
 
 #include "hv_internal.h"
 
+namespace hv {
+
+// The windows that a Pipe has enqueued. The streams of the pipelined PCA windows wait for windows up to four back,
+// from when there are as many, and find their events and buffers by the count: 64 bits, because a count that
+// wraps takes the waits away (2^31 windows of 270 us are a week).
+struct PcaWindowCount
+{
+    uint64_t n = 0;
+    bool has(unsigned back) const { return n >= back; }
+    // of window n - back (has(back)), among `slots` used in turn
+    unsigned slot(unsigned back, unsigned slots) const { return static_cast<unsigned>((n - back) % slots); }
+};
+
+}  // namespace hv
+
 struct hv_pipe
 {
     hv_frame_desc fd{};
@@ -91,7 +106,8 @@ struct hv_pipe
     // frames, the next one goes to pp_head. `ring` is not written on the way: its newest ring_stale
     // slots are rebuilt from the planes when they are asked for (refresh_ring).
     bool pp = false, pp_nested = false;
-    int pp_w = 0, pp_cap = 0, pp_head = 0, ring_stale = 0;
+    hv::PcaWindowCount pp_w;
+    int pp_cap = 0, pp_head = 0, ring_stale = 0;
     uint16_t* pp_samples = nullptr;
     double2* pp_cov[4] = {nullptr, nullptr, nullptr, nullptr};
     float2* pp_weights[2] = {nullptr, nullptr};
