@@ -62,18 +62,18 @@ __device__ __forceinline__ size_t view_target(size_t pix, int W, int H, int shif
 
 // Sum of the warp's values a and b (0 where a lane has none) as a double. An FP64 instruction
 // occupies a scheduler's FP64 unit for 64 to 76 clocks per warp here (measured), conversions from FP32
-// included, so the sum is taken in 64-bit integers: each value as a multiple of 2^(emax - 181)
-// (emax: the largest biased exponent in the warp; values within 2^31 of it lose nothing, smaller
-// ones less than 2^-54 of it), summed by three 24-bit limbs, and rounded to a double once. A warp
-// that holds an infinity or a NaN takes the FP64 tree. The partials of a 1024 x 1024 view cost
-// 3.7 us as FP64 shuffle trees.
+// included, so the sum is taken in 64-bit integers: each value as a multiple of 2^(emax - 183)
+// (emax: the largest biased exponent in the warp), summed by three 24-bit limbs, and rounded to a
+// double once. That is exact up to the one rounding where all values but zeros lie within 2^33 of the largest
+// (64 terms below 2^24 with 33 more bits stay below 2^63); a warp with smaller ones, an infinity or a NaN
+// takes the FP64 tree. The partials of a 1024 x 1024 view cost 3.7 us as FP64 shuffle trees.
 __device__ __forceinline__ long long sum_term(float v, int emax)
 {
     const unsigned int u = __float_as_uint(v);
     const int e = static_cast<int>((u >> 23) & 255u);
     const long long m = e ? (u & 0x7fffffu) | 0x800000u : u & 0x7fffffu;
-    const int right = emax - (e ? e : 1);  // 0 .. 253
-    const long long f = right < 56 ? (m << 31) >> right : 0;
+    const int right = emax - (e ? e : 1);  // 0 .. 33, or any for a zero
+    const long long f = m << ((33 - right) & 63);
     return (u >> 31) ? -f : f;
 }
 
@@ -81,8 +81,10 @@ __device__ __forceinline__ double warp_sum(float a, float b)
 {
     const unsigned int full = 0xffffffffu;
     const unsigned int ua = __float_as_uint(a) & 0x7fffffffu, ub = __float_as_uint(b) & 0x7fffffffu;
-    const int emax = static_cast<int>(__reduce_max_sync(full, ua > ub ? ua : ub) >> 23);
-    if (emax == 255)
+    const int emax = static_cast<int>(__reduce_max_sync(full, max(ua, ub)) >> 23);
+    // (a zero becomes the largest number here)
+    const int emin = static_cast<int>((__reduce_min_sync(full, min(ua - 1u, ub - 1u)) + 1u) >> 23);
+    if (emax == 255 || emax - max(emin, 1) > 33)
     {
         double d = static_cast<double>(a) + static_cast<double>(b);
 #pragma unroll
@@ -96,7 +98,7 @@ __device__ __forceinline__ double warp_sum(float a, float b)
     const unsigned int l1 = __reduce_add_sync(full, static_cast<unsigned int>(s >> 24) & 0xffffffu);
     const int l2 = __reduce_add_sync(full, static_cast<int>(s >> 48));
     const long long t = (static_cast<long long>(l2) << 48) + (static_cast<long long>(l1) << 24) + l0;
-    // t * 2^(em - 181) to the nearest double (ties to even), in integers
+    // t * 2^(em - 183) to the nearest double (ties to even), in integers
     unsigned long long mag = t < 0 ? static_cast<unsigned long long>(-t) : static_cast<unsigned long long>(t);
     if (mag == 0)
         return 0.0;
@@ -112,7 +114,7 @@ __device__ __forceinline__ double warp_sum(float a, float b)
     else
         mag <<= 52 - top;
     // mag: 53 bits (or 2^53 after rounding up, which carries into the exponent)
-    const unsigned long long ex = static_cast<unsigned long long>(top + em - 181 + 1023 - 1);
+    const unsigned long long ex = static_cast<unsigned long long>(top + em - 183 + 1023 - 1);
     const unsigned long long bits = (ex << 52) + mag;
     return __longlong_as_double(static_cast<long long>(bits | (t < 0 ? 1ull << 63 : 0ull)));
 }
