@@ -1850,43 +1850,39 @@ __global__ void __launch_bounds__(NT) k_jacobi_smem(const double2* __restrict__ 
     R floor = R(0);
     if constexpr (sizeof(R) == sizeof(float))
     {
-        // the squares' sum in pairs of floats (hi + lo, 46 bits or more)
-        __shared__ float s_hi[NT / 32], s_lo[NT / 32];
-        float hi = 0.f, lo = 0.f;
-        auto add = [&](float x) {
-            const float s = hi + x, bb = s - hi;
-            lo += (hi - (s - bb)) + (x - bb);
-            hi = s;
-        };
+        // the squares are exact in FP64, so two FP64 operations per entry; then a tree that adds each pair
+        // once (every lane of a warp's shuffle tree adds)
+        __shared__ double s_f2[NT];
+        __shared__ float s_floor;
+        double f2 = 0.0;
         for (int e = tid; e < T * T; e += NT)
         {
             const Cx<R> a = A[(e / T) * LD + e % T];
-            const float px = __fmul_rn(a.x, a.x), py = __fmul_rn(a.y, a.y);
-            lo += __fmaf_rn(a.x, a.x, -px) + __fmaf_rn(a.y, a.y, -py);
-            add(px);
-            add(py);
+            const double x = widened(a.x), y = widened(a.y);
+            f2 = fma(x, x, f2);
+            f2 = fma(y, y, f2);
         }
-        for (int o = 16; o > 0; o >>= 1)
+        s_f2[tid] = f2;
+        __syncthreads();
+        if (tid < NT / 4)
         {
-            const float oh = __shfl_xor_sync(0xffffffffu, hi, o), ol = __shfl_xor_sync(0xffffffffu, lo, o);
-            add(oh);
-            lo += ol;
-        }
-        if ((tid & 31) == 0)
-        {
-            s_hi[tid >> 5] = hi;
-            s_lo[tid >> 5] = lo;
+            f2 = (s_f2[tid] + s_f2[tid + NT / 4]) + (s_f2[tid + NT / 2] + s_f2[tid + 3 * (NT / 4)]);
+            s_f2[tid] = f2;
         }
         __syncthreads();
-        if (tid == 0)
+        if (tid < 32)
         {
-            double t2 = 0.0;
-            for (int w = 0; w < NT / 32; ++w)
-                t2 += static_cast<double>(s_hi[w]) + static_cast<double>(s_lo[w]);
-            s_hi[0] = static_cast<float>(static_cast<double>(floor_rel) * sqrt(t2));
+            f2 = 0.0;
+#pragma unroll
+            for (int i = 0; i < NT / 4; i += 32)
+                f2 += s_f2[i + tid];
+            for (int o = 16; o > 0; o >>= 1)
+                f2 += __shfl_xor_sync(0xffffffffu, f2, o);
+            if (tid == 0)
+                s_floor = static_cast<float>(static_cast<double>(floor_rel) * sqrt(f2));
         }
         __syncthreads();
-        floor = s_hi[0];
+        floor = s_floor;
     }
     if constexpr (sizeof(R) == sizeof(float))
         smem_sweeps_warps<NT, NT == JS_WIDE ? JS_MAX_T + 1 : 33>(A, V, T, Tp, sc, floor, JAC_MAX_SWEEPS);
