@@ -965,7 +965,7 @@ hv_status cov_tc(const float2* ring, int T, size_t npix, double2* cov, void* wor
         set_last_error_msg("tensor-core covariance: cuTensorMapEncodeTiled failed");
         return HV_ERR_CUDA;
     }
-    HV_CUDA_TRY(cudaFuncSetAttribute(k_cov_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    HV_CUDA_TRY(cudaFuncSetAttribute(k_cov_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, 217 * 1024));  // budget + 1 KB
     float* part = static_cast<float*>(work);
     HV_LAUNCH(k_cov_tc, grid, TC_THREADS, smem, st, map, T, npix, p.chunks_per_cta, p.ctas, p.N, p.cols, raw, p.packed,
               part, err);

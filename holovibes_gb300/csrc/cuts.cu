@@ -176,7 +176,7 @@ hv_status time_cuts(const float2* ring, int T, int W, int H, const float2* weigh
     const size_t smem = static_cast<size_t>(T) * CUT_PX * sizeof(float2);
     if (smem > 48 * 1024)
         HV_CUDA_TRY(cudaFuncSetAttribute(k_cut_values, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(smem)));
+                                         static_cast<int>(CUT_MAX_T * CUT_PX * sizeof(float2))));
     const long long blocks = (g.npix + CUT_PX - 1) / CUT_PX;
     HV_LAUNCH(k_cut_values, static_cast<unsigned>(blocks), CUT_THREADS, smem, st, ring, weights_all, g, img_type, vals);
     const long long outs = static_cast<long long>(T) * W + static_cast<long long>(H) * T;

@@ -33,6 +33,10 @@ namespace hv {
 
 constexpr int TV_THREADS = 128;  // one renormalisation partial per 128 pixels (same as the tensor-core view)
 constexpr int TV_KMAX = 16;  // bins per register chunk at most
+// Largest dynamic shared memory of the view kernels (the staged weights). Here as at every launch site, the opt-in that goes
+// to cudaFuncSetAttribute is the largest of the site, not the call's own size: it is one attribute of the kernel on the
+// device, and a smaller window's call would lower it between another thread's opt-in and its launch, which is then refused.
+constexpr size_t TV_MAX_SMEM = 200 * 1024;
 
 __device__ __forceinline__ float view_value(float2 X, int img_type)
 {
@@ -660,14 +664,14 @@ static hv_status launch_time_view(const float2* ring, int T, int W, int H, const
                                   const CycleCtl* ctl, const float* bin_w)
 {
     const size_t smem = static_cast<size_t>(T) * KC * sizeof(float2);
-    if (smem > 200 * 1024)
+    if (smem > TV_MAX_SMEM)
     {
         set_last_error_msg("time window too large for the time-view kernel");
         return HV_ERR_UNSUPPORTED;
     }
     if (smem > 48 * 1024)
         HV_CUDA_TRY(cudaFuncSetAttribute(k_time_view<KC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(smem)));
+                                         static_cast<int>(TV_MAX_SMEM)));
     const int np = time_view_partials(W, H);
     const size_t HW = static_cast<size_t>(W) * H;
     // (a ring off 16-byte alignment takes k_time_view's 8-byte loads)
@@ -675,7 +679,7 @@ static hv_status launch_time_view(const float2* ring, int T, int W, int H, const
     {
         if (smem > 48 * 1024)
             HV_CUDA_TRY(cudaFuncSetAttribute(k_time_view2<KC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             static_cast<int>(smem)));
+                                             static_cast<int>(TV_MAX_SMEM)));
         const int grid2 = static_cast<int>((HW + 2 * TV_THREADS - 1) / (2 * TV_THREADS));
         HV_LAUNCH(k_time_view2<KC>, grid2, TV_THREADS, smem, st, ring, T, W, H, weights, K, img_type, scale, shift, out,
                   partials, np, ctl, bin_w);
@@ -726,14 +730,14 @@ static hv_status launch_time_view_real(const Source& source, int T, int W, int H
                                        cudaStream_t st, const CycleCtl* ctl, const float* bin_w)
 {
     const size_t smem = static_cast<size_t>(T) * KC * sizeof(float2);
-    if (smem > 200 * 1024)
+    if (smem > TV_MAX_SMEM)
     {
         set_last_error_msg("time window too large for the time-view kernel");
         return HV_ERR_UNSUPPORTED;
     }
     auto kern = k_time_view_real<KC, Source>;
     if (smem > 48 * 1024)
-        HV_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+        HV_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(TV_MAX_SMEM)));
     const size_t HW = static_cast<size_t>(W) * H;
     const int grid = static_cast<int>((HW + 2 * TV_THREADS - 1) / (2 * TV_THREADS));
     HV_LAUNCH_BESIDE(kern, grid, TV_THREADS / Source::GROUPS, smem, st, source, T, W, H, weights, K, img_type, scale, shift, out, partials,
@@ -3317,7 +3321,8 @@ hv_status pca_eigh(double2* cov, int T, double* evals, double2* evecs, int pmin,
         const size_t smem = jacobi_smem_bytes<float>(T, warm);
         auto kern = T > 32 ? k_jacobi_smem<float, JS_WIDE> : k_jacobi_smem<float, JS_MID>;
         const int threads = T > 32 ? JS_WIDE : JS_MID;
-        HV_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+        HV_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         static_cast<int>(jacobi_smem_bytes<float>(T > 32 ? JS_MAX_T : 32, true))));
         HV_LAUNCH(kern, 1, threads, smem, st, cov, V, T, Tp, ev_unsorted, warm ? 1 : 0, floor_rel);
     }
     else if (T <= JS_MAX_T)
@@ -3325,7 +3330,7 @@ hv_status pca_eigh(double2* cov, int T, double* evals, double2* evecs, int pmin,
         const size_t smem = jacobi_smem_bytes<double>(T, false);
         if (smem > 48 * 1024)
             HV_CUDA_TRY(cudaFuncSetAttribute((k_jacobi_smem<double, JS_THREADS>), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             static_cast<int>(smem)));
+                                             static_cast<int>(jacobi_smem_bytes<double>(JS_MAX_T, false))));
         HV_LAUNCH((k_jacobi_smem<double, JS_THREADS>), 1, JS_THREADS, smem, st, cov, V, T, Tp, ev_unsorted, 0, 0.0f);
     }
     else if (T <= JC_MAX_T && prec == HV_EIG_FP32)

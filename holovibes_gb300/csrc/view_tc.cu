@@ -499,7 +499,7 @@ hv_status view_tc(const float2* ring, int T, int W, int H, int K, int img_type, 
     a.raw_stages = raw;
     const size_t smem = raw * static_cast<size_t>(V_RAW) + a_bytes + 1024;
     auto kern = bin_w ? k_view_tc<true> : k_view_tc<false>;
-    HV_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    HV_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(budget + 1024)));
     int sms = 0;
     HV_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, 0));
     int grid = a.ntiles < sms ? a.ntiles : sms;
