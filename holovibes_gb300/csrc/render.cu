@@ -710,9 +710,12 @@ hv_status log10_map(float* frame, size_t n, cudaStream_t st)
 // Bound by latency and by shared-memory atomics on few addresses (a frame's values share a handful
 // of first digits): 16 pixels per thread are loaded together, equal digits of a warp are counted by
 // one atomic, and the scan rides on the pass. 1024 x 1024: 3 x (9.0 + 5.1) us as separate histogram and
-// scan launches, 3 x 10.4 us here (serialised launch times, cold caches).
+// scan launches, 3 x 10.4 us here (serialised launch times, cold caches). With a reticle or a pitch, 4 pixels per
+// thread are loaded together and their positions take 32-bit divisions: 2048 x 2048 with a reticle of the whole height
+// 67 us as separate launches, 97 one pixel after another on the grid of the 16-byte loads, 59.6 here.
 
 constexpr int PCT_BINS = 2048;
+constexpr int PCT_SCALAR = 4;  // pixels that a thread of the passes without 16-byte loads asks for together
 
 struct PctState
 {
@@ -726,13 +729,28 @@ __device__ __forceinline__ int digit_shift(int d) { return d == 0 ? 21 : (d == 1
 __device__ __forceinline__ unsigned int digit_mask(int d) { return d == 2 ? 1023u : 2047u; }
 __device__ __forceinline__ unsigned int high_mask(int d) { return d == 0 ? 0u : (d == 1 ? 0xffe00000u : 0xfffffc00u); }
 
-__device__ __forceinline__ bool in_reticle(size_t e, int W, int H, unsigned int r2, int use)
+// Where pixel e of the frame lies in memory, and whether it counts (inside the reticle's disc); 32-bit divisions
+// where the index allows.
+__device__ __forceinline__ size_t pct_pixel(size_t e, int W, int H, int pitch, unsigned int r2, int use_reticle, bool& on)
 {
-    if (!use)
-        return true;
-    const int x = static_cast<int>(e % W), y = static_cast<int>(e / W);
-    const int dx = x - W / 2, dy = y - H / 2;
-    return static_cast<unsigned int>(dx * dx + dy * dy) <= r2;
+    int x, y;
+    if (e >> 32)
+    {
+        y = static_cast<int>(e / W);
+        x = static_cast<int>(e % W);
+    }
+    else
+    {
+        const unsigned int q = static_cast<unsigned int>(e) / static_cast<unsigned int>(W);
+        y = static_cast<int>(q);
+        x = static_cast<int>(static_cast<unsigned int>(e) - q * static_cast<unsigned int>(W));
+    }
+    if (use_reticle)
+    {
+        const int dx = x - W / 2, dy = y - H / 2;
+        on = on && static_cast<unsigned int>(dx * dx + dy * dy) <= r2;
+    }
+    return static_cast<size_t>(y) * pitch + x;
 }
 
 // Digit of rank r (0 or 1) after pass d from the histogram hh, by a CTA of EW_THREADS (PCT_BINS / 8).
@@ -823,7 +841,8 @@ __device__ void pct_select(const unsigned int* hh, PctState* st, int r, int d, f
     }
 }
 
-// VEC: rows without gaps, no reticle, 16-byte aligned, a multiple of 4 pixels.
+// VEC: rows without gaps and no reticle, so the order of the pixels does not matter: 16-byte loads from the first
+// 16-byte boundary on, the pixels before and behind them by one warp.
 template <bool VEC>
 __global__ void __launch_bounds__(EW_THREADS) k_pct_pass(const float* __restrict__ f, int W, int H, int pitch,
                                                          unsigned int r2, int use_reticle, PctState* st, int d,
@@ -871,8 +890,14 @@ __global__ void __launch_bounds__(EW_THREADS) k_pct_pass(const float* __restrict
     if constexpr (VEC)
     {
         constexpr int Q = 4;
-        const size_t n4 = n / 4, step = static_cast<size_t>(gridDim.x) * EW_THREADS;
-        const float4* f4 = reinterpret_cast<const float4*>(f);
+        const size_t head = min(n, ((16 - (reinterpret_cast<uintptr_t>(f) & 15)) & 15) / sizeof(float));
+        const size_t n4 = (n - head) / 4, step = static_cast<size_t>(gridDim.x) * EW_THREADS;
+        const float4* f4 = reinterpret_cast<const float4*>(f + head);
+        if (blockIdx.x == 0 && threadIdx.x < 32)
+        {
+            const bool on = threadIdx.x < n - 4 * n4;
+            take(on ? f[threadIdx.x < head ? threadIdx.x : 4 * n4 + threadIdx.x] : 0.f, on);
+        }
         // uniform trip count: every lane of a warp takes part in the votes
         const size_t first = blockIdx.x * static_cast<size_t>(EW_THREADS) + threadIdx.x;
         for (size_t base = 0; base < n4; base += Q * step)
@@ -897,13 +922,23 @@ __global__ void __launch_bounds__(EW_THREADS) k_pct_pass(const float* __restrict
     }
     else
     {
+        constexpr int Q = PCT_SCALAR;
         const size_t step = static_cast<size_t>(gridDim.x) * EW_THREADS;
-        for (size_t base = blockIdx.x * static_cast<size_t>(EW_THREADS); base < n; base += step)
+        for (size_t base = blockIdx.x * static_cast<size_t>(EW_THREADS); base < n; base += Q * step)
         {
-            const size_t e = base + threadIdx.x;
-            const bool on = e < n && in_reticle(e, W, H, r2, use_reticle);
-            const size_t a = pitch == W ? e : (e / W) * static_cast<size_t>(pitch) + e % W;
-            take(on ? f[a] : 0.f, on);
+            float v[Q];
+            bool on[Q];
+#pragma unroll
+            for (int q = 0; q < Q; ++q)
+            {
+                const size_t e = base + threadIdx.x + q * step;
+                on[q] = e < n;
+                const size_t a = pct_pixel(e, W, H, pitch, r2, use_reticle, on[q]);
+                v[q] = on[q] ? f[a] : 0.f;
+            }
+#pragma unroll
+            for (int q = 0; q < Q; ++q)
+                take(v[q], on[q]);
         }
     }
     __syncthreads();
@@ -959,10 +994,13 @@ hv_status percentile_pitched(const float* frame, int W, int H, int pitch, float 
             r2 = radius * radius;
         }
     }
-    const bool vec = pitch == W && !use_reticle && vec4_ok(n, {frame});
-    // 16 pixels per thread: up to two CTAs per SM
-    const size_t want = (n + 16 * EW_THREADS - 1) / (16 * EW_THREADS);
-    const int grid = static_cast<int>(want < 152 * 2 ? want : 152 * 2);
+    const bool vec = pitch == W && !use_reticle;
+    // 16 pixels per thread (VEC) or PCT_SCALAR, up to four CTAs per SM: with two, large frames wait for the votes and
+    // shared-memory atomics of a few warps (4096 x 3000: 98.8 -> 88.8 us, with a reticle 180.7 -> 131.3), with six or eight
+    // the histograms of the CTAs cost more than they bring (98.6 to 109.9 us)
+    const size_t per = static_cast<size_t>(vec ? 16 : PCT_SCALAR) * EW_THREADS, cap = 152 * 4;
+    const size_t want = (n + per - 1) / per;
+    const int grid = static_cast<int>(want < cap ? want : cap);
     for (int d = 0; d < 3; ++d)
     {
         if (vec)
