@@ -254,7 +254,7 @@ size_t footprint(const hv_frame_desc& fd, const hv_settings& s, bool served = fa
     return z.total;
 }
 
-hv_status build(hv_pipe* p)
+hv_status build_buffers(hv_pipe* p, bool pca_pipeline)
 {
     free_buffers(p);
     const hv_settings& s = p->s;
@@ -492,7 +492,7 @@ hv_status build(hv_pipe* p)
     p->render_stream = p->fast ? p->render_stream_owned : p->stream;
     p->windows = 0;
     // PCA windows over four streams (the tensor-core view's prepared weights are not double-buffered)
-    p->pp = uses_pca_pipeline(p->fd, s, p->served) && p->planes_ok && !p->view_on_tc && !p->fast;
+    p->pp = pca_pipeline && uses_pca_pipeline(p->fd, s, p->served) && p->planes_ok && !p->view_on_tc && !p->fast;
     p->pp_w = PcaWindowCount{};
     p->pp_head = p->ring_stale = 0;
     if (p->pp)
@@ -601,6 +601,16 @@ hv_status build(hv_pipe* p)
     p->out_head = p->out_count = 0;
     p->last_frame_valid = false;
     return HV_OK;
+}
+
+// Where the buffers of the pipelined PCA windows do not fit beside the rest, the windows run one after another
+// on the complex ring, with the same outputs.
+hv_status build(hv_pipe* p)
+{
+    hv_status st = build_buffers(p, true);
+    if (st == HV_ERR_OOM && p->pp && (st = build_buffers(p, false)) == HV_OK)
+        set_last_error_msg("");
+    return st;
 }
 
 // Time transform and view of one full ring, up to the renormalisation sum

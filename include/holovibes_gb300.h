@@ -180,7 +180,9 @@ typedef struct hv_pipe hv_pipe;
  * `stream` may be NULL, in which case the pipe creates and owns a non-blocking stream. */
 hv_pipe* hv_pipe_create(const hv_frame_desc* fd, const hv_settings* settings, void* stream, hv_status* status);
 void hv_pipe_destroy(hv_pipe* p);
-/* Device bytes held by a pipe with these settings (admission by HBM footprint). */
+/* Device bytes held by a pipe with these settings (admission by HBM footprint). A pipe of sliding PCA windows without a
+ * spatial transform does with less when device memory is short: without the buffers that let its windows overlap
+ * (2 (T + 2 batch) bytes per pixel and four T x T matrices), with the same outputs. */
 size_t hv_pipe_footprint(const hv_frame_desc* fd, const hv_settings* settings);
 /* Replaces BatchInputQueue::enqueue (Backend/sources/data_struct/batch_input_queue.cc:124-202)
  * followed by the compute cycles it unblocks (Pipe::exec, pipe.cc:650-676). `n` frames of
