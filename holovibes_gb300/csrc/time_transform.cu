@@ -215,11 +215,12 @@ __global__ void __launch_bounds__(TV_THREADS) k_time_view(const float2* __restri
 
 // Two adjacent pixels per thread (16-byte ring loads: 512 contiguous bytes per warp and frame;
 // HW even). 128 threads cover 256 pixels and write the two 128-pixel renormalisation partials of
-// their CTA, the same partials as k_time_view. Bound by DRAM. One bin (two accumulators per pixel)
-// has little to do between loads: it takes 16 frames per batch of loads and asks for the first
+// their CTA, the same partials as k_time_view. Bound by DRAM. One and two bins (two accumulators per pixel and
+// bin) have little to do between loads: one bin takes 16 frames per batch of loads and asks for the first
 // frames in L2 before it stages the weights (512 x 512 with the partials: T = 16 8.8 -> 7.9 us, 32 14.4
-// -> 12.8, 64 26.4 -> 23.6, 0.84 of the copy bandwidth); more bins take 8 in a plain unrolled loop (the
-// same batches slow a K = 4, T = 128 view from 44.2 to 50.3 us).
+// -> 12.8, 64 26.4 -> 23.6, 0.84 of the copy bandwidth), two bins take 8 (1024 x 1024, T = 64: 94.4 us in the plain
+// loop, 82.3 in batches; 200 frames 275.8 and 237.8; 16 per batch 236.7, but 4 frames 10.6, 10.8 and 11.4); more bins
+// take a plain loop unrolled by 8 (the batches slow a K = 4, T = 128 view from 44.2 to 50.3 us).
 template <int KC>
 __global__ void __launch_bounds__(TV_THREADS) k_time_view2(const float2* __restrict__ ring, int T, int W, int H,
                                                             const float2* __restrict__ weights, int K, int img_type,
@@ -274,7 +275,7 @@ __global__ void __launch_bounds__(TV_THREADS) k_time_view2(const float2* __restr
                     a1[kk].y = fmaf(x.z, w.y, fmaf(x.w, w.x, a1[kk].y));
                 }
             };
-            if constexpr (KC == 1)
+            if constexpr (KC <= 2)
             {
                 int t = 0;
                 // frames t .. t + N - 1: their loads go out together
@@ -289,8 +290,9 @@ __global__ void __launch_bounds__(TV_THREADS) k_time_view2(const float2* __restr
                         accumulate(x[i], t + i);
                     t += N;
                 };
-                while (t + 16 <= T)
-                    frames(std::integral_constant<int, 16>{});
+                if constexpr (KC == 1)
+                    while (t + 16 <= T)
+                        frames(std::integral_constant<int, 16>{});
                 while (t + 8 <= T)
                     frames(std::integral_constant<int, 8>{});
                 while (t + 2 <= T)
