@@ -603,10 +603,12 @@ static hv_status launch_renorm_shift_acc(const float* in, float* out, int W, int
     const size_t n = static_cast<size_t>(W) * H;
     const bool v4 = vec4_ok(n, {in, out, acc}) && (!shift || W % 8 == 0);
     // with the factors: CTAs of 1024 threads, one per SM (each sums the partials: the SM's FP64 rate
-    // bounds that, so a second CTA would double it)
+    // bounds that, so a second CTA would double it). Without 16-byte accesses large frames wait for their loads: two
+    // per SM from where each thread still has 8 pixels (2048 x 2048 46.8 -> 44.1 us, 4096 x 3000 94.4 -> 83.4, but
+    // 512 x 512 10.0 -> 10.6; with 16-byte accesses 40.5 -> 44.7 and 75.6 -> 79.4)
     const int block = sum.partials ? RN_THREADS : EW_THREADS;
     const size_t per = static_cast<size_t>(block) * (v4 ? 4 : 1);
-    const size_t want = (n + per - 1) / per, cap = sum.partials ? 152 : 152 * 32;
+    const size_t want = (n + per - 1) / per, cap = !sum.partials ? 152 * 32 : !v4 && n >= 2 * 152 * RN_THREADS * size_t(8) ? 2 * 152 : 152;
     const int grid = static_cast<int>(want < cap ? (want > 0 ? want : 1) : cap);
     if (v4)
         HV_LAUNCH(k_renorm_shift_acc<4>, grid, block, 0, st, in, out, W, H, sum, shift, acc, A, slot, start, count,
