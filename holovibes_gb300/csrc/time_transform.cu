@@ -496,7 +496,12 @@ __device__ __forceinline__ void tvp_samples(float2 (&a)[GROUPS][2][KC], const ui
 // which come from the complex ring (slots whose planes are being overwritten).
 struct PlanesSource
 {
-    static constexpr int GROUPS = 1, CTAS = 8;
+    // seven CTAs per SM (72 registers) and a loop of its own for a window without ring slots: 512 frames of 512 x 512, 4
+    // bins 98.3 us, with eight CTAs and one loop 104.0, with eight and both loops 101.3, with five or six 110 to 116 (2 and
+    // 4 bins); asking for the largest shared-memory split as the windows' kernels that run beside others do: 115.7 (1 bin
+    // 105.7 instead of 85.6)
+    static constexpr int GROUPS = 1, CTAS = 7;
+    static constexpr bool BESIDE = false;
     const uint16_t* planes;
     const float2* ring;
     int r0, rn;
@@ -504,6 +509,12 @@ struct PlanesSource
     __device__ __forceinline__ void accumulate(float2 (&a)[GROUPS][2][KC], const size_t (&pix)[GROUPS], size_t HW, int T,
                                                const float2* wsm) const
     {
+        if (rn <= 0)
+        {
+            tvp_planes<KC>(a[0], reinterpret_cast<const uint32_t*>(planes + pix[0]),
+                           reinterpret_cast<const uint32_t*>(planes + static_cast<size_t>(T) * HW + pix[0]), HW / 2, 0, T, wsm);
+            return;
+        }
         for (int t = 0; t < T;)
         {
             // slots t .. of one run, all from one source
@@ -525,6 +536,7 @@ struct PlanesSource
 struct SamplesSource
 {
     static constexpr int GROUPS = 2, CTAS = 8;
+    static constexpr bool BESIDE = true;  // the pipelined PCA windows' view
     const uint16_t* samples;
     int cap, first, slot0;
     template <int KC>
@@ -742,8 +754,8 @@ static hv_status launch_time_view_real(const Source& source, int T, int W, int H
         HV_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(TV_MAX_SMEM)));
     const size_t HW = static_cast<size_t>(W) * H;
     const int grid = static_cast<int>((HW + 2 * TV_THREADS - 1) / (2 * TV_THREADS));
-    HV_LAUNCH_BESIDE(kern, grid, TV_THREADS / Source::GROUPS, smem, st, source, T, W, H, weights, K, img_type, scale, shift, out, partials,
-              time_view_partials(W, H), ctl, bin_w);
+    HV_CUDA_TRY(launch_kernel<Source::BESIDE>(kern, grid, TV_THREADS / Source::GROUPS, smem, st, source, T, W, H, weights, K,
+                                              img_type, scale, shift, out, partials, time_view_partials(W, H), ctl, bin_w));
     count_launch();
     return HV_OK;
 }
