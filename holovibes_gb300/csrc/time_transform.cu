@@ -19,6 +19,7 @@
 // eigenvector columns (PCA); the view, the bin average, the PCA scale, the fftshift permutation
 // and the renormalisation partial sums are fused into the same kernel, so the T x HW p_acc
 // buffer of the reference never exists.
+#include <cooperative_groups.h>
 #include <math.h>
 
 #include <atomic>
@@ -2661,6 +2662,7 @@ constexpr int TS_MAX_KEEP = 16;   // top ranks served (the other 16 vectors are 
 constexpr int TS_LD = TS_P + 1;   // shared-memory row pitch (float2) of the Rayleigh-Ritz matrices
 constexpr int TS_ORTH_THREADS = 256;
 constexpr int TS_ORTH_RPT = 2;    // rows per thread of the orthonormalisation (T <= 512)
+constexpr int TS_ORTH_WARPS = TS_ORTH_THREADS / 32;
 constexpr int TS_MM_ROWS = 1;     // rows of C V per CTA
 constexpr int TS_MM_SPLIT = 16;   // warps per row (warp q sums the terms s = q mod 16)
 constexpr int TS_ITERS_COLD = 8, TS_ITERS_WARM = 1;
@@ -2782,14 +2784,45 @@ __device__ __forceinline__ float2 ts_slot(const float2 (&y)[TS_ORTH_RPT][TS_P], 
     return make_float2(re, im);
 }
 
-// Sums of the 32 slots over the CTA: a reduce-scatter across each warp (lane l ends with the warp's
+// The warps of the orthonormalisation are those of one CTA, or (CLUSTER) one-warp CTAs of a cluster. ts_warp: this
+// one's index; ts_share: `v` into this warp's `slot` for all of them (lanes with `on`), then their barrier.
+template <bool CLUSTER>
+__device__ __forceinline__ int ts_warp()
+{
+    return CLUSTER ? blockIdx.x : threadIdx.x >> 5;
+}
+
+template <bool CLUSTER, class V>
+__device__ __forceinline__ void ts_share(V* slot, V v, bool on)
+{
+    if constexpr (CLUSTER)
+    {
+        const auto cluster = cooperative_groups::this_cluster();
+        if (on)
+        {
+#pragma unroll
+            for (int r = 0; r < TS_ORTH_WARPS; ++r)
+                *cluster.map_shared_rank(slot, r) = v;
+        }
+        cluster.sync();
+    }
+    else
+    {
+        if (on)
+            *slot = v;
+        __syncthreads();
+    }
+}
+
+// Sums of the 32 slots over the warps: a reduce-scatter across each warp (lane l ends with the warp's
 // sum of slot l), then a fixed-order sum over the warps in shared memory. Every warp returns the
 // same totals (slot `lane` in its lane). `red` alternates between two buffers, so one barrier per
 // reduction suffices.
+template <bool CLUSTER>
 __device__ __forceinline__ float2 ts_reduce_slots(const float2 (&y)[TS_ORTH_RPT][TS_P],
-                                                  float2 (*red)[TS_ORTH_THREADS / 32][TS_P], int& buf)
+                                                  float2 (*red)[TS_ORTH_WARPS][TS_P], int& buf)
 {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
     float2 p[TS_P / 2];
     {
         const bool up = lane & 16;
@@ -2815,11 +2848,10 @@ __device__ __forceinline__ float2 ts_reduce_slots(const float2 (&y)[TS_ORTH_RPT]
                                keep.y + __shfl_xor_sync(0xffffffffu, send.y, w));
         }
     }
-    red[buf][warp][lane] = p[0];
-    __syncthreads();
+    ts_share<CLUSTER>(&red[buf][ts_warp<CLUSTER>()][lane], p[0], true);
     float2 s2 = red[buf][0][lane];
 #pragma unroll
-    for (int w = 1; w < TS_ORTH_THREADS / 32; ++w)
+    for (int w = 1; w < TS_ORTH_WARPS; ++w)
     {
         s2.x += red[buf][w][lane].x;
         s2.y += red[buf][w][lane].y;
@@ -2860,16 +2892,12 @@ __device__ __forceinline__ float ts_project(float2 (&y)[TS_ORTH_RPT][TS_P], floa
 // always register slot 0 and the slots rotate by one after every column, so that registers are
 // indexed by constants only. A column left without norm (Y of rank < TS_P) becomes the unit vector
 // e_k, made orthogonal at the next iteration.
-template <int CTAS>
-__global__ void __launch_bounds__(TS_ORTH_THREADS, CTAS) k_ts_orth(const float2* __restrict__ Y, int T,
-                                                                   float2* __restrict__ V, const int* __restrict__ only_if)
+template <bool CLUSTER>
+__device__ __forceinline__ void ts_orthonormalise(const float2* __restrict__ Y, int T, float2* __restrict__ V)
 {
-    wait_prior_kernels();
-    if (only_if && *only_if == 0)  // the Cholesky-QR of the warm iteration succeeded
-        return;
-    __shared__ float2 red[2][TS_ORTH_THREADS / 32][TS_P];
-    __shared__ float red1[2][TS_ORTH_THREADS / 32];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    __shared__ float2 red[2][TS_ORTH_WARPS][TS_P];
+    __shared__ float red1[2][TS_ORTH_WARPS];
+    const int lane = threadIdx.x & 31, warp = ts_warp<CLUSTER>(), tid = 32 * warp + lane;
     float2 y[TS_ORTH_RPT][TS_P];  // slot j: column TS_P - 1 - j (before the first and after the last rotation)
 #pragma unroll
     for (int r = 0; r < TS_ORTH_RPT; ++r)
@@ -2884,13 +2912,13 @@ __global__ void __launch_bounds__(TS_ORTH_THREADS, CTAS) k_ts_orth(const float2*
     for (int k = 0; k < TS_P; ++k)
     {
         const int first = TS_P - k;  // the processed columns sit in slots first .. TS_P - 1
-        const float2 s1 = ts_reduce_slots(y, red, buf);
+        const float2 s1 = ts_reduce_slots<CLUSTER>(y, red, buf);
         const float nn = __shfl_sync(0xffffffffu, s1.x, 0);
         float n2 = ts_project(y, s1, first);
         // the same totals in every warp: the branch is uniform over the CTA
         if (k > 0 && !(n2 >= 0.5f * nn))
         {
-            ts_project(y, ts_reduce_slots(y, red, buf), first);
+            ts_project(y, ts_reduce_slots<CLUSTER>(y, red, buf), first);
             float m = 0.f;
 #pragma unroll
             for (int r = 0; r < TS_ORTH_RPT; ++r)
@@ -2898,12 +2926,10 @@ __global__ void __launch_bounds__(TS_ORTH_THREADS, CTAS) k_ts_orth(const float2*
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1)
                 m += __shfl_xor_sync(0xffffffffu, m, o);
-            if (lane == 0)
-                red1[buf1][warp] = m;
-            __syncthreads();
+            ts_share<CLUSTER>(&red1[buf1][warp], m, lane == 0);
             n2 = red1[buf1][0];
 #pragma unroll
-            for (int w = 1; w < TS_ORTH_THREADS / 32; ++w)
+            for (int w = 1; w < TS_ORTH_WARPS; ++w)
                 n2 += red1[buf1][w];
             buf1 ^= 1;
         }
@@ -2933,6 +2959,26 @@ __global__ void __launch_bounds__(TS_ORTH_THREADS, CTAS) k_ts_orth(const float2*
                 V[static_cast<size_t>(t) * TS_P + (TS_P - 1 - j)] = y[r][j];
         }
     }
+}
+
+__global__ void __launch_bounds__(TS_ORTH_THREADS) k_ts_orth(const float2* __restrict__ Y, int T, float2* __restrict__ V)
+{
+    wait_prior_kernels();
+    ts_orthonormalise<false>(Y, T, V);
+}
+
+// The same, to the bit, when the Cholesky-QR failed (*fail), on eight one-warp CTAs that fit beside the covariance of
+// another window: one CTA of 256 threads takes a whole SM's registers, for which every window would wait, needed or not,
+// and limited to a quarter of them it spills (windows of fewer than 32 independent frames, which need it each
+// time: 256 x 256, T = 128, stride 16 took 600 us).
+__global__ void __cluster_dims__(TS_ORTH_WARPS, 1, 1) __launch_bounds__(32)
+    k_ts_orth_failed(const float2* __restrict__ Y, int T, float2* __restrict__ V, const int* __restrict__ fail)
+{
+    wait_prior_kernels();
+    if (*fail == 0)  // for the whole cluster
+        return;
+    cooperative_groups::this_cluster().sync();  // its CTAs have all started: their shared memory can be written
+    ts_orthonormalise<true>(Y, T, V);
 }
 
 // The warm iteration's V = orth(Y) as a Cholesky-QR: with G = Y^H Y (k_ts_gram) and D = diag(G)^-1/2,
@@ -3291,7 +3337,7 @@ hv_status pca_eigh(double2* cov, int T, double* evals, double2* evecs, int pmin,
         if (!warm)
         {
             HV_LAUNCH_BESIDE(k_ts_init, gb, 256, 0, st, C32, T, Ys);
-            HV_LAUNCH_BESIDE(k_ts_orth<1>, 1, TS_ORTH_THREADS, 0, st, Ys, T, Vs, nullptr);
+            HV_LAUNCH_BESIDE(k_ts_orth, 1, TS_ORTH_THREADS, 0, st, Ys, T, Vs);
         }
         const int iters = warm ? TS_ITERS_WARM : TS_ITERS_COLD;
         int* chol_fail = reinterpret_cast<int*>(scale + 1);
@@ -3305,12 +3351,12 @@ hv_status pca_eigh(double2* cov, int T, double* evals, double2* evecs, int pmin,
                 HV_LAUNCH_BESIDE(k_ts_gram, TS_P, TS_GRAM_WARPS * 32, 0, st, Ys, Ys, T, Hm);
                 HV_LAUNCH_BESIDE(k_ts_cholqr, 1, TS_CHOL_WARPS * 32, 0, st, Hm, Qo, chol_fail);
                 HV_LAUNCH_BESIDE(k_ts_ritz, (T + TS_RITZ_ROWS - 1) / TS_RITZ_ROWS, 32 * TS_RITZ_ROWS, 0, st, Ys, Qo, T, nullptr, Vs);
-                HV_LAUNCH_BESIDE(k_ts_orth<4>, 1, TS_ORTH_THREADS, 0, st, Ys, T, Vs, chol_fail);
+                HV_LAUNCH_BESIDE(k_ts_orth_failed, TS_ORTH_WARPS, 32, 0, st, Ys, T, Vs, chol_fail);
                 extra += 3;
             }
             else
             {
-                HV_LAUNCH_BESIDE(k_ts_orth<1>, 1, TS_ORTH_THREADS, 0, st, Ys, T, Vs, nullptr);
+                HV_LAUNCH_BESIDE(k_ts_orth, 1, TS_ORTH_THREADS, 0, st, Ys, T, Vs);
             }
         }
         HV_LAUNCH_BESIDE(k_ts_matmul, gm, mm_threads, 0, st, C32, Vs, T, Ys);
