@@ -806,8 +806,10 @@ __global__ void __launch_bounds__(W32_THREADS, 2) k_fft_cols_warp(const __grid_c
 // Raw -> complex into ring slots (space transformation NONE), 8 pixels of one frame per thread
 // (frames of a multiple of 8 pixels, 16-byte aligned rows of the raw batch); with `planes`, the
 // real rows of the ring's split-BF16 planes of those slots as well (planes[p][slot][px]: the
-// covariance operands of a ring with zero imaginary parts), so the frame is read once.
-__global__ void k_convert8(const void* in, int kind, size_t frame_px, int batch, float2* ring, FrameMap map,
+// covariance operands of a ring with zero imaginary parts), so the frame is read once. Registers for six CTAs per
+// SM: with the 32 that the compiler takes for eight the same pass is slower (64 16-bit frames of 512 x 512 49.4 -> 45.0 us, float
+// 55.6 -> 50.9, 16 8-bit frames of 2048 x 2048 210.5 -> 200.5).
+__global__ void __launch_bounds__(256, 6) k_convert8(const void* in, int kind, size_t frame_px, int batch, float2* ring, FrameMap map,
                            const CycleCtl* ctl, uint16_t* planes)
 {
     wait_prior_kernels();
