@@ -526,8 +526,8 @@ def steps_for(hv, fd, s, dev_batch, stream):
                                                                              cov.data_ptr(), cw.data_ptr(), stream),
                         T * HW * (4 if real else 8), tiles * 3 * 2 * 128 * 128 * HW))
             if real and T >= 2 * B and fd.depth <= 2:
-                # the pipe's view of a real ring pipelined over streams: the planes, except the B
-                # slots the next batch overwrites, which come from the ring
+                # the view of a real ring from its planes, B slots of it from the ring; the pipelined Pipe's own view
+                # reads a ring of 16-bit samples (half these bytes), which has no entry point of its own
                 out = [r for r in out if r[0] != "time_view"]
                 out.append(("time_view_planes", lambda: L.hv_time_view_planes(
                     planes.data_ptr(), ring.data_ptr(), S % T, B, T, W, H, wts.data_ptr(), K, s.image_type, 1.0,

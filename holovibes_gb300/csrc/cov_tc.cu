@@ -10,16 +10,22 @@
 // 2T <= 64), so three (four) BF16 MMAs with FP32 accumulation per K step recover ~16-bit-mantissa
 // accuracy.
 //
-// Kernel: one CTA per SM walks a contiguous range of 64-pixel chunks (K slices of Y):
-//   warp 17    loader: one 2-D tensor copy (TMA) per pair of chunks (T x 128 complex samples, rows
-//              of 1 KB) into a ring of R raw stages (zero fill past the frame)
-//   warps 0-15 converters: raw samples -> Yh / Yl tiles of an A stage (128-byte-swizzled K-major,
-//              rows >= 2T stay zero), each warp releasing its part of the raw and A stages
-//   warp 16    MMA issuer (M = 128 rows of Y, N = 2T rounded to 16, K = 16) into three TMEM
-//              accumulators (Yh Yh^T, Yh Yl^T, Yl Yh^T: independent chains, summed by the
-//              epilogue), tcgen05.commit frees the A stage; after the last chunk a commit to
-//              `done` releases the epilogue (warps 0-3 read the accumulator lanes 32w..32w+31)
-// Every wait is bounded in time and reports through the error flag. Per-CTA partial G tiles are
+// Kernel (k_cov_tc, T <= 64; larger windows: k_cov_tc_tiled below): the frame's 64-pixel chunks (K slices of Y) are cut
+// into parts, two per SM or whole multiples of that. A CTA (two per SM where their accumulators fit into
+// tensor memory side by side, T <= 40, else one) takes parts blockIdx.x, blockIdx.x + gridDim.x, ..., and every
+// role walks the same chunks of the same parts, counting the chunks over all of them:
+//   warp 9     loader: one 2-D tensor copy (TMA) per chunk (T x 64 complex samples, rows of 512 bytes)
+//              into a ring of R raw stages (zero fill past the frame); raw_full / raw_empty
+//   warps 0-7  converters: raw samples -> Yh / Yl tiles of one of two A stages (128-byte-swizzled K-major,
+//              rows >= 2T stay zero), each warp releasing its part of the raw and A stages; a_full / a_empty
+//   warp 8     MMA issuer (K = 16): packed (2T <= 64) one 128 x 128 MMA per step on [Yh; Yl], else M = 128, N = 2T
+//              rounded to 16 into three TMEM accumulators (Yh Yh^T, Yh Yl^T, Yl Yh^T: independent chains,
+//              summed by the epilogue); tcgen05.commit frees the A stage, after a part's last chunk a commit to
+//              `done` releases its epilogue
+//   warps 0-3  epilogue of a part: read the accumulator lanes 32w..32w+31 and write the part's partial G tile, then
+//              arrive at `acc_read`, before which the MMAs of the next part do not start (its loads and
+//              conversions do)
+// Every wait is bounded in time and reports through the error flag. The partial G tiles are
 // summed in FP64 by k_cov_tc_reduce.
 #include <algorithm>
 #include <cstring>

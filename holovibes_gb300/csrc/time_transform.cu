@@ -2988,7 +2988,7 @@ __global__ void __cluster_dims__(TS_ORTH_WARPS, 1, 1) __launch_bounds__(32)
 // j .. TS_P - 1 of Y. The warm start's C V has near-orthogonal columns (the previous window's Ritz
 // vectors times a covariance that changed by one stride), so G' is near the identity and the FP32
 // factorisation is well conditioned. A pivot below 1e-6 (Y of rank < TS_P, or columns too close to
-// dependent) sets *fail and k_ts_orth recomputes V by Gram-Schmidt. One CTA.
+// dependent) sets *fail and k_ts_orth_failed recomputes V by Gram-Schmidt. One CTA.
 //
 // Column m of L and row m of L^-1 sit in the registers of warp m mod TS_CHOL_WARPS (lane = row of L, column
 // of L^-1). Step j finishes column j and row j and every later column and row takes its term of them, in the
