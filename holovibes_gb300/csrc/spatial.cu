@@ -24,6 +24,7 @@
 
 #include <atomic>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 #include "fft_smem.cuh"
@@ -439,7 +440,10 @@ __device__ __forceinline__ float2 staged_sample(const void* row, int at, bool sw
 // block are adjacent (the multiplier rows stay in L1), else the rows of one frame. KIND: the input
 // encoding (IN_U16 for both byte orders). The input rows of the next unit land in the warp's
 // transpose block by one bulk copy; without `bulk` (input off 16-byte alignment, engine mode 2)
-// the lanes copy them there.
+// the lanes copy them there, several loads at a time (one after another: 32 x 1024 x 1024 8-bit rows 161 us, so 78,
+// 8-bit Fresnel windows of 1024 x 1024, T = 32, off alignment 351 and 270 us). Loading them into registers instead
+// is faster still without bulk copies (58 us), but made the passes with them 1 to 2 % slower, as a branch and as
+// kernels of their own.
 template <int N, int KIND, bool PREMUL>
 __global__ void __launch_bounds__(W32_THREADS, 2) k_fft_rows_warp(RowPass p, int per_frame, int nframes, int bulk)
 {
@@ -523,18 +527,23 @@ __global__ void __launch_bounds__(W32_THREADS, 2) k_fft_rows_warp(RowPass p, int
         }
         else
         {
-            const uint8_t* src = source(f, y0);
+            using E = std::conditional_t<ESIZE == 1, uint8_t,
+                                         std::conditional_t<ESIZE == 2, uint16_t, std::conditional_t<ESIZE == 4, float, float2>>>;
+            // loads that a lane issues together; whole rows are a multiple of 32 D samples
+            constexpr int D = N == 768 && KIND == IN_C64 ? 12 : 8;
+            static_assert(N % (32 * D) == 0, "rows divide into batches");
+            const E* src = reinterpret_cast<const E*>(source(f, y0)) + lane;
+            E* dst = reinterpret_cast<E*>(buf) + lane;
             const int n = min(Gm::RPW, p.rows - y0) * N;
-            for (int i = lane; i < n; i += 32)
+            for (int i = 0; i < n; i += 32 * D)
             {
-                if constexpr (KIND == IN_U8)
-                    reinterpret_cast<uint8_t*>(buf)[i] = src[i];
-                else if constexpr (KIND == IN_U16)
-                    reinterpret_cast<uint16_t*>(buf)[i] = reinterpret_cast<const uint16_t*>(src)[i];
-                else if constexpr (KIND == IN_F32)
-                    reinterpret_cast<float*>(buf)[i] = reinterpret_cast<const float*>(src)[i];
-                else
-                    buf[i] = reinterpret_cast<const float2*>(src)[i];
+                E v[D];
+#pragma unroll
+                for (int d = 0; d < D; ++d)
+                    v[d] = src[i + 32 * d];
+#pragma unroll
+                for (int d = 0; d < D; ++d)
+                    dst[i + 32 * d] = v[d];
             }
             __syncwarp();
         }
@@ -608,12 +617,16 @@ __global__ void __launch_bounds__(W32_THREADS, 2) k_fft_rows_warp(RowPass p, int
 
 // Column pass. One tile = COLS adjacent columns of one frame; the CTA walks tiles blockIdx.x,
 // + gridDim.x, ... MODE: 0 forward, 1 inverse, 2 forward * G then inverse (the AS middle pass).
-// The tile (and, for MODE 2, the transfer function's tile) lands in the transpose block by tensor
-// copies of 256 rows each; without `bulk` (alignment, engine mode 2) the threads copy it there.
-template <int N, int MODE>
+// BULK: the tile (and, for MODE 2, the transfer function's tile) lands in the transpose block by tensor
+// copies of 256 rows each; else (alignment, engine mode 2) the threads load their samples (32 x 1024 x 1024: forward
+// 117 us, 336 through the block; with G 169 and 565).
+// (The outputs of the forward and inverse modes are addressed from their base: with a running pointer, or with the
+// base computed before the wait, the pass alone takes the same time or less, and the Fresnel + PCA windows of 1024 x 1024,
+// where it runs beside three render lanes, 1 to 2 % more.)
+template <int N, int MODE, bool BULK>
 __global__ void __launch_bounds__(W32_THREADS, 2) k_fft_cols_warp(const __grid_constant__ CUtensorMap in_map,
                                                                   const __grid_constant__ CUtensorMap g_map, ColPass p,
-                                                                  int tiles_x, int ntiles, int bulk)
+                                                                  int tiles_x, int ntiles)
 {
     wait_prior_kernels();
     using Gm = W32Geom<N>;
@@ -640,7 +653,7 @@ __global__ void __launch_bounds__(W32_THREADS, 2) k_fft_cols_warp(const __grid_c
         tc::mbar_init(bar, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         tc::fence_async_smem();
-        if (bulk && static_cast<int>(blockIdx.x) < ntiles)
+        if (BULK && static_cast<int>(blockIdx.x) < ntiles)
             issue(&in_map, blockIdx.x / tiles_x, blockIdx.x % tiles_x);
     }
     stage_twiddles(tw, p.tw, Gm::TW, W32_THREADS);  // ends with a CTA barrier
@@ -650,27 +663,21 @@ __global__ void __launch_bounds__(W32_THREADS, 2) k_fft_cols_warp(const __grid_c
     const float2 scale = make_float2(p.scale, MODE != 0 ? -p.scale : p.scale);
     const bool active_b = g < K1;  // N = 768: a quarter of the threads idle in one stage
     uint32_t phase = 0;
-    // the tile (columns tx C .. of the N rows at src) is in S: every thread waits for the copies, and
-    // the CTA agrees on the outcome so that all of it leaves together; or the threads copy it
-    auto landed = [&](const float2* src, int tx) -> bool {
-        if (bulk)
-        {
-            const bool ok = tc::mbar_wait(bar, phase, abort);
-            phase ^= 1;
-            return __syncthreads_and(ok);
-        }
-        const int col = tx * C + c;
-#pragma unroll 4
-        for (int j = 0; j < NS; ++j)
-            S[(g + NG * j) * C + c] = col < p.width ? src[static_cast<size_t>(g + NG * j) * W + col] : make_float2(0.f, 0.f);
-        __syncthreads();
-        return true;
+    // the tile asked for last is in S: every thread waits for the copies, and the CTA agrees on the
+    // outcome so that all of it leaves together
+    auto landed = [&]() -> bool {
+        if constexpr (!BULK)
+            return true;
+        const bool ok = tc::mbar_wait(bar, phase, abort);
+        phase ^= 1;
+        return __syncthreads_and(ok);
     };
     // every thread has read what it needs from S: ask for the tile of the next use
     auto refill = [&](const CUtensorMap* map, int fb, int tx, bool any) {
-        tc::fence_async_smem();
+        if constexpr (BULK)
+            tc::fence_async_smem();
         __syncthreads();
-        if (bulk && any && tid == 0)
+        if (BULK && any && tid == 0)
             issue(map, fb, tx);
     };
     bool gave_up = false;
@@ -679,16 +686,28 @@ __global__ void __launch_bounds__(W32_THREADS, 2) k_fft_cols_warp(const __grid_c
         const int fb = t / tiles_x, tx = t - fb * tiles_x;
         const int tn = t + static_cast<int>(gridDim.x);
         const bool in_range = tx * C + c < p.width;
-        if (!landed(p.in + static_cast<size_t>(fb) * p.in_frame, tx))
+        if (!landed())
         {
             gave_up = true;
             break;
         }
         float2 x[32];
+        if constexpr (BULK)
+        {
 #pragma unroll
-        for (int j = 0; j < NS; ++j)
-            x[j] = S[(g + NG * j) * C + c];
-        __syncthreads();
+            for (int j = 0; j < NS; ++j)
+                x[j] = S[(g + NG * j) * C + c];
+            __syncthreads();
+        }
+        else
+        {
+            // (a column past the frame repeats the last one; it is not stored)
+            const float2* src = p.in + static_cast<size_t>(fb) * p.in_frame + static_cast<size_t>(g) * W + min(tx * C + c, p.width - 1);
+            const size_t step = static_cast<size_t>(NG) * W;
+#pragma unroll
+            for (int j = 0; j < NS; ++j, src += step)
+                x[j] = *src;
+        }
         if constexpr (MODE == 1)
         {
 #pragma unroll
@@ -731,8 +750,8 @@ __global__ void __launch_bounds__(W32_THREADS, 2) k_fft_cols_warp(const __grid_c
             if (p.stream_out)
             {
 #pragma unroll
-                for (int k2 = 0; k2 < 32; ++k2, o += step)
-                    __stcs(o, fft::pmul(x[k2], scale));
+                for (int k2 = 0; k2 < 32; ++k2)
+                    __stcs(o + k2 * step, fft::pmul(x[k2], scale));
             }
             else
             {
@@ -748,18 +767,21 @@ __global__ void __launch_bounds__(W32_THREADS, 2) k_fft_cols_warp(const __grid_c
             refill(&g_map, 0, tx, true);
             if (active_b)
                 fftw::dft32(x);
-            if (!landed(p.postmul, tx))
+            if (!landed())
             {
                 gave_up = true;
                 break;
             }
             if (active_b)
             {
+                const float2* gm = p.postmul + static_cast<size_t>(g) * W + min(tx * C + c, p.width - 1);
+                const size_t step = static_cast<size_t>(K1) * W;
 #pragma unroll
-                for (int k2 = 0; k2 < 32; ++k2)
-                    x[k2] = cconj(cmul_fma(x[k2], S[(g + K1 * k2) * C + c]));
+                for (int k2 = 0; k2 < 32; ++k2, gm += step)
+                    x[k2] = cconj(cmul_fma(x[k2], BULK ? S[(g + K1 * k2) * C + c] : __ldg(gm)));
             }
-            __syncthreads();
+            if constexpr (BULK)
+                __syncthreads();
             if constexpr (N == 768)
             {
                 if (active_b)
@@ -795,7 +817,7 @@ __global__ void __launch_bounds__(W32_THREADS, 2) k_fft_cols_warp(const __grid_c
                 *o = fft::pmul(x[k2], scale);
         }
     }
-    if (gave_up && tid == 0)
+    if (BULK && gave_up && tid == 0)
     {
         // the copy still in flight lands before the CTA's shared memory is released
         tc::mbar_wait(bar, phase ^ 1);
@@ -1196,9 +1218,11 @@ hv_status launch_cols_warp(const ColPass& p, int nframes, cudaStream_t st)
     if (bulk && p.mode == 2)
         bulk = (reinterpret_cast<uintptr_t>(p.postmul) & 15) == 0 &&
                tc::encode_tmap_2d_f32(&g_map, p.postmul, static_cast<uint64_t>(p.width) * 2, N, pitch, Gm::COLS * 2, 256);
-    auto kern = p.mode == 2 ? k_fft_cols_warp<N, 2> : p.mode == 1 ? k_fft_cols_warp<N, 1> : k_fft_cols_warp<N, 0>;
+    auto kern = p.mode == 2   ? (bulk ? k_fft_cols_warp<N, 2, true> : k_fft_cols_warp<N, 2, false>)
+                : p.mode == 1 ? (bulk ? k_fft_cols_warp<N, 1, true> : k_fft_cols_warp<N, 1, false>)
+                              : (bulk ? k_fft_cols_warp<N, 0, true> : k_fft_cols_warp<N, 0, false>);
     HV_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(Gm::COL_SMEM)));
-    HV_LAUNCH(kern, grid, W32_THREADS, Gm::COL_SMEM, st, in_map, g_map, q, tiles_x, ntiles, bulk ? 1 : 0);
+    HV_LAUNCH(kern, grid, W32_THREADS, Gm::COL_SMEM, st, in_map, g_map, q, tiles_x, ntiles);
     count_launch();
     return HV_OK;
 }
